@@ -14,31 +14,10 @@
 // fixed order.  tcgen05 is the tool for many rows (gemm_tc.cu); here its 128-row tiles and
 // shared-memory staging would only add latency.
 #include "gemm_epilogue.cuh"
+#include "gemm_rows_ring.cuh"
 #include "sampling_key.cuh"
 
 namespace rl {
-
-__device__ __forceinline__ void mma_bf16_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                               uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
-      "{%0, %1, %2, %3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
-// LayerNorm of float32 rows as the product's input (x == nullptr: off; K <= 1024, M <= 16):
-// a = (x - mean) * rsqrt(var + eps) * gamma + beta with two-pass float32 statistics
-// (rosellm/rosetrainer/fused_layernorm.py:99-120), rounded to bfloat16 as the separate kernel
-// stores it.  Every block normalises the few rows itself, into shared memory, after it has
-// issued its first weight loads: that costs less than a kernel of its own between two products.
-struct NormArgs {
-  const float* x;
-  long ldx;
-  const float* gamma;
-  const float* beta;
-  float eps;
-};
 
 // LayerNorm of the float32 rows `norm.x` [M, K] into shared memory as bfloat16 (row stride
 // a_stride elements), a warp a row at a time; g4 / b4: gamma and beta in shared memory.
@@ -560,6 +539,10 @@ RL_EXPORT int rl_gemm_rows_bf16(int out_dtype, const void* A, long lda, const vo
                                     rl::SampleArgs{}, status, stream);
       return e == cudaSuccess ? 0 : (int)e;
     }
+  }
+  if (out_dtype == RL_F32 || out_dtype == RL_BF16) {
+    const rl::ring::Args r{a, lda, norm, w, bias, out, ldo, M, N, K, act, residual, out_dtype == RL_F32 ? 1 : 0, kv, status};
+    if (rl::ring::takes(r)) return rl::ring::run(r, stream);
   }
 #define RL_ROWS_MT(MT)                                                                                        \
   do {                                                                                                        \
