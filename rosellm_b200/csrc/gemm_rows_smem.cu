@@ -266,6 +266,7 @@ static size_t smem_bytes(int mt, int nt, int kc) {
 // How a product is cut: tiles of eight columns a block (nt), parts of K (parts) of kc elements.
 struct Plan {
   int nt, parts, kc;
+  int rounds;  // of blocks, as many as the device holds at once
 };
 
 // The plan for a product of these sizes, nt == 0 where this kernel does not take it.  K is cut
@@ -274,7 +275,7 @@ struct Plan {
 // one is taken whose blocks go round the device in the least time (rounds x width; the wider on
 // a tie, since it re-reads the rows less).
 static Plan plan_for(int M, int N, int K, int residual, int out_f32, int act, bool to_cache) {
-  Plan none{0, 0, 0};
+  Plan none{0, 0, 0, 0};
   if (M < 1 || M > 64 || K % 8 != 0 || N < 1) return none;
   static int n_sms = 0;
   if (n_sms == 0) {
@@ -304,7 +305,7 @@ static Plan plan_for(int M, int N, int K, int residual, int out_f32, int act, bo
     const long rounds = (blocks + n_sms * per_sm - 1) / (n_sms * per_sm);
     const long cost = rounds * nt * kc;
     if (best.nt == 0 || cost < best_cost) {
-      best = Plan{nt, parts, kc};
+      best = Plan{nt, parts, kc, (int)rounds};
       best_cost = cost;
     }
   }
@@ -329,9 +330,10 @@ static int launch(const Args& p, int parts, cudaStream_t stream) {
 }  // namespace rsm
 }  // namespace rl
 
-// Whether rl_gemm_rows_smem takes a product of these sizes (see above).
+// Whether rl_gemm_rows_smem takes a product of these sizes (see above): in how many rounds of blocks, 0 when it does not.
 RL_EXPORT int rl_gemm_rows_smem_fits(int M, int N, int K, int residual, int out_f32, int act, int to_cache) {
-  return rl::rsm::plan_for(M, N, K, residual, out_f32, act, to_cache != 0).nt > 0 ? 1 : 0;
+  const rl::rsm::Plan plan = rl::rsm::plan_for(M, N, K, residual, out_f32, act, to_cache != 0);
+  return plan.nt > 0 ? plan.rounds : 0;
 }
 
 // bfloat16 A [M <= 64, K] (row stride lda, a multiple of 8) and W [N, K]; out bfloat16 or float32.

@@ -370,26 +370,37 @@ def sm_count(device: torch.device | None = None) -> int:
 def bf16_path(rows: int, n_out: int, k: int, *, residual: bool = False, out_f32: bool = False, act: int = ACT_NONE,
               to_cache: bool = False) -> str:
     """Which kernel a bfloat16 product of these sizes runs on (measured on B200 at the widths of
-    GPT-2): up to 16 rows the weight-streaming mma kernel; 17 to 64 rows the kernel that keeps
-    both operands in shared memory, unless the output alone has tiles enough to fill the SMs (the
-    head: tcgen05 tiles) or its sizes do not fit (then the weight-streaming kernel, or for a long
-    inner size the clustered tcgen05 kernel); up to 128 rows the clustered kernel when the output
-    is too narrow to give the tiled kernel work; beyond, tcgen05 tiles."""
+    GPT-2, each kernel alone): up to 16 rows the weight-streaming kernels; 17 to 64 rows the kernel that keeps
+    both operands in shared memory, where all of its blocks run at once and the output alone has not tiles
+    enough to fill the SMs (a head); beyond, and where that kernel would take several rounds or does not
+    fit, tcgen05 tiles.  (64 rows, K 1600: 4800 columns 8.5 us on tiles, 18.8 on the weight-streaming kernel;
+    ``+=`` into 1600 columns from 6400 10.3 us against 21.1 in shared memory in two rounds; 24 rows, 4800
+    columns 8.6 against 17.2.  In one round shared memory is ahead: 768 columns from 3072 at 64 rows 5.0 us against
+    7.2.  65 to 128 rows: the clustered kernel is behind the tiles or level with them from 768 columns on, 768 x 768
+    at 96 rows 9.1 against 6.0.)  Heads of less than 148 tiles stay on the kernels whose epilogue can draw a token of every
+    row.  Outputs too narrow to give the tiles work (``NARROW_OUTPUT``) go to shared
+    memory in any number of rounds, the clustered kernel or the weight-streaming one."""
     if rows < 17:
         return "mma"
+    narrow = n_out < NARROW_OUTPUT
     if rows <= 64:
         if -(-n_out // 64) >= sm_count():
             return "tc"
-        if ROWS_IN_SHARED_MEMORY and _lib().rl_gemm_rows_smem_fits(rows, n_out, k, int(residual), int(out_f32), act,
-                                                                   int(to_cache)):
+        rounds = _lib().rl_gemm_rows_smem_fits(rows, n_out, k, int(residual), int(out_f32), act,
+                                               int(to_cache)) if ROWS_IN_SHARED_MEMORY else 0
+        if rounds == 1 or (rounds and narrow):
             return "smem"
+        if not narrow and not (out_f32 and not residual and k < 2048):  # (narrow heads: their epilogue draws tokens)
+            return "tc"
         if rows > 32 and k >= 2048 and _lib().rl_gemm_tc_rows_fits(rows, n_out, k):
             return "tcr"
         return "mma"
-    if rows <= 128 and n_out <= 1024 and _lib().rl_gemm_tc_rows_fits(rows, n_out, k):
+    if rows <= 128 and narrow and _lib().rl_gemm_tc_rows_fits(rows, n_out, k):
         return "tcr"
     return "tc"
 
+
+NARROW_OUTPUT = 768  # columns: fewer are twelve tiles or less
 
 # The kernel of 17 to 64 rows that stages both operands in shared memory (csrc/gemm_rows_smem.cu);
 # switched off, those products run as they did without it (for comparisons).
@@ -692,6 +703,7 @@ def rows_bulk_kernel(on: bool) -> None:
 # The fused kernels of a decode layer (csrc/mlp_fused.cu) are taken where their sizes fit;
 # switched off, every layer runs as separate products (for comparisons and measurements).
 FUSED_ROWS = True
+
 _mlp_slices: dict[tuple, int] = {}
 
 
