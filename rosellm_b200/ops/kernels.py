@@ -704,6 +704,14 @@ def rows_bulk_kernel(on: bool) -> None:
 # switched off, every layer runs as separate products (for comparisons and measurements).
 FUSED_ROWS = True
 
+
+def separate_is_faster(rows: int, hidden: int) -> bool:
+    """Whether a layer's products of few rows run faster as kernels of their own (the ring-fed product, whose weights
+    arrive under the kernels ahead) than in the two fused kernels.  Measured on B200, a layer of GPT-2 124M with 512
+    cached tokens, us fused / separate: 16.6 / 16.5 at 1 row, 16.9 / 16.9 at 2, 18.1 / 17.5 at 4, 20.5 / 18.8 at
+    8, 24.4 / 23.2 at 12, 26.5 / 28.3 at 16; width 1024 (the feed-forward alone fused) 21.1 / 20.0 at 1, 23.9 /
+    22.8 at 8, 34.5 / 33.9 at 16."""
+    return hidden > 768 or 2 < rows <= 12
 _mlp_slices: dict[tuple, int] = {}
 
 

@@ -469,7 +469,7 @@ class CausalSelfAttention(Part):
         """A step of few decoded requests and nothing else: the whole of this part (its norm
         included) in one kernel, where the sizes fit."""
         n = ctx.n_tokens
-        return (self._out_weight_packed is not None and K.FUSED_ROWS and n <= 16
+        return (self._out_weight_packed is not None and K.FUSED_ROWS and n <= 16 and not ctx.extras.get("separate_products")
                 and isinstance(h, K.NormInput) and h.x is x and n == ctx.n_decode == ctx.n_reqs and run.writes_cache
                 and not getattr(ctx.position, "rotates", True))
 
@@ -577,7 +577,7 @@ class DenseMLP(Part):
 
     def forward(self, ctx, h, x, add: bool = True) -> None:
         # few rows: both products in one kernel, the inner activations never leave the SM
-        width = self._fused_slice if add and ctx.n_tokens <= 16 and K.FUSED_ROWS else 0
+        width = self._fused_slice if add and ctx.n_tokens <= 16 and K.FUSED_ROWS and not ctx.extras.get("separate_products") else 0
         if width:
             K.mlp_fused(x, h, self.in_weight, self.in_bias, self._out_weight_packed, self.out_bias, act=self.activation,
                         slice_width=width)
@@ -597,6 +597,8 @@ class PreNormBlock(Part):
     uses = {"norm_mixer": "norm", "mixer": "mixer", "norm_feed_forward": "norm", "feed_forward": "feed_forward"}
 
     def forward(self, ctx, run, layer, x) -> None:
+        # which form of a layer of few rows is the faster: the parts that have a fused one look here
+        ctx.extras["separate_products"] = K.separate_is_faster(ctx.n_tokens, x.shape[1])
         h = self._normed(ctx, layer.norm_mixer, x, layer.mixer)
         layer.mixer.forward(ctx, run, h, x)
         h = self._normed(ctx, layer.norm_feed_forward, x, layer.feed_forward)
