@@ -546,13 +546,13 @@ static inline void launch_decode_form(const AttnParams& p, const int* decode_req
     if (smem > 47 * 1024)  // the kernel has a little static shared memory too
       cudaFuncSetAttribute(attn_decode_kernel<T, EPL, WARPS, STAGES, DENSE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)smem);
-    if (DENSE != 0)
+    if (DENSE != 0 || WARPS > 4)  // wide blocks stand between products that ask for all of it
       cudaFuncSetAttribute(attn_decode_kernel<T, EPL, WARPS, STAGES, DENSE>,
                            cudaFuncAttributePreferredSharedMemoryCarveout,
                            DENSE == 1 ? 80 : (int)cudaSharedmemCarveoutMaxShared);
     attr_set = true;
   }
-  launch_pdl_split(DENSE == 0, attn_decode_kernel<T, EPL, WARPS, STAGES, DENSE>, dim3(n_decode, p.n_heads, n_splits),
+  launch_pdl_split(DENSE == 0 && WARPS == 4, attn_decode_kernel<T, EPL, WARPS, STAGES, DENSE>, dim3(n_decode, p.n_heads, n_splits),
                    dim3(32 * WARPS), smem, stream, p, decode_reqs, n_splits, part_o, part_ml);
 }
 
@@ -575,7 +575,24 @@ static inline long narrow_blocks_at_once(int percent) {
   return (long)n_sms * per_sm;
 }
 
-// wide: sixteen warps a block instead of four.
+// How many sixteen-warp blocks the device holds at once, by their shared memory.
+template <size_t SMEM>
+static inline long wide_blocks_at_once() {
+  static long at_once = 0;
+  if (at_once == 0) {
+    int dev = 0, n_sms = 0, shared = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaDeviceGetAttribute(&shared, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
+    const long per_sm = (long)shared / (long)(SMEM + 2048);
+    at_once = (long)(n_sms > 0 ? n_sms : 1) * (per_sm > 0 ? per_sm : 1);
+  }
+  return at_once;
+}
+
+// wide: sixteen warps a block instead of four; eight where the device would take more than one round over blocks of sixteen
+// (25 heads of 64, 8 requests of 512 keys: 200 blocks, one an SM with
+// sixteen warps and three with eight, 10.3 -> 8.6 us; of 896 keys 14.2 -> 13.4; 16 heads, 16 requests 10.9 -> 8.9).
 template <typename T, int EPL>
 static inline void launch_decode(const AttnParams& p, const int* decode_reqs, int n_decode, int n_splits,
                                  bool wide, float* part_o, float* part_ml, cudaStream_t stream) {
@@ -583,7 +600,10 @@ static inline void launch_decode(const AttnParams& p, const int* decode_reqs, in
   if (wide) {
     // a ring of one tile where two would not fit an SM's shared memory (float32 rows of 256)
     constexpr int WIDE_STAGES = DecodeTile<EPL * (int)sizeof(T) / 4, 16, 2>::SMEM <= 200 * 1024 ? 2 : 1;
-    launch_decode_form<T, EPL, 16, WIDE_STAGES>(p, decode_reqs, n_decode, n_splits, part_o, part_ml, stream);
+    if ((long)n_decode * p.n_heads * n_splits > wide_blocks_at_once<DecodeTile<EPL * (int)sizeof(T) / 4, 16, WIDE_STAGES>::SMEM>())
+      launch_decode_form<T, EPL, 8, 2>(p, decode_reqs, n_decode, n_splits, part_o, part_ml, stream);
+    else
+      launch_decode_form<T, EPL, 16, WIDE_STAGES>(p, decode_reqs, n_decode, n_splits, part_o, part_ml, stream);
   } else if ((long)n_decode * p.n_heads * n_splits > narrow_blocks_at_once<T, EPL>(80)) {
     launch_decode_form<T, EPL, 4, 2, 2>(p, decode_reqs, n_decode, n_splits, part_o, part_ml, stream);
   } else if ((long)n_decode * p.n_heads * n_splits > narrow_blocks_at_once<T, EPL>(50)) {
