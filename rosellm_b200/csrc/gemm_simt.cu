@@ -13,7 +13,7 @@
 
 namespace rl {
 
-// 64x64 output tile per block of 256 threads, 4x4 outputs per thread, K in steps of 16.
+// Tiles of bfloat16: 64x64 output tile per block of 256 threads, 4x4 outputs per thread, K in steps of 16.
 // Each output's sum runs over k in ascending order whatever M is, so a row's result does
 // not depend on which other rows share the launch.
 template <typename TIn, typename TOut>
@@ -80,7 +80,224 @@ __global__ __launch_bounds__(256) void gemm_tile_kernel(
   }
 }
 
-// Few rows (decoded tokens).  A block of four warps computes 4 / KSPLIT output columns for all
+// Both halves of c += a * b: two float32 FMAs in one instruction, each rounded as fmaf rounds.
+__device__ __forceinline__ void fma_pair(uint64_t& c, uint64_t a, uint64_t b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ float pair_sum(uint64_t c) {
+  return __uint_as_float((uint32_t)c) + __uint_as_float((uint32_t)(c >> 32));
+}
+
+// Tiles of float32.  BM x BN output tile per block, TM x TN outputs per thread (rows and columns of a thread lie a
+// thread grid apart), K in steps of 16 that travel by cp.async, as they lie in memory, through a ring of three buffers of
+// shared memory (rows 80 bytes apart: the eight rows of a 16-byte access phase hit different banks).
+// Each output is two sums over k in ascending order, of its even and its odd elements, whatever M is and whatever the tile
+// is, so a row's result does not depend on which other rows share the launch: neighbouring elements of k lie side by side in both
+// operands, and one instruction takes both (fma.rn.f32x2), which leaves issue slots for the reads of shared memory: they are the bound, 12 pieces of 16 bytes a
+// thread for 128 FMAs with 8 x 4 outputs (about 19 of the 37.2 TFMA/s; the form before, 64 x 64 tiles of 4 x 4 outputs transposed
+// through registers with two barriers a step, 9 to 16).
+template <int BM, int BN, int TM, int TN>
+__global__ __launch_bounds__((BM / TM) * (BN / TN)) void gemm_tile_f32_kernel(
+    const float* __restrict__ A, long lda, const float* __restrict__ W, const float* __restrict__ bias,
+    float* __restrict__ out, long ldo, int M, int N, int K, int act, int residual) {
+  constexpr int BK = 16, STAGES = 3, LD = 20;  // floats between two rows in shared memory
+  constexpr int GX = BN / TN, GY = BM / TM, THREADS = GX * GY;
+  constexpr int PIECES = (BM + BN) * 4 / THREADS;  // 16-byte pieces of a step a thread copies
+  static_assert((BM + BN) * 4 % THREADS == 0, "pieces are shared evenly");
+  extern __shared__ __align__(16) float tile_s[];  // [STAGES][BM + BN][LD]: rows of A, then of W
+  const int tid = threadIdx.x, tx = tid % GX, ty = tid / GX;
+  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+  const int steps = (K + BK - 1) / BK;
+  const float* src[PIECES];
+  uint32_t dst[PIECES];
+  bool there[PIECES];
+#pragma unroll
+  for (int q = 0; q < PIECES; ++q) {
+    const int i = tid + THREADS * q, row = i >> 2, piece = i & 3;
+    const bool of_a = row < BM;
+    const int r = of_a ? m0 + row : n0 + row - BM;
+    there[q] = r < (of_a ? M : N);
+    src[q] = (of_a ? A + (size_t)(there[q] ? r : 0) * lda : W + (size_t)(there[q] ? r : 0) * K) + 4 * piece;
+    dst[q] = (uint32_t)__cvta_generic_to_shared(tile_s + row * LD + 4 * piece);
+  }
+  auto copy = [&](int step) {  // what lies outside the matrices arrives as zeros
+    const uint32_t at = (uint32_t)(step % STAGES) * ((BM + BN) * LD * 4);
+#pragma unroll
+    for (int q = 0; q < PIECES; ++q) {
+      const bool in = there[q] && step * BK + 4 * (int)(tid & 3) < K;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst[q] + at), "l"(src[q] + (in ? step * BK : 0)),
+                   "r"(in ? 16 : 0)
+                   : "memory");
+    }
+  };
+  pdl_begin();
+  uint64_t acc[TM][TN];
+#pragma unroll
+  for (int i = 0; i < TM; ++i)
+#pragma unroll
+    for (int j = 0; j < TN; ++j) acc[i][j] = 0ull;
+#pragma unroll
+  for (int s = 0; s < STAGES - 1; ++s) {
+    if (s < steps) copy(s);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  for (int step = 0; step < steps; ++step) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+    __syncthreads();  // the step's pieces are there for all, and all have left the buffer that is filled now
+    if (step + STAGES - 1 < steps) copy(step + STAGES - 1);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    const float* a_s = tile_s + (step % STAGES) * ((BM + BN) * LD) + ty * LD;
+    const float* w_s = tile_s + (step % STAGES) * ((BM + BN) * LD) + (BM + tx) * LD;
+#pragma unroll
+    for (int kk = 0; kk < BK; kk += 4) {
+      ulonglong2 w[TN];
+#pragma unroll
+      for (int j = 0; j < TN; ++j) w[j] = *reinterpret_cast<const ulonglong2*>(w_s + j * GX * LD + kk);
+#pragma unroll
+      for (int i = 0; i < TM; ++i) {
+        const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(a_s + i * GY * LD + kk);
+#pragma unroll
+        for (int j = 0; j < TN; ++j) fma_pair(acc[i][j], a.x, w[j].x);
+#pragma unroll
+        for (int j = 0; j < TN; ++j) fma_pair(acc[i][j], a.y, w[j].y);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < TM; ++i) {
+    const int m = m0 + i * GY + ty;
+    if (m >= M) continue;
+#pragma unroll
+    for (int j = 0; j < TN; ++j) {
+      const int n = n0 + j * GX + tx;
+      if (n >= N) continue;
+      float v = pair_sum(acc[i][j]);
+      if (bias != nullptr) v += bias[n];
+      v = apply_act(v, act);
+      store_out<float>(out, (size_t)m * ldo + n, v, residual);
+    }
+  }
+}
+
+// Few rows of float32 (decoded tokens).  A block of eight warps stays for the product and takes groups of COLS output
+// columns in turn, ROWS rows at a time; its warps take the chunks of 128 elements of K in turn, a lane four elements of each:
+// every piece of the weights that a lane holds meets all the rows in registers (the kernel before read a piece of A for
+// every piece of W, from the first-level cache, whose bandwidth bounded it).  A lane's weights travel by cp.async into a
+// ring of its own in shared memory (it reads back only what it copied itself, so no barrier is needed), two chunks
+// ahead, and the first of them before the wait for the kernels ahead.  The COLS * ROWS sums of a lane (each of its even and its odd
+// elements, one instruction taking two) are added over the lanes by halving exchanges (each lane gives away half of what it
+// has left), then over the warps in shared memory: in an order that is the same for every row whatever M is.
+// per_turn: groups whose sums meet at one barrier, at most ROWS_GROUPS.
+constexpr int ROWS_COLS = 4, ROWS_GROUPS = 4;
+template <int ROWS>
+__global__ __launch_bounds__(256, 2) void gemm_rows_f32_kernel(
+    const float* __restrict__ A, long lda, const float* __restrict__ W, const float* __restrict__ bias,
+    float* __restrict__ out, long ldo, int M, int N, int K, int act, int residual, KvScatter kv, int per_turn) {
+  constexpr int WARPS = 8, COLS = ROWS_COLS, VALUES = COLS * ROWS, AHEAD = 2, STAGES = AHEAD + 1;
+  extern __shared__ __align__(16) float4 rows_ring[];  // [warp][stage][column][lane]
+  __shared__ float part_s[2][WARPS][ROWS_GROUPS][VALUES];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int groups = (N + COLS - 1) / COLS, chunks = (K + 127) / 128;
+  float4* mine = rows_ring + (size_t)warp * STAGES * COLS * 32 + lane;
+  // what the warp copies next: of a group its chunks, of the groups taken together each, those once for every ROWS rows,
+  // then the block's next groups
+  int c_first = warp < chunks ? (int)blockIdx.x * per_turn : groups, c_m0 = 0, c_group = c_first, c_chunk = warp, c_stage = 0;
+  auto copy = [&]() {
+    if (c_first < groups) {
+      const int k = c_chunk * 128 + 4 * lane;
+      const uint32_t dst = (uint32_t)__cvta_generic_to_shared(mine + c_stage * COLS * 32);
+#pragma unroll
+      for (int c = 0; c < COLS; ++c)  // beyond K: zeros
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + c * 512),
+                     "l"(W + (size_t)min(c_group * COLS + c, N - 1) * K + (k < K ? k : 0)), "r"(k < K ? 16 : 0)
+                     : "memory");
+      if (++c_stage == STAGES) c_stage = 0;
+      if ((c_chunk += WARPS) >= chunks) {
+        c_chunk = warp;
+        if (++c_group == min(c_first + per_turn, groups)) {
+          if ((c_m0 += ROWS) >= M) {
+            c_m0 = 0;
+            c_first += gridDim.x * per_turn;
+          }
+          c_group = c_first;
+        }
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+#pragma unroll
+  for (int s = 0; s < AHEAD; ++s) copy();
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  int buf = 0, stage = 0;
+  for (int first = blockIdx.x * per_turn; first < groups; first += gridDim.x * per_turn) {
+    const int n_here = min(per_turn, groups - first);
+    // the epilogue's thread: a column of a row of one of the groups
+    const int e_group = tid / VALUES, e_value = tid % VALUES, e_row = e_value / COLS, e_n = (first + e_group) * COLS + e_value % COLS;
+    const bool e_there = e_group < n_here && e_n < N;
+    const float b = e_there && bias != nullptr ? bias[e_n] : 0.f;
+    for (int m0 = 0; m0 < M; m0 += ROWS, buf ^= 1) {
+#pragma unroll 1
+      for (int g = 0; g < n_here; ++g) {
+        uint64_t sum[VALUES];  // [row][column]
+#pragma unroll
+        for (int i = 0; i < VALUES; ++i) sum[i] = 0ull;
+        for (int chunk = warp; chunk < chunks; chunk += WARPS) {
+          copy();  // into the stage that was read last
+          asm volatile("cp.async.wait_group %0;" ::"n"(AHEAD) : "memory");
+          ulonglong2 w[COLS];
+#pragma unroll
+          for (int c = 0; c < COLS; ++c) w[c] = *reinterpret_cast<const ulonglong2*>(mine + (stage * COLS + c) * 32);
+          if (++stage == STAGES) stage = 0;
+          const int k = chunk * 128 + 4 * lane;
+#pragma unroll
+          for (int r = 0; r < ROWS; ++r) {
+            ulonglong2 a = make_ulonglong2(0ull, 0ull);
+            if (k < K) a = *reinterpret_cast<const ulonglong2*>(A + (size_t)min(m0 + r, M - 1) * lda + k);
+#pragma unroll
+            for (int c = 0; c < COLS; ++c) {
+              fma_pair(sum[r * COLS + c], a.x, w[c].x);
+              fma_pair(sum[r * COLS + c], a.y, w[c].y);
+            }
+          }
+        }
+        float acc[VALUES];
+#pragma unroll
+        for (int i = 0; i < VALUES; ++i) acc[i] = pair_sum(sum[i]);
+        // after the exchange over lane bit o, a lane keeps the half of its values whose index has that bit as its own;
+        // with one value left the lanes add it up
+#pragma unroll
+        for (int o = 16, half = VALUES / 2; o > 0; o >>= 1, half >>= 1) {
+          const bool upper = (lane & o) != 0;
+          if (half == 0) {
+            acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);
+            continue;
+          }
+#pragma unroll
+          for (int i = 0; i < VALUES / 2; ++i) {
+            if (i >= half) break;
+            const float give = upper ? acc[i] : acc[i + half];
+            const float keep = upper ? acc[i + half] : acc[i];
+            acc[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+          }
+        }
+        part_s[buf][warp][g][lane / (32 / VALUES)] = acc[0];  // fewer values than lanes: neighbours hold the same one
+      }
+      __syncthreads();  // the other buffer takes the next sums, so one barrier is enough
+      const int m = m0 + e_row;
+      if (e_there && m < M) {
+        float v = 0.f;
+#pragma unroll
+        for (int q = 0; q < WARPS; ++q) v += part_s[buf][q][e_group][e_value];
+        v = apply_act(v + b, act);
+        if (!scatter_kv<float>(kv, m, e_n, v)) store_out<float>(out, (size_t)m * ldo + e_n, v, residual);
+      }
+    }
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+
+// Few rows of bfloat16.  A block of four warps computes 4 / KSPLIT output columns for all
 // rows: KSPLIT warps share a column, each taking a contiguous part of K, and their partial
 // sums meet in shared memory in a fixed order.  Lanes split a warp's part of K in 16-byte
 // pieces and four pieces of the weight row are in flight per lane before any is used, so that
@@ -195,6 +412,72 @@ static void launch_rows(const TIn* a, long lda, const TIn* w, const float* bias,
 #undef RL_ROWS
 }
 
+static int simt_sm_count() {
+  static int n_sms = 0;
+  if (n_sms == 0) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, dev);
+    if (n_sms <= 0) n_sms = 1;
+  }
+  return n_sms;
+}
+
+template <int BM, int BN, int TM, int TN>
+static void launch_tile_f32_form(const float* a, long lda, const float* w, const float* bias, float* o, long ldo, int M, int N, int K,
+                                 int act, int residual, cudaStream_t stream) {
+  constexpr size_t smem = 3 * (size_t)(BM + BN) * 20 * 4;
+  static bool attr_set = false;
+  if (!attr_set) {
+    if (smem > 48 * 1024)
+      note_launch(cudaFuncSetAttribute(gemm_tile_f32_kernel<BM, BN, TM, TN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    attr_set = true;
+  }
+  launch_pdl(gemm_tile_f32_kernel<BM, BN, TM, TN>, dim3((N + BN - 1) / BN, (M + BM - 1) / BM), dim3((BM / TM) * (BN / TN)), smem,
+             stream, a, lda, w, bias, o, ldo, M, N, K, act, residual);
+}
+
+// The tile that ends first, by what the forms measure at K 768 (us): a tile alone on its SM, and each further one.  (2304 x 768
+// at 1752 rows: 169, 174 and 207 us on 64 x 64, 32 x 64 and 32 x 32; 194 on the form before; 768 x 3072 287, 257, 281
+// and 440; 768 x 768 at 65 rows 37, 25, 16 and 45.  128 x 64, and 8 x 8 outputs a thread, measured slower throughout.)
+static void launch_tile_f32(const float* a, long lda, const float* w, const float* bias, float* o, long ldo, int M, int N, int K,
+                            int act, int residual, cudaStream_t stream) {
+  const int sms = simt_sm_count();
+  auto cost = [&](int bm, int bn, double alone, double further) {
+    const long tiles = (long)((M + bm - 1) / bm) * ((N + bn - 1) / bn);
+    return alone + (double)((tiles + sms - 1) / sms - 1) * further;
+  };
+  const double large = cost(64, 64, 37.0, 24.8), middle = cost(32, 64, 24.5, 13.0), small = cost(32, 32, 16.0, 9.5);
+  if (large <= middle && large <= small) launch_tile_f32_form<64, 64, 8, 4>(a, lda, w, bias, o, ldo, M, N, K, act, residual, stream);
+  else if (middle <= small) launch_tile_f32_form<32, 64, 4, 4>(a, lda, w, bias, o, ldo, M, N, K, act, residual, stream);
+  else launch_tile_f32_form<32, 32, 4, 2>(a, lda, w, bias, o, ldo, M, N, K, act, residual, stream);
+}
+
+template <int ROWS>
+static void launch_rows_f32_form(const float* a, long lda, const float* w, const float* bias, float* o, long ldo, int M, int N, int K,
+                                 int act, int residual, const KvScatter& kv, cudaStream_t stream) {
+  constexpr size_t smem = 8 * 3 * 4 * 512;  // the rings of eight warps: three stages of four columns
+  static bool attr_set = false;
+  if (!attr_set) {  // with the kernel's static part above 48 KB
+    note_launch(cudaFuncSetAttribute(gemm_rows_f32_kernel<ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    attr_set = true;
+  }
+  const int groups = (N + ROWS_COLS - 1) / ROWS_COLS, blocks = 2 * simt_sm_count();
+  // a barrier every four groups where there are many (50257 x 768, 8 rows: 69 us against 81); few are shared out singly
+  // (3072 x 768: 7.2 us against 8.0)
+  const int per_turn = groups >= 4 * ROWS_GROUPS * blocks ? ROWS_GROUPS : 1, turns = (groups + per_turn - 1) / per_turn;
+  launch_pdl(gemm_rows_f32_kernel<ROWS>, min(turns, blocks), 256, smem, stream, a, lda, w, bias, o, ldo, M, N, K, act, residual, kv,
+             per_turn);
+}
+
+static void launch_rows_f32(const float* a, long lda, const float* w, const float* bias, float* o, long ldo, int M, int N, int K,
+                            int act, int residual, const KvScatter& kv, cudaStream_t stream) {
+  if (M == 1) launch_rows_f32_form<1>(a, lda, w, bias, o, ldo, M, N, K, act, residual, kv, stream);
+  else if (M == 2) launch_rows_f32_form<2>(a, lda, w, bias, o, ldo, M, N, K, act, residual, kv, stream);
+  else if (M <= 4) launch_rows_f32_form<4>(a, lda, w, bias, o, ldo, M, N, K, act, residual, kv, stream);
+  else launch_rows_f32_form<8>(a, lda, w, bias, o, ldo, M, N, K, act, residual, kv, stream);
+}
+
 template <typename TIn, typename TOut>
 static int launch_gemm(const void* A, long lda, const void* W, const float* bias, void* out,
                        long ldo, int M, int N, int K, int act, int residual, int rows_limit,
@@ -203,14 +486,22 @@ static int launch_gemm(const void* A, long lda, const void* W, const float* bias
   const TIn* w = (const TIn*)W;
   TOut* o = (TOut*)out;
   if (M <= rows_limit) {
-    if (M == 1) launch_rows<TIn, TOut, 1>(a, lda, w, bias, o, ldo, M, N, K, act, residual, kv, stream);
-    else if (M == 2) launch_rows<TIn, TOut, 2>(a, lda, w, bias, o, ldo, M, N, K, act, residual, kv, stream);
-    else if (M <= 4) launch_rows<TIn, TOut, 4>(a, lda, w, bias, o, ldo, M, N, K, act, residual, kv, stream);
-    else launch_rows<TIn, TOut, 8>(a, lda, w, bias, o, ldo, M, N, K, act, residual, kv, stream);
+    if constexpr (sizeof(TIn) == 4) {
+      launch_rows_f32(a, lda, w, bias, o, ldo, M, N, K, act, residual, kv, stream);
+    } else {
+      if (M == 1) launch_rows<TIn, TOut, 1>(a, lda, w, bias, o, ldo, M, N, K, act, residual, kv, stream);
+      else if (M == 2) launch_rows<TIn, TOut, 2>(a, lda, w, bias, o, ldo, M, N, K, act, residual, kv, stream);
+      else if (M <= 4) launch_rows<TIn, TOut, 4>(a, lda, w, bias, o, ldo, M, N, K, act, residual, kv, stream);
+      else launch_rows<TIn, TOut, 8>(a, lda, w, bias, o, ldo, M, N, K, act, residual, kv, stream);
+    }
   } else {
     if (kv.pool != nullptr) return -5;  // the cache scatter is fused only into the row kernel
-    dim3 grid((N + 63) / 64, (M + 63) / 64);
-    launch_pdl(gemm_tile_kernel<TIn, TOut>, grid, 256, 0, stream, a, lda, w, bias, o, ldo, M, N, K, act, residual);
+    if constexpr (sizeof(TIn) == 4) {
+      launch_tile_f32(a, lda, w, bias, o, ldo, M, N, K, act, residual, stream);
+    } else {
+      dim3 grid((N + 63) / 64, (M + 63) / 64);
+      launch_pdl(gemm_tile_kernel<TIn, TOut>, grid, 256, 0, stream, a, lda, w, bias, o, ldo, M, N, K, act, residual);
+    }
   }
   return 0;
 }
