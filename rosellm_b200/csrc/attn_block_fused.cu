@@ -825,10 +825,10 @@ static int launch(const Args& p, cudaStream_t stream) {
   launch_config(&cfg, attr, p.n_heads, p.cluster, L.total, stream);
   if (stages == 3) {
     set_attributes<EPL, 3>();
-    note_launch(cudaLaunchKernelEx(&cfg, attn_rows_fused_kernel<EPL, 3>, p));
+    note_launch(launch_kernel(cfg, attn_rows_fused_kernel<EPL, 3>, p));
   } else {
     set_attributes<EPL, 2>();
-    note_launch(cudaLaunchKernelEx(&cfg, attn_rows_fused_kernel<EPL, 2>, p));
+    note_launch(launch_kernel(cfg, attn_rows_fused_kernel<EPL, 2>, p));
   }
   return take_launch_error();
 }

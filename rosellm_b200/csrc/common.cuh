@@ -4,8 +4,12 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <cstring>
 #include <mutex>
+#include <tuple>
+#include <type_traits>
 #include <unordered_set>
+#include <vector>
 
 // Element type codes of the C interface.
 #define RL_F32 0
@@ -36,6 +40,60 @@ inline int take_launch_error() {
   const int e = launch_error_noted;
   launch_error_noted = 0;
   return e;
+}
+}  // namespace rl
+
+// A step's kernel launches noted as they are made, to be issued again without the calls that led to them (launch_list.cu): the
+// kernel, its grid, attributes and a copy of its arguments, everything but the stream.  Noted by the host thread that asked.
+namespace rl {
+struct NotedLaunch {
+  const void* kernel;
+  dim3 grid, block;
+  size_t smem;
+  cudaLaunchAttribute attrs[3];
+  unsigned int n_attrs;
+  std::vector<size_t> at;            // where each argument lies in bytes
+  std::vector<unsigned char> bytes;  // of the arguments
+};
+struct LaunchNotes {
+  std::vector<NotedLaunch> launches;
+  bool whole = true;  // every launch since the beginning is in the list
+};
+inline thread_local LaunchNotes* launch_notes = nullptr;
+
+template <typename... Params>
+inline void note_kernel(LaunchNotes& notes, const cudaLaunchConfig_t& cfg, const void* kernel, const Params&... params) {
+  static_assert((std::is_trivially_copyable_v<Params> && ...), "kernel arguments are copied as bytes");
+  try {
+    NotedLaunch n;
+    n.kernel = kernel;
+    n.grid = cfg.gridDim;
+    n.block = cfg.blockDim;
+    n.smem = cfg.dynamicSmemBytes;
+    n.n_attrs = cfg.numAttrs;
+    if (cfg.numAttrs > 3) {
+      notes.whole = false;
+      return;
+    }
+    for (unsigned int i = 0; i < cfg.numAttrs; ++i) n.attrs[i] = cfg.attrs[i];
+    auto add = [&](const void* value, size_t size) {
+      const size_t at = (n.bytes.size() + 63) / 64 * 64;
+      n.bytes.resize(at + size);
+      std::memcpy(n.bytes.data() + at, value, size);
+      n.at.push_back(at);
+    };
+    (add(&params, sizeof(Params)), ...);
+    notes.launches.push_back(std::move(n));
+  } catch (...) {  // out of memory: the list is not whole and will not be used
+    notes.whole = false;
+  }
+}
+
+// Every launch of the library: made, and noted where its thread is taking notes.
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_kernel(const cudaLaunchConfig_t& cfg, void (*kernel)(KArgs...), Args... args) {
+  if (launch_notes != nullptr) note_kernel(*launch_notes, cfg, (const void*)kernel, static_cast<std::decay_t<KArgs>>(args)...);
+  return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
 }
 }  // namespace rl
 
@@ -136,7 +194,7 @@ inline cudaError_t launch_pdl_split(bool common_split, void (*kernel)(KArgs...),
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return note_launch(cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...));
+  return note_launch(launch_kernel(cfg, kernel, args...));
 }
 
 template <typename... KArgs, typename... Args>
@@ -162,7 +220,7 @@ inline cudaError_t launch_pdl_all_shared(void (*kernel)(KArgs...), dim3 grid, di
   attr[1].val.sharedMemCarveout = cudaSharedmemCarveoutMaxShared;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  return note_launch(cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...));
+  return note_launch(launch_kernel(cfg, kernel, args...));
 }
 
 // Thread-block clusters: rank of this block, the barrier of all threads of the cluster, and

@@ -802,7 +802,7 @@ static int launch_persistent(const void* A, long lda, const void* W, const float
   attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = CLUSTER ? 2 : 1;
-  note_launch(cudaLaunchKernelEx(&cfg, gemm_tc_persistent_kernel<TOut, EPI, CLUSTER>, ma, mw, mo, p));
+  note_launch(launch_kernel(cfg, gemm_tc_persistent_kernel<TOut, EPI, CLUSTER>, ma, mw, mo, p));
   return take_launch_error();
 }
 

@@ -257,7 +257,7 @@ static int launch_rows(const void* A, long lda, const void* W, const float* bias
   attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  note_launch(cudaLaunchKernelEx(&cfg, gemm_tc_rows_kernel<TOut>, mw, ma, bias, (TOut*)out, ldo, M, N, K, nt, kb_per,
+  note_launch(launch_kernel(cfg, gemm_tc_rows_kernel<TOut>, mw, ma, bias, (TOut*)out, ldo, M, N, K, nt, kb_per,
                                  tmem_cols, act, residual, kv, status));
   return take_launch_error();
 }

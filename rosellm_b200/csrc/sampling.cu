@@ -529,7 +529,7 @@ static cudaError_t launch_filtered_cluster(int cluster, int part, const float* l
   attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  return note_launch(cudaLaunchKernelEx(&cfg, sample_filtered_cluster_kernel, logits, ld, vocab, part, temperature,
+  return note_launch(launch_kernel(cfg, sample_filtered_cluster_kernel, logits, ld, vocab, part, temperature,
                                         top_k, top_p, seeds, counters, out_ids, kept));
 }
 

@@ -56,17 +56,30 @@ class LaunchList:
 
     What a step launches depends on its sizes, not on its contents (those lie in device
     buffers whose addresses stay): a step of sizes seen before can issue the recorded calls
-    again instead of walking through the parts and the checked wrappers a second time.
+    again instead of walking through the parts and the checked wrappers a second time.  Where the calls
+    launched kernels and nothing else, the library has noted those (csrc/launch_list.cu) and issues
+    them in one call.
     """
 
     def __init__(self) -> None:
         self.calls: list[tuple] = []  # (library function, arguments without the stream)
         self.launches = 0             # kernels these calls launch
         self.result = None            # whatever the recorded code returned (set by the caller)
+        self._notes = None            # the library and its handle of the noted kernels
+
+    def __del__(self) -> None:
+        if self._notes is not None:
+            self._notes[0].rl_notes_free(self._notes[1])
 
     def replay(self) -> None:
         global _launches
         stream = _stream()
+        if self._notes is not None:
+            rc = self._notes[0].rl_notes_replay(self._notes[1], stream)
+            if rc != 0:
+                raise KernelError(f"code {rc} when recorded launches were issued again")
+            _launches += self.launches
+            return
         for fn, args in self.calls:
             rc = fn(*args, stream)
             if rc != 0:
@@ -79,11 +92,17 @@ class _RecordingLib:
 
     def __init__(self, lib, into: LaunchList) -> None:
         self._lib, self._into = lib, into
+        # the library's own notes of the kernels (a stand-in for it may have none)
+        self._noting = hasattr(lib, "rl_notes_begin") and lib.rl_notes_begin() == 0
+        self._whole = True  # so far nothing but kernels has been issued
 
     def __getattr__(self, name):
         fn = getattr(self._lib, name)
         if name in _QUERIES:
             return fn
+
+        if name in _NOT_KERNELS:
+            self._whole = False
 
         def call(*args):
             self._into.calls.append((fn, args[:-1]))  # the stream is every launch's last argument
@@ -91,7 +110,17 @@ class _RecordingLib:
 
         return call
 
+    def finish(self) -> None:
+        if not self._noting:
+            return
+        handle = self._lib.rl_notes_end()
+        if handle and self._whole:
+            self._into._notes = (self._lib, handle)
+        elif handle:
+            self._lib.rl_notes_free(handle)
 
+
+_NOT_KERNELS = ("rl_copy_to_device", "rl_event_record")  # library functions that put something else on the stream
 _QUERIES = ("rl_gemm_tc_rows_fits", "rl_gemm_rows_smem_fits", "rl_mlp_fused_slice", "rl_attn_block_fused_fits", "rl_attn_block_fused_cluster",
             "rl_host_memory_on_device", "rl_latent_attention_fits", "rl_latent_decode_fits",
             "rl_moe_max_tiles", "rl_bias_attention_shape", "rl_recurrence_record", "rl_rmsnorm_add_experts_fits")  # library functions that launch nothing
@@ -111,6 +140,7 @@ class recording:
 
     def __exit__(self, *exc) -> None:
         global _recorder
+        _recorder.finish()
         _recorder = None
         self._list.launches = _launches - self._before
 
@@ -142,6 +172,11 @@ def _lib() -> ctypes.CDLL:
         lib.rl_gemm_tc_rows_fits.argtypes = [I, I, I]
         lib.rl_gemm_rows_smem.argtypes = [I, P, L, P, P, P, L, I, I, I, I, I, P, P, I, P, P, P, I, I, I, I, I, I, P, P]
         lib.rl_gemm_rows_smem_fits.argtypes = [I, I, I, I, I, I, I]
+        lib.rl_notes_begin.argtypes = lib.rl_notes_end.argtypes = []
+        lib.rl_notes_begin.restype = lib.rl_notes_replay.restype = I
+        lib.rl_notes_end.restype = P
+        lib.rl_notes_free.argtypes, lib.rl_notes_free.restype = [P], None
+        lib.rl_notes_replay.argtypes = [P, P]
         lib.rl_copy_to_device.argtypes = [P, P, L, P]
         lib.rl_event_record.argtypes = [P, P]
         lib.rl_attention.argtypes = [I, P, L, P, P, I, P, P, P, P, L, I, I, I, I, I, F, P, I, P, I, P, I, I, I, P, P, I, L, I, I, P, P]
