@@ -389,15 +389,28 @@ bool takes(const Args& p) {
 }
 
 // The weights as [K / 64][N][64]: a box is eight rows of `piece` blocks of 64 elements, a block's rows 128 bytes
-// apart and swizzled; rows beyond N and blocks beyond K read as zeros.
+// apart and swizzled; rows beyond N and blocks beyond K read as zeros.  Remembered by what they describe, as the other
+// kernels' maps are (tc::tensor_map): a step of GPT-2 1.5B asks for 192.
 static int weight_map(const Args& p, int piece, CUtensorMap* out) {
+  static std::unordered_map<tc::MapKey, CUtensorMap, tc::MapKeyHash> cache;
+  static std::mutex lock;
+  const tc::MapKey key{p.w, p.N, p.K, p.K, 8, piece, 2};
+  std::lock_guard<std::mutex> hold(lock);
+  const auto it = cache.find(key);
+  if (it != cache.end()) {
+    *out = it->second;
+    return 0;
+  }
   const cuuint64_t dim[3] = {64, (cuuint64_t)p.N, (cuuint64_t)(p.K / 64)};
   const cuuint64_t stride[2] = {(cuuint64_t)p.K * 2, 128};
   const cuuint32_t box[3] = {64, 8, (cuuint32_t)piece}, unit[3] = {1, 1, 1};
   const CUresult rc = tc::encode_fn()(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<__nv_bfloat16*>(p.w), dim, stride, box,
                                       unit, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                                       CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return rc == CUDA_SUCCESS ? 0 : -11;
+  if (rc != CUDA_SUCCESS) return -11;
+  if (cache.size() > 8192) cache.clear();
+  cache.emplace(key, *out);
+  return 0;
 }
 
 template <int HALVES, int PIECES, bool NORM>
