@@ -466,7 +466,7 @@ static inline int launch_attn_tc(const AttnParams& p, const int* tiles, int n_ti
     cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, dev);
     if (n_sms <= 0) n_sms = 1;
   }
-  const bool singly = (long)(n_tiles + 3) / 4 * p.n_heads > n_sms;
+  const bool singly = (long)(n_tiles + 3) / 4 * p.n_heads > n_sms && n_tiles <= 65535;  // (the limit of a grid's second extent)
   const dim3 grid = singly ? dim3(p.n_heads, n_tiles) : dim3(n_tiles, p.n_heads);
   launch_pdl_split(false, attn_tc_kernel, grid, ATT_THREADS, ATT_SMEM, stream, mq, mkv, p, tiles, singly ? 1 : 0);
   return 0;
