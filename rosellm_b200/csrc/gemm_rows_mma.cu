@@ -11,8 +11,8 @@
 // the elements are taken in a permuted order (a lane's eight consecutive elements serve two
 // MMA steps), which a dot product does not mind as long as A and W are permuted alike.
 // Warps that share columns (KSPLIT parts of K) add their accumulators in shared memory in a
-// fixed order.  tcgen05 is the tool for many rows (gemm_tc.cu); here its 128-row tiles and
-// shared-memory staging would only add latency.
+// fixed order.  Up to 16 rows gemm_rows_ring.cu takes what it can (inner sizes that are a multiple of 64, an even
+// width); here remain odd sizes, heads whose epilogue draws tokens, and narrow outputs of 17 to 64 rows.
 #include "gemm_epilogue.cuh"
 #include "gemm_rows_ring.cuh"
 #include "sampling_key.cuh"

@@ -25,11 +25,9 @@ STATUS_BITS = {
     8: "a bounded wait inside a kernel gave up",
 }
 
-# Rows up to which a matrix product streams the weights once per group of rows
-# instead of tiling: float32 products up to 64 rows (csrc/gemm_simt.cu), then 64x64 tiles in
-# IEEE arithmetic on the CUDA cores; bfloat16 products up to 16 rows the weight-streaming mma
-# kernel (csrc/gemm_rows_mma.cu), and up to 64 rows too unless the output is wide; otherwise
-# tcgen05, clustered (csrc/gemm_tc_rows.cu) or with 128-row tiles (csrc/gemm_tc.cu): bf16_path.
+# Rows up to which a float32 product streams the weights once per group of rows instead of
+# tiling, both in IEEE arithmetic on the CUDA cores (csrc/gemm_simt.cu); which kernel a
+# bfloat16 product runs on: bf16_path.
 ROWS_STREAMING_LIMIT = 64
 
 
@@ -485,9 +483,9 @@ def linear(a, weight, bias, out, *, act: int = ACT_NONE, residual: bool = False,
     at most 16 rows).  Otherwise
     a [rows, k] (row stride a multiple of 8), weight [n, k] contiguous, both float32 or both
     bfloat16; out [rows, n] of a's dtype or float32.  Which kernel runs: float32 up to 64 rows
-    the row kernel, above it 64x64 tiles (both IEEE FFMA); bfloat16 up to 16 rows the
-    weight-streaming mma kernel (for a very wide float32 output, a head, its form that is fed by
-    bulk copies: the library chooses), above it as ``bf16_path`` says.  ``path`` (for tests) forces
+    the row kernel, above it tiles (both IEEE FMAs); bfloat16 up to 16 rows the
+    weight-streaming kernels (fed by TMA through a ring; for a very wide float32 output, a head, by
+    bulk copies; by registers otherwise: the library chooses), above it as ``bf16_path`` says.  ``path`` (for tests) forces
     ``"rows"``, ``"tile"``, ``"mma"``, ``"smem"``, ``"tc"`` or ``"tcr"``.  ``kv``: output columns from
     ``kv.q_width`` on are written into cache pages, not ``out`` (not with ``"tile"``).
     ``tile_width`` and ``splits`` (for tests and measurements, ``"tc"`` only): the columns of an
