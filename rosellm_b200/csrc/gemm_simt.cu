@@ -80,22 +80,13 @@ __global__ __launch_bounds__(256) void gemm_tile_kernel(
   }
 }
 
-// Both halves of c += a * b: two float32 FMAs in one instruction, each rounded as fmaf rounds.
-__device__ __forceinline__ void fma_pair(uint64_t& c, uint64_t a, uint64_t b) {
-  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
-}
-__device__ __forceinline__ float pair_sum(uint64_t c) {
-  return __uint_as_float((uint32_t)c) + __uint_as_float((uint32_t)(c >> 32));
-}
-
 // Tiles of float32.  BM x BN output tile per block, TM x TN outputs per thread (rows and columns of a thread lie a
 // thread grid apart), K in steps of 16 that travel by cp.async, as they lie in memory, through a ring of three buffers of
 // shared memory (rows 80 bytes apart: the eight rows of a 16-byte access phase hit different banks).
-// Each output is two sums over k in ascending order, of its even and its odd elements, whatever M is and whatever the tile
-// is, so a row's result does not depend on which other rows share the launch: neighbouring elements of k lie side by side in both
-// operands, and one instruction takes both (fma.rn.f32x2), which leaves issue slots for the reads of shared memory: they are the bound, 12 pieces of 16 bytes a
-// thread for 128 FMAs with 8 x 4 outputs (about 19 of the 37.2 TFMA/s; the form before, 64 x 64 tiles of 4 x 4 outputs transposed
-// through registers with two barriers a step, 9 to 16).
+// Each output's sum runs over k in ascending order whatever M is and whatever the tile is, so a row's result does
+// not depend on which other rows share the launch.  What bounds it: reads of shared memory, 12 pieces of 16 bytes a thread for 128
+// FMAs with 8 x 4 outputs (about 19 of the 37.2 TFMA/s; the form before, 64 x 64 tiles of 4 x 4 outputs transposed through registers with
+// two barriers a step, 9 to 16).  Pairs of FMAs in one instruction (fma.rn.f32x2) measured the same and add up in another order.
 template <int BM, int BN, int TM, int TN>
 __global__ __launch_bounds__((BM / TM) * (BN / TN)) void gemm_tile_f32_kernel(
     const float* __restrict__ A, long lda, const float* __restrict__ W, const float* __restrict__ bias,
@@ -131,11 +122,11 @@ __global__ __launch_bounds__((BM / TM) * (BN / TN)) void gemm_tile_f32_kernel(
     }
   };
   pdl_begin();
-  uint64_t acc[TM][TN];
+  float acc[TM][TN];
 #pragma unroll
   for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < TN; ++j) acc[i][j] = 0ull;
+    for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
 #pragma unroll
   for (int s = 0; s < STAGES - 1; ++s) {
     if (s < steps) copy(s);
@@ -150,16 +141,20 @@ __global__ __launch_bounds__((BM / TM) * (BN / TN)) void gemm_tile_f32_kernel(
     const float* w_s = tile_s + (step % STAGES) * ((BM + BN) * LD) + (BM + tx) * LD;
 #pragma unroll
     for (int kk = 0; kk < BK; kk += 4) {
-      ulonglong2 w[TN];
+      float4 w[TN];
 #pragma unroll
-      for (int j = 0; j < TN; ++j) w[j] = *reinterpret_cast<const ulonglong2*>(w_s + j * GX * LD + kk);
+      for (int j = 0; j < TN; ++j) w[j] = *reinterpret_cast<const float4*>(w_s + j * GX * LD + kk);
 #pragma unroll
       for (int i = 0; i < TM; ++i) {
-        const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(a_s + i * GY * LD + kk);
+        const float4 a = *reinterpret_cast<const float4*>(a_s + i * GY * LD + kk);
 #pragma unroll
-        for (int j = 0; j < TN; ++j) fma_pair(acc[i][j], a.x, w[j].x);
+        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a.x, w[j].x, acc[i][j]);
 #pragma unroll
-        for (int j = 0; j < TN; ++j) fma_pair(acc[i][j], a.y, w[j].y);
+        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a.y, w[j].y, acc[i][j]);
+#pragma unroll
+        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a.z, w[j].z, acc[i][j]);
+#pragma unroll
+        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a.w, w[j].w, acc[i][j]);
       }
     }
   }
@@ -171,7 +166,7 @@ __global__ __launch_bounds__((BM / TM) * (BN / TN)) void gemm_tile_f32_kernel(
     for (int j = 0; j < TN; ++j) {
       const int n = n0 + j * GX + tx;
       if (n >= N) continue;
-      float v = pair_sum(acc[i][j]);
+      float v = acc[i][j];
       if (bias != nullptr) v += bias[n];
       v = apply_act(v, act);
       store_out<float>(out, (size_t)m * ldo + n, v, residual);
@@ -184,9 +179,9 @@ __global__ __launch_bounds__((BM / TM) * (BN / TN)) void gemm_tile_f32_kernel(
 // every piece of the weights that a lane holds meets all the rows in registers (the kernel before read a piece of A for
 // every piece of W, from the first-level cache, whose bandwidth bounded it).  A lane's weights travel by cp.async into a
 // ring of its own in shared memory (it reads back only what it copied itself, so no barrier is needed), two chunks
-// ahead, and the first of them before the wait for the kernels ahead.  The COLS * ROWS sums of a lane (each of its even and its odd
-// elements, one instruction taking two) are added over the lanes by halving exchanges (each lane gives away half of what it
-// has left), then over the warps in shared memory: in an order that is the same for every row whatever M is.
+// ahead, and the first of them before the wait for the kernels ahead.  The COLS * ROWS sums of a lane are added over the lanes
+// by halving exchanges (each lane gives away half of what it has left), then over the warps in shared memory: in an order
+// that is the same for every row whatever M is.
 // per_turn: groups whose sums meet at one barrier, at most ROWS_GROUPS.
 constexpr int ROWS_COLS = 4, ROWS_GROUPS = 4;
 template <int ROWS>
@@ -239,31 +234,31 @@ __global__ __launch_bounds__(256, 2) void gemm_rows_f32_kernel(
     for (int m0 = 0; m0 < M; m0 += ROWS, buf ^= 1) {
 #pragma unroll 1
       for (int g = 0; g < n_here; ++g) {
-        uint64_t sum[VALUES];  // [row][column]
+        float acc[VALUES];  // [row][column]
 #pragma unroll
-        for (int i = 0; i < VALUES; ++i) sum[i] = 0ull;
+        for (int i = 0; i < VALUES; ++i) acc[i] = 0.f;
         for (int chunk = warp; chunk < chunks; chunk += WARPS) {
           copy();  // into the stage that was read last
           asm volatile("cp.async.wait_group %0;" ::"n"(AHEAD) : "memory");
-          ulonglong2 w[COLS];
+          float4 w[COLS];
 #pragma unroll
-          for (int c = 0; c < COLS; ++c) w[c] = *reinterpret_cast<const ulonglong2*>(mine + (stage * COLS + c) * 32);
+          for (int c = 0; c < COLS; ++c) w[c] = mine[(stage * COLS + c) * 32];
           if (++stage == STAGES) stage = 0;
           const int k = chunk * 128 + 4 * lane;
 #pragma unroll
           for (int r = 0; r < ROWS; ++r) {
-            ulonglong2 a = make_ulonglong2(0ull, 0ull);
-            if (k < K) a = *reinterpret_cast<const ulonglong2*>(A + (size_t)min(m0 + r, M - 1) * lda + k);
+            float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (k < K) a = *reinterpret_cast<const float4*>(A + (size_t)min(m0 + r, M - 1) * lda + k);
 #pragma unroll
             for (int c = 0; c < COLS; ++c) {
-              fma_pair(sum[r * COLS + c], a.x, w[c].x);
-              fma_pair(sum[r * COLS + c], a.y, w[c].y);
+              float& t = acc[r * COLS + c];
+              t = fmaf(a.x, w[c].x, t);
+              t = fmaf(a.y, w[c].y, t);
+              t = fmaf(a.z, w[c].z, t);
+              t = fmaf(a.w, w[c].w, t);
             }
           }
         }
-        float acc[VALUES];
-#pragma unroll
-        for (int i = 0; i < VALUES; ++i) acc[i] = pair_sum(sum[i]);
         // after the exchange over lane bit o, a lane keeps the half of its values whose index has that bit as its own;
         // with one value left the lanes add it up
 #pragma unroll
