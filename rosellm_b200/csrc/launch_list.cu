@@ -40,7 +40,15 @@ RL_EXPORT int rl_notes_replay(void* handle, cudaStream_t stream) {
     cfg.stream = stream;
     cfg.attrs = const_cast<cudaLaunchAttribute*>(n.attrs);
     cfg.numAttrs = n.n_attrs;
-    rl::note_launch(cudaLaunchKernelExC(&cfg, n.kernel, params));
+    cudaError_t e = cudaLaunchKernelExC(&cfg, n.kernel, params);
+    if (e == cudaErrorInvalidValue && n.smem > 48 * 1024) {
+      // some kernels have their limit of shared memory set to what each launch needs: a launch since the notes were taken may
+      // have lowered it
+      cudaGetLastError();
+      cudaFuncSetAttribute(n.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)n.smem);
+      e = cudaLaunchKernelExC(&cfg, n.kernel, params);
+    }
+    rl::note_launch(e);
   }
   return rl::take_launch_error();
 }
