@@ -12,7 +12,7 @@
 // MMA steps), which a dot product does not mind as long as A and W are permuted alike.
 // Warps that share columns (KSPLIT parts of K) add their accumulators in shared memory in a
 // fixed order.  Up to 16 rows gemm_rows_ring.cu takes what it can (inner sizes that are a multiple of 64, an even
-// width); here remain odd sizes, heads whose epilogue draws tokens, and narrow outputs of 17 to 64 rows.
+// width); here remain odd sizes and narrow outputs of 17 to 64 rows.
 #include "gemm_epilogue.cuh"
 #include "gemm_rows_ring.cuh"
 #include "sampling_key.cuh"
@@ -541,7 +541,7 @@ RL_EXPORT int rl_gemm_rows_bf16(int out_dtype, const void* A, long lda, const vo
     }
   }
   if (out_dtype == RL_F32 || out_dtype == RL_BF16) {
-    const rl::ring::Args r{a, lda, norm, w, bias, out, ldo, M, N, K, act, residual, out_dtype == RL_F32 ? 1 : 0, kv, status};
+    const rl::ring::Args r{a, lda, norm, w, bias, out, ldo, M, N, K, act, residual, out_dtype == RL_F32 ? 1 : 0, kv, status, rl::SampleArgs{}};
     if (rl::ring::takes(r)) return rl::ring::run(r, stream);
   }
 #define RL_ROWS_MT(MT)                                                                                        \
@@ -597,6 +597,9 @@ RL_EXPORT int rl_gemm_rows_bf16_sample(const void* A, long lda, const void* W, c
       return e == cudaSuccess ? 0 : (int)e;
     }
   }
+  // the kernel that gives such a product's logits (rl_gemm_rows_bf16)
+  const rl::ring::Args r{a, lda, norm, w, bias, nullptr, 0, M, N, K, RL_ACT_NONE, 0, 1, kv, status, sample};
+  if (rl::ring::takes(r)) return rl::ring::run(r, stream);
   if (M <= 16)
     rl::launch_rows_mma<float, 1>(a, lda, norm, w, bias, nullptr, 0, M, N, K, RL_ACT_NONE, 0, kv, stream, sample);
   else if (M <= 32)

@@ -24,6 +24,7 @@
 // (5.2 TB/s of weights); 2048 x 8192 11.1, 7.8; 4800 x 1600 5.9, 5.5.  16 rows: += 1600 x 6400 14.0, 6.6.  A layer of a decode
 // step as a chain, 512 cached tokens, width 1600: 39.4 -> 28.0 at batch 1, 48.9 -> 35.6 at 8, 55.5 -> 38.4 at 16.
 #include "gemm_rows_ring.cuh"
+#include "sampling_key.cuh"
 #include "tc_common.cuh"
 
 namespace rl {
@@ -86,7 +87,9 @@ __device__ __forceinline__ uint32_t pack(float a, float b) {
 // HALVES: 1 for up to eight rows, 2 for up to sixteen.  PIECES: pieces of a group whose fragments of A a warp holds
 // at once (a longer K takes them in turn).  Registers: within half an SM's where a warp holds one piece of eight rows; with
 // more the 96 that this leaves a thread cost more than the neighbour gives (8 rows, 1600 x 6400: 7.9 us with them, 6.1 without).
-template <int HALVES, int PIECES, bool NORM>
+// SAMPLE: the rows' next tokens are chosen from the sums (SampleArgs) and nothing else is written: the same sums in the same
+// order as the form that writes them, so that a token is the one that the sampling kernel chooses from those logits.
+template <int HALVES, int PIECES, bool NORM, bool SAMPLE>
 __global__ __launch_bounds__(THREADS, HALVES * PIECES == 1 ? 2 : 1) void gemm_rows_ring_kernel(
     const __grid_constant__ CUtensorMap wmap, Args p, Cut cut) {
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -173,6 +176,19 @@ __global__ __launch_bounds__(THREADS, HALVES * PIECES == 1 ? 2 : 1) void gemm_ro
     }
   }
   asm volatile("griddepcontrol.wait;" ::: "memory");
+
+  // the row's sampling options, and its best entry so far
+  float temp = 0.f;
+  uint64_t seed = 0;
+  uint32_t counter = 0;
+  ArgMax best{-CUDART_INF_F, 0x7fffffff};
+  if (SAMPLE && p.sample.temperature != nullptr && e_thread && e_row < p.M) {
+    temp = p.sample.temperature[e_row];
+    if (temp > 0.f) {
+      seed = (uint64_t)p.sample.seeds[e_row];
+      counter = (uint32_t)p.sample.counters[e_row];
+    }
+  }
 
   // A's fragments: of piece b, slot i, the block kh + b * piece + 8 i + warp of 64 elements, in two steps of 32: lane j
   // holds elements 16 j ... 16 j + 7 of it for the first step and the next eight for the second.
@@ -314,6 +330,16 @@ __global__ __launch_bounds__(THREADS, HALVES * PIECES == 1 ? 2 : 1) void gemm_ro
       sum.x += v.x; sum.y += v.y;
     }
     const float v0 = apply_act(sum.x + bias.x, p.act), v1 = apply_act(sum.y + bias.y, p.act);
+    if constexpr (SAMPLE) {
+      float s0 = v0, s1 = v1;
+      if (temp > 0.f) {
+        const float inv_t = 1.0f / temp;
+        s0 = sample_key(soft_capped(v0, p.sample.soft_cap), inv_t, seed, counter, (uint32_t)n);
+        s1 = sample_key(soft_capped(v1, p.sample.soft_cap), inv_t, seed, counter, (uint32_t)(n + 1));
+      }
+      best = better(better(best, ArgMax{s0, n}), ArgMax{s1, n + 1});
+      continue;
+    }
     if (p.kv.pool != nullptr && n >= p.kv.q_width) {
       if (kv_page < 0) continue;
       const int cidx = n - p.kv.q_width;
@@ -327,10 +353,34 @@ __global__ __launch_bounds__(THREADS, HALVES * PIECES == 1 ? 2 : 1) void gemm_ro
       float* dst = (float*)p.out + (size_t)e_row * p.ldo + n;
       if (p.residual)  // one addition an element, or one a part of K (in no fixed order)
         asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(dst), "f"(v0), "f"(v1) : "memory");
-      else
+      else if (((uintptr_t)dst & 7) == 0)
         *reinterpret_cast<float2*>(dst) = make_float2(v0, v1);
+      else  // rows an odd number of elements apart
+        dst[0] = v0, dst[1] = v1;
     } else {
       *reinterpret_cast<__nv_bfloat162*>((__nv_bfloat16*)p.out + (size_t)e_row * p.ldo + n) = __floats2bfloat162_rn(v0, v1);
+    }
+  }
+  if constexpr (SAMPLE) {
+    // the four lanes of a row agree, a warp's best per row is offered once; then one ticket a block
+#pragma unroll
+    for (int o = 1; o <= 2; o <<= 1) {
+      const ArgMax b{__shfl_xor_sync(0xffffffffu, best.v, o), __shfl_xor_sync(0xffffffffu, best.i, o)};
+      best = better(best, b);
+    }
+    if (j == 0 && best.i != 0x7fffffff) {  // (only rows that are there have one)
+      const unsigned long long word = ((unsigned long long)ordered_bits(best.v) << 32) | (unsigned long long)(~(uint32_t)best.i);
+      if (word > __ldcg(p.sample.best + e_row)) {
+        atomicMax(p.sample.best + e_row, word);
+        __threadfence();
+      }
+    }
+    consumers_sync();
+    if (warp == 0) {
+      int last_block = 0;
+      if (lane == 0) last_block = atomicAdd(p.sample.ticket, 1) == (int)gridDim.x - 1;  // (K is not cut here)
+      last_block = __shfl_sync(0xffffffffu, last_block, 0);
+      if (last_block) sample_finish(p.sample, p.M, lane);
     }
   }
 }
@@ -374,8 +424,11 @@ static Cut cut_for(const Args& p) {
 }
 
 bool takes(const Args& p) {
-  if (p.M < 1 || p.M > 16 || p.K % 64 != 0 || p.K < 64 || p.N % 2 != 0 || p.ldo % 2 != 0 || p.status == nullptr) return false;
-  if ((uintptr_t)p.w % 16 != 0 || (uintptr_t)p.out % (p.out_f32 ? 8 : 4) != 0 || (p.bias != nullptr && (uintptr_t)p.bias % 8 != 0))
+  if (p.M < 1 || p.M > 16 || p.K % 64 != 0 || p.K < 64 || p.N % 2 != 0 || p.status == nullptr) return false;
+  // pairs of outputs are stored together; float32 ones that are not added to, logits among them, singly where need be (whether
+  // a head's tokens are asked for or its logits may not decide which kernel takes it)
+  if ((p.residual || !p.out_f32) && (p.ldo % 2 != 0 || (uintptr_t)p.out % (p.out_f32 ? 8 : 4) != 0)) return false;
+  if ((uintptr_t)p.w % 16 != 0 || (p.bias != nullptr && (uintptr_t)p.bias % 8 != 0))
     return false;
   if (p.norm.x == nullptr && (p.lda % 8 != 0 || (uintptr_t)p.a % 16 != 0)) return false;
   if (p.norm.x != nullptr && (p.K > MAX_PIECE * 64 || p.norm.ldx % 4 != 0 || (uintptr_t)p.norm.x % 16 != 0 ||
@@ -413,18 +466,23 @@ static int weight_map(const Args& p, int piece, CUtensorMap* out) {
   return 0;
 }
 
-template <int HALVES, int PIECES, bool NORM>
-static void launch(const CUtensorMap& wmap, const Args& p, const Cut& cut, cudaStream_t stream) {
+template <int HALVES, int PIECES, bool NORM, bool SAMPLE>
+static void launch_form(const CUtensorMap& wmap, const Args& p, const Cut& cut, cudaStream_t stream) {
+  constexpr auto kernel = gemm_rows_ring_kernel<HALVES, PIECES, NORM, SAMPLE>;
   static bool attr_set = false;
   if (!attr_set) {
-    note_launch(cudaFuncSetAttribute(gemm_rows_ring_kernel<HALVES, PIECES, NORM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     SMEM_TARGET));
-    note_launch(cudaFuncSetAttribute(gemm_rows_ring_kernel<HALVES, PIECES, NORM>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                     cudaSharedmemCarveoutMaxShared));
+    note_launch(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_TARGET));
+    note_launch(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
     attr_set = true;
   }
-  launch_pdl_split(false, gemm_rows_ring_kernel<HALVES, PIECES, NORM>, dim3(cut.blocks_n, cut.parts), dim3(THREADS),
+  launch_pdl_split(false, kernel, dim3(cut.blocks_n, cut.parts), dim3(THREADS),
                    (size_t)cut.fixed + (size_t)cut.stages * piece_bytes(cut.piece), stream, wmap, p, cut);
+}
+
+template <int HALVES, int PIECES, bool NORM>
+static void launch(const CUtensorMap& wmap, const Args& p, const Cut& cut, cudaStream_t stream) {
+  if (p.sample.out_ids != nullptr) launch_form<HALVES, PIECES, NORM, true>(wmap, p, cut, stream);
+  else launch_form<HALVES, PIECES, NORM, false>(wmap, p, cut, stream);
 }
 
 int run(const Args& p, cudaStream_t stream) {

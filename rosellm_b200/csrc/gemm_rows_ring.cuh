@@ -39,6 +39,7 @@ struct Args {
   int M, N, K, act, residual, out_f32;
   KvScatter kv;
   int* status;
+  SampleArgs sample;       // out_ids != nullptr: the rows' next tokens instead of `out` (nullptr then)
 };
 
 // Whether the kernel takes this product (sizes and alignments; see gemm_rows_ring.cu).

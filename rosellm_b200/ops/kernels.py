@@ -401,7 +401,7 @@ def sm_count(device: torch.device | None = None) -> int:
 
 
 def bf16_path(rows: int, n_out: int, k: int, *, residual: bool = False, out_f32: bool = False, act: int = ACT_NONE,
-              to_cache: bool = False) -> str:
+              to_cache: bool = False, head: bool = False) -> str:
     """Which kernel a bfloat16 product of these sizes runs on (measured on B200 at the widths of
     GPT-2, each kernel alone): up to 16 rows the weight-streaming kernels; 17 to 64 rows the kernel that keeps
     both operands in shared memory, where all of its blocks run at once and the output alone has not tiles
@@ -410,8 +410,8 @@ def bf16_path(rows: int, n_out: int, k: int, *, residual: bool = False, out_f32:
     ``+=`` into 1600 columns from 6400 10.3 us against 21.1 in shared memory in two rounds; 24 rows, 4800
     columns 8.6 against 17.2.  In one round shared memory is ahead: 768 columns from 3072 at 64 rows 5.0 us against
     7.2.  65 to 128 rows: the clustered kernel is behind the tiles or level with them from 768 columns on, 768 x 768
-    at 96 rows 9.1 against 6.0.)  Heads of less than 148 tiles stay on the kernels whose epilogue can draw a token of every
-    row.  Outputs too narrow to give the tiles work (``NARROW_OUTPUT``) go to shared
+    at 96 rows 9.1 against 6.0.)  A ``head`` of less than 148 tiles runs at 17 to 64 rows on what its tokens are drawn from as well: the
+    weight-streaming kernel, where the others do not take it.  Outputs too narrow to give the tiles work (``NARROW_OUTPUT``) go to shared
     memory in any number of rounds, the clustered kernel or the weight-streaming one."""
     if rows < 17:
         return "mma"
@@ -423,7 +423,7 @@ def bf16_path(rows: int, n_out: int, k: int, *, residual: bool = False, out_f32:
                                                int(to_cache)) if ROWS_IN_SHARED_MEMORY else 0
         if rounds == 1 or (rounds and narrow):
             return "smem"
-        if not narrow and not (out_f32 and not residual and k < 2048):  # (narrow heads: their epilogue draws tokens)
+        if not narrow and not head and not (out_f32 and not residual and k < 2048):
             return "tc"
         if rows > 32 and k >= 2048 and _lib().rl_gemm_tc_rows_fits(rows, n_out, k):
             return "tcr"
@@ -476,7 +476,7 @@ class KvTarget:
 
 
 def linear(a, weight, bias, out, *, act: int = ACT_NONE, residual: bool = False, path: str | None = None,
-           kv: KvTarget | None = None, tile_width: int = 0, splits: int = 0) -> None:
+           kv: KvTarget | None = None, tile_width: int = 0, splits: int = 0, head: bool = False) -> None:
     """out = act(a @ weight.T + bias), or out += ... when residual (out float32).
 
     ``a`` may be a ``NormInput``: the product then normalises float32 rows itself (bfloat16,
@@ -491,6 +491,8 @@ def linear(a, weight, bias, out, *, act: int = ACT_NONE, residual: bool = False,
     ``tile_width`` and ``splits`` (for tests and measurements, ``"tc"`` only): the columns of an
     output tile, a multiple of 32 up to 256, and the parts the inner size is cut into (1, 2, 3, 4, 6
     or 8: the blocks of a cluster take one each), instead of what the kernel would choose.
+    ``head``: the outputs are logits, whose tokens ``linear_sample`` may be asked for in their place: the same sums in
+    the same order as there, bit for bit (tiles then never cut the inner size).
     """
     norm = a if isinstance(a, NormInput) else None
     _need(weight, "weight")
@@ -533,9 +535,12 @@ def linear(a, weight, bias, out, *, act: int = ACT_NONE, residual: bool = False,
     bf16 = a_dtype == torch.bfloat16
     if path is None:
         if bf16:
-            path = bf16_path(m, n, k, residual=residual, out_f32=out.dtype == torch.float32, act=act, to_cache=kv is not None)
+            path = bf16_path(m, n, k, residual=residual, out_f32=out.dtype == torch.float32, act=act, to_cache=kv is not None,
+                             head=head)
         else:
             path = "rows" if m <= ROWS_STREAMING_LIMIT else "tile"
+    if head and path == "tc" and not splits:
+        splits = 1
     if path in ("mma", "tc", "tcr", "smem") and not bf16:
         raise KernelError("linear: the tensor-core kernels take bfloat16 inputs")
     if path == "mma" and m > 64:
@@ -641,13 +646,13 @@ def sampling_product_possible(rows: int, n_out: int, k: int, dtype: torch.dtype,
     24 against 33), so such batches are left to that."""
     if dtype != torch.bfloat16 or not 0 < rows <= SAMPLING_PRODUCT_MAX_ROWS or k % 8:
         return False
-    path = bf16_path(rows, n_out, k, out_f32=True)
+    path = bf16_path(rows, n_out, k, out_f32=True, head=True)
     return path == "mma" or (path == "tc" and not with_temperature)
 
 
 def linear_sample(a, weight, bias, into: SampleInto, soft_cap: float = 0.0) -> None:
-    """``into.out_ids[r]`` = the token ``sample`` would choose from row r of ``a @ weight.T + bias``
-    (arg-max, or with a temperature the arg-max of logit / temperature + Gumbel noise), without
+    """``into.out_ids[r]`` = the token ``sample`` would choose from row r of ``a @ weight.T + bias`` as ``linear(...,
+    head=True)`` gives it (arg-max, or with a temperature the arg-max of logit / temperature + Gumbel noise), without
     the logits being written anywhere.  bfloat16, where ``sampling_product_possible``;
     ``a`` may be a ``NormInput`` as for ``linear``.  Rows with top-k or top-p need their logits:
     they are not for this call.  ``soft_cap`` > 0: rows with a temperature draw from soft_cap * tanh(logit / soft_cap)
@@ -676,7 +681,7 @@ def linear_sample(a, weight, bias, into: SampleInto, soft_cap: float = 0.0) -> N
     if not sampling_product_possible(m, n, k, torch.bfloat16) or weight.data_ptr() % 16:
         raise KernelError("linear_sample: rows and an output width that the weight-streaming or the tcgen05 product "
                           "takes, an inner size that is a multiple of 8 and weights on a 16-byte boundary")
-    path = bf16_path(m, n, k, out_f32=True)
+    path = bf16_path(m, n, k, out_f32=True, head=True)
     if norm is not None and path != "mma":
         raise KernelError("linear_sample: a LayerNorm is fused only into the weight-streaming product")
     if bias is not None:

@@ -756,7 +756,7 @@ class TiedHead(Part):
     def forward(self, ctx, h) -> torch.Tensor:
         n_rows = h.x.shape[0] if isinstance(h, K.NormInput) else h.shape[0]
         logits = ctx.workspace.get("logits", (n_rows, self.vocab_size), torch.float32)
-        K.linear(h, self.weight, None, logits)
+        K.linear(h, self.weight, None, logits, head=True)
         if self.soft_cap:
             K.soft_cap(logits, self.soft_cap)
         return logits
