@@ -43,7 +43,9 @@ constexpr int ATT_Q_BYTES = ATT_Q * ATT_DH * 2;        // 16 KB
 constexpr int ATT_KV_BYTES = ATT_KV * ATT_DH * 2;      // 16 KB: keys or values of a tile
 constexpr int ATT_P_BYTES = ATT_Q * ATT_KV * 2;        // 32 KB: two K blocks of 64 keys
 constexpr int ATT_STAGES = 3;                          // tiles of keys and values in shared memory
-constexpr int ATT_SMEM = 2 * ATT_Q_BYTES + ATT_STAGES * 2 * ATT_KV_BYTES + ATT_P_BYTES + 128 + 3 * 4 * ATT_Q * 4 + 1024;
+// The probabilities lie in two buffers: those of tile g are written while the P V of tile g - 1 may still read its own (only the
+// P V of g - 2 has been waited for by then).  The block has its SM to itself either way.
+constexpr int ATT_SMEM = 2 * ATT_Q_BYTES + ATT_STAGES * 2 * ATT_KV_BYTES + 2 * ATT_P_BYTES + 128 + 3 * 4 * ATT_Q * 4 + 1024;
 
 // Instruction descriptor of kind::f16, bfloat16 x bfloat16 -> float32, M = 128; b_mn: the B
 // operand has its N dimension contiguous in shared memory (values as they lie in the cache).
@@ -112,11 +114,11 @@ __global__ __launch_bounds__(ATT_THREADS, 1) void attn_tc_kernel(const __grid_co
   uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)att_smem_raw + 1023) & ~(uintptr_t)1023);
   const uint32_t q_addr = smem_u32(smem);                            // [2 turns][128 queries]
   const uint32_t kv_addr = q_addr + 2 * ATT_Q_BYTES;                 // [stage][keys 16 KB, values 16 KB]
-  const uint32_t p_addr = kv_addr + ATT_STAGES * 2 * ATT_KV_BYTES;   // [2 K blocks][128 rows][128 bytes]
-  const uint32_t bar_base = p_addr + ATT_P_BYTES;
+  const uint32_t p_addr = kv_addr + ATT_STAGES * 2 * ATT_KV_BYTES;   // [2 tiles][2 K blocks][128 rows][128 bytes]
+  const uint32_t bar_base = p_addr + 2 * ATT_P_BYTES;
   const uint32_t q_full0 = bar_base, kv_full0 = bar_base + 16, kv_empty0 = bar_base + 40, s_full0 = bar_base + 64,
                  p_ready = bar_base + 80, pv_full0 = bar_base + 88;
-  uint8_t* after_p = smem + 2 * ATT_Q_BYTES + ATT_STAGES * 2 * ATT_KV_BYTES + ATT_P_BYTES;
+  uint8_t* after_p = smem + 2 * ATT_Q_BYTES + ATT_STAGES * 2 * ATT_KV_BYTES + 2 * ATT_P_BYTES;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(after_p + 112);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
@@ -265,7 +267,8 @@ __global__ __launch_bounds__(ATT_THREADS, 1) void attn_tc_kernel(const __grid_co
         const uint32_t v_addr = kv_addr + (uint32_t)(g % ATT_STAGES) * 2u * ATT_KV_BYTES + ATT_KV_BYTES;
 #pragma unroll
         for (int k = 0; k < ATT_KV / 16; ++k)  // 16 keys a step: two groups of eight value rows
-          mma_f16(tmem_pv + (uint32_t)(g & 1) * 64u, smem_desc(p_addr + (uint32_t)(k >> 2) * (ATT_Q * 128) + (k & 3) * 32),
+          mma_f16(tmem_pv + (uint32_t)(g & 1) * 64u,
+                  smem_desc(p_addr + (uint32_t)(g & 1) * ATT_P_BYTES + (uint32_t)(k >> 2) * (ATT_Q * 128) + (k & 3) * 32),
                   smem_desc_mn(v_addr + (uint32_t)k * 2048u), idesc_o, k != 0 ? 1u : 0u);
         mma_commit(kv_empty0 + 8 * (g % ATT_STAGES));
         mma_commit(pv_full0 + 8 * (g & 1));
@@ -281,7 +284,7 @@ __global__ __launch_bounds__(ATT_THREADS, 1) void attn_tc_kernel(const __grid_co
     const float sl2 = p.scale * 1.4426950408889634f;  // scores in units of log 2
     float* mx_s = reinterpret_cast<float*>(after_p + 128);  // [2 tiles][4 parts][128], then the sums [4 parts][128]
     float* sum_s = mx_s + 2 * 4 * ATT_Q;
-    // this thread's 32 probabilities of a tile: 64 bytes of the row in K block part / 2
+    // this thread's 32 probabilities of a tile: 64 bytes of the row in K block part / 2 (of the even tiles' buffer)
     uint8_t* p_row = smem + 2 * ATT_Q_BYTES + ATT_STAGES * 2 * ATT_KV_BYTES + (size_t)(part >> 1) * (ATT_Q * 128) + (size_t)row * 128;
     const int sw = row & 7;  // swizzle of 16-byte chunks
     auto row_sync = [&]() { asm volatile("bar.sync 1, 512;" ::: "memory"); };
@@ -374,7 +377,7 @@ __global__ __launch_bounds__(ATT_THREADS, 1) void attn_tc_kernel(const __grid_co
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           const int chunk = (part & 1) * 4 + c;
-          *reinterpret_cast<uint4*>(p_row + ((chunk ^ sw) << 4)) =
+          *reinterpret_cast<uint4*>(p_row + (g & 1) * ATT_P_BYTES + ((chunk ^ sw) << 4)) =
               make_uint4(packed[4 * c], packed[4 * c + 1], packed[4 * c + 2], packed[4 * c + 3]);
         }
         l = l * alpha + sum;
