@@ -9,8 +9,18 @@
 // From here on this thread's launches are noted, until rl_notes_end.  0, or -2 when they are being noted already.
 RL_EXPORT int rl_notes_begin() {
   if (rl::launch_notes != nullptr) return -2;
-  rl::launch_notes = new (std::nothrow) rl::LaunchNotes();
-  return rl::launch_notes != nullptr ? 0 : -3;
+  rl::LaunchNotes* notes = new (std::nothrow) rl::LaunchNotes();
+  if (notes == nullptr) return -3;
+  try {  // room for a step of twelve layers
+    notes->launches.reserve(96);
+    notes->at.reserve(2048);
+    notes->bytes.reserve(64 * 1024);
+  } catch (...) {
+    delete notes;
+    return -3;
+  }
+  rl::launch_notes = notes;
+  return 0;
 }
 
 // The notes are complete: a handle for rl_notes_replay and rl_notes_free, or nullptr where a launch could not be noted.
@@ -29,10 +39,11 @@ RL_EXPORT void rl_notes_free(void* handle) { delete (rl::LaunchNotes*)handle; }
 // The noted launches again, on `stream`, in order.  0 or the first error.
 RL_EXPORT int rl_notes_replay(void* handle, cudaStream_t stream) {
   constexpr size_t MOST = 64;
-  for (const rl::NotedLaunch& n : ((rl::LaunchNotes*)handle)->launches) {
+  const rl::LaunchNotes& notes = *(const rl::LaunchNotes*)handle;
+  for (const rl::NotedLaunch& n : notes.launches) {
     void* params[MOST];
-    if (n.at.size() > MOST) return -2;
-    for (size_t i = 0; i < n.at.size(); ++i) params[i] = (void*)(n.bytes.data() + n.at[i]);
+    if (n.n_args > MOST) return -2;
+    for (size_t i = 0; i < n.n_args; ++i) params[i] = (void*)(notes.bytes.data() + notes.at[n.first_arg + i]);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = n.grid;
     cfg.blockDim = n.block;

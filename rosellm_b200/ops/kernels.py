@@ -114,6 +114,7 @@ class _RecordingLib:
         handle = self._lib.rl_notes_end()
         if handle and self._whole:
             self._into._notes = (self._lib, handle)
+            self._into.calls = []  # what would be issued one by one is not needed any more
         elif handle:
             self._lib.rl_notes_free(handle)
 
