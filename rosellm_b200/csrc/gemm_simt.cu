@@ -439,7 +439,8 @@ static void launch_tile_f32(const float* a, long lda, const float* w, const floa
                             int act, int residual, cudaStream_t stream) {
   const int sms = simt_sm_count();
   auto cost = [&](int bm, int bn, double alone, double further) {
-    const long tiles = (long)((M + bm - 1) / bm) * ((N + bn - 1) / bn);
+    const long down = (M + bm - 1) / bm, tiles = down * ((N + bn - 1) / bn);
+    if (down > 65535) return 1e30;  // the limit of a grid's second extent: the tiles of 64 rows go furthest
     return alone + (double)((tiles + sms - 1) / sms - 1) * further;
   };
   const double large = cost(64, 64, 37.0, 24.8), middle = cost(32, 64, 24.5, 13.0), small = cost(32, 32, 16.0, 9.5);

@@ -55,3 +55,14 @@ def test_tiles(m, n, k):
     want = x.double() + ref
     K.linear(a, w, b, x, residual=True)
     _close(x, want, k)
+
+
+# more rows than a grid has tiles of 32 downwards
+@pytest.mark.parametrize("n", [1, 33])
+def test_very_many_rows(n):
+    m, k = 32 * 65535 + 1, 8
+    a, w, b = _data(m, n, k)
+    out = torch.full((m, n), float("nan"), device=DEV)
+    K.linear(a, w, b, out)
+    ref = torch.addmm(b.double(), a.double(), w.double().T)
+    _close(out, ref, k)
