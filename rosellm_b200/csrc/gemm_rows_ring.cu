@@ -423,6 +423,20 @@ static Cut cut_for(const Args& p) {
   return best;
 }
 
+// Whether the rows of W are so short that the register-fed kernel of gemm_rows_mma.cu is ahead: a piece costs about
+// 0.33 us (0.36 beyond eight rows) however short it is, which several groups of columns a block then pay one after the other,
+// and some tenths of a microsecond more than the other kernel before the first.  Measured up to 512 elements (us, register-fed
+// / here): 64 x 18944 at 8 rows 2.95 / 6.16, 64 x 2368 1.57 / 1.93; 256 x 9472 2.89 / 3.72 and 512 x 18944 6.15 / 6.40, but 256 x 7104 3.79 /
+// 3.28 and 512 x 7104 3.96 / 3.32 (six groups a block); 16 rows 256 x 1184 1.90 / 2.14, 512 x 9472 at 9 rows 4.31 / 4.56.  Added into
+// the stream only the shortest: 256 x 256 at 16 rows 2.3 / 1.9.  A LayerNorm of one or two rows costs the other
+// kernel's warps little as well: 256 x 9472 3.89 / 4.58 at one, 128 x 4736 2.91 / 3.30 at two, 3.97 / 3.36 at four.  From 576
+// elements on this kernel is ahead or level everywhere (576 x 37888 at 8 rows 12.86 / 11.81).
+static bool short_rows(int M, int N, int K, bool residual, bool norm) {
+  if (K > 512) return false;
+  if (norm) return K <= 256 && (M == 1 || (M == 2 && K >= 128));
+  return K < (residual ? 128 : 256) || (M > 8 && !residual) || (N + 7) / 8 > 6 * n_sms();
+}
+
 bool takes(const Args& p) {
   if (p.M < 1 || p.M > 16 || p.K % 64 != 0 || p.K < 64 || p.N % 2 != 0 || p.status == nullptr) return false;
   // pairs of outputs are stored together; float32 ones that are not added to, logits among them, singly where need be (whether
@@ -438,6 +452,7 @@ bool takes(const Args& p) {
   if (p.kv.pool != nullptr && (p.out_f32 || p.act != RL_ACT_NONE || p.kv.head_dim % 8 != 0 || p.kv.q_width % 8 != 0 ||
                                p.kv.kv_width % 8 != 0))
     return false;
+  if (short_rows(p.M, p.N, p.K, p.residual != 0, p.norm.x != nullptr)) return false;
   return tc::encode_fn() != nullptr;
 }
 
@@ -503,3 +518,9 @@ int run(const Args& p, cudaStream_t stream) {
 
 }  // namespace ring
 }  // namespace rl
+
+// Whether the sizes of a product of up to 16 rows are for this kernel (operands on the usual boundaries, even strides).
+RL_EXPORT int rl_gemm_rows_ring_fits(int M, int N, int K, int residual, int norm) {
+  return M >= 1 && M <= 16 && K % 64 == 0 && K >= 64 && N % 2 == 0 && !(norm && K > rl::ring::MAX_PIECE * 64) &&
+         !rl::ring::short_rows(M, N, K, residual != 0, norm != 0);
+}

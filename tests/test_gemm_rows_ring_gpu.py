@@ -85,3 +85,29 @@ def test_weights_that_are_not_finite_stay_in_their_column():
     assert torch.isnan(out[:, ::2]).all()
     _close(out[:, 1::2], (a.double() @ w.double().T + b.double())[:, 1::2], k)
 
+
+# short rows of W go through the ring only where a block has few groups of columns and the rows of A are few, or where the
+# result is added to the stream: both sides of each line (gemm_rows_ring.cu: short_rows; six groups a block on 148 SMs)
+@pytest.mark.parametrize("m,n,k,residual,norm,ring", [
+    (8, 7104, 256, False, False, True), (8, 7106, 256, False, False, False), (8, 4736, 192, False, False, False),
+    (9, 2368, 512, False, False, False), (9, 2368, 576, False, False, True), (8, 7106, 512, False, False, False),
+    (8, 16384, 576, False, False, True), (16, 256, 256, True, False, True), (16, 256, 128, True, False, True),
+    (16, 256, 64, True, False, False), (8, 7106, 512, True, False, False), (1, 2304, 256, False, True, False),
+    (1, 2304, 320, False, True, True), (2, 2304, 128, False, True, False), (2, 2304, 64, False, True, True),
+    (3, 2304, 128, False, True, True), (8, 10, 64, False, False, False)])
+def test_where_the_ring_begins(m, n, k, residual, norm, ring):
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert K.rows_are_ring_fed(m, n, k, residual=residual, norm=norm) == ring
+    a, w, b = _data(m, n, k, 4)
+    x = torch.randn(m, n, device=DEV) if residual else torch.full((m, n), float("nan"), device=DEV)
+    if norm:
+        inp = K.NormInput(a, torch.randn(k, device=DEV), None, 1e-5)
+        h = torch.nn.functional.layer_norm(a.double(), (k,), inp.gamma.double(), None, 1e-5).bfloat16().double()
+        # as in test_normalised_inside
+        tol = 8 * 2.0 ** -9
+    else:
+        inp, h, tol = a.bfloat16(), a.bfloat16().double(), 8 * k * 2.0 ** -24 + 1e-6
+    ref = h @ w.double().T + b.double() + (x.double() if residual else 0.0)
+    K.linear(inp, w, b, x, residual=residual)
+    assert (x.double() - ref).abs().max().item() <= tol
+    K.check_status(torch.device(DEV))
