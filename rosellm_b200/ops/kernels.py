@@ -404,17 +404,22 @@ def sm_count(device: torch.device | None = None) -> int:
 
 def bf16_path(rows: int, n_out: int, k: int, *, residual: bool = False, out_f32: bool = False, act: int = ACT_NONE,
               to_cache: bool = False, head: bool = False) -> str:
-    """Which kernel a bfloat16 product of these sizes runs on (measured on B200 at the widths of
-    GPT-2, each kernel alone): up to 16 rows the weight-streaming kernels; 17 to 64 rows the kernel that keeps
-    both operands in shared memory, where all of its blocks run at once and the output alone has not tiles
-    enough to fill the SMs (a head); beyond, and where that kernel would take several rounds or does not
-    fit, tcgen05 tiles.  (64 rows, K 1600: 4800 columns 8.5 us on tiles, 18.8 on the weight-streaming kernel;
-    ``+=`` into 1600 columns from 6400 10.3 us against 21.1 in shared memory in two rounds; 24 rows, 4800
-    columns 8.6 against 17.2.  In one round shared memory is ahead: 768 columns from 3072 at 64 rows 5.0 us against
-    7.2.  65 to 128 rows: the clustered kernel is behind the tiles or level with them from 768 columns on, 768 x 768
-    at 96 rows 9.1 against 6.0.)  A ``head`` of less than 148 tiles runs at 17 to 64 rows on what its tokens are drawn from as well: the
-    weight-streaming kernel, where the others do not take it.  Outputs too narrow to give the tiles work (``NARROW_OUTPUT``) go to shared
-    memory in any number of rounds, the clustered kernel or the weight-streaming one."""
+    """Which kernel a bfloat16 product of these sizes runs on (measured on B200, each kernel alone, us).
+
+    Up to 16 rows the weight-streaming kernels.  17 to 64 rows: tcgen05 tiles where the output has tiles enough to fill the
+    SMs; the kernel that keeps both operands in shared memory where all of its blocks run at once (768 columns from
+    3072 at 64 rows 5.0 against 7.2 on tiles; the weight-streaming kernel is ahead of it for some short rows, 2304 x 768 at 24
+    rows 3.7 against 4.0).  Where it would take several rounds or does not fit, tiles (64 rows, K 1600: 4800
+    columns 8.4 against 18.6 on the weight-streaming kernel; ``+=`` into 1600 columns from 6400 10.2 against 21.1 in shared
+    memory in two rounds; 24 rows, 4800 columns 8.4 against 17.2), but for two kinds.  Products that do not fit and
+    whose weights are few (``_few_weights``) run on the weight-streaming kernel, or with more than 32 rows and a long
+    inner size on the clustered one.  Float32 outputs that are not added to, with K below 2048, and every ``head``: in shared memory, and up to 32
+    rows on the weight-streaming kernel (5000 x 768 at 17 rows 5.8 against 7.2; at 48 10.7 against 9.7), unless the output is
+    wide and two rounds are enough (9400 x 1600 at 17 rows 17.5 against 12.4).  So a head runs on kernels whose
+    sums its tokens are drawn from as well, or on one that draws none.  65 to 128 rows: tiles; the clustered kernel is behind
+    or level with them from 768 columns on (768 x 768 at 96 rows 8.7 against 6.0).  Outputs too narrow to give the
+    tiles work (``NARROW_OUTPUT``) go to shared memory in any number of rounds, the clustered kernel or
+    the weight-streaming one."""
     if rows < 17:
         return "mma"
     narrow = n_out < NARROW_OUTPUT
@@ -425,14 +430,28 @@ def bf16_path(rows: int, n_out: int, k: int, *, residual: bool = False, out_f32:
                                                int(to_cache)) if ROWS_IN_SHARED_MEMORY else 0
         if rounds == 1 or (rounds and narrow):
             return "smem"
-        if not narrow and not head and not (out_f32 and not residual and k < 2048):
+        logits = head or (out_f32 and not residual and k < 2048)
+        if logits and rounds:
+            return "mma" if rows <= 32 and not (rounds == 2 and n_out > 8192 and k >= 1024) else "smem"
+        clustered = rows > 32 and k >= 2048 and bool(_lib().rl_gemm_tc_rows_fits(rows, n_out, k))
+        if not narrow and not logits and (rounds or residual or not _few_weights(rows, n_out, k, clustered)):
             return "tc"
-        if rows > 32 and k >= 2048 and _lib().rl_gemm_tc_rows_fits(rows, n_out, k):
-            return "tcr"
-        return "mma"
+        return "tcr" if clustered else "mma"
     if rows <= 128 and narrow and _lib().rl_gemm_tc_rows_fits(rows, n_out, k):
         return "tcr"
     return "tc"
+
+
+def _few_weights(rows: int, n_out: int, k: int, clustered: bool) -> bool:
+    """Whether a product of 17 to 64 rows that does not fit shared memory is too small for tiles (us, tiles against the
+    other kernel): up to 32 rows the weight-streaming kernel is ahead to 1024 columns (1024 x 4096 at 17 rows 7.5 against 5.4;
+    1600 x 4096 7.9 against 8.6), with rows of W up to 3072 elements to 2304 (2304 x 3072 at 17 rows 8.4 against 7.1; 2304 x 4096 level).  With
+    more rows the clustered kernel to 1600 columns (1600 x 2048 at 64 rows 7.3 against 6.9; 2304 x 2048 8.3 against
+    12.9), and where it does not go, below 2048 elements, the weight-streaming one to 1024 (1024 x 1600 at 33 rows 6.4 against 5.1;
+    1600 x 1600 at 64 rows 6.7 against 8.4)."""
+    if rows <= 32:
+        return n_out <= 1024 or (n_out <= 2304 and k <= 3072)
+    return n_out <= 1600 if clustered else n_out <= 1024 and k < 2048
 
 
 NARROW_OUTPUT = 768  # columns: fewer are twelve tiles or less
