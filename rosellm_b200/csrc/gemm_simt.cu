@@ -432,20 +432,46 @@ static void launch_tile_f32_form(const float* a, long lda, const float* w, const
              stream, a, lda, w, bias, o, ldo, M, N, K, act, residual);
 }
 
-// The tile that ends first, by what the forms measure at K 768 (us): a tile alone on its SM, and each further one.  (2304 x 768
-// at 1752 rows: 169, 174 and 207 us on 64 x 64, 32 x 64 and 32 x 32; 194 on the form before; 768 x 3072 287, 257, 281
-// and 440; 768 x 768 at 65 rows 37, 25, 16 and 45.  128 x 64, and 8 x 8 outputs a thread, measured slower throughout.)
-static void launch_tile_f32(const float* a, long lda, const float* w, const float* bias, float* o, long ldo, int M, int N, int K,
-                            int act, int residual, cudaStream_t stream) {
+// What a form of tile takes at K 768 (us) by how many of its tiles fall to an SM, measured in a chain of products and straight in
+// between; another K scales all forms alike.  A block alone is bound by its own chain of steps, and up to four, four and
+// six blocks an SM run beside one another; already from a third of the SMs on some SMs are given two (the next
+// launch's blocks are placed while the one ahead still runs).
+struct TileTime {
+  double tiles, us;
+};
+constexpr TileTime TIME_64X64[] = {{0.33, 32.2}, {0.6, 44.4}, {0.85, 69.8}, {1.1, 79.3}, {2.5, 90.1}, {4, 94.5}, {5, 128}, {8, 180}, {11, 250}};
+constexpr TileTime TIME_32X64[] = {{0.35, 20.6}, {0.65, 30.8}, {0.85, 35.4}, {1.1, 51.3}, {1.5, 52.7}, {2, 58.5}, {4.5, 63.8}, {5.2, 78.1},
+                                   {8, 104.6}, {14, 174.5}};
+constexpr TileTime TIME_32X32[] = {{0.5, 17.1}, {0.8, 21.7}, {1.2, 29.5}, {1.7, 38.5}, {2.1, 51.1}, {3, 52.4}, {4, 61.5}, {6.4, 61.5},
+                                   {8, 69.4}, {14, 109.7}, {30, 225.7}};
+
+template <int POINTS>
+static double tile_time(const TileTime (&time)[POINTS], double tiles) {
+  if (tiles <= time[0].tiles) return time[0].us;
+  int i = 1;
+  while (i < POINTS - 1 && tiles > time[i].tiles) ++i;
+  return time[i - 1].us + (time[i].us - time[i - 1].us) * (tiles - time[i - 1].tiles) / (time[i].tiles - time[i - 1].tiles);
+}
+
+// The tile that ends first.  Over 161 products of 65 to 2048 rows (64 to 4096 columns, K 256 to 6400) the choice is 1% behind the
+// fastest form on average; by counting rounds of tiles it was 7%, up to 45% (1600 x 1600 at 300 rows: 146, 99 and 120 us on 64 x 64,
+// 32 x 64 and 32 x 32; 768 x 768 at 600 rows 66, 56 and 59).  128 x 64, and 8 x 8 outputs a thread, measured slower throughout.
+static dim3 tile_f32_for(int M, int N) {
   const int sms = simt_sm_count();
-  auto cost = [&](int bm, int bn, double alone, double further) {
+  auto cost = [&](int bm, int bn, const auto& time) {
     const long down = (M + bm - 1) / bm, tiles = down * ((N + bn - 1) / bn);
     if (down > 65535) return 1e30;  // the limit of a grid's second extent: the tiles of 64 rows go furthest
-    return alone + (double)((tiles + sms - 1) / sms - 1) * further;
+    return tile_time(time, (double)tiles / sms);
   };
-  const double large = cost(64, 64, 37.0, 24.8), middle = cost(32, 64, 24.5, 13.0), small = cost(32, 32, 16.0, 9.5);
-  if (large <= middle && large <= small) launch_tile_f32_form<64, 64, 8, 4>(a, lda, w, bias, o, ldo, M, N, K, act, residual, stream);
-  else if (middle <= small) launch_tile_f32_form<32, 64, 4, 4>(a, lda, w, bias, o, ldo, M, N, K, act, residual, stream);
+  const double large = cost(64, 64, TIME_64X64), middle = cost(32, 64, TIME_32X64), small = cost(32, 32, TIME_32X32);
+  return large <= middle && large <= small ? dim3(64, 64) : middle <= small ? dim3(32, 64) : dim3(32, 32);
+}
+
+static void launch_tile_f32(const float* a, long lda, const float* w, const float* bias, float* o, long ldo, int M, int N, int K,
+                            int act, int residual, cudaStream_t stream) {
+  const dim3 tile = tile_f32_for(M, N);  // rows, columns
+  if (tile.x == 64) launch_tile_f32_form<64, 64, 8, 4>(a, lda, w, bias, o, ldo, M, N, K, act, residual, stream);
+  else if (tile.y == 64) launch_tile_f32_form<32, 64, 4, 4>(a, lda, w, bias, o, ldo, M, N, K, act, residual, stream);
   else launch_tile_f32_form<32, 32, 4, 2>(a, lda, w, bias, o, ldo, M, N, K, act, residual, stream);
 }
 
@@ -532,4 +558,10 @@ RL_EXPORT int rl_gemm_simt(int in_dtype, int out_dtype, const void* A, long lda,
   if (rc != 0) return rc;
   RL_CHECK_LAUNCH();
   return 0;
+}
+
+// The tile that a float32 product of so many rows and columns runs in: 100 x its rows + its columns.
+RL_EXPORT int rl_gemm_tile_f32_for(int M, int N) {
+  const dim3 tile = rl::tile_f32_for(M, N);
+  return (int)(100 * tile.x + tile.y);
 }

@@ -122,7 +122,7 @@ class _RecordingLib:
 _NOT_KERNELS = ("rl_copy_to_device", "rl_event_record")  # library functions that put something else on the stream
 _QUERIES = ("rl_gemm_tc_rows_fits", "rl_gemm_rows_smem_fits", "rl_mlp_fused_slice", "rl_attn_block_fused_fits", "rl_attn_block_fused_cluster",
             "rl_host_memory_on_device", "rl_latent_attention_fits", "rl_latent_decode_fits",
-            "rl_gemm_rows_ring_fits", "rl_moe_max_tiles", "rl_bias_attention_shape", "rl_recurrence_record", "rl_rmsnorm_add_experts_fits")  # library functions that launch nothing
+            "rl_gemm_rows_ring_fits", "rl_gemm_tile_f32_for", "rl_moe_max_tiles", "rl_bias_attention_shape", "rl_recurrence_record", "rl_rmsnorm_add_experts_fits")  # library functions that launch nothing
 
 
 class recording:
@@ -172,6 +172,7 @@ def _lib() -> ctypes.CDLL:
         lib.rl_gemm_rows_smem.argtypes = [I, P, L, P, P, P, L, I, I, I, I, I, P, P, I, P, P, P, I, I, I, I, I, I, P, P]
         lib.rl_gemm_rows_smem_fits.argtypes = [I, I, I, I, I, I, I]
         lib.rl_gemm_rows_ring_fits.argtypes = [I, I, I, I, I]
+        lib.rl_gemm_tile_f32_for.argtypes = [I, I]
         lib.rl_notes_begin.argtypes = lib.rl_notes_end.argtypes = []
         lib.rl_notes_begin.restype = lib.rl_notes_replay.restype = I
         lib.rl_notes_end.restype = P
@@ -455,6 +456,11 @@ def _few_weights(rows: int, n_out: int, k: int, clustered: bool) -> bool:
 
 
 NARROW_OUTPUT = 768  # columns: fewer are twelve tiles or less
+
+def f32_tile(rows: int, n_out: int) -> tuple[int, int]:
+    """Rows and columns of the output tile that a block takes of a float32 product of more than ``ROWS_STREAMING_LIMIT`` rows."""
+    return divmod(_lib().rl_gemm_tile_f32_for(rows, n_out), 100)
+
 
 def rows_are_ring_fed(rows: int, n_out: int, k: int, *, residual: bool = False, norm: bool = False) -> bool:
     """Whether a bfloat16 product of up to 16 rows runs on the kernel whose weights come through a ring in shared memory

@@ -66,3 +66,11 @@ def test_very_many_rows(n):
     K.linear(a, w, b, out)
     ref = torch.addmm(b.double(), a.double(), w.double().T)
     _close(out, ref, k)
+
+
+# the fastest of the three where they are far apart (csrc/gemm_simt.cu: launch_tile_f32)
+@pytest.mark.parametrize("m,n,tile", [(300, 1600, (32, 64)), (100, 768, (32, 32)), (65, 256, (32, 32)), (1300, 768, (32, 64)),
+                                      (2048, 3072, (64, 64)), (32 * 65535 + 1, 1, (64, 64))])
+def test_which_tile(m, n, tile):
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert K.f32_tile(m, n) == tile
