@@ -776,13 +776,46 @@ def rows_bulk_kernel(on: bool) -> None:
 FUSED_ROWS = True
 
 
-def separate_is_faster(rows: int, hidden: int) -> bool:
-    """Whether a layer's products of few rows run faster as kernels of their own (the ring-fed product, whose weights
-    arrive under the kernels ahead) than in the two fused kernels.  Measured on B200, a layer of GPT-2 124M with 512
-    cached tokens, us fused / separate: 16.6 / 16.5 at 1 row, 16.9 / 16.9 at 2, 18.1 / 17.5 at 4, 20.5 / 18.8 at
-    8, 24.4 / 23.2 at 12, 26.5 / 28.3 at 16; width 1024 (the feed-forward alone fused) 21.1 / 20.0 at 1, 23.9 /
-    22.8 at 8, 34.5 / 33.9 at 16."""
-    return hidden > 768 or 2 < rows <= 12
+# The widest stream whose layers are worth their fused form; beyond, separate kernels are ahead (see below).
+FUSED_LAYER_MAX_WIDTH = 960
+
+
+def separate_is_faster(rows: int, hidden: int, attention_fused: bool) -> bool:
+    """Whether a pre-norm layer's products of few rows run as kernels of their own (the ring-fed product, whose weights
+    arrive under the kernels ahead) and not in the two fused kernels; ``attention_fused``: the step's attention can be one
+    of them (a decode step that its sizes fit), else it is the feed-forward alone.  A captured step serves every context, so
+    the form with no context at which it is clearly behind is taken.  Measured on B200 at 32 / 256 / 512 / 1000
+    cached tokens, us a layer, fused > separate:
+
+    both fused, width 576, 8 rows    16.4 > 17.1   17.3 > 17.1   18.7 > 18.2   21.8 > 20.5
+                704, 5               16.6 > 16.8   17.4 > 16.8   18.7 > 17.8   21.3 > 20.1
+                768, 1               16.7 > 15.3   16.7 > 15.6   16.7 > 16.7   16.9 > 18.9
+                768, 4               16.8 > 16.7   17.1 > 16.7   17.8 > 17.7   19.4 > 20.0
+                768, 8               18.0 > 17.5   19.9 > 17.6   20.3 > 18.8   23.2 > 21.1
+                768, 12              18.8 > 21.0   21.4 > 21.3   23.8 > 22.7   29.3 > 25.1
+                832, 8               18.7 > 18.4   19.7 > 18.4   21.5 > 19.5   24.6 > 22.0
+                896, 1               17.7 > 17.9   17.6 > 18.0   17.8 > 19.1   17.9 > 21.5
+                960, 5               19.0 > 19.6   19.8 > 19.7   21.3 > 20.7   23.8 > 23.1
+    feed-forward,     128, 1         12.1 > 12.6   12.2 > 12.7   13.0 > 13.8   15.4 > 16.2
+                256, 8               15.0 > 14.8   15.2 > 15.1   16.0 > 16.1   18.3 > 18.2
+                384, 9               17.1 > 18.4   17.2 > 18.7   18.9 > 20.0   21.1 > 22.3
+                768, 1               18.2 > 15.6   18.3 > 15.7   19.7 > 16.6   22.1 > 18.9
+                768, 12              21.9 > 20.9   22.2 > 21.3   22.9 > 22.8   26.0 > 25.2
+                768, 16              22.4 > 21.4   23.3 > 23.2   25.6 > 26.7   31.2 > 33.2
+                1024, 1              19.8 > 18.8   20.3 > 19.0   21.0 > 19.5   23.5 > 21.9
+                1024, 8              22.0 > 20.9   22.2 > 20.9   23.4 > 22.0   25.7 > 24.6
+                1024, 16             25.5 > 24.2   28.2 > 26.2   29.9 > 29.7   34.8 > 36.3
+
+    Both at 1024 columns are not to be had (sixteen heads of clusters are more than the device holds).  There the separate
+    form is taken for all rows, though from eleven to fifteen rows and 512 tokens on it is up to 9% behind."""
+    if hidden > FUSED_LAYER_MAX_WIDTH:
+        return True
+    middle = 704 <= hidden <= 832
+    if attention_fused:
+        return middle and 5 <= rows <= 8
+    return (hidden >= 256 and rows <= 8) or (middle and rows <= 12)
+
+
 _mlp_slices: dict[tuple, int] = {}
 
 

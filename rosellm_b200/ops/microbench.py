@@ -175,6 +175,20 @@ def _layer_ring(a, dev, dt, entries):
     return ring, ctx, x, layer_bytes
 
 
+def _fused_kernels_of(run) -> list[str]:
+    """The names of the fused decode kernels that ``run()`` launches."""
+    names, real = [], {}
+    for name in ("attn_block_fused", "mlp_fused"):
+        real[name] = getattr(K, name)
+        setattr(K, name, lambda *a, name=name, **kw: (names.append(name), real[name](*a, **kw))[1])
+    try:
+        run()
+    finally:
+        for name, fn in real.items():
+            setattr(K, name, fn)
+    return names
+
+
 def main(argv=None) -> int:
     p = argparse.ArgumentParser(description=__doc__.split("\n\n")[0])
     p.add_argument("--op", required=True, choices=["linear", "attention-decode", "attention-prefill", "layernorm", "sample", "head", "decode-layer", "prefill-layer", "mlp"])
@@ -202,6 +216,8 @@ def main(argv=None) -> int:
     p.add_argument("--slice", type=int, default=0, help="mlp: slice of the inner width a block takes (0: as the library chooses)")
     p.add_argument("--unfused", action="store_true",
                    help="decode-layer: the fused kernels of few rows switched off (every product a kernel of its own)")
+    p.add_argument("--fused", action="store_true",
+                   help="decode-layer: the fused kernels wherever their sizes fit (not only where they are taken to be the faster form)")
     p.add_argument("--phases", action="store_true",
                    help="print the clock stamps of the fused decode kernels' phases (a library built with "
                         "ROSELLM_B200_NVCC_EXTRA=-DRL_PHASE_TIMING; all zero otherwise)")
@@ -326,6 +342,8 @@ def main(argv=None) -> int:
         assert h * dh == hid
         ring, ctx, x, layer_bytes = _layer_ring(a, dev, dt, [(r, a.context - 1, [0], []) for r in range(rows)])
         K.FUSED_ROWS = not a.unfused
+        if a.fused:
+            K.separate_is_faster = lambda rows, hidden, attention_fused: False
         if a.splits or a.wide:
             ctx.extras["decode_plan"] = (max(1, a.splits), a.wide)
 
@@ -333,8 +351,9 @@ def main(argv=None) -> int:
             run, parts = ring[i % len(ring)]
             parts.block.forward(ctx, run, parts, x)
 
+        ran = _fused_kernels_of(lambda: layer(0))
         us = _time(layer, a.reps, graph=not a.eager)
-        rec.update(batch=rows, context=a.context, hidden=hid, inner=inner, fused=not a.unfused,
+        rec.update(batch=rows, context=a.context, hidden=hid, inner=inner, fused=ran,
                    plan=ctx.extras.get("decode_plan"), us=round(us, 2), gbytes_per_s=round(layer_bytes / us / 1e3, 1))
     else:
         h, hk, dh, ps = a.heads, a.kv_heads or a.heads, a.head_dim, a.page_size

@@ -465,16 +465,16 @@ class CausalSelfAttention(Part):
             if cluster:
                 self._out_weight_packed = K.attn_pack_out_weight(w, self.num_heads, self.head_dim, cluster)
 
-    def _fused_decode(self, ctx, run, h, x) -> bool:
+    def fits_one_kernel(self, ctx, run, h, x) -> bool:
         """A step of few decoded requests and nothing else: the whole of this part (its norm
-        included) in one kernel, where the sizes fit."""
+        included) can be one kernel, where the sizes fit."""
         n = ctx.n_tokens
-        return (self._out_weight_packed is not None and K.FUSED_ROWS and n <= 16 and not ctx.extras.get("separate_products")
+        return (self._out_weight_packed is not None and K.FUSED_ROWS and n <= 16
                 and isinstance(h, K.NormInput) and h.x is x and n == ctx.n_decode == ctx.n_reqs and run.writes_cache
                 and not getattr(ctx.position, "rotates", True))
 
     def forward(self, ctx, run, h, x, add: bool = True) -> None:
-        if add and self._fused_decode(ctx, run, h, x):
+        if add and not ctx.extras.get("separate_products") and self.fits_one_kernel(ctx, run, h, x):
             K.attn_block_fused(x, h, self.qkv_weight, self.qkv_bias, self._out_weight_packed, self.out_bias,
                                ctx.kv_pool(run.cache_key), ctx.block_table(run.cache_key), ctx.positions, ctx.slots,
                                n_heads=self.num_heads, scale=self.scale, max_pos=ctx.cache.max_seq_len)
@@ -597,9 +597,10 @@ class PreNormBlock(Part):
     uses = {"norm_mixer": "norm", "mixer": "mixer", "norm_feed_forward": "norm", "feed_forward": "feed_forward"}
 
     def forward(self, ctx, run, layer, x) -> None:
-        # which form of a layer of few rows is the faster: the parts that have a fused one look here
-        ctx.extras["separate_products"] = K.separate_is_faster(ctx.n_tokens, x.shape[1])
         h = self._normed(ctx, layer.norm_mixer, x, layer.mixer)
+        # which form of a layer of few rows is the faster: the parts that have a fused one look here
+        fits = getattr(layer.mixer, "fits_one_kernel", None)
+        ctx.extras["separate_products"] = K.separate_is_faster(ctx.n_tokens, x.shape[1], fits is not None and fits(ctx, run, h, x))
         layer.mixer.forward(ctx, run, h, x)
         h = self._normed(ctx, layer.norm_feed_forward, x, layer.feed_forward)
         layer.feed_forward.forward(ctx, h, x)
