@@ -67,7 +67,10 @@ def _build_layer(ls) -> Layer:
                 f"block {ls.block.kind!r} arranges a {cat} called {name!r}; the layer's spec gives "
                 f"{ {n: c for n, c in cats.items()} }"
             )
-    return Layer(block, parts, cats)
+    layer = Layer(block, parts, cats)
+    if hasattr(block, "arrange"):
+        block.arrange(layer)
+    return layer
 
 
 def _parts_with_specs(spec: ModelSpec, model: "Model | None" = None):

@@ -776,7 +776,8 @@ def rows_bulk_kernel(on: bool) -> None:
 FUSED_ROWS = True
 
 
-# The widest stream whose layers are worth their fused form; beyond, separate kernels are ahead (see below).
+# The widest stream whose layers are worth their fused form; beyond, separate kernels are ahead (see below), and the weights
+# that the fused kernels read in a layout of their own are not kept.
 FUSED_LAYER_MAX_WIDTH = 960
 
 
@@ -807,7 +808,8 @@ def separate_is_faster(rows: int, hidden: int, attention_fused: bool) -> bool:
                 1024, 16             25.5 > 24.2   28.2 > 26.2   29.9 > 29.7   34.8 > 36.3
 
     Both at 1024 columns are not to be had (sixteen heads of clusters are more than the device holds).  There the separate
-    form is taken for all rows, though from eleven to fifteen rows and 512 tokens on it is up to 9% behind."""
+    form is taken for all rows, though from eleven to fifteen rows and 512 tokens on it is up to 9% behind: the fused
+    feed-forward reads a copy of its output weights, 250 MB for the 24 layers of GPT-2 355M."""
     if hidden > FUSED_LAYER_MAX_WIDTH:
         return True
     middle = 704 <= hidden <= 832

@@ -357,6 +357,7 @@ class CausalSelfAttention(Part):
     graph_safe = True
     launches_replayable = True
     takes_norm_input = True  # h may be a K.NormInput: the qkv product then normalises its own input
+    keeps_fused_weights = True  # as in DenseMLP
 
     def __init__(self, hidden_size: int, num_heads: int, head_dim: int, num_kv_heads: int | None = None,
                  window: int | None = None, scale: float | None = None, bias: bool = True,
@@ -459,7 +460,7 @@ class CausalSelfAttention(Part):
         # the fused kernel of a decode step reads W_out slice by slice: laid out for it once, here
         self._out_weight_packed = None
         w = self.out_weight
-        if (w is not None and w.is_cuda and self.window is None and self.num_kv_heads == self.num_heads
+        if (w is not None and w.is_cuda and self.keeps_fused_weights and self.window is None and self.num_kv_heads == self.num_heads
                 and self.q_width == self.hidden_size):
             cluster = K.attn_block_fused_cluster(self.hidden_size, self.num_heads, self.head_dim, w.dtype)
             if cluster:
@@ -532,6 +533,10 @@ class DenseMLP(Part):
     launches_replayable = True
     takes_norm_input = True
 
+    # whether the output weights are laid out a second time for the fused kernel of few rows (a block that never
+    # runs it says no before the weights come)
+    keeps_fused_weights = True
+
     def __init__(self, hidden_size: int, inner_size: int, activation: str, bias: bool = True,
                  weights_in_out: bool = False) -> None:
         if activation not in K.ACTIVATIONS or activation == "none":
@@ -570,7 +575,7 @@ class DenseMLP(Part):
                 self.in_bias = torch.nn.functional.pad(self.in_bias, (0, pad)).contiguous()
         # the fused kernel of few rows reads W_out slice by slice: laid out for it once, here
         self._fused_slice, self._out_weight_packed = 0, None
-        if self.out_weight.is_cuda:
+        if self.out_weight.is_cuda and self.keeps_fused_weights:
             self._fused_slice = K.mlp_fused_slice(1, self.hidden_size, self.inner_padded, True, self.out_weight.dtype)
             if self._fused_slice:
                 self._out_weight_packed = K.mlp_pack_out_weight(self.out_weight, self._fused_slice)
@@ -595,6 +600,13 @@ class PreNormBlock(Part):
     launches_replayable = True
     # the sub-parts of a layer this block arranges, by name and category
     uses = {"norm_mixer": "norm", "mixer": "mixer", "norm_feed_forward": "norm", "feed_forward": "feed_forward"}
+
+    def arrange(self, layer) -> None:
+        """Told of the layer before its weights come: where the stream is too wide for the fused kernels, its parts keep
+        no weights for them."""
+        for part in (layer.mixer, layer.feed_forward):
+            if getattr(part, "hidden_size", 0) > K.FUSED_LAYER_MAX_WIDTH and hasattr(part, "keeps_fused_weights"):
+                part.keeps_fused_weights = False
 
     def forward(self, ctx, run, layer, x) -> None:
         h = self._normed(ctx, layer.norm_mixer, x, layer.mixer)

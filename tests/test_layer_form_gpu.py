@@ -1,4 +1,4 @@
-"""Which form a decode layer of few rows takes (two fused kernels or kernels of its own)."""
+"""Which form a decode layer of few rows takes (two fused kernels or kernels of its own), and what the parts keep for it."""
 import pytest
 import torch
 
@@ -36,6 +36,9 @@ def _layer(hidden, heads):
     (1024, 16, {1: [], 8: [], 16: []}, {4: [], 16: []})])
 def test_form_of_a_layer(hidden, heads, decoded, prompt):
     layer = _layer(hidden, heads)
+    # the second copy of the output weights is kept only where some row count reads it
+    kept = hidden <= K.FUSED_LAYER_MAX_WIDTH
+    assert (layer.mixer._out_weight_packed is not None) == kept and (layer.feed_forward._out_weight_packed is not None) == kept
     cache = make_cache({0: layer.mixer.cache_spec()}, page=16, pages=80, slots=18, seq=64, dtype=torch.bfloat16)
     slots = [cache.new_request() for _ in range(16)]
     for s in slots:
