@@ -67,3 +67,25 @@ def test_decode_attention_in_blocks_of_eight_warps(dtype, n_req, heads, dh):
     """More blocks than the device holds of sixteen warps; contexts of one key, beside a round of a block's keys and beyond."""
     lens = [[1, 33, 127, 128, 129, 257, 600][i % 7] for i in range(n_req)]
     run_attention(K, dtype, [1] * n_req, lens, heads, heads, dh, 16, None, seed=dh, decode_wide=True)
+
+
+def test_a_kernel_whose_limit_of_shared_memory_has_been_lowered_since_is_issued_again():
+    """The norm of rows of some sizes has its kernel's limit set to what each launch needs: one of shorter rows lowers it."""
+    def row(n):
+        x = torch.randn(3, n, device=DEV)
+        return x, torch.randn(n, device=DEV), torch.randn(n, device=DEV), torch.empty(3, n, device=DEV)
+
+    long, short = row(30001), row(14001)  # 117 and 55 KB, both above the limit that needs no raising
+    with K.recording() as launches:
+        K.layernorm(*long[:3], 1e-5, long[3])
+    assert launches._notes is not None
+    K.layernorm(*short[:3], 1e-5, short[3])
+    long[0].mul_(2).add_(1)
+    long[3].fill_(float("nan"))
+    launches.replay()
+    for x, gamma, beta, out in (long, short):
+        want = torch.nn.functional.layer_norm(x.double(), x.shape[1:], gamma.double(), beta.double(), 1e-5)
+        assert (out.double() - want).abs().max().item() < 1e-4  # float32 statistics of numbers of order 1
+    K.layernorm(*short[:3], 1e-5, short[3])
+    launches.replay()  # and once more after the limit was lowered a second time
+    torch.cuda.synchronize()
