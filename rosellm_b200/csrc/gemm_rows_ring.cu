@@ -4,11 +4,12 @@
 //
 // Such a product is its weight stream and, in a step, the wait for the kernel ahead.  One block an
 // SM owns some groups of eight output columns (and, for an `out += ...`, perhaps a part of K).  The
-// weight rows of a group, up to 1024 elements of each at a time, are copied by the copy engine
-// (cp.async.bulk, a copy a row) into a ring of stages in shared memory, and the first of them before
-// the block waits for the kernels ahead, since no kernel writes weights.  A block's shared memory and registers are kept below
-// half of an SM's, so that the next product's block stands beside this one and its weights arrive
-// while this one computes: in a chain of products the memory is busy through the kernel boundaries.
+// weight rows of a group, up to 1024 elements of each at a time, are brought by TMA (one box of eight rows
+// a piece: cp.async.bulk.tensor; a bulk copy a row measured 19.7 us where this takes 13) into a ring of stages in shared memory,
+// and the first of them before the block waits for the kernels ahead, since no kernel writes weights.  A block's shared
+// memory is kept below half of an SM's, and where a warp holds one piece of eight rows its registers too, so
+// that the next product's block stands beside this one and its weights arrive while this one computes: in a chain of
+// products the memory is busy through the kernel boundaries.  Short rows of W stay with gemm_rows_mma.cu (short_rows).
 // Eight warps share K (blocks of 64 elements in turn), so that a warp's part of the rows of A, as mma.sync
 // fragments, stays in its registers for all of the block's columns: the rows are read (and normalised,
 // through shared memory) once a block.  A ninth warp keeps the ring full.  The loop over the pieces is kept to some tens of
@@ -477,7 +478,10 @@ static int weight_map(const Args& p, int piece, CUtensorMap* out) {
                                       CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (rc != CUDA_SUCCESS) return -11;
   if (cache.size() > 8192) cache.clear();
-  cache.emplace(key, *out);
+  try {
+    cache.emplace(key, *out);
+  } catch (...) {  // no memory to remember it by: the caller is a C entry
+  }
   return 0;
 }
 

@@ -266,7 +266,10 @@ inline int tensor_map(const void* ptr, long rows, long cols, long ld, int box_ro
                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (rc != CUDA_SUCCESS) return -11;
   if (cache.size() > 8192) cache.clear();
-  cache.emplace(key, m);
+  try {
+    cache.emplace(key, m);
+  } catch (...) {  // no memory to remember it by: the caller is a C entry
+  }
   *out = m;
   return 0;
 }
