@@ -6,8 +6,9 @@
 // head_dim: a multiple of 16, at most 256.  tiles: [n_tiles][2] = (request, first query of the
 // tile within the request's portion); tiles_wide: the same for 64-query tiles, which the
 // tensor-core kernel takes (bfloat16, head_dim <= 128; other cases use `tiles`).
-// decode_reqs: requests with a single query; decode_wide: their blocks have sixteen warps
-// instead of four (few requests: a block then covers 256 keys a round).  With
+// decode_reqs: requests with a single query; decode_wide != 0: their blocks have sixteen warps
+// instead of four (few requests: a block then covers 256 keys a round), or (1, not 2) eight where
+// the device would take a second round over blocks of sixteen.  With
 // n_splits > 1, part_o holds n_decode*heads*n_splits*head_dim floats and part_ml
 // n_decode*heads*n_splits*2.  n_tokens: rows of q; n_pages: pages of the pool (both bound the
 // TMA tensor maps of the tcgen05 kernel).
@@ -37,7 +38,7 @@ RL_EXPORT int rl_attention(int dtype, const void* q, long q_stride, const void* 
                    out_stride, n_heads, n_kv_heads, head_dim, page_size, window, scale, status, old_keys_settled};
   int rc;
   if (dtype == RL_F32)
-    rc = rl::dispatch_attention<float>(p, tiles, n_tiles, decode_reqs, n_decode, n_splits, decode_wide != 0, part_o, part_ml, stream);
+    rc = rl::dispatch_attention<float>(p, tiles, n_tiles, decode_reqs, n_decode, n_splits, decode_wide, part_o, part_ml, stream);
   else {
     // prompt portions: tcgen05 where its sizes fit (prefill_path 0: as fits, 1: mma.sync, 2: tcgen05
     // or refuse), else mma.sync, else (head sizes above 128) the CUDA-core tiles below
@@ -49,7 +50,7 @@ RL_EXPORT int rl_attention(int dtype, const void* q, long q_stride, const void* 
       if (!done) done = rl::dispatch_mma_tiles(p, tiles_wide, n_tiles_wide, stream);
       if (done) n_tiles = 0;  // the prompt portions are done
     }
-    rc = rl::dispatch_attention<__nv_bfloat16>(p, tiles, n_tiles, decode_reqs, n_decode, n_splits, decode_wide != 0, part_o, part_ml, stream);
+    rc = rl::dispatch_attention<__nv_bfloat16>(p, tiles, n_tiles, decode_reqs, n_decode, n_splits, decode_wide, part_o, part_ml, stream);
   }
   if (rc != 0) return rc;
   RL_CHECK_LAUNCH();

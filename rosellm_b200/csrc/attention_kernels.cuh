@@ -541,18 +541,22 @@ template <typename T, int EPL, int WARPS, int STAGES, int DENSE = 0>
 static inline void launch_decode_form(const AttnParams& p, const int* decode_reqs, int n_decode, int n_splits,
                                       float* part_o, float* part_ml, cudaStream_t stream) {
   constexpr size_t smem = DecodeTile<EPL * (int)sizeof(T) / 4, WARPS, STAGES>::SMEM;
+  // Eight-warp blocks are taken for several an SM, and sixteen-warp blocks that need more than the common split gives stand
+  // between products that ask for all of it; smaller ones gain from the L1 (3 heads of 32, 16 requests of 1000 keys 5.9 us
+  // against 6.6 without it).
+  constexpr bool ALL_SHARED = WARPS == 8 || (WARPS == 16 && smem > RL_CARVEOUT_UP_TO);
   static bool attr_set = false;
   if (!attr_set) {
     if (smem > 47 * 1024)  // the kernel has a little static shared memory too
       cudaFuncSetAttribute(attn_decode_kernel<T, EPL, WARPS, STAGES, DENSE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)smem);
-    if (DENSE != 0 || WARPS > 4)  // wide blocks stand between products that ask for all of it
+    if (ALL_SHARED || DENSE != 0)
       cudaFuncSetAttribute(attn_decode_kernel<T, EPL, WARPS, STAGES, DENSE>,
                            cudaFuncAttributePreferredSharedMemoryCarveout,
                            DENSE == 1 ? 80 : (int)cudaSharedmemCarveoutMaxShared);
     attr_set = true;
   }
-  launch_pdl_split(DENSE == 0 && WARPS == 4, attn_decode_kernel<T, EPL, WARPS, STAGES, DENSE>, dim3(n_decode, p.n_heads, n_splits),
+  launch_pdl_split(DENSE == 0 && !ALL_SHARED, attn_decode_kernel<T, EPL, WARPS, STAGES, DENSE>, dim3(n_decode, p.n_heads, n_splits),
                    dim3(32 * WARPS), smem, stream, p, decode_reqs, n_splits, part_o, part_ml);
 }
 
@@ -590,17 +594,17 @@ static inline long wide_blocks_at_once() {
   return at_once;
 }
 
-// wide: sixteen warps a block instead of four; eight where the device would take more than one round over blocks of sixteen
-// (25 heads of 64, 8 requests of 512 keys: 200 blocks, one an SM with
-// sixteen warps and three with eight, 10.3 -> 8.6 us; of 896 keys 14.2 -> 13.4; 16 heads, 16 requests 10.9 -> 8.9).
+// wide: sixteen warps a block instead of four (0); 1: eight where the device would take more than one round over blocks of
+// sixteen (of bfloat16 heads of 64 an SM holds one block of sixteen and three of eight), 2: sixteen all the same.  Which is
+// ahead then depends on the keys a block walks, which only the caller knows.
 template <typename T, int EPL>
 static inline void launch_decode(const AttnParams& p, const int* decode_reqs, int n_decode, int n_splits,
-                                 bool wide, float* part_o, float* part_ml, cudaStream_t stream) {
+                                 int wide, float* part_o, float* part_ml, cudaStream_t stream) {
   const int dh = p.head_dim;
   if (wide) {
     // a ring of one tile where two would not fit an SM's shared memory (float32 rows of 256)
     constexpr int WIDE_STAGES = DecodeTile<EPL * (int)sizeof(T) / 4, 16, 2>::SMEM <= 200 * 1024 ? 2 : 1;
-    if ((long)n_decode * p.n_heads * n_splits > wide_blocks_at_once<DecodeTile<EPL * (int)sizeof(T) / 4, 16, WIDE_STAGES>::SMEM>())
+    if (wide == 1 && (long)n_decode * p.n_heads * n_splits > wide_blocks_at_once<DecodeTile<EPL * (int)sizeof(T) / 4, 16, WIDE_STAGES>::SMEM>())
       launch_decode_form<T, EPL, 8, 2>(p, decode_reqs, n_decode, n_splits, part_o, part_ml, stream);
     else
       launch_decode_form<T, EPL, 16, WIDE_STAGES>(p, decode_reqs, n_decode, n_splits, part_o, part_ml, stream);
@@ -619,7 +623,7 @@ static inline void launch_decode(const AttnParams& p, const int* decode_reqs, in
 
 template <typename T>
 static inline int dispatch_attention(const AttnParams& p, const int* tiles, int n_tiles,
-                                     const int* decode_reqs, int n_decode, int n_splits, bool decode_wide,
+                                     const int* decode_reqs, int n_decode, int n_splits, int decode_wide,
                                      float* part_o, float* part_ml, cudaStream_t stream) {
   if (p.head_dim % 16 != 0 || p.head_dim > 256) return -2;
   if (n_tiles > 0) {

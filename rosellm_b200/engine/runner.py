@@ -394,11 +394,14 @@ class ModelRunner:
         plans = self._graph_decode_plans(b)
         return max(plans.values()) if plans else None
 
+    def _graph_span(self) -> int:
+        """The context a captured step is laid out for: a request's is anywhere below the limit."""
+        return self.max_model_len // 2
+
     def _graph_decode_plans(self, b: int) -> dict:
         """The same per part (by ``id``): a model whose layers attend in different ways (over all keys, over a
         window, over latents) cuts each kind's keys as that kind wants them."""
-        span = self.max_model_len // 2  # a request's context is anywhere below the limit
-        return {id(part): part.decode_plan_for(b, span, self.dtype) for l in self.model.layers for part in l.parts.values()
+        return {id(part): part.decode_plan_for(b, self._graph_span(), self.dtype) for l in self.model.layers for part in l.parts.values()
                 if hasattr(part, "decode_plan_for")}
 
     def _stage_decode(self, hb: HostBatch, b: int) -> None:
@@ -445,6 +448,7 @@ class ModelRunner:
             ctx.workspace = ws
             ctx.extras["decode_plan"] = plan
             ctx.extras["decode_plans"] = plans
+            ctx.extras["decode_span"] = self._graph_span()
             if sample_into is not None:
                 ctx.extras["sample_into"] = sample_into
             return ctx

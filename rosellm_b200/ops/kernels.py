@@ -991,7 +991,8 @@ def kv_write(k, v, pool, block_table, positions, req_of_token, slots, max_pos: i
 def attention(q, pool, block_table, q_start, kv_len, slots, out, *, n_heads: int, scale: float,
               window: int | None, tiles, n_tiles: int, decode_reqs, n_decode: int,
               n_splits: int = 1, part_o=None, part_ml=None, tiles_wide=None, n_tiles_wide: int = 0,
-              decode_wide: bool = False, prefill_path: str | None = None, old_keys_settled: bool = False) -> None:
+              decode_wide: bool = False, prefill_path: str | None = None, old_keys_settled: bool = False,
+              decode_sixteen: bool = False) -> None:
     """Causal attention of the step's queries over the paged cache (see csrc/attention.cu).
 
     q [tokens, heads*head dim] (a view with a row stride), out the same shape; ``tiles``
@@ -999,7 +1000,8 @@ def attention(q, pool, block_table, q_start, kv_len, slots, out, *, n_heads: int
     ``decode_reqs`` int32 [n_decode] the requests with one query.  ``tiles_wide``: the
     portions again as 64-query tiles, used instead of ``tiles`` by the tensor-core kernel
     (bfloat16, head size up to 128).  ``decode_wide``: the blocks of decoded requests have
-    sixteen warps instead of four (few requests, so that their keys need no split).
+    sixteen warps instead of four (few requests, so that their keys need no split), or eight where
+    the device would take a second round over blocks of sixteen (``decode_sixteen``: sixteen all the same).
     ``prefill_path`` (for tests): ``"tc"`` or ``"mma"`` forces the kernel of the prompt portions.
     ``old_keys_settled``: the caller promises that the block table and the keys and values below
     each decoded request's last position were written by work that was over before the kernel
@@ -1028,7 +1030,7 @@ def attention(q, pool, block_table, q_start, kv_len, slots, out, *, n_heads: int
                              _ptr(q_start), _ptr(kv_len), _ptr(slots), _ptr(out), out.stride(0),
                              n_heads, n_kv, dh, page_size, int(window or 0), float(scale),
                              _ptr(tiles), n_tiles, _ptr(tiles_wide), n_tiles_wide if tiles_wide is not None else 0,
-                             _ptr(decode_reqs), n_decode, n_splits, int(decode_wide),
+                             _ptr(decode_reqs), n_decode, n_splits, (2 if decode_sixteen else 1) if decode_wide else 0,
                              _ptr(part_o), _ptr(part_ml), q.shape[0], pool.shape[0],
                              {None: 0, "mma": 1, "tc": 2}[prefill_path], int(old_keys_settled),
                              _ptr(status_word(q.device)), _stream())

@@ -371,10 +371,12 @@ def main(argv=None) -> int:
         splits, wide = _decode_plan(a, a.batch, h, dh) if decode else (1, False)
         po = torch.empty(max(1, a.batch * h * splits * dh), device=dev)
         pm = torch.empty(max(1, a.batch * h * splits * 2), device=dev)
+        from ..parts.standard import CausalSelfAttention
+        sixteen = CausalSelfAttention(h * dh, h, dh, hk).decode_sixteen_for(splits, a.context, dt)
         args = dict(n_heads=h, scale=dh ** -0.5, window=None, tiles=i32(hb.tiles.reshape(-1)), n_tiles=len(hb.tiles),
                     decode_reqs=i32(hb.decode_reqs), n_decode=len(hb.decode_reqs), n_splits=splits, part_o=po,
                     part_ml=pm, tiles_wide=i32(hb.tiles_wide.reshape(-1)), n_tiles_wide=len(hb.tiles_wide),
-                    decode_wide=wide, old_keys_settled=True)  # as inside the engine: the cache is of earlier steps
+                    decode_wide=wide, decode_sixteen=sixteen, old_keys_settled=True)  # as inside the engine: the cache is of earlier steps
         qs, kl, sl = i32(hb.q_start), i32(hb.kv_len), i32(hb.slots)
         us = _time(lambda i: K.attention(q, pools[i % len(pools)], table, qs, kl, sl, out, **args), a.reps, graph=not a.eager)
         kv_bytes = a.batch * a.context * 2 * hk * dh * el

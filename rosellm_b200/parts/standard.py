@@ -442,6 +442,28 @@ class CausalSelfAttention(Part):
     def decode_plan(self, ctx) -> tuple[int, bool]:
         return self.decode_plan_for(ctx.n_decode, ctx.max_kv_len, ctx.act_dtype)
 
+    # Keys up to which a wide block of eight warps is ahead of one of sixteen, by the bytes of a key and its value, where blocks of
+    # sixteen would take a second round: several blocks of eight stand on an SM, but each walks twice as long.  Measured
+    # on B200, us, sixteen / eight warps: 25 heads of 64 in bfloat16, 8 requests of 32 keys 6.2 / 3.1, of 512 10.5 / 8.7, of
+    # 1023 15.1 / 12.8; 16 heads on 4, 10 requests of 768 11.4 / 11.3, of 1023 13.8 / 14.6, of 4000 40 / 51.  8 heads
+    # of 128, 28 requests of 256 12.1 / 11.3, of 512 17.3 / 20.0, of 4000 84 / 132.  In 32 bits: 12 heads of 64, 18
+    # requests of 320 12.7 / 11.5, of 512 16.3 / 17.5; 8 heads of 128, 28 requests of 64 11.2 / 10.0, of 96 13.3 / 14.1, of 1023
+    # 65 / 113; 6 heads of 256, 36 requests of 448 109 / 107, of 1023 208 / 218.
+    EIGHT_WARPS_KEYS = {256: 960, 512: 320, 1024: 64, 2048: 400}
+
+    def decode_sixteen_for(self, splits: int, span: int, act_dtype: torch.dtype) -> bool:
+        """Whether wide blocks keep sixteen warps even where the device takes a second round over them."""
+        if self.window is not None:
+            span = min(span, self.window)
+        key_bytes = 2 * self.head_dim * (2 if act_dtype == torch.bfloat16 else 4)
+        limit = next((keys for size, keys in self.EIGHT_WARPS_KEYS.items() if key_bytes <= size), 0)
+        return -(-span // max(1, splits)) > limit
+
+    @staticmethod
+    def _decode_span(ctx) -> int:
+        """The context that a step's decode attention is laid out for (a captured step's serves every context)."""
+        return ctx.extras.get("decode_span") or ctx.max_kv_len
+
     @staticmethod
     def _tc_prompt_attention(ctx) -> bool:
         """Whether the step's prompt portions go to the tcgen05 kernel: decided by the longest
@@ -450,9 +472,10 @@ class CausalSelfAttention(Part):
         return ctx.max_tile_kv_len >= TC_ATTENTION_MIN_CONTEXT
 
     def launch_key(self, ctx) -> tuple:
-        """The longest context decides how decoded requests are split over blocks and which
-        kernel takes the prompt portions."""
-        return (ctx.extras.get("decode_plan") or self.decode_plan(ctx) if ctx.n_decode else None,
+        """The longest context decides how decoded requests are split over blocks, how many warps those have, and
+        which kernel takes the prompt portions."""
+        plan = ctx.extras.get("decode_plan") or self.decode_plan(ctx) if ctx.n_decode else None
+        return (plan, self.decode_sixteen_for(plan[0], self._decode_span(ctx), ctx.act_dtype) if plan else None,
                 self._tc_prompt_attention(ctx) if ctx.n_tiles else None)
 
     def bind(self, tensors) -> None:
@@ -513,7 +536,7 @@ class CausalSelfAttention(Part):
                     scale=self.scale, window=self.window, tiles=ctx.tiles, n_tiles=ctx.n_tiles,
                     decode_reqs=ctx.decode_reqs, n_decode=ctx.n_decode, n_splits=splits,
                     part_o=part_o, part_ml=part_ml, tiles_wide=ctx.tiles_wide, n_tiles_wide=ctx.n_tiles_wide,
-                    decode_wide=wide,
+                    decode_wide=wide, decode_sixteen=self.decode_sixteen_for(splits, self._decode_span(ctx), ctx.act_dtype),
                     # what decoded requests read of the cache beside their newest key is of earlier
                     # steps, and a step begins with a copy to the device that separates it from them
                     old_keys_settled=True,

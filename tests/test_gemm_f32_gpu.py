@@ -21,7 +21,7 @@ def _close(got, ref, k):
 
 
 # rows kernel: one row, eight, nine, 64; one chunk of K (128), a ragged one, more than the warps take at once (1024);
-# four and eight columns a block, ragged
+# groups of four columns, ragged
 @pytest.mark.parametrize("m", [1, 8, 9, 64])
 @pytest.mark.parametrize("n,k", [(1, 8), (5, 136), (769, 768), (2401, 1032), (768, 3072), (50257, 64)])
 def test_few_rows(m, n, k):

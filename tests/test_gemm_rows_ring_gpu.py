@@ -27,7 +27,8 @@ def _close(got, ref, k):
 
 
 # K: below a warp's 32, ragged, a stage exactly, one beyond it, two stages, more than a warp's fragments hold;
-# N: a pair, a ragged group, one group a block, several rounds of groups
+# N: a pair, a ragged group, one group a block, several rounds of groups (inner sizes that are no multiple of 64, and short
+# ones, run on the register-fed kernel: test_where_the_ring_begins)
 @pytest.mark.parametrize("m", [1, 8, 9, 16])
 @pytest.mark.parametrize("n,k", [(2, 8), (10, 40), (66, 1000), (1600, 1024), (4800, 1088), (6400, 1600), (72, 2048),
                                  (130, 2112), (2048, 8192), (16384, 256), (10, 64)])
@@ -74,9 +75,10 @@ def test_normalised_inside(m, k):
     K.check_status(torch.device(DEV))
 
 
-def test_weights_that_are_not_finite_stay_in_their_column():
+@pytest.mark.parametrize("k", [64, 320, 1088])  # register-fed; five blocks for eight warps; a second piece of one block
+def test_weights_that_are_not_finite_stay_in_their_column(k):
     """What a stage held before, and blocks of K that a warp does not have, never reach a sum."""
-    m, n, k = 8, 4000, 64
+    m, n = 8, 4000
     a, w, b = _data(m, n, k, 3)
     a = a.bfloat16()
     w[::2] = float("nan")
