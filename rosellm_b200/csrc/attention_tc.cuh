@@ -458,10 +458,11 @@ static inline int launch_attn_tc(const AttnParams& p, const int* tiles, int n_ti
     cudaFuncSetAttribute(attn_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ATT_SMEM);
     attr_set = true;
   }
-  // Pairs all walk about as many key tiles: a round of them is full to its end, and a second round, of which only a few blocks are left,
-  // costs as much as the first.  Where the pairs (about a quarter of the 64-query tiles, for every head) do not fit one round, the
-  // pieces go singly, and an SM takes the next as soon as it is free (25 heads, 2 prompts of 1024: 200 pairs on 148
-  // SMs, 41.5 -> 37.1 us; 4 of 512 29.5 -> 27.5).
+  // Pairs all walk about as many key tiles: a round of them is full to its end, and a last round of only a few blocks
+  // costs as much as the first.  Where the rounds that the pairs (about a quarter of the 64-query tiles, for every head) take
+  // would stand empty by a sixth or more, the pieces go singly, and an SM takes the next as soon as it is free (us, pairs / singly: 25
+  // heads, 2 prompts of 1024, 200 pairs on 148 SMs 41.9 / 37.8, 4 of 512 29.8 / 27.9; 20 heads, 2048 tokens 64.0 / 44.8;
+  // 40 heads, 2 of 1024 62.0 / 57.1).  Fuller rounds go in pairs: 32 heads, 256 pairs, 4 prompts of 512 32.3 / 34.0, 8 of 256 26.5 / 29.3.
   static int n_sms = 0;
   if (n_sms == 0) {
     int dev = 0;
@@ -469,7 +470,8 @@ static inline int launch_attn_tc(const AttnParams& p, const int* tiles, int n_ti
     cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, dev);
     if (n_sms <= 0) n_sms = 1;
   }
-  const bool singly = (long)(n_tiles + 3) / 4 * p.n_heads > n_sms && n_tiles <= 65535;  // (the limit of a grid's second extent)
+  const long pairs = (long)(n_tiles + 3) / 4 * p.n_heads, places = (pairs + n_sms - 1) / n_sms * n_sms;
+  const bool singly = pairs > n_sms && 5 * places > 6 * pairs && n_tiles <= 65535;  // (the limit of a grid's second extent)
   const dim3 grid = singly ? dim3(p.n_heads, n_tiles) : dim3(n_tiles, p.n_heads);
   launch_pdl_split(false, attn_tc_kernel, grid, ATT_THREADS, ATT_SMEM, stream, mq, mkv, p, tiles, singly ? 1 : 0);
   return 0;
