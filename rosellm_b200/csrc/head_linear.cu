@@ -11,6 +11,7 @@
 // An output gate may ride on the epilogue (fused): out[t, h, n] *= sigmoid(gate[t, h, n]) with float32 logits
 // reached by strides of their own (a column stride of 0: one logit a head), so a mixer that gates its merged heads needs
 // no kernel for it.
+#include "head_rows.cuh"
 #include "mma_tile.cuh"
 #include "tile_gemm.cuh"
 
@@ -83,6 +84,48 @@ __global__ __launch_bounds__(128) void head_linear_mma_kernel(const __nv_bfloat1
   });
 }
 
+// At most 16 rows of bfloat16 (a decode step of few requests): eight warps a block, each eight columns and KB blocks of 64
+// elements of K; `parts` warps share columns, their sums meeting in shared memory in a fixed order.  What bounds it is latency:
+// one round trip for the input's rows after the wait.  Eight rows, 16 heads, 512 to 128 columns: 10.3 us on 64 x 64
+// tiles (32 blocks, sixteen steps of K one after the other).
+constexpr int HR_WARPS = 8, HR_MAX_K = 4 * 64 * HR_WARPS;
+template <int KB>
+__global__ __launch_bounds__(32 * HR_WARPS) void head_rows_kernel(const __nv_bfloat16* __restrict__ in, long in_tok, long in_head,
+                                                                  const __nv_bfloat16* __restrict__ w, long w_head, long w_n,
+                                                                  __nv_bfloat16* __restrict__ out, long out_tok, long out_head,
+                                                                  int n_tokens, int n_total, int parts, const float* __restrict__ gate,
+                                                                  long gate_tok, long gate_head, long gate_n) {
+  __shared__ float part_s[HR_WARPS][32][4];
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, j = lane & 3;
+  const int h = blockIdx.y, per_block = HR_WARPS / parts;
+  const int part = warp / per_block, n0 = (blockIdx.x * per_block + warp % per_block) * 8, k0 = part * KB * 64;
+  HeadRowsWeights<KB> weights;
+  weights.load(w + (size_t)h * w_head + (size_t)min(n0 + g, n_total - 1) * w_n + k0);
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const __nv_bfloat16* in_h = in + (size_t)h * in_head + k0;
+  float c[4];
+  weights.multiply(in_h + (size_t)min(g, n_tokens - 1) * in_tok, in_h + (size_t)min(g + 8, n_tokens - 1) * in_tok, c);
+  if (parts > 1) {
+    *reinterpret_cast<float4*>(part_s[warp][lane]) = make_float4(c[0], c[1], c[2], c[3]);
+    __syncthreads();
+    if (part != 0) return;
+    for (int q = 1; q < parts; ++q) {
+      const float4 o = *reinterpret_cast<const float4*>(part_s[q * per_block + warp][lane]);
+      c[0] += o.x, c[1] += o.y, c[2] += o.z, c[3] += o.w;
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int t = g + (i >> 1) * 8, n = n0 + 2 * j + (i & 1);
+    if (t < n_tokens && n < n_total) {
+      float v = c[i];
+      if (gate != nullptr) v *= 1.0f / (1.0f + expf(-gate[(size_t)t * gate_tok + (size_t)h * gate_head + n * gate_n]));
+      out[(size_t)t * out_tok + (size_t)h * out_head + n] = __float2bfloat16_rn(v);
+    }
+  }
+}
+
 }  // namespace rl
 
 // in: element (t, h, k) at in + t*in_tok + h*in_head + k; w: element (h, k, n) at
@@ -103,6 +146,22 @@ RL_EXPORT int rl_head_linear(int dtype, const void* in, long in_tok, long in_hea
   else if (w_k == 1) {
     const bool vec = k_total % 8 == 0 && in_tok % 8 == 0 && in_head % 8 == 0 && w_head % 8 == 0 && w_n % 8 == 0 &&
                      ((uintptr_t)in % 16) == 0 && ((uintptr_t)w % 16) == 0;
+    const int kbs = k_total / 64;
+    if (vec && n_tokens <= 16 && k_total % 64 == 0 && k_total <= rl::HR_MAX_K) {
+      // two blocks of 64 a warp while eight warps reach that far, else four; a power of two of warps along K
+      int parts = 1;
+      while (parts < rl::HR_WARPS && parts * 2 < kbs) parts *= 2;
+      const int kb = kbs / parts;
+      if (kb * parts == kbs && (kb == 1 || kb == 2 || kb == 4)) {
+        const int columns = 8 * (rl::HR_WARPS / parts);
+        auto kernel = kb == 1 ? rl::head_rows_kernel<1> : kb == 2 ? rl::head_rows_kernel<2> : rl::head_rows_kernel<4>;
+        rl::launch_pdl(kernel, dim3((n_total + columns - 1) / columns, n_heads), 32 * rl::HR_WARPS, 0, stream, (const __nv_bfloat16*)in,
+                       in_tok, in_head, (const __nv_bfloat16*)w, w_head, w_n, (__nv_bfloat16*)out, out_tok, out_head, n_tokens, n_total,
+                       parts, gate, gate_tok, gate_head, gate_n);
+        RL_CHECK_LAUNCH();
+        return 0;
+      }
+    }
     auto kernel = vec ? rl::head_linear_mma_kernel<true> : rl::head_linear_mma_kernel<false>;
     rl::launch_pdl(kernel, grid, 128, 0, stream, (const __nv_bfloat16*)in, in_tok, in_head, (const __nv_bfloat16*)w,
                    w_head, w_n, (__nv_bfloat16*)out, out_tok, out_head, n_tokens, k_total, n_total, gate, gate_tok, gate_head, gate_n);

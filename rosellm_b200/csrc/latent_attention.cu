@@ -29,6 +29,7 @@
 
 #include "common.cuh"
 #include "gemm_vec.cuh"
+#include "head_rows.cuh"
 
 namespace rl {
 
@@ -104,6 +105,113 @@ __global__ __launch_bounds__(128) void latent_q_rope_kernel(
       v = to_f32(qr[j]);
     }
     rows[(size_t)n * rows_stride + (size_t)h * row_width + rank + j] = from_f32<T>(v);
+  }
+}
+
+// All that lies between a step's projections and its attention, for at most 16 rows of bfloat16 (a decode step of few
+// requests), in one launch: the queries' product with W_uk, their rotated part, and the new rows of the cache.  Grid (slices of
+// 64 latent entries and one more, heads): block (s, h) makes entries [64 s, 64 s + 64) of head h's query rows, the last one of a
+// head turns its rotated part and writes the cache rows of tokens h, h + heads, ...  As kernels of their own the three took
+// 4.6, 5.7 and 5.4 us a layer of 8 requests with 16 heads, latent 512, bound by round trips one after the other
+// (positions, slots, table, rows), which are now made before the wait for the kernels ahead, or side by side.
+struct LatentPrepare {
+  const __nv_bfloat16* q;  // query of token n, head h: q + n * q_stride + h * head_in: plain entries, then the rotated part
+  long q_stride;
+  int head_in;
+  const __nv_bfloat16* uk;  // [heads][rank][plain]
+  __nv_bfloat16* rows;      // row of token n, head h: rows + n * rows_stride + h * row_width
+  long rows_stride;
+  int row_width, rank, rot_dim, rot_dims;
+  const float* inv_freq;
+  float rot_mult;
+  const int* positions;
+  int n_tokens, n_heads;
+  // the cache rows (dkv null: none are written)
+  const float* dkv;
+  long ld;
+  const float* gamma;
+  float eps;
+  __nv_bfloat16* pool;
+  const int* block_table;
+  int bt_stride;
+  const int* req_of_token;
+  const int* slots;
+  int page_size, max_pos;
+  int* status;
+};
+
+template <int KB>
+__global__ __launch_bounds__(256) void latent_prepare_kernel(const LatentPrepare p) {
+  __shared__ float scratch[33];
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  constexpr int PLAIN = 64 * KB;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, h = blockIdx.y;
+  if (blockIdx.x + 1 < gridDim.x) {
+    const int g = lane >> 2, j = lane & 3, n0 = blockIdx.x * 64 + warp * 8;
+    HeadRowsWeights<KB> weights;
+    weights.load(p.uk + ((size_t)h * p.rank + min(n0 + g, p.rank - 1)) * PLAIN);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const __nv_bfloat16* q = p.q + (size_t)h * p.head_in;
+    float c[4];
+    weights.multiply(q + (size_t)min(g, p.n_tokens - 1) * p.q_stride, q + (size_t)min(g + 8, p.n_tokens - 1) * p.q_stride, c);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int t = g + (i >> 1) * 8, n = n0 + 2 * j + (i & 1);
+      if (t < p.n_tokens && n < p.rank) p.rows[(size_t)t * p.rows_stride + (size_t)h * p.row_width + n] = __float2bfloat16_rn(c[i]);
+    }
+    return;
+  }
+  const int tail = p.row_width - p.rank;
+  // the places of this block's first token in the cache: read before the wait, like the positions
+  auto place_of = [&](int n) -> long long {
+    const int slot = p.slots[p.req_of_token[n]], pos = p.positions[n];
+    if (slot < 0) return -1;  // padding of a fixed-size batch
+    if (pos < 0 || pos >= p.max_pos) {
+      if (tid == 0) atomicOr(p.status, RL_STATUS_BAD_POSITION);
+      return -1;
+    }
+    const int page = p.block_table[(size_t)slot * p.bt_stride + pos / p.page_size];
+    if (page < 0) {
+      if (tid == 0) atomicOr(p.status, RL_STATUS_BAD_PAGE);
+      return -1;
+    }
+    return ((long long)page * p.page_size + pos % p.page_size) * p.row_width;
+  };
+  long long place = p.dkv != nullptr && h < p.n_tokens ? place_of(h) : -1;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  for (int i = tid; i < p.n_tokens * tail; i += 256) {
+    const int n = i / tail, e = i - n * tail;
+    const __nv_bfloat16* qr = p.q + (size_t)n * p.q_stride + (size_t)h * p.head_in + PLAIN;
+    float v = 0.f;
+    if (e < p.rot_dims) {
+      const int pair = e >> 1;
+      v = rotate_element(to_f32(qr[2 * pair]), to_f32(qr[2 * pair + 1]), (float)p.positions[n] * p.inv_freq[pair], e & 1) * p.rot_mult;
+    } else if (e < p.rot_dim) {
+      v = to_f32(qr[e]);
+    }
+    p.rows[(size_t)n * p.rows_stride + (size_t)h * p.row_width + p.rank + e] = __float2bfloat16_rn(v);
+  }
+  if (p.dkv == nullptr) return;
+  for (int n = h; n < p.n_tokens; n += p.n_heads) {
+    if (n != h) place = place_of(n);
+    if (place < 0) continue;  // (the same for the whole block)
+    const float* src = p.dkv + (size_t)n * p.ld;
+    float s = 0.f;
+    for (int d = tid; d < p.rank; d += 256) s = fmaf(src[d], src[d], s);
+    const float r = 1.0f / sqrtf(block_sum(s, scratch) / (float)p.rank + p.eps);
+    __nv_bfloat16* dst = p.pool + place;
+    for (int d = tid; d < p.rank; d += 256) dst[d] = __float2bfloat16_rn(src[d] * r * p.gamma[d]);
+    const float* kr = src + p.rank;
+    for (int e = tid; e < tail; e += 256) {
+      float v = 0.f;
+      if (e < p.rot_dims) {
+        const int i = e >> 1;
+        v = rotate_element(kr[2 * i], kr[2 * i + 1], (float)p.positions[n] * p.inv_freq[i], e & 1) * p.rot_mult;
+      } else if (e < p.rot_dim) {
+        v = kr[e];
+      }
+      dst[p.rank + e] = __float2bfloat16_rn(v);
+    }
   }
 }
 
@@ -461,7 +569,8 @@ __global__ __launch_bounds__(128) void latent_attn_mma_kernel(LatentParams p, co
   using bf16 = __nv_bfloat16;
   constexpr int RB = 16 * (4 / DVS), LM_KT = 8 * NKT;
   extern __shared__ __align__(16) unsigned char latent_smem[];
-  pdl_begin();
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  // (the step's description and the block table are written by none of its kernels: read before the wait below)
   const int W = p.row_width, H = p.n_heads;
   const int Wk = (W + 15) & ~15, LD = Wk + 8, W8 = Wk >> 3;
   bf16* q_s = reinterpret_cast<bf16*>(latent_smem);  // [RB][LD]
@@ -487,6 +596,7 @@ __global__ __launch_bounds__(128) void latent_attn_mma_kernel(LatentParams p, co
   bf16* out = (bf16*)p.out;
   const int slot = p.slots[req];
   if (slot < 0) {  // padding of a fixed-size batch
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     if (sp == 0)
       for (int i = tid; i < min(RB, rows_total - row0) * p.rank; i += blockDim.x) {
         const int gr = row0 + i / p.rank;
@@ -503,14 +613,35 @@ __global__ __launch_bounds__(128) void latent_attn_mma_kernel(LatentParams p, co
     beg = sp * chunk;
     end = min(kv_len, beg + chunk);
   }
+  // Where a tile's keys lie: lane i of every warp looks up keys i and (tiles of 64) i + 32, a row of the pool each (-1: none).
+  // A row's pieces are then copied by the lanes of one warp: one dependent read of the table a tile, asked for a tile ahead
+  // (with a look-up a piece, a thread's eighteen copies waited for one another).
+  auto pool_rows = [&](int kt, int (&row)[(LM_KT + 31) / 32]) {
+#pragma unroll
+    for (int u = 0; u < (LM_KT + 31) / 32; ++u) {
+      const int key = kt + u * 32 + lane;
+      row[u] = -1;
+      if (key < end) {
+        const int page = bt[key / p.page_size];
+        if (page >= 0) row[u] = page * p.page_size + key % p.page_size;
+        else if (warp == 0) atomicOr(p.status, RL_STATUS_BAD_PAGE);
+      }
+    }
+  };
+  int next_rows[(LM_KT + 31) / 32];
+  pool_rows(beg, next_rows);
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   const bf16* q = (const bf16*)p.q;
-  for (int i = tid; i < RB * W8; i += 128) {
-    const int r = i / W8, c = (i - r * W8) * 8;
+  for (int r = warp; r < RB; r += 4) {
     const int gr = row0 + r;
-    uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    if (gr < rows_total && c < W)
-      v = *reinterpret_cast<const uint4*>(q + (size_t)(qs + t0 + gr / H) * p.q_stride + (size_t)(gr % H) * W + c);
-    *reinterpret_cast<uint4*>(q_s + r * LD + c) = v;
+    const bf16* src = q + (size_t)(qs + t0 + gr / H) * p.q_stride + (size_t)(gr % H) * W;
+    for (int c = lane * 8; c < Wk; c += 256) {
+      if (gr < rows_total && c < W)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(q_s + r * LD + c)), "l"(src + c)
+                     : "memory");
+      else
+        *reinterpret_cast<uint4*>(q_s + r * LD + c) = make_uint4(0u, 0u, 0u, 0u);
+    }
   }
   const int rg = warp / DVS, vh = warp % DVS;
   const int row_a = row0 + rg * 16 + g, row_b = row_a + 8;
@@ -527,27 +658,24 @@ __global__ __launch_bounds__(128) void latent_attn_mma_kernel(LatentParams p, co
   const uint32_t q_s_addr = (uint32_t)__cvta_generic_to_shared(q_s);
   const uint32_t k_s_addr = (uint32_t)__cvta_generic_to_shared(k_s);
 
-  // a tile of keys into stage `st`: valid 16-byte pieces by cp.async, the rest zeros
+  // the tile whose rows have been looked up into stage `st`: valid 16-byte pieces by cp.async, the rest zeros; then the
+  // rows of the tile after it are looked up
   auto stage_keys = [&](int kt, int st) {
     bf16* dst = k_s + st * LM_KT * LD;
-    for (int i = tid; i < LM_KT * W8; i += 128) {
-      const int j = i / W8, c = (i - j * W8) * 8;
-      const int key = kt + j;
-      int page = -1;
-      if (key < end && c < W) {
-        page = bt[key / p.page_size];
-        if (page < 0) atomicOr(p.status, RL_STATUS_BAD_PAGE);
-      }
-      if (page >= 0) {
-        const bf16* src = (const bf16*)p.pool + ((size_t)page * p.page_size + key % p.page_size) * W + c;
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + j * LD + c)),
-                     "l"(src)
-                     : "memory");
-      } else {
-        *reinterpret_cast<uint4*>(dst + j * LD + c) = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll 4
+    for (int j = warp; j < LM_KT; j += 4) {
+      const int row = __shfl_sync(0xffffffffu, next_rows[j >> 5], j & 31);
+      const bf16* src = (const bf16*)p.pool + (size_t)max(row, 0) * W;
+      for (int c = lane * 8; c < Wk; c += 256) {
+        if (row >= 0 && c < W)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + j * LD + c)), "l"(src + c)
+                       : "memory");
+        else
+          *reinterpret_cast<uint4*>(dst + j * LD + c) = make_uint4(0u, 0u, 0u, 0u);
       }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
+    pool_rows(kt + LM_KT, next_rows);
   };
   if (beg < end) stage_keys(beg, 0);
   int st = 0;
@@ -652,6 +780,7 @@ __global__ __launch_bounds__(128) void latent_attn_mma_kernel(LatentParams p, co
     }
     __syncthreads();  // the stage may be written again
   }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");  // a part without keys has not waited for its queries
 #pragma unroll
   for (int half = 0; half < 2; ++half) {
     const int gr = half ? row_b : row_a;
@@ -843,6 +972,30 @@ RL_EXPORT int rl_latent_kv_write(int dtype, const float* dkv, long ld, const flo
     rl::launch_pdl(rl::latent_kv_write_kernel<__nv_bfloat16>, n_tokens, 128, 0, stream, dkv, ld, gamma, eps, inv_freq,
                    rot_dims, (__nv_bfloat16*)pool, block_table, bt_stride, positions, req_of_token, slots, n_tokens,
                    rank, rot_dim, row_width, page_size, max_pos, rot_mult, status);
+  RL_CHECK_LAUNCH();
+  return 0;
+}
+
+// The product of at most 16 rows' queries with W_uk, their rotation and the new rows of the cache in one launch (bfloat16; see
+// LatentPrepare).  dkv null: no rows are written.  Returns -2 for sizes it does not take (the caller then makes the three calls).
+RL_EXPORT int rl_latent_prepare(const void* q, long q_stride, int head_in, int plain, const void* uk, void* rows, long rows_stride,
+                                int row_width, int rank, int rot_dim, int rot_dims, const float* inv_freq, float rot_mult,
+                                const int* positions, int n_tokens, int n_heads, const float* dkv, long ld, const float* gamma, float eps,
+                                void* pool, const int* block_table, int bt_stride, const int* req_of_token, const int* slots, int page_size,
+                                int max_pos, int* status, cudaStream_t stream) {
+  if (n_tokens <= 0) return 0;
+  if (n_tokens > 16 || n_heads <= 0 || n_heads > 65535 || plain % 64 != 0 || plain <= 0 || plain > 256 || plain == 192 || head_in % 8 != 0 ||
+      q_stride % 8 != 0 || (uintptr_t)q % 16 != 0 || (uintptr_t)uk % 16 != 0)
+    return -2;
+  if (rank <= 0 || rot_dim < 0 || rot_dims < 0 || rot_dims > rot_dim || (rot_dims & 1) || row_width < rank + rot_dim || plain + rot_dim > head_in ||
+      status == nullptr)
+    return -2;
+  using bf16 = __nv_bfloat16;
+  const rl::LatentPrepare p{(const bf16*)q, q_stride, head_in, (const bf16*)uk, (bf16*)rows, rows_stride, row_width, rank, rot_dim, rot_dims,
+                            inv_freq, rot_mult, positions, n_tokens, n_heads, dkv, ld, gamma, eps, (bf16*)pool, block_table, bt_stride,
+                            req_of_token, slots, page_size, max_pos, status};
+  auto kernel = plain == 64 ? rl::latent_prepare_kernel<1> : plain == 128 ? rl::latent_prepare_kernel<2> : rl::latent_prepare_kernel<4>;
+  rl::launch_pdl(kernel, dim3((rank + 63) / 64 + 1, n_heads), 256, 0, stream, p);
   RL_CHECK_LAUNCH();
   return 0;
 }

@@ -194,6 +194,8 @@ def _lib() -> ctypes.CDLL:
         lib.rl_latent_attention_fits.argtypes = [I, I, I]
         lib.rl_latent_decode_fits.argtypes = [I, I, I]
         lib.rl_latent_kv_write.argtypes = [I, P, L, P, F, P, I, P, P, I, P, P, P, I, I, I, I, I, I, F, P, P]
+        lib.rl_latent_prepare.argtypes = [P, L, I, I, P, P, L, I, I, I, I, P, F, P, I, I, P, L, P, F, P, P, I, P, P, I, I, P, P]
+        lib.rl_latent_prepare.restype = I
         lib.rl_latent_q_rope.argtypes = [I, P, L, I, I, P, L, I, I, I, I, P, P, I, I, F, P]
         lib.rl_latent_attention.argtypes = [I, P, L, P, P, I, P, P, P, P, L, P, I, I, I, I, F, P, I, P, I, I, I, P, P, I, P, P]
         lib.rl_head_linear.argtypes = [I, P, L, L, P, L, L, L, P, L, L, I, I, I, I, P, L, L, L, P]
@@ -1173,6 +1175,45 @@ def latent_kv_write(dkv, gamma, eps: float, inv_freq, rot_dims: int, pool, block
                                    _ptr(req_of_token), _ptr(slots), dkv.shape[0], rank, rot_dim, row_width, page_size,
                                    max_pos, float(rot_mult), _ptr(status_word(pool.device)), _stream())
     _ok(rc, "latent_kv_write")
+
+
+def latent_prepare_possible(rows: int, plain: int, head_in: int, dtype: torch.dtype) -> bool:
+    """Whether ``latent_prepare`` takes a step of so many rows."""
+    return rows <= 16 and dtype == torch.bfloat16 and plain in (64, 128, 256) and head_in % 8 == 0
+
+
+def latent_prepare(q, uk, rows, inv_freq, positions, *, n_heads: int, head_in: int, plain: int, rank: int, rot_dim: int, rot_dims: int,
+                   row_width: int, rot_mult: float = 1.0, dkv=None, gamma=None, eps: float = 0.0, pool=None, block_table=None,
+                   req_of_token=None, slots=None, max_pos: int = 0) -> None:
+    """In one launch, for at most 16 rows of bfloat16: ``rows[t, h, :rank] = q_plain W_uk,h^T`` (``uk`` [heads, rank, plain],
+    weights: read before the kernels ahead have ended), ``latent_q_rope``, and (``dkv`` given) ``latent_kv_write``."""
+    _need(q, "q", torch.bfloat16, contiguous=False)
+    _need(rows, "rows", torch.bfloat16, contiguous=False)
+    _need(uk, "uk", torch.bfloat16)
+    n = q.shape[0]
+    if q.shape[1] != n_heads * head_in or rows.shape[1] != n_heads * row_width or q.stride(1) != 1 or rows.stride(1) != 1 \
+            or rows.shape[0] != n or uk.numel() != n_heads * rank * plain:
+        raise KernelError("latent_prepare: widths do not fit the heads")
+    if rot_dims:
+        _need(inv_freq, "inv_freq", torch.float32)
+        if inv_freq.numel() < rot_dims // 2:
+            raise KernelError("latent_prepare: a frequency for every rotated pair")
+    kx = (None, 0, None, 0.0, None, None, 0, None, None, 1, 0)
+    if dkv is not None:
+        _need(dkv, "dkv", torch.float32, contiguous=False)
+        _need(gamma, "gamma", torch.float32)
+        _need(pool, "pool", torch.bfloat16)
+        _need(block_table, "block_table", torch.int32)
+        _, planes, heads, page_size, width = pool.shape
+        if planes != 1 or heads != 1 or width != row_width or dkv.shape[1] < rank + rot_dim or dkv.stride(1) != 1 \
+                or gamma.numel() != rank or dkv.shape[0] != n:
+            raise KernelError("latent_prepare: the pool holds one row a token; dkv holds the latent and the rotated part")
+        kx = (_ptr(dkv), dkv.stride(0), _ptr(gamma), float(eps), _ptr(pool), _ptr(block_table), block_table.stride(0),
+              _ptr(req_of_token), _ptr(slots), page_size, max_pos)
+    rc = _lib().rl_latent_prepare(_ptr(q), q.stride(0), head_in, plain, _ptr(uk), _ptr(rows), rows.stride(0), row_width, rank, rot_dim,
+                                  rot_dims, _ptr(inv_freq), float(rot_mult), _ptr(positions), n, n_heads, *kx,
+                                  _ptr(status_word(q.device)), _stream())
+    _ok(rc, "latent_prepare")
 
 
 def latent_q_rope(q, rows, inv_freq, positions, *, n_heads: int, head_in: int, plain: int, rank: int, rot_dim: int,

@@ -159,19 +159,15 @@ class LatentAttention(Part):
                 cq_buf = ws.get("latent_cq", (n, self.q_rank_padded), act)
             K.rmsnorm(proj[:, off["dq"]:off["dq"] + self.q_rank], self.dq_norm, self.norm_eps, cq_buf[:, :self.q_rank])
             K.linear(cq_buf, self.q_weight, None, q)
-        if run.writes_cache:
-            dkv = proj[:, off["dkv"]:off["dkv"] + rank + self.rot_dim]
-            K.latent_kv_write(dkv, self.dkv_norm, self.norm_eps, freq, self.rotary.dims, pool, table, ctx.positions,
-                              ctx.req_of_token, ctx.slots, rank=rank, rot_dim=self.rot_dim,
-                              max_pos=ctx.cache.max_seq_len, rot_mult=self.rotary.mult)
-        # the query rows [q_plain W_uk | rotated part] of every head
+        dkv = proj[:, off["dkv"]:off["dkv"] + rank + self.rot_dim] if run.writes_cache else None
         rows = ws.get("latent_q_rows", (n, H * W), act)
-        K.head_linear(q, self.uk_weight, rows, n_tokens=n, n_heads=H, k=self.plain_dim, n=rank,
-                      in_strides=(q.stride(0), self.head_in), w_strides=(self.plain_dim * rank, 1, self.plain_dim),
-                      out_strides=(H * W, W))
-        K.latent_q_rope(q, rows, freq, ctx.positions, n_heads=H, head_in=self.head_in, plain=self.plain_dim,
-                        rank=rank, rot_dim=self.rot_dim, rot_dims=self.rotary.dims, row_width=W,
-                        rot_mult=self.rotary.mult)
+        if K.latent_prepare_possible(n, self.plain_dim, self.head_in, act):  # the rest up to the attention in one launch
+            K.latent_prepare(q, self.uk_weight, rows, freq, ctx.positions, n_heads=H, head_in=self.head_in, plain=self.plain_dim,
+                             rank=rank, rot_dim=self.rot_dim, rot_dims=self.rotary.dims, row_width=W, rot_mult=self.rotary.mult,
+                             dkv=dkv, gamma=self.dkv_norm, eps=self.norm_eps, pool=pool, block_table=table,
+                             req_of_token=ctx.req_of_token, slots=ctx.slots, max_pos=ctx.cache.max_seq_len)
+        else:
+            self._prepare(ctx, q, dkv, rows, freq, pool, table)
         o_lat = ws.get("latent_o", (n, H * rank), act)
         by_request = ctx.n_decode > 0 and K.latent_decode_fits(H, rank, W)
         splits = step_decode_plan(self, ctx)[0] if by_request else 1
@@ -197,6 +193,20 @@ class LatentAttention(Part):
                       in_strides=(H * rank, rank), w_strides=(self.value_dim * rank, 1, rank),
                       out_strides=(self.heads_padded, self.value_dim), gate=gate, gate_strides=gate_strides)
         K.linear(o, self.o_weight, None, x, residual=add)
+
+    def _prepare(self, ctx, q, dkv, rows, freq, pool, table) -> None:
+        """The new rows of the cache and the query rows ``[q_plain W_uk | rotated part]`` of every head, a kernel each."""
+        n, H, W, rank = ctx.n_tokens, self.num_heads, self.row_width, self.kv_rank
+        if dkv is not None:
+            K.latent_kv_write(dkv, self.dkv_norm, self.norm_eps, freq, self.rotary.dims, pool, table, ctx.positions,
+                              ctx.req_of_token, ctx.slots, rank=rank, rot_dim=self.rot_dim,
+                              max_pos=ctx.cache.max_seq_len, rot_mult=self.rotary.mult)
+        K.head_linear(q, self.uk_weight, rows, n_tokens=n, n_heads=H, k=self.plain_dim, n=rank,
+                      in_strides=(q.stride(0), self.head_in), w_strides=(self.plain_dim * rank, 1, self.plain_dim),
+                      out_strides=(H * W, W))
+        K.latent_q_rope(q, rows, freq, ctx.positions, n_heads=H, head_in=self.head_in, plain=self.plain_dim,
+                        rank=rank, rot_dim=self.rot_dim, rot_dims=self.rotary.dims, row_width=W,
+                        rot_mult=self.rotary.mult)
 
 
 def K_fits(n_heads: int, rank: int, row_width: int) -> bool:
