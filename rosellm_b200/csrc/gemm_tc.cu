@@ -34,8 +34,13 @@
 // The accumulator is double-buffered in tensor memory, so the epilogue of tile i runs under the
 // MMAs of tile i+1.  Every wait on a barrier is bounded: after about two seconds the kernel sets
 // a status bit, raises a block-wide abort flag and leaves, freeing its tensor memory on the way
-// out.  No multicast and no clusters are used.  (A one-tile-per-block form with K split over
+// out.  No load is multicast.  (A one-tile-per-block form with K split over
 // blocks was tried for outputs of few tiles and measured about half as fast.)
+//
+// The issuing warps walk their loops whole, with values that are the same in all lanes, and elect a lane for the issue itself: a
+// copy's and a product's operands are taken from uniform registers, and with one lane in a branch of its own each had to
+// be moved there first.  A K block of 64 at 64 columns 0.29 -> 0.19 us: 768 x 768 at 2048 rows 8.0 -> 6.9 us, 3072 x 768 13.9 -> 12.4,
+// 2304 x 768 at 512 rows 7.3 -> 6.4, += 1600 x 6400 64 columns wide 32.4 -> 24.2.
 #include "gemm_epilogue.cuh"
 #include "sampling_key.cuh"
 #include "tc_common.cuh"
@@ -86,19 +91,29 @@ struct PArgs {
   SampleArgs sample;  // EPI_SAMPLE only
 };
 
-__host__ __device__ inline int stage_bytes(int bn) { return A_BYTES + bn * BK * 2; }
+// How blocks share a tile: each has its own; the blocks of a cluster take the parts of K of one tile (one unit a block, no
+// walk) and add them up through distributed shared memory; the two blocks of a cluster (a pair of SMs) walk tiles of 256 rows.
+constexpr int FORM_SINGLE = 0, FORM_PARTS = 1, FORM_PAIR = 2;
 
-// Shared memory: stages | staging | barriers.  CLUSTER: the blocks of a cluster take the parts of
-// K of one tile (one unit a block, no walk) and add them up through distributed shared memory.
-template <typename TOut, int EPI, bool CLUSTER>
+__host__ __device__ inline int stage_bytes(int bn, bool pair) { return A_BYTES + (pair ? bn / 2 : bn) * BK * 2; }
+
+// Shared memory: stages | staging | barriers.
+//
+// FORM_PAIR (cta_group::2): each block brings its own 128 rows of A and half of the tile's rows of W, the first block's lane
+// issues products of 256 rows that read both blocks' shared memory, and each block's tensor memory gets its own 128 rows of
+// the result.  A K block of a 256-column tile then costs an SM 32 KB of operands instead of 48.  The copies of both blocks
+// count on the first one's "full" barriers; a product's end arrives at both blocks' "empty" and accumulator barriers.
+template <typename TOut, int EPI, int FORM>
 __global__ __launch_bounds__(PTHREADS, 1) void gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a,
                                                                       const __grid_constant__ CUtensorMap map_w,
                                                                       const __grid_constant__ CUtensorMap map_out,
                                                                       const PArgs p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  constexpr bool CLUSTER = FORM == FORM_PARTS, PAIR = FORM == FORM_PAIR;
+  constexpr int TM = PAIR ? 2 * BM : BM;  // rows of a tile
   const int BN = p.bn, PSTAGES = p.stages;
-  const int STAGE = stage_bytes(BN);
+  const int STAGE = stage_bytes(BN, PAIR);
   const uint32_t smem_base = smem_u32(smem);
   const int staging_offset = PSTAGES * STAGE;
   const int bar_offset = staging_offset + staging_bytes<TOut, EPI>();
@@ -110,10 +125,15 @@ __global__ __launch_bounds__(PTHREADS, 1) void gemm_tc_persistent_kernel(const _
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + bar_offset + (2 * MAX_STAGES + 4) * 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // the warp's number as a value that the compiler knows to be the same in all lanes
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int M = p.M, N = p.N;
-  const int m_tiles = (M + BM - 1) / BM, n_tiles = (N + BN - 1) / BN;
+  const int m_tiles = (M + TM - 1) / TM, n_tiles = (N + BN - 1) / BN;
   const int splits = p.splits;
+  const int half = PAIR ? (int)cluster_rank() : 0;  // which of the pair's blocks this is: of the tile's rows, and of its rows of W
+  const int first_unit = PAIR ? (int)blockIdx.x >> 1 : (int)blockIdx.x, unit_step = PAIR ? (int)gridDim.x >> 1 : (int)gridDim.x;
+  // the barrier that the operands of stage s are counted on: the first block's
+  auto operands_bar = [&](int s) { return PAIR ? peer_addr(full_bar(s), 0) : full_bar(s); };
   const int total_units = m_tiles * n_tiles * splits;  // a unit: a tile and a part of K
   const int num_kb = (p.K + BK - 1) / BK;
   const uint32_t acc_stride = (uint32_t)p.tmem_cols / 2;
@@ -127,7 +147,7 @@ __global__ __launch_bounds__(PTHREADS, 1) void gemm_tc_persistent_kernel(const _
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(acc_full(b), 1);
-      mbar_init(acc_empty(b), PEPI_WARPS);  // one arrival per epilogue warp
+      mbar_init(acc_empty(b), PAIR ? 2 * PEPI_WARPS : PEPI_WARPS);  // one arrival per epilogue warp
     }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -137,64 +157,81 @@ __global__ __launch_bounds__(PTHREADS, 1) void gemm_tc_persistent_kernel(const _
     if (EPI == EPI_TMA) tma_prefetch_map(&map_out);
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"((uint32_t)p.tmem_cols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    if constexpr (PAIR) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                   "r"((uint32_t)p.tmem_cols)
+                   : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                   "r"((uint32_t)p.tmem_cols)
+                   : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  if constexpr (PAIR) {
+    __syncwarp();
+    cluster_sync();  // the first block's barriers are there before the other one's copies count on them
+  }
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   RL_PHASE(1);
 
   if (warp == 0) {
-    if (lane == 0) {
-      // before the wait for the kernels ahead: the W tiles of the first stages of the first tile
-      int ahead = 0;
-      if ((int)blockIdx.x < total_units) {
-        const int tile = (int)blockIdx.x / splits, kb0 = ((int)blockIdx.x - tile * splits) * p.kb_per;
-        const int n0 = (tile / m_tiles) * BN;
-        const int kbs = min(num_kb - kb0, p.kb_per);
-        ahead = kbs < PSTAGES ? kbs : PSTAGES;
-        for (int s = 0; s < ahead; ++s) {
-          mbar_expect_tx(full_bar(s), (uint32_t)STAGE);
-          tma_load_2d(smem_base + s * STAGE + A_BYTES, &map_w, full_bar(s), (kb0 + s) * BK, n0);
+    // before the wait for the kernels ahead: the W tiles of the first stages of the first tile
+    int ahead = 0;
+    if (first_unit < total_units) {
+      const int tile = first_unit / splits, kb0 = (first_unit - tile * splits) * p.kb_per;
+      const int n0 = (tile / m_tiles) * BN + half * (BN / 2);
+      const int kbs = min(num_kb - kb0, p.kb_per);
+      ahead = kbs < PSTAGES ? kbs : PSTAGES;
+      for (int s = 0; s < ahead; ++s)
+        if (elect_one()) {
+          if (half == 0) mbar_expect_tx(full_bar(s), (uint32_t)(PAIR ? 2 * STAGE : STAGE));
+          tma_load<PAIR>(smem_base + s * STAGE + A_BYTES, &map_w, operands_bar(s), (kb0 + s) * BK, n0);
         }
-      }
-      asm volatile("griddepcontrol.wait;" ::: "memory");
-      RL_PHASE(2);
-      // K blocks issued so far, over all tiles, and where the next one goes: ring position, its
-      // phase and its address are stepped along, never divided out (the lane's own instructions
-      // are what the copies wait for)
-      uint32_t it = 0, s = 0, ph = 0, a_dst = smem_base;
-      bool ok = true;
-      for (int unit = blockIdx.x; unit < total_units && ok; unit += gridDim.x) {
-        const int tile = unit / splits, kb0 = (unit - tile * splits) * p.kb_per;
-        const int kb1 = min(num_kb, kb0 + p.kb_per);
-        const int m0 = (tile % m_tiles) * BM, n0 = (tile / m_tiles) * BN;
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
-          if (it >= (uint32_t)ahead) {
-            ok = mbar_wait(empty_bar(s), ph ^ 1u, abort_flag, p.status);
-            if (!ok) break;
-            mbar_expect_tx(full_bar(s), (uint32_t)STAGE);
-            tma_load_2d(a_dst + A_BYTES, &map_w, full_bar(s), kb * BK, n0);
-          }
-          if (it == 0) RL_PHASE(3);
-          if (it + 1 == (uint32_t)num_kb) RL_PHASE(4);
-          if (++s == (uint32_t)PSTAGES) {
-            s = 0;
-            ph ^= 1u;
-            a_dst = smem_base;
-          } else {
-            a_dst += STAGE;
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    RL_PHASE(2);
+    // K blocks issued so far, over all tiles, and where the next one goes: ring position, its
+    // phase and its address are stepped along, never divided out (the warp's own instructions
+    // are what the copies wait for)
+    uint32_t it = 0, s = 0, ph = 0, a_dst = smem_base;
+    bool ok = true;
+    for (int unit = first_unit; unit < total_units && ok; unit += unit_step) {
+      const int tile = unit / splits, kb0 = (unit - tile * splits) * p.kb_per;
+      const int kb1 = min(num_kb, kb0 + p.kb_per);
+      const int n0 = (tile / m_tiles) * BN + half * (BN / 2);
+      for (int kb = kb0; kb < kb1; ++kb, ++it) {
+        if (it >= (uint32_t)ahead) {
+          ok = mbar_wait_warp(empty_bar(s), ph ^ 1u, abort_flag, p.status);
+          if (!ok) break;
+          if (elect_one()) {
+            if (half == 0) mbar_expect_tx(full_bar(s), (uint32_t)(PAIR ? 2 * STAGE : STAGE));
+            tma_load<PAIR>(a_dst + A_BYTES, &map_w, operands_bar(s), kb * BK, n0);
           }
         }
+        if (it == 0) RL_PHASE(3);
+        if (it + 1 == (uint32_t)num_kb) RL_PHASE(4);
+        if (++s == (uint32_t)PSTAGES) {
+          s = 0;
+          ph ^= 1u;
+          a_dst = smem_base;
+        } else {
+          a_dst += STAGE;
+        }
       }
-      if (*abort_flag) {
-        for (uint32_t k = it > (uint32_t)PSTAGES ? it - PSTAGES : 0; k < it; ++k)
-          mbar_wait_quiet(full_bar(k % PSTAGES), (k / PSTAGES) & 1u);
-      }
+    }
+    if constexpr (PAIR) {
+      // the products that read the last stages have arrived at this block's barriers before it may end
+      for (uint32_t k = it > (uint32_t)PSTAGES ? it - PSTAGES : 0; k < it && ok; ++k)
+        ok = mbar_wait_warp(empty_bar(k % PSTAGES), (k / PSTAGES) & 1u, abort_flag, p.status);
+    }
+    if (*abort_flag && half == 0) {
+      for (uint32_t k = it > (uint32_t)PSTAGES ? it - PSTAGES : 0; k < it; ++k)
+        mbar_wait_quiet(full_bar(k % PSTAGES), (k / PSTAGES) & 1u);
     }
     if constexpr (CLUSTER) {  // the cluster's two barriers are reached by every thread on every path
       __syncwarp();
@@ -202,36 +239,34 @@ __global__ __launch_bounds__(PTHREADS, 1) void gemm_tc_persistent_kernel(const _
       cluster_sync();
     }
   } else if (warp == A_WARP) {
-    // The tiles of A, by a lane of their own: issuing a stage's two copies, with the wait and the
+    // The tiles of A, by a warp of their own: issuing a stage's two copies, with the wait and the
     // announcement before them, took one lane longer than the tensor pipe needs for the stage.
-    // Both lanes wait for the same empty slot and their copies count on the same barrier, whose
-    // expected bytes (the whole stage) the other lane announces; bytes that land before the
+    // Both warps wait for the same empty slot and their copies count on the same barrier, whose
+    // expected bytes (the whole stage) the other one announces; bytes that land before the
     // announcement are counted all the same.
-    if (lane == 0) {
-      asm volatile("griddepcontrol.wait;" ::: "memory");  // A is what the kernel ahead wrote
-      uint32_t it = 0, s = 0, ph = 0, a_dst = smem_base;
-      bool ok = true;
-      for (int unit = blockIdx.x; unit < total_units && ok; unit += gridDim.x) {
-        const int tile = unit / splits, kb0 = (unit - tile * splits) * p.kb_per;
-        const int kb1 = min(num_kb, kb0 + p.kb_per);
-        const int m0 = (tile % m_tiles) * BM;
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
-          ok = mbar_wait(empty_bar(s), ph ^ 1u, abort_flag, p.status);  // a slot's first use: passes at once
-          if (!ok) break;
-          tma_load_2d(a_dst, &map_a, full_bar(s), kb * BK, m0);
-          if (++s == (uint32_t)PSTAGES) {
-            s = 0;
-            ph ^= 1u;
-            a_dst = smem_base;
-          } else {
-            a_dst += STAGE;
-          }
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // A is what the kernel ahead wrote
+    uint32_t it = 0, s = 0, ph = 0, a_dst = smem_base;
+    bool ok = true;
+    for (int unit = first_unit; unit < total_units && ok; unit += unit_step) {
+      const int tile = unit / splits, kb0 = (unit - tile * splits) * p.kb_per;
+      const int kb1 = min(num_kb, kb0 + p.kb_per);
+      const int m0 = (tile % m_tiles) * TM + half * BM;
+      for (int kb = kb0; kb < kb1; ++kb, ++it) {
+        ok = mbar_wait_warp(empty_bar(s), ph ^ 1u, abort_flag, p.status);  // a slot's first use: passes at once
+        if (!ok) break;
+        if (elect_one()) tma_load<PAIR>(a_dst, &map_a, operands_bar(s), kb * BK, m0);
+        if (++s == (uint32_t)PSTAGES) {
+          s = 0;
+          ph ^= 1u;
+          a_dst = smem_base;
+        } else {
+          a_dst += STAGE;
         }
       }
-      if (*abort_flag) {
-        for (uint32_t k = it > (uint32_t)PSTAGES ? it - PSTAGES : 0; k < it; ++k)
-          mbar_wait_quiet(full_bar(k % PSTAGES), (k / PSTAGES) & 1u);
-      }
+    }
+    if (*abort_flag && half == 0) {
+      for (uint32_t k = it > (uint32_t)PSTAGES ? it - PSTAGES : 0; k < it; ++k)
+        mbar_wait_quiet(full_bar(k % PSTAGES), (k / PSTAGES) & 1u);
     }
     if constexpr (CLUSTER) {
       __syncwarp();
@@ -239,38 +274,43 @@ __global__ __launch_bounds__(PTHREADS, 1) void gemm_tc_persistent_kernel(const _
       cluster_sync();
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (half == 0) {
       // The tensor pipe takes a 128 x 256 x 16 product every 129 clocks, and a narrower one
-      // sooner: the lane must not need longer than that to issue the next.  So ring position,
+      // sooner: issuing the next must not take longer than that.  So the whole warp walks the loop,
+      // with values that are the same in all lanes (a product's operands are taken from uniform registers; with one lane in
+      // a branch of its own every one of them had to be moved there), and only the issue itself is one lane's; ring position,
       // phase and the operands' descriptors are stepped along (a descriptor's address field
       // counts 16-byte units: the next K step of 32 bytes is +2, the next stage +STAGE/16), and
       // nothing is divided or built from scratch between two products.
-      const uint32_t idesc = instr_desc(BN);
+      const uint32_t idesc = instr_desc(BN, TM);
       const uint64_t desc_first = smem_desc(smem_base);
       constexpr uint32_t STEP16 = 32 >> 4;
       const uint32_t stage16 = (uint32_t)STAGE >> 4, b16 = (uint32_t)A_BYTES >> 4;
       uint32_t it = 0, local = 0, s = 0, ph = 0;
       uint64_t a_desc = desc_first;
       bool ok = true;
-      for (int unit = blockIdx.x; unit < total_units && ok; unit += gridDim.x, ++local) {
+      for (int unit = first_unit; unit < total_units && ok; unit += unit_step, ++local) {
         const int buf = local & 1;
         const int kb0 = (unit % splits) * p.kb_per, kb1 = min(num_kb, kb0 + p.kb_per);
-        ok = mbar_wait(acc_empty(buf), ((local >> 1) & 1u) ^ 1u, abort_flag, p.status);
+        ok = mbar_wait_warp(acc_empty(buf), ((local >> 1) & 1u) ^ 1u, abort_flag, p.status);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t d_addr = tmem_base + (uint32_t)buf * acc_stride;
         for (int kb = kb0; kb < kb1; ++kb, ++it) {
-          ok = mbar_wait(full_bar(s), ph, abort_flag, p.status);
+          ok = mbar_wait_warp(full_bar(s), ph, abort_flag, p.status);
           if (!ok) break;
           if (it < 16) RL_PHASE_OF(10 + it, 32);
           // (no tcgen05 fence here: the copies that completed this barrier and the products that
           // read what they brought both go through the async proxy; the fence after the wait for
           // the accumulator orders the products against the epilogue's reads of tensor memory)
           const uint64_t b_desc = a_desc + b16;
-          mma_f16(d_addr, a_desc, b_desc, idesc, kb > kb0 ? 1u : 0u);
+          if (elect_one()) {
+            mma<PAIR>(d_addr, a_desc, b_desc, idesc, kb > kb0 ? 1u : 0u);
 #pragma unroll
-          for (int k = 1; k < BK / 16; ++k) mma_f16(d_addr, a_desc + k * STEP16, b_desc + k * STEP16, idesc, 1u);
-          mma_commit(empty_bar(s));
+            for (int k = 1; k < BK / 16; ++k) mma<PAIR>(d_addr, a_desc + k * STEP16, b_desc + k * STEP16, idesc, 1u);
+            commit<PAIR>(empty_bar(s));
+          }
+          __syncwarp();
           if (++s == (uint32_t)PSTAGES) {
             s = 0;
             ph ^= 1u;
@@ -279,7 +319,8 @@ __global__ __launch_bounds__(PTHREADS, 1) void gemm_tc_persistent_kernel(const _
             a_desc += stage16;
           }
         }
-        if (ok) mma_commit(acc_full(buf));
+        if (ok && elect_one()) commit<PAIR>(acc_full(buf));
+        __syncwarp();
         if (local == 0) RL_PHASE_OF(5, 32);
       }
     }
@@ -302,7 +343,7 @@ __global__ __launch_bounds__(PTHREADS, 1) void gemm_tc_persistent_kernel(const _
       // offers it once the tile is through.  Nothing is staged and nothing written but the offers.
       const SampleArgs& sm = p.sample;
       bool offered = false;
-      for (int unit = blockIdx.x; unit < total_units && ok; unit += gridDim.x, ++local) {
+      for (int unit = first_unit; unit < total_units && ok; unit += unit_step, ++local) {
         const int m0 = (unit % m_tiles) * BM, n0 = (unit / m_tiles) * BN;
         const int row = m0 + quarter * 32 + lane;
         const int buf = local & 1;
@@ -384,7 +425,7 @@ __global__ __launch_bounds__(PTHREADS, 1) void gemm_tc_persistent_kernel(const _
       long long row_base = -1;
       bool tile_to_cache = false;
       auto begin_tile = [&](int tile) {
-        m0 = (tile % m_tiles) * BM;
+        m0 = (tile % m_tiles) * TM + half * BM;
         n0 = (tile / m_tiles) * BN;
         row0 = m0 + quarter * 32;
         row = row0 + lane;
@@ -542,7 +583,7 @@ __global__ __launch_bounds__(PTHREADS, 1) void gemm_tc_persistent_kernel(const _
         }
         RL_PHASE_OF(7, 64);
       } else {
-        for (int unit = blockIdx.x; unit < total_units && ok; unit += gridDim.x, ++local) {
+        for (int unit = first_unit; unit < total_units && ok; unit += unit_step, ++local) {
           begin_tile(unit);  // no parts of K here: a unit is a tile
           const int buf = local & 1;
           // the bias of this warp's (at most two) pieces, lane i that of column i: asked for
@@ -572,7 +613,13 @@ __global__ __launch_bounds__(PTHREADS, 1) void gemm_tc_persistent_kernel(const _
           // the buffer may be overwritten by the MMAs of the tile after next
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
           __syncwarp();
-          if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(acc_empty(buf)) : "memory");
+          if (lane == 0) {
+            if constexpr (PAIR)  // the first block's lane issues the products of both
+              asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(peer_addr(acc_empty(buf), 0))
+                           : "memory");
+            else
+              asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(acc_empty(buf)) : "memory");
+          }
           if (local == 0) RL_PHASE_OF(7, 64);
         }
       }
@@ -659,11 +706,23 @@ __global__ __launch_bounds__(PTHREADS, 1) void gemm_tc_persistent_kernel(const _
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  if constexpr (PAIR) {
+    // a block that gave up lets the other one know, whose waits look at the flag; neither ends, nor frees its tensor memory,
+    // while the other may still read its operands or arrive at its barriers
+    if (*abort_flag)
+      asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(peer_addr(smem_u32(tmem_slot + 1), (uint32_t)(half ^ 1))), "r"(1) : "memory");
+    __syncwarp();
+    cluster_sync();
+  }
   __syncthreads();
   RL_PHASE(8);
   if (warp == 1) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)p.tmem_cols)
-                 : "memory");
+    if constexpr (PAIR)
+      asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)p.tmem_cols)
+                   : "memory");
+    else
+      asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)p.tmem_cols)
+                   : "memory");
   }
 }
 
@@ -678,20 +737,24 @@ static int sm_count() {
   return n_sms;
 }
 
-// How a product is cut: the width of a tile and the parts of K.  A block takes about the same
-// time for a K block of 64 whatever the tile's width (measured: 0.37 us from 32 to 256 columns),
-// so what counts is how many K blocks fall to the busiest SM; a tile costs its epilogue, and
-// parts of K the trip of the accumulators through the cluster.  Parts are taken only where all
-// the clusters run at once (the product of a narrow output and a long inner size: mlp.c_proj of
-// a prompt portion, whose few tiles would leave most SMs idle).  Times in nanoseconds, from
-// measurements of 2048-row products.  force_bn / force_splits != 0 fix one or both (for tests
-// and measurements).
+// How a product is cut: the width of a tile, the parts of K, and whether tiles are of 256 rows over pairs of SMs.  A K block
+// takes an SM what its operands take to arrive, about 116 bytes a nanosecond (64 bytes a clock), and no less than 0.16 us; so a
+// wide tile is bound by its 16 KB of A and 32 KB of W, of which a pair's block brings half, and a pair by the tensor pipe
+// under the power limit (0.37 us for 256 columns).  What counts then is how many K blocks fall to the busiest SM; a tile
+// costs its epilogue, a pair the two meetings of its blocks, and parts of K the trip of the accumulators through the
+// cluster.  Measured over 45 products of 384 to 2048 rows in every width, single and in pairs, us: the choice is within 0.5% of
+// the best on average.  2048 rows: += 1600 x 6400 single 37.4, pairs 33.6; 4800 x 1600 28.5, 26.6; 3072 x 2048 24.5, 22.1; += 1024 x
+// 4096 19.6, 18.4; 2304 x 768 9.8, 11.2; 512 rows: 4096 x 1024 8.2, 9.0; 6400 x 1600 12.9, 12.8.  Parts are taken only
+// where all the clusters run at once (the product of a narrow output and a long inner size, whose few tiles would leave most
+// SMs idle).  Times in nanoseconds.  force_bn / force_splits != 0 fix one or both (for tests and measurements; FORCE_PAIR: pairs).
 struct Cut {
   int bn, splits, kb_per;
+  bool pair;
 };
-static int ring_stages(int bn, int staging) {
+constexpr int FORCE_PAIR = -2;  // in the place of the parts of K: tiles on pairs of SMs
+static int ring_stages(int bn, int staging, bool pair) {
   const int room = SMEM_BUDGET - 1024 - staging - BAR_BYTES;
-  const int stages = room / stage_bytes(bn);
+  const int stages = room / stage_bytes(bn, pair);
   return stages > MAX_STAGES ? MAX_STAGES : stages;
 }
 // How many clusters of `size` blocks of this kernel the device holds at once (a block fills an
@@ -700,7 +763,7 @@ static int clusters_at_once(int size) {
   static int known[MAX_CLUSTER + 1] = {0};
   if (size < 1 || size > MAX_CLUSTER) return 0;
   if (known[size] == 0) {
-    cudaFuncSetAttribute(gemm_tc_persistent_kernel<float, EPI_TMA, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaFuncSetAttribute(gemm_tc_persistent_kernel<float, EPI_TMA, FORM_PARTS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          SMEM_BUDGET);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(size * 64);
@@ -714,7 +777,7 @@ static int clusters_at_once(int size) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, gemm_tc_persistent_kernel<float, EPI_TMA, true>, &cfg) != cudaSuccess || n < 1) {
+    if (cudaOccupancyMaxActiveClusters(&n, gemm_tc_persistent_kernel<float, EPI_TMA, FORM_PARTS>, &cfg) != cudaSuccess || n < 1) {
       cudaGetLastError();
       n = -1;
     }
@@ -723,13 +786,32 @@ static int clusters_at_once(int size) {
   return known[size] > 0 ? known[size] : 0;
 }
 
-static Cut plan_cut(int M, int N, int K, bool may_split, int staging, int force_bn, int force_splits) {
+static Cut plan_cut(int M, int N, int K, bool may_split, bool may_pair, int staging, int force_bn, int force_splits) {
   const long m_tiles = (M + BM - 1) / BM;
   const int num_kb = (K + BK - 1) / BK;
   const int n_sms = sm_count();
-  Cut best{256, 1, num_kb};
+  Cut best{256, 1, num_kb, false};
   long best_cost = -1;
   static const int kSplits[] = {1, 2, 3, 4, 6, 8};
+  // TMA writes the output (staging of a piece a warp): a float32 piece takes twice as long
+  auto cost_of = [&](long rounds, int bn, int kbs, bool pair) {
+    long kb_ns = stage_bytes(bn, pair) / 116;
+    if (pair && kb_ns < 370L * bn / 256) kb_ns = 370L * bn / 256;
+    if (kb_ns < 160) kb_ns = 160;
+    return rounds * (kb_ns * kbs + 500) + 2500 + (staging > staging_bytes<__nv_bfloat16, EPI_TMA>() ? 1400L : 1000L) * bn / 256;
+  };
+  if (may_pair && (force_splits == 0 || force_splits == FORCE_PAIR) && (M > BM || force_splits == FORCE_PAIR)) {
+    const long down = (M + 2 * BM - 1) / (2 * BM), pairs = n_sms / 2;
+    for (int bn = 256; bn >= 64; bn -= 32) {
+      if (force_bn != 0 && bn != force_bn) continue;
+      const long cost = cost_of(((N + bn - 1) / bn * down + pairs - 1) / pairs, bn, num_kb, true) + 2100;
+      if (best_cost < 0 || cost < best_cost) {
+        best = Cut{bn, 1, num_kb, true};
+        best_cost = cost;
+      }
+    }
+    if (force_splits == FORCE_PAIR) return best;
+  }
   for (int bn = 256; bn >= 64; bn -= 32) {
     if (force_bn != 0 && bn != force_bn) continue;
     const long tiles = (long)((N + bn - 1) / bn) * m_tiles;
@@ -741,32 +823,32 @@ static Cut plan_cut(int M, int N, int K, bool may_split, int staging, int force_
       if (splits > 1) {
         // the pieces sent round the cluster lie in the receiver's ring
         const int owned_max = (bn / 32 + splits - 1) / splits;
-        if (!may_split || (long)splits * 4 * owned_max * 4096 > (long)ring_stages(bn, staging) * stage_bytes(bn)) continue;
+        if (!may_split || (long)splits * 4 * owned_max * 4096 > (long)ring_stages(bn, staging, false) * stage_bytes(bn, false)) continue;
         if (clusters_at_once(splits) < 1) continue;
         if (force_splits == 0 && (tiles > clusters_at_once(splits) || splits * 2 > num_kb)) continue;
       }
       const long rounds = (tiles * splits + n_sms - 1) / n_sms;
-      long cost = rounds * (300L * kb_per + 600) + 1000 + 1500L * bn / 256;
-      if (splits > 1) cost += 2500;
+      const long cost = cost_of(rounds, bn, kb_per, false) + (splits > 1 ? 2300 : 0);
       if (best_cost < 0 || cost < best_cost) {
-        best = Cut{bn, splits, kb_per};
+        best = Cut{bn, splits, kb_per, false};
         best_cost = cost;
       }
     }
   }
-  if (best_cost < 0) best = Cut{force_bn != 0 ? force_bn : 256, 1, num_kb};  // what was forced cannot be had
+  if (best_cost < 0) best = Cut{force_bn != 0 ? force_bn : 256, 1, num_kb, false};  // what was forced cannot be had
   return best;
 }
 
-template <typename TOut, int EPI, bool CLUSTER>
+template <typename TOut, int EPI, int FORM>
 static int launch_persistent(const void* A, long lda, const void* W, const float* bias, void* out, long ldo, int M,
                              int N, int K, int act, int residual, const KvScatter& kv, int* status, const Cut& cut,
                              cudaStream_t stream, const SampleArgs& sample = SampleArgs{}) {
+  constexpr bool CLUSTER = FORM == FORM_PARTS, PAIR = FORM == FORM_PAIR;
   const int bn = cut.bn;
   CUtensorMap ma, mw, mo;
   int rc = tensor_map(A, M, K, lda, BM, &ma);
   if (rc != 0) return rc;
-  rc = tensor_map(W, N, K, K, bn, &mw);
+  rc = tensor_map(W, N, K, K, PAIR ? bn / 2 : bn, &mw);
   if (rc != 0) return rc;
   if (EPI == EPI_TMA) {
     // in a packed qkv product only the queries go to `out`: its map ends where they end
@@ -777,19 +859,21 @@ static int launch_persistent(const void* A, long lda, const void* W, const float
   }
   static bool attr_set = false;
   if (!attr_set) {
-    note_launch(cudaFuncSetAttribute(gemm_tc_persistent_kernel<TOut, EPI, CLUSTER>,
+    note_launch(cudaFuncSetAttribute(gemm_tc_persistent_kernel<TOut, EPI, FORM>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BUDGET));
     attr_set = true;
   }
   constexpr int STAGING_BYTES = staging_bytes<TOut, EPI>();
-  const int stages = ring_stages(bn, STAGING_BYTES);
+  const int stages = ring_stages(bn, STAGING_BYTES, PAIR);
   if (stages < 2) return -2;
-  const size_t smem = 1024 + (size_t)stages * stage_bytes(bn) + STAGING_BYTES + BAR_BYTES;
+  const size_t smem = 1024 + (size_t)stages * stage_bytes(bn, PAIR) + STAGING_BYTES + BAR_BYTES;
   PArgs p{bias, out, ldo, M, N, K, act, residual, bn, stages, bn > 128 ? 512 : (bn > 64 ? 256 : 128),
           cut.splits, cut.kb_per, kv, status, sample};
-  const int units = ((M + BM - 1) / BM) * ((N + bn - 1) / bn) * cut.splits;
+  const int tile_rows = PAIR ? 2 * BM : BM;
+  const int units = ((M + tile_rows - 1) / tile_rows) * ((N + bn - 1) / bn) * cut.splits;
+  const int pairs = sm_count() / 2;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(CLUSTER ? units : (units < sm_count() ? units : sm_count()));
+  cfg.gridDim = dim3(CLUSTER ? units : PAIR ? 2 * (units < pairs ? units : pairs) : (units < sm_count() ? units : sm_count()));
   cfg.blockDim = dim3(PTHREADS);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
@@ -797,12 +881,12 @@ static int launch_persistent(const void* A, long lda, const void* W, const float
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = CLUSTER ? cut.splits : 1;
+  attr[1].val.clusterDim.x = CLUSTER ? cut.splits : PAIR ? 2 : 1;
   attr[1].val.clusterDim.y = 1;
   attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = CLUSTER ? 2 : 1;
-  note_launch(launch_kernel(cfg, gemm_tc_persistent_kernel<TOut, EPI, CLUSTER>, ma, mw, mo, p));
+  cfg.numAttrs = CLUSTER || PAIR ? 2 : 1;
+  note_launch(launch_kernel(cfg, gemm_tc_persistent_kernel<TOut, EPI, FORM>, ma, mw, mo, p));
   return take_launch_error();
 }
 
@@ -831,7 +915,7 @@ RL_EXPORT int rl_gemm_tc_cut(int out_dtype, const void* A, long lda, const void*
   if (kv_pool != nullptr && (kv_head_dim % 4 != 0 || kv_q_width % 4 != 0 || kv_width % 4 != 0 || act != 0 || residual))
     return -8;
   if (tile_width != 0 && (tile_width % 32 != 0 || tile_width < 32 || tile_width > 256)) return -2;
-  if (splits < 0 || splits > 8 || status == nullptr) return -2;
+  if ((splits < 0 && splits != rl::tc::FORCE_PAIR) || splits > 8 || status == nullptr) return -2;
   const rl::KvScatter kv{kv_pool, kv_block_table, kv_bt_stride, kv_positions, kv_req_of_token, kv_slots,
                          kv_q_width, kv_width, kv_head_dim, kv_page_size, kv_heads, kv_max_pos, status};
   // the output goes through a tensor map where its rows start on 16-byte boundaries (and keys
@@ -843,11 +927,14 @@ RL_EXPORT int rl_gemm_tc_cut(int out_dtype, const void* A, long lda, const void*
   using namespace rl::tc;
 #define RL_TC(T, E)                                                                                                  \
   do {                                                                                                               \
-    const Cut cut = plan_cut(M, N, K, E != EPI_PLAIN, staging_bytes<T, E>(), tile_width, splits);                     \
+    const Cut cut = plan_cut(M, N, K, E == EPI_TMA, E == EPI_TMA, staging_bytes<T, E>(), tile_width, splits);         \
     if (E != EPI_PLAIN && cut.splits > 1)                                                                            \
-      return launch_persistent<T, E == EPI_PLAIN ? EPI_TMA : E, true>(A, lda, W, bias, out, ldo, M, N, K, act, residual, kv, \
-                                                                     status, cut, stream);                           \
-    return launch_persistent<T, E, false>(A, lda, W, bias, out, ldo, M, N, K, act, residual, kv, status, cut, stream); \
+      return launch_persistent<T, E == EPI_PLAIN ? EPI_TMA : E, FORM_PARTS>(A, lda, W, bias, out, ldo, M, N, K, act, residual, \
+                                                                           kv, status, cut, stream);                 \
+    if (E != EPI_PLAIN && cut.pair)                                                                                  \
+      return launch_persistent<T, E == EPI_PLAIN ? EPI_TMA : E, FORM_PAIR>(A, lda, W, bias, out, ldo, M, N, K, act, residual, \
+                                                                          kv, status, cut, stream);                  \
+    return launch_persistent<T, E, FORM_SINGLE>(A, lda, W, bias, out, ldo, M, N, K, act, residual, kv, status, cut, stream); \
   } while (0)
   if (out_dtype == RL_F32) {
     if (tma_out) RL_TC(float, EPI_TMA);
@@ -884,8 +971,8 @@ RL_EXPORT int rl_gemm_tc_sample(const void* A, long lda, const void* W, const fl
   const rl::KvScatter kv{};
   if (host_ring != nullptr && (ring_step == nullptr || ring_stride < M)) return -7;
   const rl::SampleArgs sample{out_ids, temperature, seeds, counters, best, ticket, host_ring, ring_stride, ring_step, soft_cap};
-  const Cut cut = plan_cut(M, N, K, false, 0, 0, 0);
-  return launch_persistent<float, EPI_SAMPLE, false>(A, lda, W, bias, nullptr, 0, M, N, K, RL_ACT_NONE, 0, kv, status, cut,
+  const Cut cut = plan_cut(M, N, K, false, false, 0, 0, 0);
+  return launch_persistent<float, EPI_SAMPLE, FORM_SINGLE>(A, lda, W, bias, nullptr, 0, M, N, K, RL_ACT_NONE, 0, kv, status, cut,
                                                      stream, sample);
 }
 
