@@ -1,0 +1,385 @@
+// float32 products of many rows (prompt portions of the 32-bit mode) on the tensor cores of sm_100a:
+//
+//   out[M,N] = A[M,K] * W[N,K]^T  (+ bias[N]) (GELU) (or out += ..., the float32 residual stream)
+//
+// the products and epilogues of gemm_simt.cu (rosellm/rosetrainer/model.py:95, 220, 334-337; fused_mlp.py:79-113).  An
+// operand is cut into two parts of eleven significant bits, x = hi + lo, hi the nearest tf32 number to x and lo the
+// nearest to the rest, which leaves at most 2^-24 of x (half a unit in its last place).  Of the four products of the parts
+// three are made, hi hi, hi lo and lo hi, each exact in the multiplier; lo lo is below 2^-22 of the product and
+// left out (its sign is random: over a sum it stays far below one rounding).  What costs a sum on this unit its bits is the
+// accumulator, which cuts off instead of rounding: so hi hi and the two small products have an accumulator each, the small
+// one losing nothing that counts, and after CHUNK K blocks of 32 both are drained and added in registers with ordinary
+// float32 additions.  (With two blocks between the additions 5% faster, but sums of 128 positive products were further from 64 bits
+// than single FMAs.)
+//
+// One block per SM walks tiles of 128 rows x BN columns.  Its warps:
+//   warp 0      one lane copies tiles of A and W (K blocks of 32 floats = 128 bytes, 128-byte swizzle) by TMA into a ring of
+//               stages; those of W for the first stages before the wait for the kernels ahead;
+//   warps 2-9   cut what arrived: hi takes the place of x, lo goes to the stage's second half, byte for byte at the same
+//               place, so that the swizzle needs no thought;
+//   warp 1      one lane issues tcgen05.mma kind::tf32, twelve of K 8 a K block;
+//   warps 10-17 drain the accumulators (two pairs in turn) and write the tile.
+// Shared memory is what bounds it: a K block of a 128 x 128 tile is read once and written twice by the cutting warps (96 KB)
+// and read three times by the products (96 KB), about 1,500 clocks of its 128 bytes a clock where the tensor pipe needs 770.
+//
+// Measured on B200 between the other kernels of a layer, 1,752 rows of GPT-2 124M, us (the CUDA-core tiles before, now): 2304 x 768
+// 160, 3072 x 768 226, now 82 on average; += 768 x 768 and += 768 x 3072 161 on average, now 73.  Error against 64 bits (2-norm of
+// the difference over that of the result) of those tiles and of this kernel: K 768 2.4e-7, 1.0e-7; K 3072 7.5e-7, 1.8e-7.
+//
+// Numbers that cannot be cut (infinities, NaN, magnitudes that round to infinity) are noticed while cutting: a block that
+// has met one works its tiles out anew with FMAs from memory, in the order of the CUDA-core kernels.
+// Every wait on a barrier is bounded (status bit, abort flag), as in gemm_tc.cu.
+#include "gemm_epilogue.cuh"
+#include "gemm_f32_tc.cuh"
+#include "tc_common.cuh"
+
+namespace rl {
+namespace f32tc {
+
+constexpr int BM = 128, BK = 32;
+constexpr int CUT_WARPS = 8, EPI_WARPS = 8, THREADS = 32 * (2 + CUT_WARPS + EPI_WARPS);
+constexpr int CHUNK = 1;  // K blocks between two additions in registers
+constexpr int MAX_STAGES = 4;
+constexpr int A_BYTES = BM * BK * 4;
+__host__ __device__ constexpr int operand_bytes(int bn) { return A_BYTES + bn * BK * 4; }
+__host__ __device__ constexpr int stages_of(int bn) {
+  const int fit = (227 * 1024 - 2048) / (2 * operand_bytes(bn));
+  return fit > MAX_STAGES ? MAX_STAGES : fit;
+}
+// 1024 for alignment | stages of (hi, in x's place | lo) | barriers full, cut, empty [MAX_STAGES], acc_full, acc_empty [2],
+// the tensor-memory address, the abort flag and the flag of a number that cannot be cut
+__host__ __device__ constexpr int smem_bytes(int bn) { return 1024 + stages_of(bn) * 2 * operand_bytes(bn) + (3 * MAX_STAGES + 4) * 8 + 16; }
+
+struct Args {
+  const float* a;
+  long lda;
+  const float* w;
+  const float* bias;
+  float* out;
+  long ldo;
+  int M, N, K, act, residual;
+  int* status;
+};
+
+__device__ __forceinline__ void mma_tf32(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// tf32 x tf32 -> float32, both operands K-major
+__host__ __device__ constexpr uint32_t instr_desc_tf32(int n) {
+  return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+}
+// The nearest number of eleven significant bits, halves away from zero (an infinity stays one; the largest magnitudes become one).
+__device__ __forceinline__ float to_tf32(float x) { return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u); }
+// A call, not sixteen inlined copies, of four values at a time: one after the other their latencies would add up.
+__device__ __noinline__ float4 act_call(float4 v, int act) {
+  return make_float4(apply_act(v.x, act), apply_act(v.y, act), apply_act(v.z, act), apply_act(v.w, act));
+}
+
+template <int BN>
+__global__ __launch_bounds__(THREADS, 1) void gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a,
+                                                                 const __grid_constant__ CUtensorMap map_w, const Args p) {
+  constexpr int OPERANDS = operand_bytes(BN), STAGE = 2 * OPERANDS, STAGES = stages_of(BN);
+  constexpr uint32_t TMEM_COLS = 4 * BN;  // two pairs of accumulators
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  const uint32_t smem_base = tc::smem_u32(smem), bar_base = smem_base + STAGES * STAGE;
+  auto full_bar = [&](int s) { return bar_base + 8u * s; };
+  auto cut_bar = [&](int s) { return bar_base + 8u * (MAX_STAGES + s); };
+  auto empty_bar = [&](int s) { return bar_base + 8u * (2 * MAX_STAGES + s); };
+  auto acc_full = [&](int b) { return bar_base + 8u * (3 * MAX_STAGES + b); };
+  auto acc_empty = [&](int b) { return bar_base + 8u * (3 * MAX_STAGES + 2 + b); };
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + STAGES * STAGE + (3 * MAX_STAGES + 4) * 8);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  volatile int* uncut_flag = reinterpret_cast<volatile int*>(tmem_slot + 2);
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  const int m_tiles = (p.M + BM - 1) / BM, units = m_tiles * ((p.N + BN - 1) / BN), kbs = (p.K + BK - 1) / BK;
+
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (tid == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      tc::mbar_init(full_bar(s), 1);
+      tc::mbar_init(cut_bar(s), CUT_WARPS);
+      tc::mbar_init(empty_bar(s), 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      tc::mbar_init(acc_full(b), 1);
+      tc::mbar_init(acc_empty(b), EPI_WARPS);
+    }
+    *abort_flag = 0;
+    *uncut_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    tc::tma_prefetch_map(&map_a);
+    tc::tma_prefetch_map(&map_w);
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc::smem_u32(tmem_slot)), "r"(TMEM_COLS)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+
+  // The copying and the issuing warp walk their loops whole, with values that are the same in all lanes; one lane issues.
+  if (warp == 0) {
+    int ahead = 0;  // stages whose W tiles are asked for before the kernels ahead have ended
+    if ((int)blockIdx.x < units) {
+      ahead = kbs < STAGES ? kbs : STAGES;
+      const int n0 = ((int)blockIdx.x / m_tiles) * BN;
+      for (int s = 0; s < ahead; ++s)
+        if (tc::elect_one()) {
+          tc::mbar_expect_tx(full_bar(s), OPERANDS);
+          tc::tma_load_2d(smem_base + s * STAGE + A_BYTES, &map_w, full_bar(s), s * BK, n0);
+        }
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    int it = 0, s = 0;
+    uint32_t ph = 0;
+    bool ok = true;
+    for (int unit = blockIdx.x; unit < units && ok; unit += gridDim.x) {
+      const int m0 = (unit % m_tiles) * BM, n0 = (unit / m_tiles) * BN;
+      for (int kb = 0; kb < kbs; ++kb, ++it) {
+        if (it >= ahead) {
+          ok = tc::mbar_wait_warp(empty_bar(s), ph ^ 1u, abort_flag, p.status);  // a stage's first use: passes at once
+          if (!ok) break;
+        }
+        if (tc::elect_one()) {
+          if (it >= ahead) {
+            tc::mbar_expect_tx(full_bar(s), OPERANDS);
+            tc::tma_load_2d(smem_base + s * STAGE + A_BYTES, &map_w, full_bar(s), kb * BK, n0);
+          }
+          tc::tma_load_2d(smem_base + s * STAGE, &map_a, full_bar(s), kb * BK, m0);
+        }
+        __syncwarp();
+        if (++s == STAGES) s = 0, ph ^= 1u;
+      }
+    }
+    if (*abort_flag)
+      for (int k = it > STAGES ? it - STAGES : 0; k < it; ++k) tc::mbar_wait_quiet(full_bar(k % STAGES), (uint32_t)(k / STAGES) & 1u);
+  } else if (warp == 1) {
+    constexpr uint32_t idesc = instr_desc_tf32(BN);
+    const uint64_t desc0 = tc::smem_desc(smem_base);
+    int s = 0, chunk = 0;
+    uint32_t ph = 0;
+    bool ok = true;
+    for (int unit = blockIdx.x; unit < units && ok; unit += gridDim.x)
+      for (int kb0 = 0; kb0 < kbs && ok; kb0 += CHUNK, ++chunk) {
+        const int buf = chunk & 1;
+        ok = tc::mbar_wait_warp(acc_empty(buf), ((uint32_t)(chunk >> 1) & 1u) ^ 1u, abort_flag, p.status);
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t main = tmem_base + (uint32_t)(buf * 2 * BN), small = main + BN;
+        for (int kb = kb0; kb < min(kb0 + CHUNK, kbs); ++kb) {
+          ok = tc::mbar_wait_warp(cut_bar(s), ph, abort_flag, p.status);
+          if (!ok) break;
+          const uint64_t a_hi = desc0 + (uint64_t)(s * (STAGE >> 4)), w_hi = a_hi + (A_BYTES >> 4);
+          const uint64_t a_lo = a_hi + (OPERANDS >> 4), w_lo = w_hi + (OPERANDS >> 4);
+          if (tc::elect_one()) {
+#pragma unroll
+            for (int k = 0; k < BK / 8; ++k) {  // K steps of 8 floats: 32 bytes, two units of a descriptor
+              const uint32_t more = kb > kb0 || k > 0 ? 1u : 0u;
+              mma_tf32(small, a_lo + 2 * k, w_hi + 2 * k, idesc, more);
+              mma_tf32(small, a_hi + 2 * k, w_lo + 2 * k, idesc, 1u);
+              mma_tf32(main, a_hi + 2 * k, w_hi + 2 * k, idesc, more);
+            }
+            tc::mma_commit(empty_bar(s));
+          }
+          __syncwarp();
+          if (++s == STAGES) s = 0, ph ^= 1u;
+        }
+        if (ok && tc::elect_one()) tc::mma_commit(acc_full(buf));
+        __syncwarp();
+      }
+  } else if (warp < 2 + CUT_WARPS) {
+    constexpr int PIECES = OPERANDS / 16 / (32 * CUT_WARPS);  // 16-byte pieces of a K block a thread cuts
+    static_assert(OPERANDS % (16 * 32 * CUT_WARPS) == 0, "pieces are shared evenly");
+    int s = 0;
+    uint32_t ph = 0;
+    bool ok = true;
+    for (int unit = blockIdx.x; unit < units && ok; unit += gridDim.x)
+      for (int kb = 0; kb < kbs; ++kb) {
+        ok = tc::mbar_wait(full_bar(s), ph, abort_flag, p.status);
+        if (!ok) break;
+        float4* x = reinterpret_cast<float4*>(smem + s * STAGE) + (tid - 64);
+        float4* low = reinterpret_cast<float4*>(smem + s * STAGE + OPERANDS) + (tid - 64);
+        float4 v[PIECES];
+#pragma unroll
+        for (int i = 0; i < PIECES; ++i) v[i] = x[i * 32 * CUT_WARPS];
+        float odd = 0.f;  // becomes NaN where a rest is not finite
+#pragma unroll
+        for (int i = 0; i < PIECES; ++i) {
+          const float4 hi = make_float4(to_tf32(v[i].x), to_tf32(v[i].y), to_tf32(v[i].z), to_tf32(v[i].w));
+          const float4 lo = make_float4(v[i].x - hi.x, v[i].y - hi.y, v[i].z - hi.z, v[i].w - hi.w);
+          odd = fmaf(lo.x, 0.f, odd), odd = fmaf(lo.y, 0.f, odd), odd = fmaf(lo.z, 0.f, odd), odd = fmaf(lo.w, 0.f, odd);
+          x[i * 32 * CUT_WARPS] = hi;
+          low[i * 32 * CUT_WARPS] = make_float4(to_tf32(lo.x), to_tf32(lo.y), to_tf32(lo.z), to_tf32(lo.w));
+        }
+        if (odd != 0.f) *uncut_flag = 1;  // (a NaN is not equal to zero)
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(cut_bar(s)) : "memory");
+        if (++s == STAGES) s = 0, ph ^= 1u;
+      }
+  } else {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    constexpr int COLS = BN / 2;                    // of a thread: its row's, in one half of the tile
+    constexpr int STEP = 16;
+    const int quarter = warp & 3, part = (warp - 2 - CUT_WARPS) >> 2;
+    const bool vec = p.ldo % 4 == 0 && (uintptr_t)p.out % 16 == 0;
+    int chunk = 0;
+    bool ok = true;
+    for (int unit = blockIdx.x; unit < units && ok; unit += gridDim.x) {
+      const int row = (unit % m_tiles) * BM + quarter * 32 + lane, n0 = (unit / m_tiles) * BN + part * COLS;
+      float acc[COLS];
+#pragma unroll
+      for (int i = 0; i < COLS; ++i) acc[i] = 0.f;
+      for (int kb0 = 0; kb0 < kbs; kb0 += CHUNK, ++chunk) {
+        const int buf = chunk & 1;
+        ok = __all_sync(0xffffffffu, tc::mbar_wait(acc_full(buf), (uint32_t)(chunk >> 1) & 1u, abort_flag, p.status));
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t main = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * 2 * BN + part * COLS);
+#pragma unroll
+        for (int c = 0; c < COLS; c += STEP) {
+          uint32_t big[STEP], small[STEP];
+          tc::tmem_load16(main + c, big);
+          tc::tmem_load16(main + BN + c, small);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int i = 0; i < STEP; ++i) acc[c + i] += __uint_as_float(big[i]) + __uint_as_float(small[i]);
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(acc_empty(buf)) : "memory");
+      }
+      if (!ok) break;
+      if (row >= p.M) continue;
+      if (*uncut_flag) {
+        const float* a = p.a + (size_t)row * p.lda;
+#pragma unroll
+        for (int i = 0; i < COLS; ++i) {
+          const float* w = p.w + (size_t)min(n0 + i, p.N - 1) * p.K;
+          float t = 0.f;
+#pragma unroll 1
+          for (int k = 0; k < p.K; ++k) t = fmaf(a[k], w[k], t);
+          acc[i] = t;
+        }
+      }
+      float* out = p.out + (size_t)row * p.ldo + n0;
+#pragma unroll
+      for (int c = 0; c < COLS; c += 4) {
+        if (n0 + c >= p.N) break;
+        float v[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          v[i] = acc[c + i];
+          if (p.bias != nullptr && n0 + c + i < p.N) v[i] += p.bias[n0 + c + i];
+        }
+        if (p.act != RL_ACT_NONE) {
+          const float4 t = act_call(make_float4(v[0], v[1], v[2], v[3]), p.act);
+          v[0] = t.x, v[1] = t.y, v[2] = t.z, v[3] = t.w;
+        }
+        if (vec && n0 + c + 3 < p.N) {
+          float4 t = make_float4(v[0], v[1], v[2], v[3]);
+          if (p.residual) {
+            const float4 old = *reinterpret_cast<const float4*>(out + c);
+            t.x += old.x, t.y += old.y, t.z += old.z, t.w += old.w;
+          }
+          *reinterpret_cast<float4*>(out + c) = t;
+        } else {
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            if (n0 + c + i < p.N) out[c + i] = p.residual ? out[c + i] + v[i] : v[i];
+        }
+      }
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 1)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
+}
+
+static int sm_count() {
+  static int n_sms = 0;
+  if (n_sms == 0) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, dev);
+    if (n_sms <= 0) n_sms = 1;
+  }
+  return n_sms;
+}
+
+template <int BN>
+static int launch(const Args& p, cudaStream_t stream) {
+  CUtensorMap ma, mw;
+  int rc = tc::tensor_map(p.a, p.M, p.K, p.lda, BM, &ma, BK, 4);
+  if (rc == 0) rc = tc::tensor_map(p.w, p.N, p.K, p.K, BN, &mw, BK, 4);
+  if (rc != 0) return rc;
+  static bool attr_set = false;
+  if (!attr_set) {
+    note_launch(cudaFuncSetAttribute(gemm_f32_tc_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(BN)));
+    attr_set = true;
+  }
+  const int n_sms = sm_count();
+  const long units = (long)((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN);
+  launch_pdl_split(false, gemm_f32_tc_kernel<BN>, dim3((unsigned)(units < n_sms ? units : n_sms)), dim3(THREADS), smem_bytes(BN), stream, ma,
+                   mw, p);
+  return take_launch_error();
+}
+
+bool takes(const void* a, long lda, const void* w, int K, const int* status) {
+  return K > 0 && K % 4 == 0 && lda % 4 == 0 && (uintptr_t)a % 16 == 0 && (uintptr_t)w % 16 == 0 && status != nullptr &&
+         tc::encode_fn() != nullptr;
+}
+
+// A tile: a fixed time (launch, first copies, the epilogue) and one a K block; a round of tiles more costs its epilogue too.
+struct WidthTime {
+  int bn;
+  double fixed, kb, round;
+};
+constexpr WidthTime WIDTHS[] = {{32, 5.1, 0.62, 1.2}, {64, 7.0, 0.67, 3.0}, {128, 10.5, 0.85, 7.0}};
+
+double time_us(int M, int N, int K, int* width) {
+  const long down = ((long)M + BM - 1) / BM;
+  const int kbs = (K + BK - 1) / BK, sms = sm_count();
+  double best = 1e30;
+  for (const WidthTime& w : WIDTHS) {
+    const long tiles = down * ((N + w.bn - 1) / w.bn), rounds = (tiles + sms - 1) / sms;
+    const double us = w.fixed + rounds * kbs * w.kb + (rounds - 1) * w.round;
+    if (us < best && tiles <= 0x7fffffff) {
+      best = us;
+      *width = w.bn;
+    }
+  }
+  return best;
+}
+
+int run(const float* a, long lda, const float* w, const float* bias, float* out, long ldo, int M, int N, int K, int act, int residual,
+        int width, int* status, cudaStream_t stream) {
+  const Args p{a, lda, w, bias, out, ldo, M, N, K, act, residual, status};
+  return width == 32 ? launch<32>(p, stream) : width == 64 ? launch<64>(p, stream) : launch<128>(p, stream);
+}
+
+}  // namespace f32tc
+}  // namespace rl
+
+// float32 A [M, K] (row stride lda) and W [N, K], out float32; residual != 0: out += result.  tile_width: 0 = chosen here, else
+// the columns of a tile (32, 64 or 128; for tests and measurements).  Operands on 16-byte boundaries, K and lda multiples of 4.
+RL_EXPORT int rl_gemm_f32_tc(const float* A, long lda, const float* W, const float* bias, float* out, long ldo, int M, int N, int K,
+                             int act, int residual, int tile_width, int* status, cudaStream_t stream) {
+  if (M <= 0 || N <= 0) return 0;
+  if (!rl::f32tc::takes(A, lda, W, K, status)) return -2;
+  int width = tile_width;
+  if (width == 0) rl::f32tc::time_us(M, N, K, &width);
+  if (width != 32 && width != 64 && width != 128) return -2;
+  return rl::f32tc::run(A, lda, W, bias, out, ldo, M, N, K, act, residual, width, status, stream);
+}

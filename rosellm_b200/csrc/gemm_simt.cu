@@ -10,6 +10,7 @@
 //   gelu_erf(u)  = 0.5 u (1 + erf(u / sqrt 2))                       model.py:345-346 (F.gelu)
 //   x = x + y (residual)                  model.py:412-413, 424-428; fused_mlp.py:91-113
 #include "gemm_epilogue.cuh"
+#include "gemm_f32_tc.cuh"
 
 namespace rl {
 
@@ -456,7 +457,7 @@ static double tile_time(const TileTime (&time)[POINTS], double tiles) {
 // The tile that ends first.  Over 161 products of 65 to 2048 rows (64 to 4096 columns, K 256 to 6400) the choice is 1% behind the
 // fastest form on average; by counting rounds of tiles it was 7%, up to 45% (1600 x 1600 at 300 rows: 146, 99 and 120 us on 64 x 64,
 // 32 x 64 and 32 x 32; 768 x 768 at 600 rows 66, 56 and 59).  128 x 64, and 8 x 8 outputs a thread, measured slower throughout.
-static dim3 tile_f32_for(int M, int N) {
+static dim3 tile_f32_for(int M, int N, double* us = nullptr) {
   const int sms = simt_sm_count();
   auto cost = [&](int bm, int bn, const auto& time) {
     const long down = (M + bm - 1) / bm, tiles = down * ((N + bn - 1) / bn);
@@ -464,6 +465,7 @@ static dim3 tile_f32_for(int M, int N) {
     return tile_time(time, (double)tiles / sms);
   };
   const double large = cost(64, 64, TIME_64X64), middle = cost(32, 64, TIME_32X64), small = cost(32, 32, TIME_32X32);
+  if (us != nullptr) *us = fmin(fmin(large, middle), small);
   return large <= middle && large <= small ? dim3(64, 64) : middle <= small ? dim3(32, 64) : dim3(32, 32);
 }
 
@@ -547,6 +549,15 @@ RL_EXPORT int rl_gemm_simt(int in_dtype, int out_dtype, const void* A, long lda,
   rl::KvScatter kv{kv_pool, kv_block_table, kv_bt_stride, kv_positions, kv_req_of_token, kv_slots,
                    kv_q_width, kv_width, kv_head_dim, kv_page_size, kv_heads, kv_max_pos, status};
   int rc;
+  if (in_dtype == RL_F32 && out_dtype == RL_F32 && M > rows_limit && kv_pool == nullptr && K >= rl::f32tc::MIN_K &&
+      rl::f32tc::takes(A, lda, W, K, status)) {
+    // many rows: the tensor cores where they are the faster (gemm_f32_tc.cu), which they are but for few tiles
+    double tiles_us = 0.0;
+    rl::tile_f32_for(M, N, &tiles_us);
+    int width = 0;
+    if (rl::f32tc::time_us(M, N, K, &width) < 0.95 * tiles_us * K / 768.0)
+      return rl::f32tc::run((const float*)A, lda, (const float*)W, bias, (float*)out, ldo, M, N, K, act, residual, width, status, stream);
+  }
   if (in_dtype == RL_F32 && out_dtype == RL_F32)
     rc = rl::launch_gemm<float, float>(A, lda, W, bias, out, ldo, M, N, K, act, residual, rows_limit, kv, stream);
   else if (in_dtype == RL_BF16 && out_dtype == RL_BF16)

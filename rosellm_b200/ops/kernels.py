@@ -173,6 +173,8 @@ def _lib() -> ctypes.CDLL:
         lib.rl_gemm_rows_smem_fits.argtypes = [I, I, I, I, I, I, I]
         lib.rl_gemm_rows_ring_fits.argtypes = [I, I, I, I, I]
         lib.rl_gemm_tile_f32_for.argtypes = [I, I]
+        lib.rl_gemm_f32_tc.argtypes = [P, L, P, P, P, L, I, I, I, I, I, I, P, P]
+        lib.rl_gemm_f32_tc.restype = I
         lib.rl_notes_begin.argtypes = lib.rl_notes_end.argtypes = []
         lib.rl_notes_begin.restype = lib.rl_notes_replay.restype = I
         lib.rl_notes_end.restype = P
@@ -596,7 +598,13 @@ def linear(a, weight, bias, out, *, act: int = ACT_NONE, residual: bool = False,
             raise KernelError("linear: the packed qkv width does not fit the cache's heads")
         kx = (kv.pool.data_ptr(), kv.block_table.data_ptr(), kv.block_table.stride(0), kv.positions.data_ptr(),
               kv.req_of_token.data_ptr(), kv.slots.data_ptr(), kv.q_width, n_kv * dh, dh, page_size, n_kv, kv.max_pos)
-    if path == "smem":
+    if path == "f32tc":
+        rc = _lib().rl_gemm_f32_tc(a_ptr, lda, _ptr(weight), _ptr(bias), _ptr(out), out.stride(0), m, n, k, act, int(residual),
+                                   tile_width, status, _stream())
+        if rc in (-10, -11):
+            raise KernelError("linear: the driver refused to encode a TMA tensor map for these operands")
+        _ok(rc, "linear (float32 on tcgen05)")
+    elif path == "smem":
         rc = _lib().rl_gemm_rows_smem(_code(out), a_ptr, lda, _ptr(weight), _ptr(bias), _ptr(out),
                                       out.stride(0), m, n, k, act, int(residual), *kx, status, _stream())
         if rc == -2:
