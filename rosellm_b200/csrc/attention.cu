@@ -32,7 +32,8 @@ RL_EXPORT int rl_attention(int dtype, const void* q, long q_stride, const void* 
                            cudaStream_t stream) {
   if (head_dim % 16 != 0 || head_dim <= 0 || head_dim > 256) return -2;
   if (n_kv_heads <= 0 || n_heads % n_kv_heads != 0) return -3;
-  if (n_splits < 1 || n_splits > 65535 || (n_splits > 1 && (part_o == nullptr || part_ml == nullptr))) return -4;
+  if (n_splits < 1 || n_splits > 65535 || ((n_splits > 8 || decode_wide == 0) && n_splits > 1 && (part_o == nullptr || part_ml == nullptr)))
+    return -4;
   if (status == nullptr) return -6;
   rl::AttnParams p{q, q_stride, pool, block_table, bt_stride, q_start, kv_len, slots, out,
                    out_stride, n_heads, n_kv_heads, head_dim, page_size, window, scale, status, old_keys_settled};

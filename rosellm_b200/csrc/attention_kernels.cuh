@@ -249,7 +249,11 @@ struct DecodeTile {
 // memory (launch_decode_form): 80 % (DENSE 1: five four-warp blocks of 33 KB an SM instead of
 // three) or all of it (DENSE 2: six), each block somewhat slower the less L1 is left, for grids
 // that would otherwise need a second, partly empty round.
-template <typename T, int EPL, int WARPS, int STAGES, int DENSE = 0>
+// CLUSTER: the parts of a request's keys are the blocks of a cluster, whose results meet in the first one's hands through
+// distributed shared memory, instead of in part_o and a kernel of their own.  Requests of up to DECODE_CLUSTER_KEYS keys are
+// walked by the first block alone: the meeting costs 0.5 us, a round of the eight warps (128 keys) about 0.8.
+constexpr int DECODE_CLUSTER_KEYS = 256;
+template <typename T, int EPL, int WARPS, int STAGES, int DENSE = 0, bool CLUSTER = false>
 __global__ __launch_bounds__(32 * WARPS) void attn_decode_kernel(
     AttnParams p, const int* __restrict__ decode_reqs, int n_splits, float* __restrict__ part_o,
     float* __restrict__ part_ml) {
@@ -261,8 +265,10 @@ __global__ __launch_bounds__(32 * WARPS) void attn_decode_kernel(
   // exponentials are single ex2 instructions; float32 keeps the library's expf
   constexpr bool BASE2 = sizeof(T) == 2;
   auto ex = [](float x) { return BASE2 ? exp2f(x) : expf(x); };
-  extern __shared__ __align__(16) uint32_t ring[];      // [warps][STAGES][2][SUB][32 lanes][WORDS]
-  __shared__ float ml_s[WARPS][2];
+  // [warps][STAGES][2][SUB][32 lanes][WORDS], behind the static part; on a boundary of 128 bytes: 16 bytes off one of 32, the
+  // copies' sectors were cut in two and every form took 17% longer
+  extern __shared__ __align__(128) uint32_t ring[];
+  __shared__ float ml_s[CLUSTER ? WARPS + 1 : WARPS][2];  // of the warps (then of the block)
   // The batch's description (written by the host before the step) and the keys and values of
   // earlier steps do not depend on the kernels ahead: they are fetched before the wait for
   // those.  What the kernel ahead does write is read after it: the query, and the key and
@@ -287,6 +293,13 @@ __global__ __launch_bounds__(32 * WARPS) void attn_decode_kernel(
   const int kv_len = p.kv_len[req];
   const int kv_lo = p.window > 0 ? max(0, kv_len - p.window) : 0;
   const int total = kv_len - kv_lo;
+  if constexpr (CLUSTER) {
+    // few keys: the first block alone (all of the cluster's blocks come to the same answer; none waits for another then)
+    if (total <= DECODE_CLUSTER_KEYS) {
+      if (sp > 0) return;
+      n_splits = 1;
+    }
+  }
   const int chunk = ((total + n_splits - 1) / n_splits + 31) / 32 * 32;
   const int beg = kv_lo + sp * chunk;
   const int end = min(kv_len, beg + chunk);
@@ -444,6 +457,45 @@ __global__ __launch_bounds__(32 * WARPS) void attn_decode_kernel(
     f[w] = ml_s[w][0] == -CUDART_INF_F ? 0.f : ex(ml_s[w][0] - mm);
     ll += ml_s[w][1] * f[w];
   }
+  if (CLUSTER && n_splits > 1) {
+    // the block's result to its own shared memory, behind the warps'; the first block adds the parts up in their order
+    float* o_block = o_s + WARPS * dh;
+    for (int d = tid; d < dh; d += blockDim.x) {
+      float acc = 0.f;
+#pragma unroll
+      for (int w = 0; w < WARPS; ++w) acc = fmaf(o_s[w * dh + d], f[w], acc);
+      o_block[d] = acc;
+    }
+    if (tid == 0) {
+      ml_s[WARPS][0] = mm;
+      ml_s[WARPS][1] = ll;
+    }
+    cluster_sync();
+    for (int d = sp == 0 ? tid : dh; d < dh; d += blockDim.x) {
+      float mp[8], lp[8], op[8];
+      const uint32_t ml_a = (uint32_t)__cvta_generic_to_shared(&ml_s[WARPS][0]), o_a = (uint32_t)__cvta_generic_to_shared(o_block + d);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {  // unconditional (the last block's again): all on their way before the first is used
+        const uint32_t r = (uint32_t)min(q, n_splits - 1);
+        asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(mp[q]), "=f"(lp[q]) : "r"(peer_addr(ml_a, r)) : "memory");
+        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(op[q]) : "r"(peer_addr(o_a, r)) : "memory");
+      }
+      float top = -CUDART_INF_F;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) top = fmaxf(top, mp[q]);
+      float den = 0.f, acc = 0.f;
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if (q < n_splits && mp[q] != -CUDART_INF_F) {  // a part may be without keys
+          const float e = ex(mp[q] - top);
+          den = fmaf(lp[q], e, den);
+          acc = fmaf(op[q], e, acc);
+        }
+      ((T*)p.out)[(size_t)n * p.out_stride + h * dh + d] = from_f32<T>(acc / den);
+    }
+    cluster_sync();  // no block ends while the first may still read its result
+    return;
+  }
   const size_t base = ((size_t)di * p.n_heads + h) * n_splits + sp;
   for (int d = tid; d < dh; d += blockDim.x) {
     float acc = 0.f;
@@ -560,6 +612,34 @@ static inline void launch_decode_form(const AttnParams& p, const int* decode_req
                    dim3(32 * WARPS), smem, stream, p, decode_reqs, n_splits, part_o, part_ml);
 }
 
+// The same over clusters of n_splits (2 to 8) blocks.
+template <typename T, int EPL, int WARPS, int STAGES>
+static inline void launch_decode_cluster(const AttnParams& p, const int* decode_reqs, int n_decode, int n_splits, cudaStream_t stream) {
+  constexpr auto kernel = attn_decode_kernel<T, EPL, WARPS, STAGES, 0, true>;
+  constexpr size_t smem = DecodeTile<EPL * (int)sizeof(T) / 4, WARPS, STAGES>::SMEM;
+  static bool attr_set = false;
+  if (!attr_set) {
+    if (smem > 47 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
+    attr_set = true;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(n_decode, p.n_heads, n_splits);
+  cfg.blockDim = dim3(32 * WARPS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = 1;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = n_splits;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  note_launch(launch_kernel(cfg, kernel, p, decode_reqs, n_splits, (float*)nullptr, (float*)nullptr));
+}
+
 // How many narrow (four-warp) blocks of these sizes the device holds at once with this share
 // (percent) of an SM's memory as shared memory; half is the split every small kernel asks for.
 template <typename T, int EPL>
@@ -601,6 +681,10 @@ template <typename T, int EPL>
 static inline void launch_decode(const AttnParams& p, const int* decode_reqs, int n_decode, int n_splits,
                                  int wide, float* part_o, float* part_ml, cudaStream_t stream) {
   const int dh = p.head_dim;
+  if (n_splits > 1 && part_o == nullptr) {  // the parts as clusters
+    launch_decode_cluster<T, EPL, 8, 2>(p, decode_reqs, n_decode, n_splits, stream);
+    return;
+  }
   if (wide) {
     // a ring of one tile where two would not fit an SM's shared memory (float32 rows of 256)
     constexpr int WIDE_STAGES = DecodeTile<EPL * (int)sizeof(T) / 4, 16, 2>::SMEM <= 200 * 1024 ? 2 : 1;

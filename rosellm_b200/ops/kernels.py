@@ -1013,6 +1013,8 @@ def attention(q, pool, block_table, q_start, kv_len, slots, out, *, n_heads: int
     sixteen warps instead of four (few requests, so that their keys need no split), or eight where
     the device would take a second round over blocks of sixteen (``decode_sixteen``: sixteen all the same).
     ``prefill_path`` (for tests): ``"tc"`` or ``"mma"`` forces the kernel of the prompt portions.
+    With ``n_splits`` of 2 to 8, ``decode_wide`` and no ``part_o`` the parts of a request's keys are the blocks of a
+    cluster, of eight warps each, and meet there.
     ``old_keys_settled``: the caller promises that the block table and the keys and values below
     each decoded request's last position were written by work that was over before the kernel
     preceding this call on the stream began (true inside the engine, whose steps are separated
@@ -1030,7 +1032,7 @@ def attention(q, pool, block_table, q_start, kv_len, slots, out, *, n_heads: int
         raise KernelError(f"attention: {n_heads} heads are not a multiple of {n_kv} key/value heads")
     if q.shape[1] != n_heads * dh or q.stride(1) != 1 or out.stride(1) != 1:
         raise KernelError("attention: q does not fit heads * head size")
-    if n_splits > 1:
+    if n_splits > 1 and not (part_o is None and n_splits <= 8 and decode_wide):
         need = n_decode * n_heads * n_splits
         if part_o is None or part_ml is None or part_o.numel() < need * dh or part_ml.numel() < need * 2:
             raise KernelError("attention: scratch for the split partial results is too small")

@@ -408,6 +408,18 @@ class CausalSelfAttention(Part):
         units = n_decode * self.num_heads
         sms = K.sm_count()
         if units <= 2 * sms:
+            # Parts of up to eight are the blocks of a cluster (eight warps each).  Measured on B200 with heads of 64 in
+            # bfloat16, us, whole (sixteen warps a block, or eight) / in parts: 25 heads of one request, 544 keys 5.3 / 4.2, 900
+            # 7.0 / 4.6, four requests of 12 heads 5.7 / 5.1 and 8.5 / 6.4 (six parts); 200 heads, 320 keys 7.8 / 7.2, 544
+            # 11.7 / 9.4, 900 16.9 / 13.3 (two); 96 to 144 heads stand at one block an SM each and gain nothing
+            # (6.4 / 6.8, 900 keys 8.7 / 8.7), nor do 288 (13.0 / 15.1).  Up to 256 keys the kernel takes them whole.
+            if span >= 300 and 2 * self.head_dim * (2 if act_dtype == torch.bfloat16 else 4) <= 512 and span <= 8192:
+                if units <= sms // 4:
+                    return max(3, min(8, span // 100)), True
+                if units <= sms * 9 // 20 and span >= 500:
+                    return 6, True
+                if sms < units <= sms * 3 // 2:
+                    return 2, True
             return max(1, min(span // 1024, 2 * sms // units, 32)), True   # up to four rounds a block
         # Narrow blocks: a few fit on an SM (shared memory); where they do not all run at once the
         # kernel takes its dense form (twice as many an SM, each slower), and what is still left
@@ -528,7 +540,7 @@ class CausalSelfAttention(Part):
         o = ctx.workspace.get("attn_out", (n, self.q_width), ctx.act_dtype)
         splits, wide = ctx.extras.get("decode_plan") or self.decode_plan(ctx)
         part_o = part_ml = None
-        if splits > 1:
+        if splits > 8 or (splits > 1 and not wide):
             rows = ctx.n_decode * self.num_heads * splits
             part_o = ctx.workspace.get("attn_part_o", (rows, self.head_dim), torch.float32)
             part_ml = ctx.workspace.get("attn_part_ml", (rows, 2), torch.float32)
