@@ -501,6 +501,10 @@ static void launch_rows_mma(const __nv_bfloat16* a, long lda, const NormArgs& no
 #undef RL_MMA
 }
 
+// A head of long rows leaves a block of the bulk-fed kernel room for few warps, each with two buffers of eight rows: below four of
+// them the ring-fed kernel is ahead (32000 x 2048, 8 rows, two warps: 42.6 us, the ring-fed kernel 67 MB of such rows in 12.9).
+constexpr int BULK_WARPS = 4;
+
 }  // namespace rl
 
 // bfloat16 A [M <= 64, K] (row stride lda) and W [N, K]; out bfloat16 or float32 [M, N].
@@ -528,10 +532,11 @@ RL_EXPORT int rl_gemm_rows_bf16(int out_dtype, const void* A, long lda, const vo
                    kv_q_width, kv_width, kv_head_dim, kv_page_size, kv_heads, kv_max_pos, status};
   const __nv_bfloat16* a = (const __nv_bfloat16*)A;
   const __nv_bfloat16* w = (const __nv_bfloat16*)W;
+  const rl::ring::Args r{a, lda, norm, w, bias, out, ldo, M, N, K, act, residual, out_dtype == RL_F32 ? 1 : 0, kv, status, rl::SampleArgs{}};
   // a very wide float32 output of few rows (a head): the weights by bulk copies into shared memory
   if (out_dtype == RL_F32 && !residual && act == RL_ACT_NONE && kv_pool == nullptr && status != nullptr) {
     const int warps = rl::bulk::plan_warps(M, N, K, norm_x != nullptr, rl::rows_sm_count());
-    if (warps > 0) {
+    if (warps >= rl::BULK_WARPS || (warps > 0 && !rl::ring::takes(r))) {
       const cudaError_t e = norm_x != nullptr
           ? rl::bulk::launch<true>(warps, rl::rows_sm_count(), a, lda, norm, w, bias, (float*)out, ldo, M, N, K,
                                    rl::SampleArgs{}, status, stream)
@@ -540,10 +545,7 @@ RL_EXPORT int rl_gemm_rows_bf16(int out_dtype, const void* A, long lda, const vo
       return e == cudaSuccess ? 0 : (int)e;
     }
   }
-  if (out_dtype == RL_F32 || out_dtype == RL_BF16) {
-    const rl::ring::Args r{a, lda, norm, w, bias, out, ldo, M, N, K, act, residual, out_dtype == RL_F32 ? 1 : 0, kv, status, rl::SampleArgs{}};
-    if (rl::ring::takes(r)) return rl::ring::run(r, stream);
-  }
+  if ((out_dtype == RL_F32 || out_dtype == RL_BF16) && rl::ring::takes(r)) return rl::ring::run(r, stream);
 #define RL_ROWS_MT(MT)                                                                                        \
   do {                                                                                                        \
     if (out_dtype == RL_F32)                                                                                  \
@@ -588,17 +590,17 @@ RL_EXPORT int rl_gemm_rows_bf16_sample(const void* A, long lda, const void* W, c
   const rl::SampleArgs sample{out_ids, temperature, seeds, counters, best, ticket, host_ring, ring_stride, ring_step, soft_cap};
   const __nv_bfloat16* a = (const __nv_bfloat16*)A;
   const __nv_bfloat16* w = (const __nv_bfloat16*)W;
+  // the kernel that gives such a product's logits (rl_gemm_rows_bf16)
+  const rl::ring::Args r{a, lda, norm, w, bias, nullptr, 0, M, N, K, RL_ACT_NONE, 0, 1, kv, status, sample};
   if (status != nullptr) {
     const int warps = rl::bulk::plan_warps(M, N, K, norm_x != nullptr, rl::rows_sm_count());
-    if (warps > 0) {
+    if (warps >= rl::BULK_WARPS || (warps > 0 && !rl::ring::takes(r))) {
       const cudaError_t e = norm_x != nullptr
           ? rl::bulk::launch<true>(warps, rl::rows_sm_count(), a, lda, norm, w, bias, nullptr, 0, M, N, K, sample, status, stream)
           : rl::bulk::launch<false>(warps, rl::rows_sm_count(), a, lda, norm, w, bias, nullptr, 0, M, N, K, sample, status, stream);
       return e == cudaSuccess ? 0 : (int)e;
     }
   }
-  // the kernel that gives such a product's logits (rl_gemm_rows_bf16)
-  const rl::ring::Args r{a, lda, norm, w, bias, nullptr, 0, M, N, K, RL_ACT_NONE, 0, 1, kv, status, sample};
   if (rl::ring::takes(r)) return rl::ring::run(r, stream);
   if (M <= 16)
     rl::launch_rows_mma<float, 1>(a, lda, norm, w, bias, nullptr, 0, M, N, K, RL_ACT_NONE, 0, kv, stream, sample);
