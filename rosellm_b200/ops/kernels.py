@@ -438,13 +438,32 @@ def bf16_path(rows: int, n_out: int, k: int, *, residual: bool = False, out_f32:
         logits = head or (out_f32 and not residual and k < 2048)
         if logits and rounds:
             return "mma" if rows <= 32 and not (rounds == 2 and n_out > 8192 and k >= 1024) else "smem"
-        clustered = rows > 32 and k >= 2048 and bool(_lib().rl_gemm_tc_rows_fits(rows, n_out, k))
+        clustered = rows > 32 and k >= 2048 and _parts_held_whole(rows, k)
         if not narrow and not logits and (rounds or residual or not _few_weights(rows, n_out, k, clustered)):
             return "tc"
         return "tcr" if clustered else "mma"
-    if rows <= 128 and narrow and _lib().rl_gemm_tc_rows_fits(rows, n_out, k):
+    if rows <= 128 and narrow and _parts_held_whole(rows, k):
         return "tcr"
     return "tc"
+
+
+def _parts_held_whole(rows: int, k: int) -> bool:
+    """Whether eight blocks hold their parts of K, 64 elements of 128 columns and of all rows at a time, and the float32 sums in
+    200 KB each: the sizes up to which the clustered kernel was measured against the others for narrow outputs."""
+    padded, parts = -(-rows // 16) * 16, -(-k // (64 * 8))
+    return parts * (128 + padded) * 128 + padded * 512 + 2100 + 8 * parts <= 200 * 1024
+
+
+def clustered_is_ahead(rows: int, n_out: int, k: int, *, out_f32: bool = False, residual: bool = False) -> bool:
+    """Whether a product that ``bf16_path`` gives to shared memory or to tiles runs on the clustered tcgen05 kernel
+    instead (csrc/gemm_tc_rows.cu), by what it takes between the other kernels of a layer (GPT-2 of three sizes at 64 rows, us, the
+    other kernel / clustered): 3072 x 1024 7.4 / 6.7, 4096 x 1024 6.9 / 6.3, 4800 x 1600 9.0 / 8.7, 6400 x 1600 9.6 / 8.1, += 1600 x
+    6400 11.5 / 10.9.  Smaller products lose what their clusters wait for places that the kernels ahead leave: 2304 x 768 5.6 / 6.8, += 768 x
+    768 5.2 / 6.4, += 1600 x 1600 6.0 / 7.6, though in chains of their own they gain as well (3072 x 768 6.2 / 4.8).  Float32 outputs that
+    are not added to, logits among them, stay with the kernels that tokens are drawn from."""
+    if not 17 <= rows <= 64 or k > 8192 or (out_f32 and not residual) or -(-n_out // 64) >= sm_count():
+        return False
+    return n_out >= 1600 and k >= 6400 if residual else n_out >= 3072 and k >= 1024
 
 
 def _few_weights(rows: int, n_out: int, k: int, clustered: bool) -> bool:
@@ -574,6 +593,9 @@ def linear(a, weight, bias, out, *, act: int = ACT_NONE, residual: bool = False,
         if bf16:
             path = bf16_path(m, n, k, residual=residual, out_f32=out.dtype == torch.float32, act=act, to_cache=kv is not None,
                              head=head)
+            if path in ("smem", "tc") and not head and clustered_is_ahead(m, n, k, out_f32=out.dtype == torch.float32,
+                                                                          residual=residual):
+                path = "tcr"
         else:
             path = "rows" if m <= ROWS_STREAMING_LIMIT else "tile"
     if head and path == "tc" and not splits:

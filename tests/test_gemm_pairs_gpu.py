@@ -1,4 +1,5 @@
-"""tcgen05 products on pairs of SMs (tiles of 256 rows over two blocks)."""
+"""tcgen05 products on pairs of SMs (tiles of 256 rows over two blocks), and the clustered kernel of few rows whose ring is
+shorter than its part of K."""
 import pytest
 import torch
 
@@ -52,3 +53,34 @@ def test_chosen(m, n, k):
     K.linear(a, w, b, x, residual=True)
     _close(x, want, k)
     K.check_status(torch.device(DEV))
+
+
+# rows at the edges of the 16 that they are rounded up to; one block a cluster to eight, parts of K longer than the ring, the last
+# one short; an output that ends inside a tile
+@pytest.mark.parametrize("m", [1, 16, 17, 33, 64, 65, 128])
+@pytest.mark.parametrize("n,k", [(200, 104), (768, 768), (3072, 1024), (130, 6400), (6400, 200), (1000, 1608)])
+def test_rows_in_clusters(m, n, k):
+    a, w, b = _data(m, n, k)
+    ref = a.double() @ w.double().T + b.double()
+    out = torch.full((m, n), float("nan"), device=DEV)
+    K.linear(a, w, b, out, path="tcr")
+    _close(out, ref, k)
+    again = torch.empty_like(out)
+    K.linear(a, w, b, again, path="tcr")
+    assert torch.equal(again, out)
+    x = torch.randn(m, n, device=DEV)
+    want = x.double() + ref
+    K.linear(a, w, b, x, residual=True, path="tcr")
+    _close(x, want, k)
+    half = torch.full((m, n), float("nan"), dtype=torch.bfloat16, device=DEV)
+    K.linear(a, w, b, half, path="tcr")
+    assert torch.equal(half, out.bfloat16())
+    K.check_status(torch.device(DEV))
+
+
+@pytest.mark.parametrize("rows,n,k,kw,clustered", [
+    (16, 3072, 1024, {}, False), (17, 3072, 1024, {}, True), (64, 3072, 1024, {}, True), (65, 3072, 1024, {}, False), (64, 3071, 1024, {}, False),
+    (64, 3072, 1023, {}, False), (64, 4800, 1600, dict(out_f32=True), False), (64, 1600, 6400, dict(residual=True, out_f32=True), True),
+    (64, 1600, 6399, dict(residual=True, out_f32=True), False), (64, 4800, 8256, {}, False), (64, 9472, 1600, {}, False)])
+def test_which_products_go_to_clusters(rows, n, k, kw, clustered):
+    assert K.clustered_is_ahead(rows, n, k, **kw) == clustered
