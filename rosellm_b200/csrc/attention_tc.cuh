@@ -9,21 +9,23 @@
 //   warp 0     looks up the pages of each tile, a lane a page, and issues their TMA loads (a page
 //              of one head is a contiguous [page size x 64] piece of the pool: one box a page)
 //              for keys and values into a ring of three stages, and the load of the queries;
-//   warp 1     allocates tensor memory (two score tiles of 128 columns, two P V tiles of 64); one
-//              lane issues S = Q K^T (M=128, N=128, four steps of K=16) for the next tile as
-//              soon as its keys have arrived, and P V (M=128, N=64, eight steps; V is read
-//              as it lies in the cache, head dimension contiguous: the MN-major form of the B
+//   warp 1     allocates tensor memory (two score tiles of 128 columns, two P V tiles of 64); the
+//              whole warp walks, one lane issues S = Q K^T (M=128, N=128, four steps of K=16) for the
+//              next tile as soon as its keys have arrived, and P V (M=128, N=64, eight steps; V is
+//              read as it lies in the cache, head dimension contiguous: the MN-major form of the B
 //              operand) once the probabilities of the tile are in shared memory;
-//   warps 2-17 softmax, four threads a query row (one for each quarter of a tile's keys and of
-//              the output's columns; tensor memory lets a warp read only the lanes of its
-//              quarter, so warps w, w + 4, w + 8 and w + 12 share rows): read the scores from
-//              tensor memory, mask by
-//              position, agree on the row's maximum through shared memory, update the running
+//   warps 2-17 softmax, two groups of eight warps on alternate key tiles, two threads a query row
+//              (one for each half of a tile's keys and of the output's columns; tensor memory lets a
+//              warp read only the lanes of its quarter): read the scores from tensor memory, mask by
+//              position, agree on the row's maximum through shared memory, update the group's
 //              maximum and sum in float32, write the probabilities as bfloat16 in the swizzled
-//              K-major layout the second product reads, and, once the next tile's
-//              probabilities are handed over, add each tile's P V (read back from tensor
-//              memory) to the row's output, which they keep in registers and rescale there
-//              when the maximum rose.
+//              K-major layout the second product reads, and, at the group's next tile, add
+//              the P V (read back from tensor memory) to the row's output, which they keep in
+//              registers and rescale there when the maximum rose.  At a turn's end the two
+//              groups' outputs are added up through shared memory.
+// What bounds it is the softmax's chain (a tile: scores ready, maximum 0.3 us, exponentials 1 us, product 0.4) and its
+// arithmetic, not the tensor cores; hence the two chains side by side, 16 columns of scores on their way while the 16 before are
+// worked on, and instructions that take two float32 values or three.
 // Keys past the request's last visible key may hold anything (a partly filled page): their
 // scores are masked by index, and their value rows are zeroed in shared memory before the
 // second product, so that 0 * value stays 0.  Every wait on a barrier is bounded.
@@ -45,7 +47,7 @@ constexpr int ATT_P_BYTES = ATT_Q * ATT_KV * 2;        // 32 KB: two K blocks of
 constexpr int ATT_STAGES = 3;                          // tiles of keys and values in shared memory
 // The probabilities lie in two buffers: those of tile g are written while the P V of tile g - 1 may still read its own (only the
 // P V of g - 2 has been waited for by then).  The block has its SM to itself either way.
-constexpr int ATT_SMEM = 2 * ATT_Q_BYTES + ATT_STAGES * 2 * ATT_KV_BYTES + 2 * ATT_P_BYTES + 128 + 3 * 4 * ATT_Q * 4 + 1024;
+constexpr int ATT_SMEM = 2 * ATT_Q_BYTES + ATT_STAGES * 2 * ATT_KV_BYTES + 2 * ATT_P_BYTES + 128 + 13 * ATT_Q * 4 + 1024;
 
 // Instruction descriptor of kind::f16, bfloat16 x bfloat16 -> float32, M = 128; b_mn: the B
 // operand has its N dimension contiguous in shared memory (values as they lie in the cache).
@@ -85,6 +87,36 @@ __device__ __forceinline__ bool att_wait(uint32_t bar, uint32_t parity, volatile
   }
 }
 
+// Waits for tensor-memory loads, naming the registers that the last one fills: what is computed from them cannot move ahead.
+__device__ __forceinline__ void att_loads_wait(uint32_t (&r)[16]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]),
+                 "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+               :
+               : "memory");
+}
+__device__ __forceinline__ float att_max3(float a, float b, float c) {
+  float m;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(m) : "f"(a), "f"(b), "f"(c));
+  return m;
+}
+// Two float32 values as one register pair, for the instructions that take two at a time.
+__device__ __forceinline__ uint64_t att_pair(float lo, float hi) {
+  return (uint64_t)__float_as_uint(lo) | ((uint64_t)__float_as_uint(hi) << 32);
+}
+__device__ __forceinline__ uint64_t att_fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t att_add2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ float att_lo(uint64_t v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float att_hi(uint64_t v) { return __uint_as_float((uint32_t)(v >> 32)); }
+
 __device__ __forceinline__ float att_ex2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -117,12 +149,13 @@ __global__ __launch_bounds__(ATT_THREADS, 1) void attn_tc_kernel(const __grid_co
   const uint32_t p_addr = kv_addr + ATT_STAGES * 2 * ATT_KV_BYTES;   // [2 tiles][2 K blocks][128 rows][128 bytes]
   const uint32_t bar_base = p_addr + 2 * ATT_P_BYTES;
   const uint32_t q_full0 = bar_base, kv_full0 = bar_base + 16, kv_empty0 = bar_base + 40, s_full0 = bar_base + 64,
-                 p_ready = bar_base + 80, pv_full0 = bar_base + 88;
+                 p_ready0 = bar_base + 80, pv_full0 = bar_base + 96;
   uint8_t* after_p = smem + 2 * ATT_Q_BYTES + ATT_STAGES * 2 * ATT_KV_BYTES + 2 * ATT_P_BYTES;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(after_p + 112);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // the warp's number as a value that the compiler knows to be the same in all lanes
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int tile = singly ? gridDim.y - 1 - blockIdx.y : gridDim.x - 1 - blockIdx.x;
   const int req = tiles[2 * tile], entry_t0 = tiles[2 * tile + 1];
   if (entry_t0 % ATT_Q != 0) return;  // the second half of a piece
@@ -156,8 +189,8 @@ __global__ __launch_bounds__(ATT_THREADS, 1) void attn_tc_kernel(const __grid_co
     for (int s = 0; s < 2; ++s) {
       mbar_init(s_full0 + 8 * s, 1);
       mbar_init(pv_full0 + 8 * s, 1);
+      mbar_init(p_ready0 + 8 * s, ATT_SOFTMAX_THREADS / 64);  // one arrival a warp of the tile's group
     }
-    mbar_init(p_ready, ATT_SOFTMAX_THREADS);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -171,10 +204,18 @@ __global__ __launch_bounds__(ATT_THREADS, 1) void attn_tc_kernel(const __grid_co
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   const uint32_t tmem_pv = tmem_base + 256u;  // two tiles of 64 columns
   RL_PHASE(1);
-  pdl_begin();
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  // the pages of the first tile (the block table is written by no kernel of a step): looked up before the wait
+  const int* bt = p.block_table + (size_t)slot * p.bt_stride;
+  const int pages_per_tile = ATT_KV / p.page_size;
+  auto pages_of_tile = [&](int kv_hi, int t) { return min(pages_per_tile, (kv_hi - t * ATT_KV + p.page_size - 1) / p.page_size); };
+  auto entry_of_tile = [&](int kv_hi, int t) { return lane < pages_of_tile(kv_hi, t) ? bt[t * pages_per_tile + lane] : 0; };
+  int next_page = 0;
+  if (warp == 0) next_page = entry_of_tile(queries_of(0).kv_hi, 0);
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   RL_PHASE(2);
 
   // Key tiles are counted through both turns (g): stages, score and P V buffers and the phases
@@ -190,12 +231,7 @@ __global__ __launch_bounds__(ATT_THREADS, 1) void attn_tc_kernel(const __grid_co
         tma_load_2d(q_addr + turn * ATT_Q_BYTES, &map_q, q_full0 + 8 * turn, h * ATT_DH, qs + queries_of(turn).t0);
       }
     }
-    const int* bt = p.block_table + (size_t)slot * p.bt_stride;
-    const int pages_per_tile = ATT_KV / p.page_size;
     const uint32_t page_bytes = (uint32_t)p.page_size * ATT_DH * 2;
-    auto pages_of_tile = [&](int kv_hi, int t) { return min(pages_per_tile, (kv_hi - t * ATT_KV + p.page_size - 1) / p.page_size); };
-    auto entry_of_tile = [&](int kv_hi, int t) { return lane < pages_of_tile(kv_hi, t) ? bt[t * pages_per_tile + lane] : 0; };
-    int next_page = entry_of_tile(queries_of(0).kv_hi, 0);
     bool ok = true;
     int g = 0;
     for (int turn = 0; turn < n_turns && ok; ++turn) {
@@ -230,156 +266,191 @@ __global__ __launch_bounds__(ATT_THREADS, 1) void attn_tc_kernel(const __grid_co
       for (int k = max(0, g - ATT_STAGES); k < g; ++k) mbar_wait_quiet(kv_full0 + 8 * (k % ATT_STAGES), (k / ATT_STAGES) & 1u);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc_s = att_instr_desc(ATT_KV, false);
-      constexpr uint32_t idesc_o = att_instr_desc(ATT_DH, true);
-      const int n_first = queries_of(0).n_tiles;
-      const int n_all = n_first + (n_turns > 1 ? queries_of(1).n_tiles : 0);
-      bool ok = true;
-      // S = Q K^T of tile g (of the turn it falls in), once its keys (and that turn's queries) have arrived
-      auto issue_s = [&](int g) {
-        const int turn = g < n_first ? 0 : 1;
-        if (g == 0 || g == n_first) ok = att_wait(q_full0 + 8 * turn, 0u, abort_flag, p.status, 1);
-        if (ok) ok = att_wait(kv_full0 + 8 * (g % ATT_STAGES), (g / ATT_STAGES) & 1u, abort_flag, p.status, 2);
-        if (!ok) return;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t k_addr = kv_addr + (uint32_t)(g % ATT_STAGES) * 2u * ATT_KV_BYTES;
-        const uint32_t qa = q_addr + (uint32_t)turn * ATT_Q_BYTES;
+    // The whole warp walks, with values that are the same in all lanes (a product's operands are taken from uniform
+    // registers); one lane issues.
+    constexpr uint32_t idesc_s = att_instr_desc(ATT_KV, false);
+    constexpr uint32_t idesc_o = att_instr_desc(ATT_DH, true);
+    const int n_first = queries_of(0).n_tiles;
+    const int n_all = n_first + (n_turns > 1 ? queries_of(1).n_tiles : 0);
+    const uint64_t q_desc = smem_desc(q_addr), k_desc = smem_desc(kv_addr), p_desc = smem_desc(p_addr),
+                   v_desc = smem_desc_mn(kv_addr + ATT_KV_BYTES);
+    bool ok = true;
+    auto wait = [&](uint32_t bar, uint32_t parity, int which) {
+      return __all_sync(0xffffffffu, att_wait(bar, parity, abort_flag, p.status, which));
+    };
+    // S = Q K^T of tile g (of the turn it falls in), once its keys (and that turn's queries) have arrived
+    auto issue_s = [&](int g) {
+      const int turn = g < n_first ? 0 : 1;
+      if (g == 0 || g == n_first) ok = wait(q_full0 + 8 * turn, 0u, 1);
+      if (ok) ok = wait(kv_full0 + 8 * (g % ATT_STAGES), (g / ATT_STAGES) & 1u, 2);
+      if (!ok) return;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      // descriptors count 16-byte units; a K step of 32 bytes is +2
+      const uint64_t kd = k_desc + (uint64_t)((g % ATT_STAGES) * (2 * ATT_KV_BYTES >> 4)), qd = q_desc + (uint64_t)(turn * (ATT_Q_BYTES >> 4));
+      if (elect_one()) {
 #pragma unroll
         for (int k = 0; k < ATT_DH / 16; ++k)
-          mma_f16(tmem_base + (uint32_t)(g & 1) * 128u, smem_desc(qa + k * 32), smem_desc(k_addr + k * 32), idesc_s,
-                  k != 0 ? 1u : 0u);
+          mma_f16(tmem_base + (uint32_t)(g & 1) * 128u, qd + 2 * k, kd + 2 * k, idesc_s, k != 0 ? 1u : 0u);
         mma_commit(s_full0 + 8 * (g & 1));
-      };
-      if (n_all > 0) issue_s(0);
-      RL_PHASE_OF(6, 32);
-      for (int g = 0; g < n_all && ok; ++g) {
-        // the scores of the next tile, while the softmax works on this one (its place was last
-        // read for tile g - 1, whose probabilities have been waited for)
-        if (g + 1 < n_all) {
-          issue_s(g + 1);
-          if (!ok) break;
-        }
-        ok = att_wait(p_ready, g & 1u, abort_flag, p.status, 3);
+      }
+      __syncwarp();
+    };
+    if (n_all > 0) issue_s(0);
+    RL_PHASE_OF(6, 32);
+    for (int g = 0; g < n_all && ok; ++g) {
+      // the scores of the next tile, while the softmax works on this one (its place was last
+      // read for tile g - 1, whose probabilities have been waited for)
+      if (g + 1 < n_all) {
+        issue_s(g + 1);
         if (!ok) break;
-        if (g < 6) RL_PHASE_OF(10 + g, 32);
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t v_addr = kv_addr + (uint32_t)(g % ATT_STAGES) * 2u * ATT_KV_BYTES + ATT_KV_BYTES;
+      }
+      ok = wait(p_ready0 + 8 * (g & 1), (g >> 1) & 1u, 3);
+      if (!ok) break;
+      if (g < 6) RL_PHASE_OF(10 + g, 32);
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint64_t vd = v_desc + (uint64_t)((g % ATT_STAGES) * (2 * ATT_KV_BYTES >> 4)), pd = p_desc + (uint64_t)((g & 1) * (ATT_P_BYTES >> 4));
+      if (elect_one()) {
 #pragma unroll
         for (int k = 0; k < ATT_KV / 16; ++k)  // 16 keys a step: two groups of eight value rows
-          mma_f16(tmem_pv + (uint32_t)(g & 1) * 64u,
-                  smem_desc(p_addr + (uint32_t)(g & 1) * ATT_P_BYTES + (uint32_t)(k >> 2) * (ATT_Q * 128) + (k & 3) * 32),
-                  smem_desc_mn(v_addr + (uint32_t)k * 2048u), idesc_o, k != 0 ? 1u : 0u);
+          mma_f16(tmem_pv + (uint32_t)(g & 1) * 64u, pd + (uint64_t)((k >> 2) * (ATT_Q * 128 >> 4) + (k & 3) * 2),
+                  vd + (uint64_t)(k * (2048 >> 4)), idesc_o, k != 0 ? 1u : 0u);
         mma_commit(kv_empty0 + 8 * (g % ATT_STAGES));
         mma_commit(pv_full0 + 8 * (g & 1));
       }
+      __syncwarp();
     }
   } else {
-    // four threads a query row: warp w reads the tensor-memory lanes of its quarter (w % 4);
-    // `part` says which 32 keys of a tile and which 16 columns of the output are this thread's
-    const int quarter = warp & 3, part = (warp - 2) >> 2;
+    // Two groups of eight warps take the key tiles in turn, each with a running maximum, sum and output of its own, so that
+    // the chain of one tile (scores, maximum over the row, exponentials, probabilities to shared memory, their product) lies
+    // under the other's; a turn's two results are added up at its end.  In a group two threads share a query row: warp w reads the
+    // tensor-memory lanes of its quarter (w % 4); `half` says which 64 keys of a tile and which 32 columns of the output are
+    // this thread's.  (With all sixteen warps on one tile the 2 x 1024 tokens of GPT-2 124M took 22.6 us a layer.)
+    const int quarter = warp & 3, group = (warp - 2) >> 3, half = ((warp - 2) >> 2) & 1;
     const int row = quarter * 32 + lane;
-    const int st = threadIdx.x - 64;  // 0..511 among the softmax threads
+    const int st = (threadIdx.x - 64) & (ATT_SOFTMAX_THREADS / 2 - 1);  // 0..255 in the group
     const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
     const float sl2 = p.scale * 1.4426950408889634f;  // scores in units of log 2
-    float* mx_s = reinterpret_cast<float*>(after_p + 128);  // [2 tiles][4 parts][128], then the sums [4 parts][128]
-    float* sum_s = mx_s + 2 * 4 * ATT_Q;
-    // this thread's 32 probabilities of a tile: 64 bytes of the row in K block part / 2 (of the even tiles' buffer)
-    uint8_t* p_row = smem + 2 * ATT_Q_BYTES + ATT_STAGES * 2 * ATT_KV_BYTES + (size_t)(part >> 1) * (ATT_Q * 128) + (size_t)row * 128;
+    float* mx_s = reinterpret_cast<float*>(after_p + 128);  // maxima [2 groups][2 tiles][2 halves][128]
+    float* l_s = mx_s + 8 * ATT_Q;                           // at a turn's end: sums [2 groups][2 halves][128], then
+    float* m_s = l_s + 4 * ATT_Q;                            // the second group's maxima [128]
+    // this thread's 64 probabilities of a tile: the row's 128 bytes in K block `half` of the group's buffer
+    uint8_t* p_row = smem + 2 * ATT_Q_BYTES + ATT_STAGES * 2 * ATT_KV_BYTES + (size_t)group * ATT_P_BYTES + (size_t)half * (ATT_Q * 128) +
+                     (size_t)row * 128;
+    // the second group's outputs at a turn's end, in the place of its probabilities: [16 pieces of four columns][128 rows] float4
+    float4* o_s = reinterpret_cast<float4*>(smem + 2 * ATT_Q_BYTES + ATT_STAGES * 2 * ATT_KV_BYTES + ATT_P_BYTES);
     const int sw = row & 7;  // swizzle of 16-byte chunks
-    auto row_sync = [&]() { asm volatile("bar.sync 1, 512;" ::: "memory"); };
-    float o[ATT_DH / 4];
-    // adds tile g's P V (this thread's 16 columns) to the row's output, after its product has finished
+    auto group_sync = [&]() { asm volatile("bar.sync %0, 256;" ::"r"(1 + group) : "memory"); };
+    auto all_sync = [&]() { asm volatile("bar.sync 3, 512;" ::: "memory"); };
+    float o[ATT_DH / 2];
+    // adds tile g's P V (this thread's 32 columns) to the row's output, after its product has finished
     auto take_pv = [&](int g) -> bool {
-      const bool arrived = __all_sync(0xffffffffu, att_wait(pv_full0 + 8 * (g & 1), (g >> 1) & 1u, abort_flag, p.status, 5));
+      const bool arrived = __all_sync(0xffffffffu, att_wait(pv_full0 + 8 * group, (g >> 1) & 1u, abort_flag, p.status, 5));
       if (!arrived) return false;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      uint32_t r[16];
-      tmem_load16(tmem_pv + lane_base + (uint32_t)(g & 1) * 64u + (uint32_t)part * 16u, r);
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-      for (int i = 0; i < 16; ++i) o[i] += __uint_as_float(r[i]);
+      for (int c = 0; c < 32; c += 16) {
+        uint32_t r[16];
+        tmem_load16(tmem_pv + lane_base + (uint32_t)group * 64u + (uint32_t)half * 32u + (uint32_t)c, r);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int i = 0; i < 16; ++i) o[c + i] += __uint_as_float(r[i]);
+      }
       return true;
     };
-    // Every softmax thread passes the row barrier once a tile and once at the end of a turn, also
-    // after a wait gave up (ok false): the work is skipped then, the barrier never.
+    // Every softmax thread passes its group's barrier once a tile of the group and the common one twice a turn, also
+    // after a wait gave up (ok false): the work is skipped then, the barriers never.
     bool ok = true;
-    int g = 0;
+    int g0 = 0;  // tiles of the turns before
     for (int turn = 0; turn < n_turns; ++turn) {
       const AttQueries q = queries_of(turn);
       const bool row_ok = row < q.rows;
       const int qpos = q.first_pos + row;
       float m = -CUDART_INF_F, l = 0.f;  // l: the sum over this thread's keys
 #pragma unroll
-      for (int d = 0; d < ATT_DH / 4; ++d) o[d] = 0.f;
-      for (int t = 0; t < q.n_tiles; ++t, ++g) {
-        const int kt = t * ATT_KV + part * 32;  // first key of this thread's quarter of the tile
-        if (ok) ok = __all_sync(0xffffffffu, att_wait(s_full0 + 8 * (g & 1), (g >> 1) & 1u, abort_flag, p.status, 4));
+      for (int d = 0; d < ATT_DH / 2; ++d) o[d] = 0.f;
+      int last = -1;  // the group's last tile of this turn
+      for (int t = (group - g0) & 1; t < q.n_tiles; t += 2) {
+        const int g = g0 + t;
+        const int kt = t * ATT_KV + half * 64;  // first key of this thread's half of the tile
+        if (ok) ok = __all_sync(0xffffffffu, att_wait(s_full0 + 8 * group, (g >> 1) & 1u, abort_flag, p.status, 4));
         if (g < 4) RL_PHASE_OF(16 + 4 * g, 64);
-        const uint32_t s_addr = tmem_base + lane_base + (uint32_t)(g & 1) * 128u + (uint32_t)part * 32u;
-        // keys of this quarter the query sees: [0, n_vis); the whole warp sees all of them in
-        // every tile but the last ones
-        const int n_vis = row_ok ? max(0, min(32, qpos - kt + 1)) : 0;
-        const bool all_vis = __all_sync(0xffffffffu, n_vis == 32);
+        const uint32_t s_addr = tmem_base + lane_base + (uint32_t)group * 128u + (uint32_t)half * 64u;
+        // keys of this half the query sees: [0, n_vis); the whole warp sees all of them in every tile but the last ones
+        const int n_vis = row_ok ? max(0, min(64, qpos - kt + 1)) : 0;
+        const bool all_vis = __all_sync(0xffffffffu, n_vis == 64);
         float mx = -CUDART_INF_F;
-        uint32_t r[32];  // the scores stay in registers between the maximum and the exponentials
         if (ok) {
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          tmem_load32(s_addr, r);
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          if (all_vis) {
-            // four chains of eight instead of one of thirty-two: each fmax waits for the one before it
-            float m4[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
+          // sixteen columns at a time, the next on their way while these are looked at
+          uint32_t r[2][16];
+          tmem_load16(s_addr, r[0]);
+          float m2[2] = {-CUDART_INF_F, -CUDART_INF_F};
 #pragma unroll
-            for (int i = 0; i < 32; ++i) m4[i & 3] = fmaxf(m4[i & 3], __uint_as_float(r[i]));
-            mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
-          } else {
+          for (int c = 0; c < 4; ++c) {
+            att_loads_wait(r[c & 1]);
+            if (c < 3) tmem_load16(s_addr + (uint32_t)(c + 1) * 16u, r[(c + 1) & 1]);
+            if (all_vis) {
 #pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (i < n_vis) mx = fmaxf(mx, __uint_as_float(r[i]));
+              for (int i = 0; i < 16; i += 2)
+                m2[(i >> 1) & 1] = att_max3(m2[(i >> 1) & 1], __uint_as_float(r[c & 1][i]), __uint_as_float(r[c & 1][i + 1]));
+            } else {
+#pragma unroll
+              for (int i = 0; i < 16; ++i)
+                if (c * 16 + i < n_vis) mx = fmaxf(mx, __uint_as_float(r[c & 1][i]));
+            }
           }
+          mx = fmaxf(mx, fmaxf(m2[0], m2[1]));
         }
-        // the row's maximum over the four quarters
-        float* mx_t = mx_s + (g & 1) * 4 * ATT_Q + row;
-        mx_t[part * ATT_Q] = mx;
-        row_sync();
-        mx = fmaxf(fmaxf(mx_t[0], mx_t[ATT_Q]), fmaxf(mx_t[2 * ATT_Q], mx_t[3 * ATT_Q]));
+        // the row's maximum over the two halves
+        float* mx_t = mx_s + (group * 2 + ((g >> 1) & 1)) * 2 * ATT_Q + row;  // (written again two of the group's tiles on)
+        mx_t[half * ATT_Q] = mx;
+        group_sync();
+        mx = fmaxf(mx_t[0], mx_t[ATT_Q]);
         if (g < 4) RL_PHASE_OF(17 + 4 * g, 64);
         const float m_new = fmaxf(m, mx * sl2);
         const float alpha = m_new == -CUDART_INF_F ? 1.f : att_ex2(m - m_new);
         const float neg_m = m_new == -CUDART_INF_F ? 0.f : -m_new;
-        if (!ok) continue;
-        // probabilities of this thread's 32 keys, as bfloat16, into the operand of the second product
-        float sum = 0.f;
-        uint32_t packed[16];
-        if (all_vis) {
-          float s4[4] = {0.f, 0.f, 0.f, 0.f};  // four chains of additions, as for the maximum
+        // the P V of the group's tile before: its probabilities lie where this tile's go
+        if (ok && last >= 0) {
+          ok = take_pv(last);
+          if (ok && __any_sync(0xffffffffu, alpha != 1.f)) {
 #pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            const float p0 = att_ex2(fmaf(__uint_as_float(r[2 * i]), sl2, neg_m));
-            const float p1 = att_ex2(fmaf(__uint_as_float(r[2 * i + 1]), sl2, neg_m));
-            s4[i & 3] += p0 + p1;
-            const __nv_bfloat162 hh = __floats2bfloat162_rn(p0, p1);
-            packed[i] = *reinterpret_cast<const uint32_t*>(&hh);
-          }
-          sum = (s4[0] + s4[1]) + (s4[2] + s4[3]);
-        } else {
-#pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            const float p0 = 2 * i < n_vis ? att_ex2(fmaf(__uint_as_float(r[2 * i]), sl2, neg_m)) : 0.f;
-            const float p1 = 2 * i + 1 < n_vis ? att_ex2(fmaf(__uint_as_float(r[2 * i + 1]), sl2, neg_m)) : 0.f;
-            sum += p0 + p1;
-            const __nv_bfloat162 hh = __floats2bfloat162_rn(p0, p1);
-            packed[i] = *reinterpret_cast<const uint32_t*>(&hh);
+            for (int d = 0; d < ATT_DH / 2; ++d) o[d] *= alpha;
           }
         }
-        // 32 keys = 64 bytes = four 16-byte chunks of the row: the first or the second half of it
+        last = g;
+        if (!ok) continue;
+        // probabilities of this thread's 64 keys, as bfloat16, into the operand of the second product (the scores are read again:
+        // held from the first reading, they would not fit the registers beside the output)
+        const uint64_t sl2_2 = att_pair(sl2, sl2), neg_m2 = att_pair(neg_m, neg_m);
+        uint64_t sum2[2] = {0ull, 0ull};  // two chains of pairs of sums
+        uint32_t r[2][16];
+        tmem_load16(s_addr, r[0]);
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-          const int chunk = (part & 1) * 4 + c;
-          *reinterpret_cast<uint4*>(p_row + (g & 1) * ATT_P_BYTES + ((chunk ^ sw) << 4)) =
-              make_uint4(packed[4 * c], packed[4 * c + 1], packed[4 * c + 2], packed[4 * c + 3]);
+          att_loads_wait(r[c & 1]);
+          if (c < 3) tmem_load16(s_addr + (uint32_t)(c + 1) * 16u, r[(c + 1) & 1]);
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {  // eight keys = a 16-byte chunk of the row
+            uint32_t packed[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const int k = 8 * e + 2 * i;
+              const uint64_t x = att_fma2((uint64_t)r[c & 1][k] | ((uint64_t)r[c & 1][k + 1] << 32), sl2_2, neg_m2);
+              float p0 = att_ex2(att_lo(x)), p1 = att_ex2(att_hi(x));
+              if (!all_vis) {
+                if (c * 16 + k >= n_vis) p0 = 0.f;
+                if (c * 16 + k + 1 >= n_vis) p1 = 0.f;
+              }
+              sum2[i & 1] = att_add2(sum2[i & 1], att_pair(p0, p1));
+              const __nv_bfloat162 hh = __floats2bfloat162_rn(p0, p1);
+              packed[i] = *reinterpret_cast<const uint32_t*>(&hh);
+            }
+            *reinterpret_cast<uint4*>(p_row + (((c * 2 + e) ^ sw) << 4)) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+          }
         }
+        const uint64_t both = att_add2(sum2[0], sum2[1]);
+        const float sum = att_lo(both) + att_hi(both);
         l = l * alpha + sum;
         m = m_new;
         // value rows of keys no query of the turn sees: zero, so that 0 * value stays 0
@@ -388,45 +459,46 @@ __global__ __launch_bounds__(ATT_THREADS, 1) void attn_tc_kernel(const __grid_co
           // keys and values come under one barrier
           uint8_t* v_s = smem + 2 * ATT_Q_BYTES + (size_t)(g % ATT_STAGES) * 2 * ATT_KV_BYTES + ATT_KV_BYTES;
           const int first_bad = q.kv_hi - t * ATT_KV;
-          for (int i = st + first_bad * 8; i < ATT_KV * 8; i += ATT_SOFTMAX_THREADS)
+          for (int i = st + first_bad * 8; i < ATT_KV * 8; i += ATT_SOFTMAX_THREADS / 2)
             *reinterpret_cast<uint4*>(v_s + (size_t)i * 16) = make_uint4(0u, 0u, 0u, 0u);
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(p_ready) : "memory");
+        __syncwarp();
+        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(p_ready0 + 8 * group) : "memory");
         if (g < 4) RL_PHASE_OF(18 + 4 * g, 64);
-        // Only now the P V of the tile before (whose product ran while this tile's exponentials
-        // were taken: the second product waits for the probabilities, never the probabilities
-        // for the second product): add it, then bring the output to the new maximum.
-        if (t > 0) {
-          ok = take_pv(g - 1);
-          if (ok && __any_sync(0xffffffffu, alpha != 1.f)) {
-#pragma unroll
-            for (int d = 0; d < ATT_DH / 4; ++d) o[d] *= alpha;
-          }
-        }
-        if (g < 4) RL_PHASE_OF(19 + 4 * g, 64);
       }
-      if (ok && q.n_tiles > 0) ok = take_pv(g - 1);
+      g0 += q.n_tiles;
+      if (ok && last >= 0) ok = take_pv(last);
       if (turn == 0) RL_PHASE_OF(7, 64);
-      // the row's sum over the four quarters (every softmax thread comes here, also after a wait gave up)
-      sum_s[part * ATT_Q + row] = l;
-      row_sync();
-      l = (sum_s[row] + sum_s[ATT_Q + row]) + (sum_s[2 * ATT_Q + row] + sum_s[3 * ATT_Q + row]);
-      if (ok && row_ok) {
-        const float inv = l > 0.f ? 1.0f / l : 0.f;
-        __nv_bfloat16* out = (__nv_bfloat16*)p.out + (size_t)(qs + q.t0 + row) * p.out_stride + h * ATT_DH + part * 16;
+      // the turn's end: the second group's outputs, maxima and sums to shared memory, the first group adds its own
+      l_s[(group * 2 + half) * ATT_Q + row] = l;
+      if (group == 1) {
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          uint32_t w[4];
+        for (int i = 0; i < 8; ++i) o_s[(half * 8 + i) * ATT_Q + row] = make_float4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
+        if (half == 0) m_s[row] = m;
+      }
+      all_sync();
+      if (group == 0 && ok && row_ok) {
+        const float m1 = m_s[row], top = fmaxf(m, m1);
+        const float f0 = m == -CUDART_INF_F ? 0.f : att_ex2(m - top), f1 = m1 == -CUDART_INF_F ? 0.f : att_ex2(m1 - top);
+        const float all = (l_s[row] + l_s[ATT_Q + row]) * f0 + (l_s[2 * ATT_Q + row] + l_s[3 * ATT_Q + row]) * f1;
+        const float inv = all > 0.f ? 1.0f / all : 0.f;
+        const float s0 = f0 * inv, s1 = f1 * inv;
+        __nv_bfloat16* out = (__nv_bfloat16*)p.out + (size_t)(qs + q.t0 + row) * p.out_stride + h * ATT_DH + half * 32;
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const __nv_bfloat162 hh = __floats2bfloat162_rn(o[8 * i + 2 * e] * inv, o[8 * i + 2 * e + 1] * inv);
-            w[e] = *reinterpret_cast<const uint32_t*>(&hh);
-          }
-          *reinterpret_cast<uint4*>(out + i * 8) = make_uint4(w[0], w[1], w[2], w[3]);
+        for (int i = 0; i < 4; ++i) {
+          const float4 u = o_s[(half * 8 + 2 * i) * ATT_Q + row], v = o_s[(half * 8 + 2 * i + 1) * ATT_Q + row];
+          const __nv_bfloat162 a0 = __floats2bfloat162_rn(o[8 * i] * s0 + u.x * s1, o[8 * i + 1] * s0 + u.y * s1);
+          const __nv_bfloat162 a1 = __floats2bfloat162_rn(o[8 * i + 2] * s0 + u.z * s1, o[8 * i + 3] * s0 + u.w * s1);
+          const __nv_bfloat162 a2 = __floats2bfloat162_rn(o[8 * i + 4] * s0 + v.x * s1, o[8 * i + 5] * s0 + v.y * s1);
+          const __nv_bfloat162 a3 = __floats2bfloat162_rn(o[8 * i + 6] * s0 + v.z * s1, o[8 * i + 7] * s0 + v.w * s1);
+          *reinterpret_cast<uint4*>(out + i * 8) =
+              make_uint4(*reinterpret_cast<const uint32_t*>(&a0), *reinterpret_cast<const uint32_t*>(&a1),
+                         *reinterpret_cast<const uint32_t*>(&a2), *reinterpret_cast<const uint32_t*>(&a3));
         }
       }
+      all_sync();  // the next turn's probabilities and maxima take their places
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -471,7 +543,10 @@ static inline int launch_attn_tc(const AttnParams& p, const int* tiles, int n_ti
     if (n_sms <= 0) n_sms = 1;
   }
   const long pairs = (long)(n_tiles + 3) / 4 * p.n_heads, places = (pairs + n_sms - 1) / n_sms * n_sms;
-  const bool singly = pairs > n_sms && 5 * places > 6 * pairs && n_tiles <= 65535;  // (the limit of a grid's second extent)
+  // Up to eight pieces to five SMs go singly as well: their longest, started first, end before a pair of a long and a short
+  // piece does (12 heads, 2 prompts of 1024: eight key tiles against nine).
+  const bool few = 2 * pairs * 5 <= 8 * n_sms;
+  const bool singly = (few || (pairs > n_sms && 5 * places > 6 * pairs)) && n_tiles <= 65535;  // (the limit of a grid's second extent)
   const dim3 grid = singly ? dim3(p.n_heads, n_tiles) : dim3(n_tiles, p.n_heads);
   launch_pdl_split(false, attn_tc_kernel, grid, ATT_THREADS, ATT_SMEM, stream, mq, mkv, p, tiles, singly ? 1 : 0);
   return 0;

@@ -336,10 +336,11 @@ def narrow_decode_blocks_at_once(head_dim: int, element_bytes: int, percent: int
 NARROW_FORMS = ((50, 1.0), (80, 1.15), (100, 1.3))
 
 
-# Longest context of a step from which prompt portions go to the tcgen05 attention kernel
-# (measured on B200, 12 heads of 64: 48 against 56 TFLOP/s at 256 tokens, 101 against 86 at
-# 1024, 131 against 96 at 2048).
-TC_ATTENTION_MIN_CONTEXT = 512
+# Longest context of a step from which prompt portions go to the tcgen05 attention kernel (measured on B200, whole prompt
+# steps, us, mma.sync / tcgen05: 12 heads, one prompt of 500 tokens 793 / 679, four of 380 to 500 1009 / 942, one of 300
+# 680 / 632, eight of 200 to 280 1062 / 1091; 16 heads, sixteen of 100 to 511 6612 / 6397; 25 heads, one of 400 4020 / 3716, eight
+# of 200 to 300 7063 / 7280, 32 of 63 to 511 36042 / 35702).
+TC_ATTENTION_MIN_CONTEXT = 320
 
 
 @register_part("mixer", "causal_self_attention")
