@@ -75,6 +75,15 @@ __global__ __launch_bounds__(128) void head_linear_mma_kernel(const __nv_bfloat1
   mma_tile<VEC>(
       acc, k_total, [&](int m) { return m0 + m < n_tokens ? in_h + (size_t)(m0 + m) * in_tok : nullptr; },
       [&](int n) { return n0 + n < n_total ? w_h + (size_t)(n0 + n) * w_n : nullptr; }, s);
+  if (gate == nullptr && (((uintptr_t)out & 3) | (uintptr_t)((out_tok | out_head | n_total) & 1)) == 0) {
+    // neighbouring columns together: single bfloat16 stores were what a prompt's product waited for
+    mma_for_each(acc, [&](int m, int n, int mi, int ni, int c) {
+      if ((c & 1) == 0 && m0 + m < n_tokens && n0 + n < n_total)
+        *reinterpret_cast<__nv_bfloat162*>(out + (size_t)(m0 + m) * out_tok + (size_t)h * out_head + n0 + n) =
+            __floats2bfloat162_rn(acc[mi][ni][c], acc[mi][ni][c + 1]);
+    });
+    return;
+  }
   mma_for_each(acc, [&](int m, int n, int mi, int ni, int c) {
     if (m0 + m < n_tokens && n0 + n < n_total) {
       float v = acc[mi][ni][c];

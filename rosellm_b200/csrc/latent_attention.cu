@@ -561,13 +561,13 @@ __device__ __forceinline__ float quad_sum(float v) {
   return v + __shfl_xor_sync(0xffffffffu, v, 2);
 }
 
-template <int NVW, int DVS, int NKT>
-__global__ __launch_bounds__(128) void latent_attn_mma_kernel(LatentParams p, const int* __restrict__ tiles,
+template <int NVW, int DVS, int NKT, int WARPS = 4>
+__global__ __launch_bounds__(32 * WARPS) void latent_attn_mma_kernel(LatentParams p, const int* __restrict__ tiles,
                                                               const int* __restrict__ decode_reqs, int decode,
                                                               int n_splits, float* __restrict__ part_o,
                                                               float* __restrict__ part_ml) {
   using bf16 = __nv_bfloat16;
-  constexpr int RB = 16 * (4 / DVS), LM_KT = 8 * NKT;
+  constexpr int RB = 16 * (WARPS / DVS), LM_KT = 8 * NKT;
   extern __shared__ __align__(16) unsigned char latent_smem[];
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   // (the step's description and the block table are written by none of its kernels: read before the wait below)
@@ -613,26 +613,23 @@ __global__ __launch_bounds__(128) void latent_attn_mma_kernel(LatentParams p, co
     beg = sp * chunk;
     end = min(kv_len, beg + chunk);
   }
-  // Where a tile's keys lie: lane i of every warp looks up keys i and (tiles of 64) i + 32, a row of the pool each (-1: none).
-  // A row's pieces are then copied by the lanes of one warp: one dependent read of the table a tile, asked for a tile ahead
-  // (with a look-up a piece, a thread's eighteen copies waited for one another).
-  auto pool_rows = [&](int kt, int (&row)[(LM_KT + 31) / 32]) {
+  // Where a tile's keys lie: lane i of every warp looks up the pages of keys i and (tiles of 64) i + 32; a key's row is then
+  // copied by the lanes of one warp.  One dependent read of the table a tile, asked for a tile ahead and looked at only when the tile
+  // is copied (with a look-up a piece, a thread's eighteen copies waited for one another).
+  constexpr int LOOKS = (LM_KT + 31) / 32;
+  const int pshift = (p.page_size & (p.page_size - 1)) == 0 ? 31 - __clz(p.page_size) : -1;
+  int pages[LOOKS];
+  auto look_up = [&](int kt) {
 #pragma unroll
-    for (int u = 0; u < (LM_KT + 31) / 32; ++u) {
-      const int key = kt + u * 32 + lane;
-      row[u] = -1;
-      if (key < end) {
-        const int page = bt[key / p.page_size];
-        if (page >= 0) row[u] = page * p.page_size + key % p.page_size;
-        else if (warp == 0) atomicOr(p.status, RL_STATUS_BAD_PAGE);
-      }
+    for (int u = 0; u < LOOKS; ++u) {
+      const int key = max(min(kt + u * 32 + lane, end - 1), 0);
+      pages[u] = bt[pshift >= 0 ? key >> pshift : key / p.page_size];
     }
   };
-  int next_rows[(LM_KT + 31) / 32];
-  pool_rows(beg, next_rows);
+  look_up(beg);
   asm volatile("griddepcontrol.wait;" ::: "memory");
   const bf16* q = (const bf16*)p.q;
-  for (int r = warp; r < RB; r += 4) {
+  for (int r = warp; r < RB; r += WARPS) {
     const int gr = row0 + r;
     const bf16* src = q + (size_t)(qs + t0 + gr / H) * p.q_stride + (size_t)(gr % H) * W;
     for (int c = lane * 8; c < Wk; c += 256) {
@@ -658,13 +655,21 @@ __global__ __launch_bounds__(128) void latent_attn_mma_kernel(LatentParams p, co
   const uint32_t q_s_addr = (uint32_t)__cvta_generic_to_shared(q_s);
   const uint32_t k_s_addr = (uint32_t)__cvta_generic_to_shared(k_s);
 
-  // the tile whose rows have been looked up into stage `st`: valid 16-byte pieces by cp.async, the rest zeros; then the
-  // rows of the tile after it are looked up
+  // the tile whose pages have been looked up into stage `st`: valid 16-byte pieces by cp.async, the rest zeros; then the
+  // pages of the tile after it are looked up
   auto stage_keys = [&](int kt, int st) {
     bf16* dst = k_s + st * LM_KT * LD;
+    int rows[LOOKS];  // of the pool, -1: none
+#pragma unroll
+    for (int u = 0; u < LOOKS; ++u) {
+      const int key = kt + u * 32 + lane;
+      const int place = pshift >= 0 ? key & (p.page_size - 1) : key % p.page_size;
+      rows[u] = key < end && pages[u] >= 0 ? pages[u] * p.page_size + place : -1;
+      if (key < end && pages[u] < 0 && warp == 0) atomicOr(p.status, RL_STATUS_BAD_PAGE);
+    }
 #pragma unroll 4
-    for (int j = warp; j < LM_KT; j += 4) {
-      const int row = __shfl_sync(0xffffffffu, next_rows[j >> 5], j & 31);
+    for (int j = warp; j < LM_KT; j += WARPS) {
+      const int row = __shfl_sync(0xffffffffu, rows[j >> 5], j & 31);
       const bf16* src = (const bf16*)p.pool + (size_t)max(row, 0) * W;
       for (int c = lane * 8; c < Wk; c += 256) {
         if (row >= 0 && c < W)
@@ -675,7 +680,7 @@ __global__ __launch_bounds__(128) void latent_attn_mma_kernel(LatentParams p, co
       }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
-    pool_rows(kt + LM_KT, next_rows);
+    look_up(kt + LM_KT);
   };
   if (beg < end) stage_keys(beg, 0);
   int st = 0;
@@ -716,16 +721,36 @@ __global__ __launch_bounds__(128) void latent_attn_mma_kernel(LatentParams p, co
         mma_16x8x16(acc[ni + 1], a, b2, b3);
       }
     };
-    int ks = 0;
-    for (; ks + 32 <= Wk; ks += 32) {
+    // four or eight warps that share their rows (a decoded token's heads) take a part of the inner size each; their sums meet
+    // in shared memory, in the warps' order
+    constexpr bool IN_PARTS = DVS >= 4;
+    const int k_steps = Wk >> 4, k_first = IN_PARTS ? vh * k_steps / DVS : 0, k_last = IN_PARTS ? (vh + 1) * k_steps / DVS : k_steps;
+    int ks = k_first * 16;
+    for (; ks + 32 <= k_last * 16; ks += 32) {
       score_step(ks, s);
       score_step(ks + 16, s2);
     }
-    if (ks < Wk) score_step(ks, s);
+    if (ks < k_last * 16) score_step(ks, s);
 #pragma unroll
     for (int ni = 0; ni < NKT; ++ni)
 #pragma unroll
       for (int c = 0; c < 4; ++c) s[ni][c] += s2[ni][c];
+    if constexpr (IN_PARTS) {
+      float4* part = reinterpret_cast<float4*>(k_s + 2 * LM_KT * LD) + lane;  // [warp][NKT][32 lanes]
+#pragma unroll
+      for (int ni = 0; ni < NKT; ++ni) part[(vh * NKT + ni) * 32] = make_float4(s[ni][0], s[ni][1], s[ni][2], s[ni][3]);
+      __syncthreads();
+#pragma unroll
+      for (int ni = 0; ni < NKT; ++ni) {
+        float4 t = part[ni * 32];
+#pragma unroll
+        for (int v = 1; v < DVS; ++v) {
+          const float4 a = part[(v * NKT + ni) * 32];
+          t.x += a.x, t.y += a.y, t.z += a.z, t.w += a.w;
+        }
+        s[ni][0] = t.x, s[ni][1] = t.y, s[ni][2] = t.z, s[ni][3] = t.w;
+      }
+    }
     // mask by each row's own position, online softmax in base 2
     float top_a = -CUDART_INF_F, top_b = -CUDART_INF_F;
 #pragma unroll
@@ -812,12 +837,17 @@ __global__ __launch_bounds__(128) void latent_attn_mma_kernel(LatentParams p, co
   }
 }
 
-// DVS_DEC, NVW_DEC: the form of the kernel that decoded tokens take (few heads: the value columns
-// spread over all four warps, so that none of them idles on rows that do not exist).
+constexpr size_t LATENT_PART_BYTES = 4 * 32 * 16;  // a warp's partial scores, tiles of 32 keys
+
+// DVS_DEC, NVW_DEC: the form of the kernel that decoded tokens take.  Up to 16 heads are the rows of one 16-row tile: the value
+// columns, and the inner size of the scores, are spread over four warps, or eight where the latents are wide enough (16 heads, latents
+// of 512, 8 requests of 544 keys in 8 parts, us among the kernels of a layer: four warps that each did all of the scores 15.3, four with
+// a part each 14.1, eight 12.1).
 template <int NVW, int DVS, int NKT, int NVW_DEC, int DVS_DEC>
 static inline void launch_latent_mma(const LatentParams& p, const int* tiles, int n_tiles, const int* decode_reqs,
                                      int n_decode, int n_splits, float* part_o, float* part_ml, cudaStream_t stream) {
-  constexpr int RB = 16 * (4 / DVS), RB_DEC = 16 * (4 / DVS_DEC), LM_KT = 8 * NKT, KT_DEC = 32;
+  constexpr int WARPS_DEC = DVS_DEC > 4 ? DVS_DEC : 4;
+  constexpr int RB = 16 * (4 / DVS), RB_DEC = 16 * (WARPS_DEC / DVS_DEC), LM_KT = 8 * NKT, KT_DEC = 32;
   const int Wk = (p.row_width + 15) & ~15;
   const size_t smem = (size_t)(RB + 2 * LM_KT) * (Wk + 8) * 2;
   static size_t granted = 0;
@@ -839,15 +869,15 @@ static inline void launch_latent_mma(const LatentParams& p, const int* tiles, in
     launch_pdl_split(false, latent_attn_mma_kernel<NVW, DVS, NKT>, dim3((LT_Q * p.n_heads + RB - 1) / RB, n_tiles), 128, smem, stream, p,
                tiles, decode_reqs, 0, 1, part_o, part_ml);
   if (n_decode > 0) {
-    const size_t smem_dec = (size_t)(RB_DEC + 2 * KT_DEC) * (Wk + 8) * 2;
+    const size_t smem_dec = (size_t)(RB_DEC + 2 * KT_DEC) * (Wk + 8) * 2 + (DVS_DEC >= 4 ? DVS_DEC * LATENT_PART_BYTES : 0);
     static size_t granted_dec = 0;
     if (smem_dec > 48 * 1024 && smem_dec > granted_dec) {
-      cudaFuncSetAttribute(latent_attn_mma_kernel<NVW_DEC, DVS_DEC, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      cudaFuncSetAttribute(latent_attn_mma_kernel<NVW_DEC, DVS_DEC, 4, WARPS_DEC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)smem_dec);
       granted_dec = smem_dec;
     }
-    launch_pdl(latent_attn_mma_kernel<NVW_DEC, DVS_DEC, 4>, dim3(n_decode, (p.n_heads + RB_DEC - 1) / RB_DEC, n_splits),
-               128, smem_dec, stream, p, tiles, decode_reqs, 1, n_splits, part_o, part_ml);
+    launch_pdl(latent_attn_mma_kernel<NVW_DEC, DVS_DEC, 4, WARPS_DEC>, dim3(n_decode, (p.n_heads + RB_DEC - 1) / RB_DEC, n_splits),
+               32 * WARPS_DEC, smem_dec, stream, p, tiles, decode_reqs, 1, n_splits, part_o, part_ml);
     if (n_splits > 1)
       launch_pdl(latent_attn_merge_kernel<__nv_bfloat16>, dim3(n_decode, p.n_heads), 128, 0, stream,
                  (const float*)part_o, (const float*)part_ml, n_splits, decode_reqs, p.q_start, p.slots,
@@ -868,23 +898,24 @@ static inline bool dispatch_latent_mma(const LatentParams& p, const int* tiles, 
   if ((size_t)(rows + 2 * keys) * (Wk + 8) * 2 > 200 * 1024) return false;
   // decoded tokens: up to 16 heads are one warp's rows, up to 32 two warps'
   const bool few = p.n_heads <= 16, some = p.n_heads <= 32;
-#define RL_LATENT_MMA(NVW, DVS, NKT, NVW4, NVW2)                                                                         \
+  // NVWF, DVSF: the form of up to 16 heads, four warps or (latents beyond 64) eight
+#define RL_LATENT_MMA(NVW, DVS, NKT, NVWF, DVSF, NVW2)                                                                   \
   do {                                                                                                                   \
-    if (few) launch_latent_mma<NVW, DVS, NKT, NVW4, 4>(p, tiles, n_tiles, decode_reqs, n_decode, n_splits, part_o, part_ml, stream); \
+    if (few) launch_latent_mma<NVW, DVS, NKT, NVWF, DVSF>(p, tiles, n_tiles, decode_reqs, n_decode, n_splits, part_o, part_ml, stream); \
     else if (some) launch_latent_mma<NVW, DVS, NKT, NVW2, 2>(p, tiles, n_tiles, decode_reqs, n_decode, n_splits, part_o, part_ml, stream); \
     else launch_latent_mma<NVW, DVS, NKT, NVW, DVS>(p, tiles, n_tiles, decode_reqs, n_decode, n_splits, part_o, part_ml, stream); \
   } while (0)
   // latent_prefill_form (for measurements): 0 the rule below; 1: latents of 129 to 256 with their
   // value columns over two warps; 2: the same with key tiles of 64
-  if (n8 <= 2) RL_LATENT_MMA(2, 1, 8, 2, 2);
-  else if (n8 <= 4) RL_LATENT_MMA(4, 1, 8, 2, 2);
-  else if (n8 <= 8) RL_LATENT_MMA(8, 1, 8, 2, 4);
-  else if (n8 <= 16) RL_LATENT_MMA(16, 1, 8, 4, 8);
-  else if (n8 <= 32 && latent_prefill_form == 1) RL_LATENT_MMA(16, 2, 4, 8, 16);
+  if (n8 <= 2) RL_LATENT_MMA(2, 1, 8, 2, 4, 2);
+  else if (n8 <= 4) RL_LATENT_MMA(4, 1, 8, 2, 4, 2);
+  else if (n8 <= 8) RL_LATENT_MMA(8, 1, 8, 2, 4, 4);
+  else if (n8 <= 16) RL_LATENT_MMA(16, 1, 8, 2, 8, 8);
+  else if (n8 <= 32 && latent_prefill_form == 1) RL_LATENT_MMA(16, 2, 4, 4, 8, 16);
   else if (n8 <= 32 && latent_prefill_form == 2 && (size_t)(32 + 128) * (Wk + 8) * 2 <= 200 * 1024)
-    RL_LATENT_MMA(16, 2, 8, 8, 16);
-  else if (n8 <= 32) RL_LATENT_MMA(32, 1, 4, 8, 16);
-  else if (n8 <= 64) RL_LATENT_MMA(32, 2, 4, 16, 32);
+    RL_LATENT_MMA(16, 2, 8, 4, 8, 16);
+  else if (n8 <= 32) RL_LATENT_MMA(32, 1, 4, 4, 8, 16);
+  else if (n8 <= 64) RL_LATENT_MMA(32, 2, 4, 8, 8, 32);
   else return false;
 #undef RL_LATENT_MMA
   return true;

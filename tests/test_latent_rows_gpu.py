@@ -97,3 +97,47 @@ def test_norm_added_with_the_row_in_registers(width):
     wide[:, :width] = base
     K.rmsnorm_add(y, gamma, 1e-5, wide[:, :width], 0.5, None)
     assert ((wide[:, :width] - x).abs() <= 4e-6 * (1 + x.abs())).all()
+
+
+# one warp's rows in four warps and in eight, two warps' rows, four's; latents that end inside a slice and rows that end inside a step of
+# 32; pages of a power of two and of 24; requests of one key, of part of a tile of keys, of whole tiles, of parts without a key
+@pytest.mark.parametrize("splits", [1, 3])
+@pytest.mark.parametrize("heads,rank,rot,page", [(16, 512, 64, 16), (3, 40, 8, 24), (16, 100, 20, 8), (5, 200, 8, 24), (20, 512, 40, 16), (40, 128, 24, 16)])
+def test_decoded_tokens_in_parts(heads, rank, rot, page, splits):
+    lens, width = [1, 31, 33, 64, 200, 371], rank + rot
+    n, width = len(lens), width + (-width) % 8
+    g = torch.Generator(device=DEV).manual_seed(heads * 7 + rank)
+    per = -(-max(lens) // page)
+    table = torch.randperm(n * per, generator=g, device=DEV).int().view(n, per).contiguous()
+    pool = torch.randn(n * per, 1, 1, page, width, generator=g, device=DEV).bfloat16()
+    q = torch.randn(n, heads * width, generator=g, device=DEV).bfloat16()
+    sink, scale = torch.randn(heads, generator=g, device=DEV), width ** -0.5
+    out = torch.full((n, heads * rank), float("nan"), device=DEV).bfloat16()
+    ids, scratch = _ints(list(range(n))), [torch.empty(n * heads * splits, w, device=DEV) for w in (rank, 2)]
+    K.latent_attention(q, pool, table, _ints(list(range(n + 1))), _ints(lens), ids, out, sink=sink, n_heads=heads, rank=rank, scale=scale,
+                       tiles=None, n_tiles=0, decode_reqs=ids, n_decode=n, decode_by_request=True, n_splits=splits, part_o=scratch[0],
+                       part_ml=scratch[1])
+    K.check_status(torch.device(DEV))
+    for r, length in enumerate(lens):
+        rows = pool[table[r].long()].view(-1, width)[:length].double()
+        scores = q[r].view(heads, width).double() @ rows.T * scale
+        p = torch.softmax(torch.cat([scores, sink.double()[:, None]], 1), 1)[:, :-1]
+        want, most = p @ rows[:, :rank], p @ rows[:, :rank].abs()
+        # probabilities and the result each rounded to bfloat16, the parts' maxima apart from the whole's
+        assert ((out[r].view(heads, rank).double() - want).abs() <= 2.0 ** -8 * (want.abs() + 1.5 * most) + 1e-5).all()
+
+
+# whole pairs of columns and an odd last one, a stride between heads that is odd: two columns stored together or each by itself
+@pytest.mark.parametrize("n,gap", [(40, 0), (41, 0), (40, 3)])
+def test_head_product_of_many_rows(n, gap):
+    t, h, k = 37, 3, 72
+    g = torch.Generator(device=DEV).manual_seed(n + gap)
+    x = torch.randn(t, h * k, generator=g, device=DEV).bfloat16()
+    w = (torch.randn(h, k, n, generator=g, device=DEV) * k ** -0.5).bfloat16()
+    out = torch.full((t, h, n + gap), 5.0, device=DEV).bfloat16()
+    K.head_linear(x, w, out, n_tokens=t, n_heads=h, k=k, n=n, in_strides=(h * k, k), w_strides=(k * n, n, 1),
+                  out_strides=(h * (n + gap), n + gap))
+    want = torch.einsum("thk,hkn->thn", x.view(t, h, k).double(), w.double())
+    # a bfloat16 rounding, and float32 sums of products of order 1
+    assert ((out[..., :n].double() - want).abs() <= want.abs() * 2.0 ** -8 + 1e-5).all()
+    assert (out[..., n:] == 5.0).all()
