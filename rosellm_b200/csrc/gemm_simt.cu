@@ -293,6 +293,98 @@ __global__ __launch_bounds__(256, 2) void gemm_rows_f32_kernel(
   asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
+// The same where there are many more groups of columns than warps (a head): a warp takes a group for itself, all of K, so that
+// its sums are added over the lanes once a group and never meet another warp's (at K 768 the kernel above does the 31 exchanges of
+// that addition after every single chunk: 50257 x 768, 8 rows 69 us, where the weights take 24).  The order of a sum is the same for
+// every row whatever M is.
+constexpr int WIDE_STAGES = 4;
+template <int ROWS>
+__global__ __launch_bounds__(256, 2) void gemm_rows_f32_wide_kernel(const float* __restrict__ A, long lda, const float* __restrict__ W,
+                                                                    const float* __restrict__ bias, float* __restrict__ out, long ldo,
+                                                                    int M, int N, int K, int act, int residual) {
+  constexpr int COLS = ROWS_COLS, VALUES = COLS * ROWS, AHEAD = WIDE_STAGES - 1;
+  extern __shared__ __align__(16) float4 wide_ring[];  // [warp][stage][column][lane]
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int groups = (N + COLS - 1) / COLS, chunks = (K + 127) / 128, stride = (int)gridDim.x * 8;
+  float4* mine = wide_ring + (size_t)warp * WIDE_STAGES * COLS * 32 + lane;
+  const uint32_t mine_addr = (uint32_t)__cvta_generic_to_shared(mine);
+  // what the warp copies next: of a group its chunks, those once for every ROWS rows, then its next group
+  int c_group = (int)blockIdx.x * 8 + warp, c_chunk = 0, c_m0 = 0, c_stage = 0;
+  auto copy = [&]() {
+    if (c_group < groups) {
+      const int k = c_chunk * 128 + 4 * lane;
+#pragma unroll
+      for (int c = 0; c < COLS; ++c)  // beyond K: zeros
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(mine_addr + (uint32_t)(c_stage * COLS + c) * 512),
+                     "l"(W + (size_t)min(c_group * COLS + c, N - 1) * K + (k < K ? k : 0)), "r"(k < K ? 16 : 0)
+                     : "memory");
+      if (++c_stage == WIDE_STAGES) c_stage = 0;
+      if (++c_chunk == chunks) {
+        c_chunk = 0;
+        if ((c_m0 += ROWS) >= M) c_m0 = 0, c_group += stride;
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+#pragma unroll
+  for (int s = 0; s < AHEAD; ++s) copy();
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  int stage = 0;
+  const int value = lane / (32 / VALUES), row = value / COLS;  // what this lane holds after the exchanges (fewer values: neighbours alike)
+  for (int group = (int)blockIdx.x * 8 + warp; group < groups; group += stride) {
+    const int n = group * COLS + value % COLS;
+    const float b = n < N && bias != nullptr ? bias[n] : 0.f;
+    for (int m0 = 0; m0 < M; m0 += ROWS) {
+      float acc[VALUES];  // [row][column]
+#pragma unroll
+      for (int i = 0; i < VALUES; ++i) acc[i] = 0.f;
+      for (int chunk = 0; chunk < chunks; ++chunk) {
+        copy();  // into the stage that was read last
+        asm volatile("cp.async.wait_group %0;" ::"n"(AHEAD) : "memory");
+        float4 w[COLS];
+#pragma unroll
+        for (int c = 0; c < COLS; ++c) w[c] = mine[(stage * COLS + c) * 32];
+        if (++stage == WIDE_STAGES) stage = 0;
+        const int k = chunk * 128 + 4 * lane;
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) {
+          float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (k < K) a = *reinterpret_cast<const float4*>(A + (size_t)min(m0 + r, M - 1) * lda + k);
+#pragma unroll
+          for (int c = 0; c < COLS; ++c) {
+            float& t = acc[r * COLS + c];
+            t = fmaf(a.x, w[c].x, t);
+            t = fmaf(a.y, w[c].y, t);
+            t = fmaf(a.z, w[c].z, t);
+            t = fmaf(a.w, w[c].w, t);
+          }
+        }
+      }
+      // after the exchange over lane bit o, a lane keeps the half of its values whose index has that bit as its own;
+      // with one value left the lanes add it up
+#pragma unroll
+      for (int o = 16, half = VALUES / 2; o > 0; o >>= 1, half >>= 1) {
+        const bool upper = (lane & o) != 0;
+        if (half == 0) {
+          acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);
+          continue;
+        }
+#pragma unroll
+        for (int i = 0; i < VALUES / 2; ++i) {
+          if (i >= half) break;
+          const float give = upper ? acc[i] : acc[i + half];
+          const float keep = upper ? acc[i + half] : acc[i];
+          acc[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+      }
+      const int m = m0 + row;
+      if (lane % (32 / VALUES) == 0 && n < N && m < M) store_out<float>(out, (size_t)m * ldo + n, apply_act(acc[0] + b, act), residual);
+    }
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+
 // Few rows of bfloat16.  A block of four warps computes 4 / KSPLIT output columns for all
 // rows: KSPLIT warps share a column, each taking a contiguous part of K, and their partial
 // sums meet in shared memory in a fixed order.  Lanes split a warp's part of K in 16-byte
@@ -487,7 +579,19 @@ static void launch_rows_f32_form(const float* a, long lda, const float* w, const
     attr_set = true;
   }
   const int groups = (N + ROWS_COLS - 1) / ROWS_COLS, blocks = 2 * simt_sm_count();
-  // a barrier every four groups where there are many (50257 x 768, 8 rows: 69 us against 81); few are shared out singly
+  if (kv.pool == nullptr && groups >= 4 * 8 * blocks) {  // four groups a warp and more
+    constexpr size_t wide = 8 * WIDE_STAGES * 4 * 512;
+    static bool wide_set = false;
+    if (!wide_set) {
+      note_launch(cudaFuncSetAttribute(gemm_rows_f32_wide_kernel<ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wide));
+      note_launch(cudaFuncSetAttribute(gemm_rows_f32_wide_kernel<ROWS>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                       (int)cudaSharedmemCarveoutMaxShared));  // two blocks an SM
+      wide_set = true;
+    }
+    launch_pdl_split(false, gemm_rows_f32_wide_kernel<ROWS>, blocks, 256, wide, stream, a, lda, w, bias, o, ldo, M, N, K, act, residual);
+    return;
+  }
+  // a barrier every four groups where there are many (but fewer than above); few are shared out singly
   // (3072 x 768: 7.2 us against 8.0)
   const int per_turn = groups >= 4 * ROWS_GROUPS * blocks ? ROWS_GROUPS : 1, turns = (groups + per_turn - 1) / per_turn;
   launch_pdl(gemm_rows_f32_kernel<ROWS>, min(turns, blocks), 256, smem, stream, a, lda, w, bias, o, ldo, M, N, K, act, residual, kv,
