@@ -175,48 +175,38 @@ __global__ __launch_bounds__((BM / TM) * (BN / TN)) void gemm_tile_f32_kernel(
   }
 }
 
-// Few rows of float32 (decoded tokens).  A block of eight warps stays for the product and takes groups of COLS output
-// columns in turn, ROWS rows at a time; its warps take the chunks of 128 elements of K in turn, a lane four elements of each:
-// every piece of the weights that a lane holds meets all the rows in registers (the kernel before read a piece of A for
-// every piece of W, from the first-level cache, whose bandwidth bounded it).  A lane's weights travel by cp.async into a
-// ring of its own in shared memory (it reads back only what it copied itself, so no barrier is needed), two chunks
-// ahead, and the first of them before the wait for the kernels ahead.  The COLS * ROWS sums of a lane are added over the lanes
-// by halving exchanges (each lane gives away half of what it has left), then over the warps in shared memory: in an order
-// that is the same for every row whatever M is.
-// per_turn: groups whose sums meet at one barrier, at most ROWS_GROUPS.
-constexpr int ROWS_COLS = 4, ROWS_GROUPS = 4;
-template <int ROWS>
-__global__ __launch_bounds__(256, 2) void gemm_rows_f32_kernel(
-    const float* __restrict__ A, long lda, const float* __restrict__ W, const float* __restrict__ bias,
-    float* __restrict__ out, long ldo, int M, int N, int K, int act, int residual, KvScatter kv, int per_turn) {
-  constexpr int WARPS = 8, COLS = ROWS_COLS, VALUES = COLS * ROWS, AHEAD = 2, STAGES = AHEAD + 1;
-  extern __shared__ __align__(16) float4 rows_ring[];  // [warp][stage][column][lane]
-  __shared__ float part_s[2][WARPS][ROWS_GROUPS][VALUES];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int groups = (N + COLS - 1) / COLS, chunks = (K + 127) / 128;
-  float4* mine = rows_ring + (size_t)warp * STAGES * COLS * 32 + lane;
-  // what the warp copies next: of a group its chunks, of the groups taken together each, those once for every ROWS rows,
-  // then the block's next groups
-  int c_first = warp < chunks ? (int)blockIdx.x * per_turn : groups, c_m0 = 0, c_group = c_first, c_chunk = warp, c_stage = 0;
+// Few rows of float32 (decoded tokens).  PARTS of a block's eight warps share a group of COLS output columns, ROWS rows at a
+// time: they take the chunks of 128 elements of K in turn, a lane four elements of each, so that every piece of the weights that a
+// lane holds meets all the rows in registers.  A lane's weights travel by cp.async into a ring of its own in shared memory (it
+// reads back only what it copied itself, so no barrier is needed), two chunks ahead, and the first of them before the wait
+// for the kernels ahead.  The COLS * ROWS sums of a lane are added over the lanes by halving exchanges (each lane gives away half
+// of what it has left), then over the group's warps in shared memory: in an order that is the same for every row whatever M is.
+constexpr int ROWS_COLS = 4, ROWS_STAGES = 3;
+template <int ROWS, int PARTS>
+__global__ __launch_bounds__(256, 2) void gemm_rows_f32_kernel(const float* __restrict__ A, long lda, const float* __restrict__ W,
+                                                               const float* __restrict__ bias, float* __restrict__ out, long ldo,
+                                                               int M, int N, int K, int act, int residual, KvScatter kv) {
+  constexpr int COLS = ROWS_COLS, STAGES = ROWS_STAGES, VALUES = COLS * ROWS, AHEAD = STAGES - 1, GROUPS = 8 / PARTS;
+  extern __shared__ __align__(128) float4 rows_ring[];  // [warp][stage][column][lane]
+  __shared__ __align__(128) float part_s[2][GROUPS][PARTS][VALUES];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, mine = warp / PARTS, part = warp % PARTS;
+  const int groups = (N + COLS - 1) / COLS, chunks = (K + 127) / 128, stride = (int)gridDim.x * GROUPS;
+  float4* ring = rows_ring + (size_t)warp * STAGES * COLS * 32 + lane;
+  const uint32_t ring_addr = (uint32_t)__cvta_generic_to_shared(ring);
+  // what the warp copies next: of a group its chunks, those once for every ROWS rows, then its next group
+  int c_group = part < chunks ? (int)blockIdx.x * GROUPS + mine : groups, c_chunk = part, c_m0 = 0, c_stage = 0;
   auto copy = [&]() {
-    if (c_first < groups) {
+    if (c_group < groups) {
       const int k = c_chunk * 128 + 4 * lane;
-      const uint32_t dst = (uint32_t)__cvta_generic_to_shared(mine + c_stage * COLS * 32);
 #pragma unroll
       for (int c = 0; c < COLS; ++c)  // beyond K: zeros
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + c * 512),
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(ring_addr + (uint32_t)(c_stage * COLS + c) * 512),
                      "l"(W + (size_t)min(c_group * COLS + c, N - 1) * K + (k < K ? k : 0)), "r"(k < K ? 16 : 0)
                      : "memory");
       if (++c_stage == STAGES) c_stage = 0;
-      if ((c_chunk += WARPS) >= chunks) {
-        c_chunk = warp;
-        if (++c_group == min(c_first + per_turn, groups)) {
-          if ((c_m0 += ROWS) >= M) {
-            c_m0 = 0;
-            c_first += gridDim.x * per_turn;
-          }
-          c_group = c_first;
-        }
+      if ((c_chunk += PARTS) >= chunks) {
+        c_chunk = part;
+        if ((c_m0 += ROWS) >= M) c_m0 = 0, c_group += stride;
       }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
@@ -226,24 +216,24 @@ __global__ __launch_bounds__(256, 2) void gemm_rows_f32_kernel(
   for (int s = 0; s < AHEAD; ++s) copy();
   asm volatile("griddepcontrol.wait;" ::: "memory");
   int buf = 0, stage = 0;
-  for (int first = blockIdx.x * per_turn; first < groups; first += gridDim.x * per_turn) {
-    const int n_here = min(per_turn, groups - first);
-    // the epilogue's thread: a column of a row of one of the groups
-    const int e_group = tid / VALUES, e_value = tid % VALUES, e_row = e_value / COLS, e_n = (first + e_group) * COLS + e_value % COLS;
-    const bool e_there = e_group < n_here && e_n < N;
-    const float b = e_there && bias != nullptr ? bias[e_n] : 0.f;
+  // the epilogue's thread: a column of a row of one of the groups
+  const int e_mine = tid / VALUES, e_value = tid % VALUES;
+  for (int first = (int)blockIdx.x * GROUPS; first < groups; first += stride) {
+    const bool there = first + mine < groups;
+    const int n = (first + e_mine) * COLS + e_value % COLS;
+    const bool n_there = e_mine < GROUPS && n < N;
+    const float b = n_there && bias != nullptr ? bias[n] : 0.f;
     for (int m0 = 0; m0 < M; m0 += ROWS, buf ^= 1) {
-#pragma unroll 1
-      for (int g = 0; g < n_here; ++g) {
-        float acc[VALUES];  // [row][column]
+      float acc[VALUES];  // [row][column]
 #pragma unroll
-        for (int i = 0; i < VALUES; ++i) acc[i] = 0.f;
-        for (int chunk = warp; chunk < chunks; chunk += WARPS) {
+      for (int i = 0; i < VALUES; ++i) acc[i] = 0.f;
+      if (there)
+        for (int chunk = part; chunk < chunks; chunk += PARTS) {
           copy();  // into the stage that was read last
           asm volatile("cp.async.wait_group %0;" ::"n"(AHEAD) : "memory");
           float4 w[COLS];
 #pragma unroll
-          for (int c = 0; c < COLS; ++c) w[c] = mine[(stage * COLS + c) * 32];
+          for (int c = 0; c < COLS; ++c) w[c] = ring[(stage * COLS + c) * 32];
           if (++stage == STAGES) stage = 0;
           const int k = chunk * 128 + 4 * lane;
 #pragma unroll
@@ -260,107 +250,6 @@ __global__ __launch_bounds__(256, 2) void gemm_rows_f32_kernel(
             }
           }
         }
-        // after the exchange over lane bit o, a lane keeps the half of its values whose index has that bit as its own;
-        // with one value left the lanes add it up
-#pragma unroll
-        for (int o = 16, half = VALUES / 2; o > 0; o >>= 1, half >>= 1) {
-          const bool upper = (lane & o) != 0;
-          if (half == 0) {
-            acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);
-            continue;
-          }
-#pragma unroll
-          for (int i = 0; i < VALUES / 2; ++i) {
-            if (i >= half) break;
-            const float give = upper ? acc[i] : acc[i + half];
-            const float keep = upper ? acc[i + half] : acc[i];
-            acc[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
-          }
-        }
-        part_s[buf][warp][g][lane / (32 / VALUES)] = acc[0];  // fewer values than lanes: neighbours hold the same one
-      }
-      __syncthreads();  // the other buffer takes the next sums, so one barrier is enough
-      const int m = m0 + e_row;
-      if (e_there && m < M) {
-        float v = 0.f;
-#pragma unroll
-        for (int q = 0; q < WARPS; ++q) v += part_s[buf][q][e_group][e_value];
-        v = apply_act(v + b, act);
-        if (!scatter_kv<float>(kv, m, e_n, v)) store_out<float>(out, (size_t)m * ldo + e_n, v, residual);
-      }
-    }
-  }
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
-}
-
-// The same where there are many more groups of columns than warps (a head): a warp takes a group for itself, all of K, so that
-// its sums are added over the lanes once a group and never meet another warp's (at K 768 the kernel above does the 31 exchanges of
-// that addition after every single chunk: 50257 x 768, 8 rows 69 us, where the weights take 24).  The order of a sum is the same for
-// every row whatever M is.
-constexpr int WIDE_STAGES = 4;
-template <int ROWS>
-__global__ __launch_bounds__(256, 2) void gemm_rows_f32_wide_kernel(const float* __restrict__ A, long lda, const float* __restrict__ W,
-                                                                    const float* __restrict__ bias, float* __restrict__ out, long ldo,
-                                                                    int M, int N, int K, int act, int residual) {
-  constexpr int COLS = ROWS_COLS, VALUES = COLS * ROWS, AHEAD = WIDE_STAGES - 1;
-  extern __shared__ __align__(16) float4 wide_ring[];  // [warp][stage][column][lane]
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int groups = (N + COLS - 1) / COLS, chunks = (K + 127) / 128, stride = (int)gridDim.x * 8;
-  float4* mine = wide_ring + (size_t)warp * WIDE_STAGES * COLS * 32 + lane;
-  const uint32_t mine_addr = (uint32_t)__cvta_generic_to_shared(mine);
-  // what the warp copies next: of a group its chunks, those once for every ROWS rows, then its next group
-  int c_group = (int)blockIdx.x * 8 + warp, c_chunk = 0, c_m0 = 0, c_stage = 0;
-  auto copy = [&]() {
-    if (c_group < groups) {
-      const int k = c_chunk * 128 + 4 * lane;
-#pragma unroll
-      for (int c = 0; c < COLS; ++c)  // beyond K: zeros
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(mine_addr + (uint32_t)(c_stage * COLS + c) * 512),
-                     "l"(W + (size_t)min(c_group * COLS + c, N - 1) * K + (k < K ? k : 0)), "r"(k < K ? 16 : 0)
-                     : "memory");
-      if (++c_stage == WIDE_STAGES) c_stage = 0;
-      if (++c_chunk == chunks) {
-        c_chunk = 0;
-        if ((c_m0 += ROWS) >= M) c_m0 = 0, c_group += stride;
-      }
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-#pragma unroll
-  for (int s = 0; s < AHEAD; ++s) copy();
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  int stage = 0;
-  const int value = lane / (32 / VALUES), row = value / COLS;  // what this lane holds after the exchanges (fewer values: neighbours alike)
-  for (int group = (int)blockIdx.x * 8 + warp; group < groups; group += stride) {
-    const int n = group * COLS + value % COLS;
-    const float b = n < N && bias != nullptr ? bias[n] : 0.f;
-    for (int m0 = 0; m0 < M; m0 += ROWS) {
-      float acc[VALUES];  // [row][column]
-#pragma unroll
-      for (int i = 0; i < VALUES; ++i) acc[i] = 0.f;
-      for (int chunk = 0; chunk < chunks; ++chunk) {
-        copy();  // into the stage that was read last
-        asm volatile("cp.async.wait_group %0;" ::"n"(AHEAD) : "memory");
-        float4 w[COLS];
-#pragma unroll
-        for (int c = 0; c < COLS; ++c) w[c] = mine[(stage * COLS + c) * 32];
-        if (++stage == WIDE_STAGES) stage = 0;
-        const int k = chunk * 128 + 4 * lane;
-#pragma unroll
-        for (int r = 0; r < ROWS; ++r) {
-          float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (k < K) a = *reinterpret_cast<const float4*>(A + (size_t)min(m0 + r, M - 1) * lda + k);
-#pragma unroll
-          for (int c = 0; c < COLS; ++c) {
-            float& t = acc[r * COLS + c];
-            t = fmaf(a.x, w[c].x, t);
-            t = fmaf(a.y, w[c].y, t);
-            t = fmaf(a.z, w[c].z, t);
-            t = fmaf(a.w, w[c].w, t);
-          }
-        }
-      }
       // after the exchange over lane bit o, a lane keeps the half of its values whose index has that bit as its own;
       // with one value left the lanes add it up
 #pragma unroll
@@ -378,8 +267,16 @@ __global__ __launch_bounds__(256, 2) void gemm_rows_f32_wide_kernel(const float*
           acc[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
         }
       }
-      const int m = m0 + row;
-      if (lane % (32 / VALUES) == 0 && n < N && m < M) store_out<float>(out, (size_t)m * ldo + n, apply_act(acc[0] + b, act), residual);
+      part_s[buf][mine][part][lane / (32 / VALUES)] = acc[0];  // fewer values than lanes: neighbours hold the same one
+      __syncthreads();  // the other buffer takes the next sums, so one barrier is enough
+      const int m = m0 + e_value / COLS;
+      if (n_there && m < M) {
+        float v = 0.f;
+#pragma unroll
+        for (int q = 0; q < PARTS; ++q) v += part_s[buf][e_mine][q][e_value];
+        v = apply_act(v + b, act);
+        if (!scatter_kv<float>(kv, m, n, v)) store_out<float>(out, (size_t)m * ldo + n, v, residual);
+      }
     }
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -569,33 +466,39 @@ static void launch_tile_f32(const float* a, long lda, const float* w, const floa
   else launch_tile_f32_form<32, 32, 4, 2>(a, lda, w, bias, o, ldo, M, N, K, act, residual, stream);
 }
 
+template <int ROWS, int PARTS>
+static void launch_rows_f32_parts(const float* a, long lda, const float* w, const float* bias, float* o, long ldo, int M, int N, int K,
+                                  int act, int residual, const KvScatter& kv, int blocks, cudaStream_t stream) {
+  constexpr size_t smem = 8 * ROWS_STAGES * ROWS_COLS * 512;  // the rings of eight warps
+  static bool attr_set = false;
+  if (!attr_set) {  // with the kernel's static part above 48 KB
+    note_launch(cudaFuncSetAttribute(gemm_rows_f32_kernel<ROWS, PARTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    attr_set = true;
+  }
+  launch_pdl(gemm_rows_f32_kernel<ROWS, PARTS>, blocks, 256, smem, stream, a, lda, w, bias, o, ldo, M, N, K, act, residual, kv);
+}
+
 template <int ROWS>
 static void launch_rows_f32_form(const float* a, long lda, const float* w, const float* bias, float* o, long ldo, int M, int N, int K,
                                  int act, int residual, const KvScatter& kv, cudaStream_t stream) {
-  constexpr size_t smem = 8 * 3 * 4 * 512;  // the rings of eight warps: three stages of four columns
-  static bool attr_set = false;
-  if (!attr_set) {  // with the kernel's static part above 48 KB
-    note_launch(cudaFuncSetAttribute(gemm_rows_f32_kernel<ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attr_set = true;
+  // Warps that share a group, by the rounds of groups and what a round takes: a part that does not change with K and one for each chunk
+  // a warp walks (in 8 rows about 1 us and 0.75).  Measured, 8 rows, us, two / four / eight warps: 768 x 768 3.6 / 2.9 / 2.4, 2304 x 768
+  // 4.1 / 3.3 / 4.0, 3072 x 768 4.5 / 5.5 / 5.7, 4096 x 1024 5.5 / 6.2 / 7.6, 1600 x 1600 7.0 / 5.1 / 5.3, 4800 x 1600 12.2 / 11.2 / 10.8,
+  // 6400 x 1600 13.4 / 12.3 / 14.2, 1600 x 6400 20.5 / 13.0 / 15.1, 50257 x 768 35.7 / 49.6 / 68.7 (43.0 with a warp a group).
+  const int groups = (N + ROWS_COLS - 1) / ROWS_COLS, chunks = (K + 127) / 128, places = 2 * simt_sm_count();
+  int parts = 8, turns = groups;
+  float least = 0.f;
+  for (int p = 8; p >= 2; p /= 2) {
+    const int t = (groups + 8 / p - 1) / (8 / p);
+    const float cost = (float)((t + places - 1) / places) * (1.f + 0.75f * (float)((chunks + p - 1) / p));
+    if (p == 8 || cost < 0.95f * least) parts = p, turns = t, least = cost;
   }
-  const int groups = (N + ROWS_COLS - 1) / ROWS_COLS, blocks = 2 * simt_sm_count();
-  if (kv.pool == nullptr && groups >= 4 * 8 * blocks) {  // four groups a warp and more
-    constexpr size_t wide = 8 * WIDE_STAGES * 4 * 512;
-    static bool wide_set = false;
-    if (!wide_set) {
-      note_launch(cudaFuncSetAttribute(gemm_rows_f32_wide_kernel<ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wide));
-      note_launch(cudaFuncSetAttribute(gemm_rows_f32_wide_kernel<ROWS>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                       (int)cudaSharedmemCarveoutMaxShared));  // two blocks an SM
-      wide_set = true;
-    }
-    launch_pdl_split(false, gemm_rows_f32_wide_kernel<ROWS>, blocks, 256, wide, stream, a, lda, w, bias, o, ldo, M, N, K, act, residual);
-    return;
-  }
-  // a barrier every four groups where there are many (but fewer than above); few are shared out singly
-  // (3072 x 768: 7.2 us against 8.0)
-  const int per_turn = groups >= 4 * ROWS_GROUPS * blocks ? ROWS_GROUPS : 1, turns = (groups + per_turn - 1) / per_turn;
-  launch_pdl(gemm_rows_f32_kernel<ROWS>, min(turns, blocks), 256, smem, stream, a, lda, w, bias, o, ldo, M, N, K, act, residual, kv,
-             per_turn);
+#define RL_PARTS(PARTS) \
+  launch_rows_f32_parts<ROWS, PARTS>(a, lda, w, bias, o, ldo, M, N, K, act, residual, kv, min(turns, places), stream)
+  if (parts == 2) RL_PARTS(2);
+  else if (parts == 4) RL_PARTS(4);
+  else RL_PARTS(8);
+#undef RL_PARTS
 }
 
 static void launch_rows_f32(const float* a, long lda, const float* w, const float* bias, float* o, long ldo, int M, int N, int K,
