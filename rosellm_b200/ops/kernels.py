@@ -25,9 +25,9 @@ STATUS_BITS = {
     8: "a bounded wait inside a kernel gave up",
 }
 
-# Rows up to which a float32 product streams the weights once per group of rows on the CUDA cores
-# (csrc/gemm_simt.cu) instead of tiling, there or on the tensor cores (csrc/gemm_f32_tc.cu); which
-# kernel a bfloat16 product runs on: bf16_path.
+# Rows up to which a float32 product streams the weights once per group of rows instead of
+# tiling, both in IEEE arithmetic on the CUDA cores (csrc/gemm_simt.cu); which kernel a
+# bfloat16 product runs on: bf16_path.
 ROWS_STREAMING_LIMIT = 64
 
 
@@ -539,15 +539,14 @@ def linear(a, weight, bias, out, *, act: int = ACT_NONE, residual: bool = False,
     at most 16 rows).  Otherwise
     a [rows, k] (row stride a multiple of 8), weight [n, k] contiguous, both float32 or both
     bfloat16; out [rows, n] of a's dtype or float32.  Which kernel runs: float32 up to 64 rows
-    the row kernel, above it tiles of FMAs or, from an inner size of 256 where it is faster, of tf32 parts; bfloat16 up to 16 rows the
+    the row kernel, above it tiles (both IEEE FMAs); bfloat16 up to 16 rows the
     weight-streaming kernels (fed by TMA through a ring; for a very wide float32 output, a head, by
-    bulk copies; by registers otherwise: the library chooses), above it as ``bf16_path`` and ``clustered_is_ahead`` say.  ``path``
-    (for tests) forces ``"rows"``, ``"tile"``, ``"f32tc"``, ``"mma"``, ``"smem"``, ``"tc"`` or ``"tcr"``.  ``kv``: output columns from
+    bulk copies; by registers otherwise: the library chooses), above it as ``bf16_path`` says.  ``path`` (for tests) forces
+    ``"rows"``, ``"tile"``, ``"mma"``, ``"smem"``, ``"tc"`` or ``"tcr"``.  ``kv``: output columns from
     ``kv.q_width`` on are written into cache pages, not ``out`` (not with ``"tile"``).
     ``tile_width`` and ``splits`` (for tests and measurements, ``"tc"`` only): the columns of an
     output tile, a multiple of 32 up to 256, and the parts the inner size is cut into (1, 2, 3, 4, 6
-    or 8: the blocks of a cluster take one each; -2: tiles of 256 rows over pairs of SMs), instead of what the kernel would choose
-    (``tile_width`` with ``"f32tc"`` too).
+    or 8: the blocks of a cluster take one each), instead of what the kernel would choose.
     ``head``: the outputs are logits, whose tokens ``linear_sample`` may be asked for in their place: the same sums in
     the same order as there, bit for bit (tiles then never cut the inner size).
     """
@@ -823,6 +822,8 @@ def separate_is_faster(rows: int, hidden: int, attention_fused: bool) -> bool:
 
     both fused, width 576, 8 rows    16.4 > 17.1   17.3 > 17.1   18.7 > 18.2   21.8 > 20.5
                 704, 5               16.6 > 16.8   17.4 > 16.8   18.7 > 17.8   21.3 > 20.1
+                768, 1               16.7 > 15.3   16.7 > 15.6   16.7 > 16.7   16.9 > 18.9
+                768, 4               16.8 > 16.7   17.1 > 16.7   17.8 > 17.7   19.4 > 20.0
                 768, 8               18.0 > 17.5   19.9 > 17.6   20.3 > 18.8   23.2 > 21.1
                 768, 12              18.8 > 21.0   21.4 > 21.3   23.8 > 22.7   29.3 > 25.1
                 832, 8               18.7 > 18.4   19.7 > 18.4   21.5 > 19.5   24.6 > 22.0
@@ -838,17 +839,6 @@ def separate_is_faster(rows: int, hidden: int, attention_fused: bool) -> bool:
                 1024, 8              22.0 > 20.9   22.2 > 20.9   23.4 > 22.0   25.7 > 24.6
                 1024, 16             25.5 > 24.2   28.2 > 26.2   29.9 > 29.7   34.8 > 36.3
 
-    and, with a request's keys over the blocks of a cluster, a step of twelve layers and a head at 32 / 128 / 512 / 900 cached tokens:
-
-    both fused, width 704, 1 row     223 > 205     222 > 214     224 > 223     226 > 230
-                704, 2               217 > 211     219 > 219     226 > 228     231 > 238
-                704, 4               225 > 215     226 > 226     243 > 233     254 > 246
-                768, 1               227 > 207     226 > 214     228 > 224     230 > 232
-                768, 2               226 > 211     225 > 217     233 > 229     237 > 238
-                768, 3               232 > 218     231 > 229     246 > 237     256 > 250
-                832, 1               238 > 214     237 > 221     239 > 231     241 > 241
-                832, 4               244 > 228     244 > 237     262 > 246     272 > 258
-
     Both at 1024 columns are not to be had (sixteen heads of clusters are more than the device holds).  There the separate
     form is taken for all rows, though from eleven to fifteen rows and 512 tokens on it is up to 9% behind: the fused
     feed-forward reads a copy of its output weights, 250 MB for the 24 layers of GPT-2 355M."""
@@ -856,7 +846,7 @@ def separate_is_faster(rows: int, hidden: int, attention_fused: bool) -> bool:
         return True
     middle = 704 <= hidden <= 832
     if attention_fused:
-        return middle and (1 if hidden >= 768 else 3) <= rows <= 8
+        return middle and 5 <= rows <= 8
     return (hidden >= 256 and rows <= 8) or (middle and rows <= 12)
 
 
