@@ -24,7 +24,7 @@
 // shared memory: prompt portions, and decoded tokens in the 32-bit mode);
 // `latent_attn_decode_kernel` (a decoded token: one block takes all heads of a request and a
 // share of its keys, so that a cached row is read once for all heads) with
-// `latent_attn_merge_kernel`.
+// `latent_attn_merge_kernel`, which also merges more than eight parts of the tensor-core kernel.
 #include <math_constants.h>
 
 #include "common.cuh"
@@ -561,7 +561,7 @@ __device__ __forceinline__ float quad_sum(float v) {
   return v + __shfl_xor_sync(0xffffffffu, v, 2);
 }
 
-template <int NVW, int DVS, int NKT, int WARPS = 4>
+template <int NVW, int DVS, int NKT, int WARPS = 4, bool CLUSTERED = false>
 __global__ __launch_bounds__(32 * WARPS) void latent_attn_mma_kernel(LatentParams p, const int* __restrict__ tiles,
                                                               const int* __restrict__ decode_reqs, int decode,
                                                               int n_splits, float* __restrict__ part_o,
@@ -627,6 +627,7 @@ __global__ __launch_bounds__(32 * WARPS) void latent_attn_mma_kernel(LatentParam
     }
   };
   look_up(beg);
+  if constexpr (CLUSTERED) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");  // waited for before results are sent
   asm volatile("griddepcontrol.wait;" ::: "memory");
   const bf16* q = (const bf16*)p.q;
   for (int r = warp; r < RB; r += WARPS) {
@@ -806,6 +807,56 @@ __global__ __launch_bounds__(32 * WARPS) void latent_attn_mma_kernel(LatentParam
     __syncthreads();  // the stage may be written again
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");  // a part without keys has not waited for its queries
+  if constexpr (CLUSTERED) {
+    // The parts of these rows are the blocks of a cluster: part s finishes rows [s * own, (s + 1) * own), every block sends it
+    // its sums of those, [part][own][columns] float32, and their (maximum, sum), [part][own].
+    const int own = (RB + n_splits - 1) / n_splits, cols = (p.rank + 7) & ~7;
+    float* recv = reinterpret_cast<float*>(k_s + 2 * LM_KT * LD) + DVS * NKT * 128;
+    float* recv_ml = recv + n_splits * own * cols;
+    const uint32_t recv_addr = (uint32_t)__cvta_generic_to_shared(recv), ml_addr = (uint32_t)__cvta_generic_to_shared(recv_ml);
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const int row = rg * 16 + g + 8 * half, owner = row / own, at = sp * own + row - owner * own;
+      if (row0 + row >= rows_total) continue;
+      if (t == 0 && vh == 0)
+        asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(peer_addr(ml_addr + (uint32_t)at * 8u, (uint32_t)owner)),
+                     "f"(half ? m_b : m_a), "f"(half ? l_b : l_a)
+                     : "memory");
+      const uint32_t dst = peer_addr(recv_addr + (uint32_t)(at * cols + vh * NVW * 8 + 2 * t) * 4u, (uint32_t)owner);
+#pragma unroll
+      for (int nv = 0; nv < NVW; ++nv)
+        if ((vh * NVW + nv) * 8 < cols)
+          asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(dst + (uint32_t)nv * 32u), "f"(o[nv][2 * half]),
+                       "f"(o[nv][2 * half + 1])
+                       : "memory");
+    }
+    __syncwarp();
+    cluster_sync();
+    const bool pairs = (((uintptr_t)out & 3) | (uintptr_t)((p.out_stride | p.rank) & 1)) == 0;
+    for (int i = tid; i < own * (cols >> 1); i += 32 * WARPS) {
+      const int in = i / (cols >> 1), d = (i - in * (cols >> 1)) * 2, row = sp * own + in, gr = row0 + row;
+      if (row >= RB || gr >= rows_total) break;  // rows ascend with i
+      float top = -CUDART_INF_F;
+      for (int s = 0; s < n_splits; ++s) top = fmaxf(top, recv_ml[2 * (s * own + in)]);
+      float sum = 0.f, v0 = 0.f, v1 = 0.f;
+      for (int s = 0; s < n_splits; ++s) {
+        const float m = recv_ml[2 * (s * own + in)], f = m == -CUDART_INF_F ? 0.f : exp2f(m - top);
+        const float2 v = *reinterpret_cast<const float2*>(recv + (size_t)(s * own + in) * cols + d);
+        sum = fmaf(recv_ml[2 * (s * own + in) + 1], f, sum);
+        v0 = fmaf(v.x, f, v0), v1 = fmaf(v.y, f, v1);
+      }
+      const float inv = 1.0f / sum;
+      bf16* dst = out + (size_t)(qs + t0 + gr / H) * p.out_stride + (size_t)(gr % H) * p.rank + d;
+      if (pairs && d < p.rank) {
+        *reinterpret_cast<__nv_bfloat162*>(dst) = __floats2bfloat162_rn(v0 * inv, v1 * inv);
+      } else {
+        if (d < p.rank) dst[0] = __float2bfloat16_rn(v0 * inv);
+        if (d + 1 < p.rank) dst[1] = __float2bfloat16_rn(v1 * inv);
+      }
+    }
+    return;
+  }
 #pragma unroll
   for (int half = 0; half < 2; ++half) {
     const int gr = half ? row_b : row_a;
@@ -835,6 +886,17 @@ __global__ __launch_bounds__(32 * WARPS) void latent_attn_mma_kernel(LatentParam
       }
     }
   }
+}
+
+static int latent_sm_count() {
+  static int n_sms = 0;
+  if (n_sms == 0) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, dev);
+    if (n_sms <= 0) n_sms = 1;
+  }
+  return n_sms;
 }
 
 constexpr size_t LATENT_PART_BYTES = 4 * 32 * 16;  // a warp's partial scores, tiles of 32 keys
@@ -869,15 +931,46 @@ static inline void launch_latent_mma(const LatentParams& p, const int* tiles, in
     launch_pdl_split(false, latent_attn_mma_kernel<NVW, DVS, NKT>, dim3((LT_Q * p.n_heads + RB - 1) / RB, n_tiles), 128, smem, stream, p,
                tiles, decode_reqs, 0, 1, part_o, part_ml);
   if (n_decode > 0) {
+    constexpr auto kernel = latent_attn_mma_kernel<NVW_DEC, DVS_DEC, 4, WARPS_DEC>;
+    const dim3 grid(n_decode, (p.n_heads + RB_DEC - 1) / RB_DEC, n_splits);
     const size_t smem_dec = (size_t)(RB_DEC + 2 * KT_DEC) * (Wk + 8) * 2 + (DVS_DEC >= 4 ? DVS_DEC * LATENT_PART_BYTES : 0);
+    if constexpr (DVS_DEC >= 4) {
+      // Three to eight parts that stand on the SMs at once, a block each, meet as a cluster (16 heads, latents of 512, us, with a merge
+      // kernel / as a cluster: 8 requests of 544 keys in 8 parts 16.4 / 13.7, in 4 20.9 / 19.3, in 2 30.7 / 32.1; of 128 keys in 4 10.6 / 9.2; 18
+      // requests in 8, where blocks share SMs, 16.5 / 16.7).  More parts meet through memory and a kernel of their own.
+      const int own = (RB_DEC + n_splits - 1) / n_splits;
+      const size_t smem_all = smem_dec + (size_t)n_splits * own * (((p.rank + 7) & ~7) + 2) * 4;
+      if (n_splits >= 3 && n_splits <= 8 && (long)grid.x * grid.y * grid.z * 4 <= 3L * latent_sm_count() && smem_all <= 220 * 1024) {
+        constexpr auto clustered = latent_attn_mma_kernel<NVW_DEC, DVS_DEC, 4, WARPS_DEC, true>;
+        static size_t granted_all = 0;
+        if (smem_all > 48 * 1024 && smem_all > granted_all) {
+          cudaFuncSetAttribute(clustered, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_all);
+          granted_all = smem_all;
+        }
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = grid;
+        cfg.blockDim = dim3(32 * WARPS_DEC);
+        cfg.dynamicSmemBytes = smem_all;
+        cfg.stream = stream;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = 1;
+        attr[1].val.clusterDim.y = 1;
+        attr[1].val.clusterDim.z = n_splits;
+        cfg.attrs = attr;
+        cfg.numAttrs = 2;
+        note_launch(launch_kernel(cfg, clustered, p, tiles, decode_reqs, 1, n_splits, part_o, part_ml));
+        return;
+      }
+    }
     static size_t granted_dec = 0;
     if (smem_dec > 48 * 1024 && smem_dec > granted_dec) {
-      cudaFuncSetAttribute(latent_attn_mma_kernel<NVW_DEC, DVS_DEC, 4, WARPS_DEC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)smem_dec);
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_dec);
       granted_dec = smem_dec;
     }
-    launch_pdl(latent_attn_mma_kernel<NVW_DEC, DVS_DEC, 4, WARPS_DEC>, dim3(n_decode, (p.n_heads + RB_DEC - 1) / RB_DEC, n_splits),
-               32 * WARPS_DEC, smem_dec, stream, p, tiles, decode_reqs, 1, n_splits, part_o, part_ml);
+    launch_pdl(kernel, grid, 32 * WARPS_DEC, smem_dec, stream, p, tiles, decode_reqs, 1, n_splits, part_o, part_ml);
     if (n_splits > 1)
       launch_pdl(latent_attn_merge_kernel<__nv_bfloat16>, dim3(n_decode, p.n_heads), 128, 0, stream,
                  (const float*)part_o, (const float*)part_ml, n_splits, decode_reqs, p.q_start, p.slots,

@@ -101,7 +101,7 @@ def test_norm_added_with_the_row_in_registers(width):
 
 # one warp's rows in four warps and in eight, two warps' rows, four's; latents that end inside a slice and rows that end inside a step of
 # 32; pages of a power of two and of 24; requests of one key, of part of a tile of keys, of whole tiles, of parts without a key
-@pytest.mark.parametrize("splits", [1, 3])
+@pytest.mark.parametrize("splits", [1, 2, 3, 8, 9])  # whole, in clusters, more parts than a cluster takes
 @pytest.mark.parametrize("heads,rank,rot,page", [(16, 512, 64, 16), (3, 40, 8, 24), (16, 100, 20, 8), (5, 200, 8, 24), (20, 512, 40, 16), (40, 128, 24, 16)])
 def test_decoded_tokens_in_parts(heads, rank, rot, page, splits):
     lens, width = [1, 31, 33, 64, 200, 371], rank + rot
