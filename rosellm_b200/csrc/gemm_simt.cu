@@ -1,9 +1,9 @@
 // Matrix products on the CUDA cores: out[M,N] = A[M,K] * W[N,K]^T, with the epilogues the
 // model needs fused in: + bias[N]; GELU; and accumulation into a float32 residual stream.
 //
-// This is the whole matrix path of the 32-bit mode (IEEE float32 FMA, no tensor-core mode of
-// reduced precision), and the small-batch path of the bfloat16 mode, where a product streams
-// the weights once and is bound by memory, not arithmetic.  The formulas fused here:
+// This is the matrix path of the 32-bit mode (IEEE float32 FMA; products of many rows with inner sizes
+// from 256 go to gemm_f32_tc.cu, whose error is no larger), and the small-batch path of the bfloat16
+// mode, where a product streams the weights once and is bound by memory, not arithmetic.  The formulas fused here:
 //   y = a W + b                           rosellm/rosetrainer/model.py:95, 220, 334-337
 //   gelu_tanh(u) = 0.5 u (1 + tanh(sqrt(2/pi) (u + 0.044715 u^3)))   model.py:274-277,
 //                                                                    fused_mlp.py:79-89

@@ -8,16 +8,16 @@
 // not memory is the bound.  The reference leaves these products to cuBLAS through torch.
 //
 // One block per SM walks the output tiles of 128 rows x BN columns; BN (a multiple of 32 up to
-// 256) is chosen per product so that the tiles fill their rounds over the SMs (2048 x 3072 takes
-// 192 columns: 256 tiles in two rounds; 2048 x 768 takes 96: 128 tiles in one).
+// 256) is chosen per product so that the tiles fill their rounds over the SMs (2048 x 768 takes
+// 96: 128 tiles in one round); or pairs of SMs walk tiles of 256 rows, or parts of K go to the blocks of a cluster (plan_cut).
 // Its warps have fixed roles:
-//   warp 0     one lane issues the TMA loads of the W tiles (BN x 64 bfloat16, 128-byte swizzle)
+//   warp 0     issues the TMA loads of the W tiles (BN x 64 bfloat16, 128-byte swizzle)
 //              into a ring of shared-memory stages, running ahead over tiles; those of its first
 //              stages it asks for before it waits for the kernels ahead (weights are written by
 //              none of them);
-//   warp 18    one lane issues the loads of the A tiles (128 x 64) into the same stages: one lane
+//   warp 18    issues the loads of the A tiles (128 x 64) into the same stages: one warp
 //              for both took longer over a stage than the tensor pipe does;
-//   warp 1     allocates tensor memory for two accumulators; one lane issues tcgen05.mma
+//   warp 1     allocates tensor memory for two accumulators; issues tcgen05.mma
 //              (M=128, N=BN, K=16, four per stage) and commits to the stage's "empty" barrier
 //              and, after a tile's last K block, to that accumulator's "full" barrier; ring
 //              position and operand descriptors are stepped along, so that issuing a product

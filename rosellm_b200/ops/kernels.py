@@ -25,9 +25,9 @@ STATUS_BITS = {
     8: "a bounded wait inside a kernel gave up",
 }
 
-# Rows up to which a float32 product streams the weights once per group of rows instead of
-# tiling, both in IEEE arithmetic on the CUDA cores (csrc/gemm_simt.cu); which kernel a
-# bfloat16 product runs on: bf16_path.
+# Rows up to which a float32 product streams the weights once per group of rows on the CUDA cores
+# (csrc/gemm_simt.cu) instead of tiling, there or on the tensor cores (csrc/gemm_f32_tc.cu); which
+# kernel a bfloat16 product runs on: bf16_path.
 ROWS_STREAMING_LIMIT = 64
 
 
@@ -539,14 +539,15 @@ def linear(a, weight, bias, out, *, act: int = ACT_NONE, residual: bool = False,
     at most 16 rows).  Otherwise
     a [rows, k] (row stride a multiple of 8), weight [n, k] contiguous, both float32 or both
     bfloat16; out [rows, n] of a's dtype or float32.  Which kernel runs: float32 up to 64 rows
-    the row kernel, above it tiles (both IEEE FMAs); bfloat16 up to 16 rows the
+    the row kernel, above it tiles of FMAs or, from an inner size of 256 where it is faster, of tf32 parts; bfloat16 up to 16 rows the
     weight-streaming kernels (fed by TMA through a ring; for a very wide float32 output, a head, by
-    bulk copies; by registers otherwise: the library chooses), above it as ``bf16_path`` says.  ``path`` (for tests) forces
-    ``"rows"``, ``"tile"``, ``"mma"``, ``"smem"``, ``"tc"`` or ``"tcr"``.  ``kv``: output columns from
+    bulk copies; by registers otherwise: the library chooses), above it as ``bf16_path`` and ``clustered_is_ahead`` say.  ``path``
+    (for tests) forces ``"rows"``, ``"tile"``, ``"f32tc"``, ``"mma"``, ``"smem"``, ``"tc"`` or ``"tcr"``.  ``kv``: output columns from
     ``kv.q_width`` on are written into cache pages, not ``out`` (not with ``"tile"``).
     ``tile_width`` and ``splits`` (for tests and measurements, ``"tc"`` only): the columns of an
     output tile, a multiple of 32 up to 256, and the parts the inner size is cut into (1, 2, 3, 4, 6
-    or 8: the blocks of a cluster take one each), instead of what the kernel would choose.
+    or 8: the blocks of a cluster take one each; -2: tiles of 256 rows over pairs of SMs), instead of what the kernel would choose
+    (``tile_width`` with ``"f32tc"`` too).
     ``head``: the outputs are logits, whose tokens ``linear_sample`` may be asked for in their place: the same sums in
     the same order as there, bit for bit (tiles then never cut the inner size).
     """
