@@ -314,7 +314,10 @@ __global__ __launch_bounds__(32 * WARPS) void attn_decode_kernel(
   // [warps][STAGES][2][SUB][32 lanes][WORDS], behind the static part; on a boundary of 128 bytes: 16 bytes off one of 32, the
   // copies' sectors were cut in two and every form took 17% longer
   extern __shared__ __align__(128) uint32_t ring[];
-  __shared__ float ml_s[CLUSTER ? WARPS + 1 : WARPS][2];  // of the warps (then of the block)
+  __shared__ float ml_s[WARPS][2];  // of the warps
+  // what the blocks of a cluster send the first one: their outputs, and their (maximum, sum)
+  __shared__ float sent_o[CLUSTER ? 8 : 1][CLUSTER ? 8 * EPL : 1];
+  __shared__ float2 sent_ml[CLUSTER ? 8 : 1];
   // The batch's description (written by the host before the step) and the keys and values of
   // earlier steps do not depend on the kernels ahead: they are fetched before the wait for
   // those.  What the kernel ahead does write is read after it: the query, and the key and
@@ -344,6 +347,8 @@ __global__ __launch_bounds__(32 * WARPS) void attn_decode_kernel(
     if (total <= DECODE_CLUSTER_KEYS) {
       if (sp > 0) return;
       n_splits = 1;
+    } else {
+      asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");  // waited for before results are sent
     }
   }
   const int chunk = ((total + n_splits - 1) / n_splits + 31) / 32 * 32;
@@ -504,42 +509,45 @@ __global__ __launch_bounds__(32 * WARPS) void attn_decode_kernel(
     ll += ml_s[w][1] * f[w];
   }
   if (CLUSTER && n_splits > 1) {
-    // the block's result to its own shared memory, behind the warps'; the first block adds the parts up in their order
-    float* o_block = o_s + WARPS * dh;
+    // every block sends its result to the first, which adds the parts up in their order; the others have done then
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+    const uint32_t to = peer_addr((uint32_t)__cvta_generic_to_shared(&sent_o[sp][0]), 0u);
     for (int d = tid; d < dh; d += blockDim.x) {
       float acc = 0.f;
 #pragma unroll
       for (int w = 0; w < WARPS; ++w) acc = fmaf(o_s[w * dh + d], f[w], acc);
-      o_block[d] = acc;
+      asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(to + 4u * (uint32_t)d), "f"(acc) : "memory");
     }
-    if (tid == 0) {
-      ml_s[WARPS][0] = mm;
-      ml_s[WARPS][1] = ll;
-    }
-    cluster_sync();
-    for (int d = sp == 0 ? tid : dh; d < dh; d += blockDim.x) {
-      float mp[8], lp[8], op[8];
-      const uint32_t ml_a = (uint32_t)__cvta_generic_to_shared(&ml_s[WARPS][0]), o_a = (uint32_t)__cvta_generic_to_shared(o_block + d);
+    if (tid == 0)
+      asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(peer_addr((uint32_t)__cvta_generic_to_shared(&sent_ml[sp]), 0u)),
+                   "f"(mm), "f"(ll)
+                   : "memory");
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    if (sp > 0) return;
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    for (int d = tid; d < dh; d += blockDim.x) {
+      float2 ml[8];
+      float op[8];
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {  // unconditional (the last block's again): all on their way before the first is used
-        const uint32_t r = (uint32_t)min(q, n_splits - 1);
-        asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(mp[q]), "=f"(lp[q]) : "r"(peer_addr(ml_a, r)) : "memory");
-        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(op[q]) : "r"(peer_addr(o_a, r)) : "memory");
+      for (int q = 0; q < 8; ++q) {  // unconditional (the last part's again): all on their way before the first is used
+        const int r = min(q, n_splits - 1);
+        ml[q] = sent_ml[r];
+        op[q] = sent_o[r][d];
       }
       float top = -CUDART_INF_F;
 #pragma unroll
-      for (int q = 0; q < 8; ++q) top = fmaxf(top, mp[q]);
+      for (int q = 0; q < 8; ++q) top = fmaxf(top, ml[q].x);
       float den = 0.f, acc = 0.f;
 #pragma unroll
       for (int q = 0; q < 8; ++q)
-        if (q < n_splits && mp[q] != -CUDART_INF_F) {  // a part may be without keys
-          const float e = ex(mp[q] - top);
-          den = fmaf(lp[q], e, den);
+        if (q < n_splits && ml[q].x != -CUDART_INF_F) {  // a part may be without keys
+          const float e = ex(ml[q].x - top);
+          den = fmaf(ml[q].y, e, den);
           acc = fmaf(op[q], e, acc);
         }
       ((T*)p.out)[(size_t)n * p.out_stride + h * dh + d] = from_f32<T>(acc / den);
     }
-    cluster_sync();  // no block ends while the first may still read its result
     return;
   }
   const size_t base = ((size_t)di * p.n_heads + h) * n_splits + sp;
