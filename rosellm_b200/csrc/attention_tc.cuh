@@ -44,6 +44,7 @@ constexpr int ATT_SOFTMAX_THREADS = 512;
 constexpr int ATT_Q_BYTES = ATT_Q * ATT_DH * 2;        // 16 KB
 constexpr int ATT_KV_BYTES = ATT_KV * ATT_DH * 2;      // 16 KB: keys or values of a tile
 constexpr int ATT_P_BYTES = ATT_Q * ATT_KV * 2;        // 32 KB: two K blocks of 64 keys
+constexpr int ATT_PAIRED = 4;                          // pieces of 128 queries of a request that go in pairs where the grid leaves a choice
 constexpr int ATT_STAGES = 3;                          // tiles of keys and values in shared memory
 // The probabilities lie in two buffers: those of tile g are written while the P V of tile g - 1 may still read its own (only the
 // P V of g - 2 has been waited for by then).  The block has its SM to itself either way.
@@ -136,7 +137,7 @@ struct AttQueries {
 // every block walks about the same number of key tiles, and all blocks run in one round), the
 // block of the middle piece takes it alone, and the others' blocks leave at once.
 // singly (grid: heads, tiles): every piece has a block of its own, the pieces with the most keys of a request first, for
-// grids whose pairs would need a second round of blocks (see launch_attn_tc).
+// grids whose pairs would need a second round of blocks (see launch_attn_tc); 2: those of requests of more than ATT_PAIRED pieces.
 // map_q: the step's queries [tokens][heads * 64]; map_kv: this layer's pool as rows of 64
 // [pages * 2 * kv heads * page size][64], a box being one page of one head.
 __global__ __launch_bounds__(ATT_THREADS, 1) void attn_tc_kernel(const __grid_constant__ CUtensorMap map_q,
@@ -166,11 +167,12 @@ __global__ __launch_bounds__(ATT_THREADS, 1) void attn_tc_kernel(const __grid_co
   const int kv_len = p.kv_len[req];
   const int slot = p.slots[req];
   const int piece = entry_t0 / ATT_Q, n_pieces = (q_len + ATT_Q - 1) / ATT_Q;
-  if (!singly && piece > n_pieces - 1 - piece) return;  // taken by the block of its partner
-  const int n_turns = !singly && piece < n_pieces - 1 - piece ? 2 : 1;
+  const bool alone = singly == 1 || (singly == 2 && n_pieces > ATT_PAIRED);
+  if (!alone && piece > n_pieces - 1 - piece) return;  // taken by the block of its partner
+  const int n_turns = !alone && piece < n_pieces - 1 - piece ? 2 : 1;
   auto queries_of = [&](int turn) {
     AttQueries q;
-    q.t0 = (turn == 0 && !singly ? n_pieces - 1 - piece : piece) * ATT_Q;  // the longer walk first
+    q.t0 = (turn == 0 && !alone ? n_pieces - 1 - piece : piece) * ATT_Q;  // the longer walk first
     q.rows = min(ATT_Q, q_len - q.t0);
     q.first_pos = kv_len - q_len + q.t0;
     q.kv_hi = q.first_pos + q.rows;
@@ -543,12 +545,15 @@ static inline int launch_attn_tc(const AttnParams& p, const int* tiles, int n_ti
     if (n_sms <= 0) n_sms = 1;
   }
   const long pairs = (long)(n_tiles + 3) / 4 * p.n_heads, places = (pairs + n_sms - 1) / n_sms * n_sms;
-  // Up to eight pieces to five SMs go singly as well: their longest, started first, end before a pair of a long and a short
-  // piece does (12 heads, 2 prompts of 1024: eight key tiles against nine).
-  const bool few = 2 * pairs * 5 <= 8 * n_sms;
-  const bool singly = (few || (pairs > n_sms && 5 * places > 6 * pairs)) && n_tiles <= 65535;  // (the limit of a grid's second extent)
+  // Pieces that all stand on the SMs at once go singly as well, and up to eight pieces to five SMs where a request has more than four: the
+  // longest, started first, end before a pair of a long and a short piece does (us, pairs / singly: 12 heads, 2 prompts of 512 14.2 (the
+  // form before) / 10.0, 2 of 1024 19.6 / 17.1, 2 of 896 18.2 / 14.4, 3 of 640 15.7 / 15.1, one of 2048 29.3 / 25.1); shorter
+  // requests' pieces in a second round cost their blocks' start again: 4 of 512 14.8 / 16.7, 4 of 400 14.2 / 16.2.
+  const bool round = pairs > n_sms && 5 * places > 6 * pairs;
+  const int mode = n_tiles > 65535 ? 0 : (round || 2 * pairs <= n_sms) ? 1 : (2 * pairs * 5 <= 8 * n_sms) ? 2 : 0;  // (a grid's second extent)
+  const bool singly = mode != 0;
   const dim3 grid = singly ? dim3(p.n_heads, n_tiles) : dim3(n_tiles, p.n_heads);
-  launch_pdl_split(false, attn_tc_kernel, grid, ATT_THREADS, ATT_SMEM, stream, mq, mkv, p, tiles, singly ? 1 : 0);
+  launch_pdl_split(false, attn_tc_kernel, grid, ATT_THREADS, ATT_SMEM, stream, mq, mkv, p, tiles, mode);
   return 0;
 }
 
