@@ -10,7 +10,8 @@
 // instead of four (few requests: a block then covers 256 keys a round), or (1, not 2) eight where
 // the device would take a second round over blocks of sixteen.  With
 // n_splits > 1, part_o holds n_decode*heads*n_splits*head_dim floats and part_ml
-// n_decode*heads*n_splits*2.  n_tokens: rows of q; n_pages: pages of the pool (both bound the
+// n_decode*heads*n_splits*2, or (decode_wide, 2 to 8 parts) both are null and the parts are the blocks of
+// clusters.  One without the other is refused.  n_tokens: rows of q; n_pages: pages of the pool (both bound the
 // TMA tensor maps of the tcgen05 kernel).
 //
 // old_keys_settled: the decode kernel is launched with programmatic dependent launch and, when
@@ -32,8 +33,9 @@ RL_EXPORT int rl_attention(int dtype, const void* q, long q_stride, const void* 
                            cudaStream_t stream) {
   if (head_dim % 16 != 0 || head_dim <= 0 || head_dim > 256) return -2;
   if (n_kv_heads <= 0 || n_heads % n_kv_heads != 0) return -3;
-  if (n_splits < 1 || n_splits > 65535 || ((n_splits > 8 || decode_wide == 0) && n_splits > 1 && (part_o == nullptr || part_ml == nullptr)))
-    return -4;
+  if (n_splits < 1 || n_splits > 65535) return -4;
+  const bool in_clusters = n_splits <= 8 && decode_wide != 0 && part_o == nullptr && part_ml == nullptr;
+  if (n_splits > 1 && !in_clusters && (part_o == nullptr || part_ml == nullptr)) return -4;
   if (status == nullptr) return -6;
   rl::AttnParams p{q, q_stride, pool, block_table, bt_stride, q_start, kv_len, slots, out,
                    out_stride, n_heads, n_kv_heads, head_dim, page_size, window, scale, status, old_keys_settled};
