@@ -95,10 +95,14 @@ inline void note_kernel(LaunchNotes& notes, const cudaLaunchConfig_t& cfg, const
   }
 }
 
-// Every launch of the library: made, and noted where its thread is taking notes.
+// Kernels this host thread has launched so far (rl_launches_made): how many an entry point launches can hang on sizes that only it looks at.
+inline thread_local int launches_made = 0;
+
+// Every launch of the library: made, counted, and noted where its thread is taking notes.
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_kernel(const cudaLaunchConfig_t& cfg, void (*kernel)(KArgs...), Args... args) {
   if (launch_notes != nullptr) note_kernel(*launch_notes, cfg, (const void*)kernel, static_cast<std::decay_t<KArgs>>(args)...);
+  ++launches_made;
   return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
 }
 }  // namespace rl

@@ -6,6 +6,9 @@
 
 #include "common.cuh"
 
+// How many kernels the entry points have launched on this host thread (rl_notes_replay's are not among them).
+RL_EXPORT int rl_launches_made() { return rl::launches_made; }
+
 // From here on this thread's launches are noted, until rl_notes_end.  0, or -2 when they are being noted already.
 RL_EXPORT int rl_notes_begin() {
   if (rl::launch_notes != nullptr) return -2;

@@ -122,7 +122,7 @@ class _RecordingLib:
 _NOT_KERNELS = ("rl_copy_to_device", "rl_event_record")  # library functions that put something else on the stream
 _QUERIES = ("rl_gemm_tc_rows_fits", "rl_gemm_rows_smem_fits", "rl_mlp_fused_slice", "rl_attn_block_fused_fits", "rl_attn_block_fused_cluster",
             "rl_host_memory_on_device", "rl_latent_attention_fits", "rl_latent_decode_fits",
-            "rl_gemm_rows_ring_fits", "rl_gemm_tile_f32_for", "rl_moe_max_tiles", "rl_bias_attention_shape", "rl_recurrence_record", "rl_rmsnorm_add_experts_fits")  # library functions that launch nothing
+            "rl_launches_made", "rl_gemm_rows_ring_fits", "rl_gemm_tile_f32_for", "rl_moe_max_tiles", "rl_bias_attention_shape", "rl_recurrence_record", "rl_rmsnorm_add_experts_fits")  # library functions that launch nothing
 
 
 class recording:
@@ -282,9 +282,10 @@ def _need(t: torch.Tensor, name: str, dtype: torch.dtype | None = None, contiguo
         raise KernelError(f"{name} must be contiguous")
 
 
-def _ok(rc: int, what: str) -> None:
+def _ok(rc: int, what: str, made: int | None = None) -> None:
+    """``made``: what ``rl_launches_made`` said before the call, where the library alone knows how many kernels it takes."""
     global _launches
-    _launches += 1
+    _launches += 1 if made is None else _lib().rl_launches_made() - made
     if rc != 0:
         if rc > 0:
             raise KernelError(f"{what}: CUDA error {rc} at launch")
@@ -1061,6 +1062,7 @@ def attention(q, pool, block_table, q_start, kv_len, slots, out, *, n_heads: int
             raise KernelError("attention: scratch for the split partial results is too small")
         _need(part_o, "part_o", torch.float32)
         _need(part_ml, "part_ml", torch.float32)
+    made = _lib().rl_launches_made()
     rc = _lib().rl_attention(_code(q), _ptr(q), q.stride(0), _ptr(pool), _ptr(block_table), block_table.stride(0),
                              _ptr(q_start), _ptr(kv_len), _ptr(slots), _ptr(out), out.stride(0),
                              n_heads, n_kv, dh, page_size, int(window or 0), float(scale),
@@ -1072,9 +1074,7 @@ def attention(q, pool, block_table, q_start, kv_len, slots, out, *, n_heads: int
     if rc == -5:
         raise KernelError("attention: the tcgen05 kernel takes bfloat16, head size 64, no window and pages of "
                           "8 to 128 tokens that divide 128")
-    _ok(rc, "attention")
-    global _launches
-    _launches += (1 if n_tiles and n_decode else 0) + (1 if n_decode and n_splits > 1 else 0)
+    _ok(rc, "attention", made)
 
 
 def sample(logits, temperature, top_k, top_p, seeds, counters, out_ids, kept=None, filtered: bool | None = None) -> None:
@@ -1288,6 +1288,7 @@ def latent_attention(q, pool, block_table, q_start, kv_len, slots, out, *, sink,
         need = n_decode * n_heads * n_splits
         if part_o is None or part_ml is None or part_o.numel() < need * rank or part_ml.numel() < need * 2:
             raise KernelError("latent_attention: scratch for the split partial results is too small")
+    made = _lib().rl_launches_made()
     rc = _lib().rl_latent_attention(_code(q), _ptr(q), q.stride(0), _ptr(pool), _ptr(block_table), block_table.stride(0),
                                     _ptr(q_start), _ptr(kv_len), _ptr(slots), _ptr(out), out.stride(0), _ptr(sink),
                                     n_heads, rank, row_width, page_size, float(scale), _ptr(tiles), n_tiles,
@@ -1295,10 +1296,7 @@ def latent_attention(q, pool, block_table, q_start, kv_len, slots, out, *, sink,
                                     _ptr(part_ml), int(simt_only), _ptr(status_word(q.device)), _stream())
     if rc in (-2, -3):
         raise KernelError(f"latent_attention: sizes not taken (heads {n_heads}, value width {rank}, row width {row_width})")
-    _ok(rc, "latent_attention")
-    global _launches
-    if decode_by_request and n_decode:
-        _launches += (1 if n_tiles else 0) + (1 if n_splits > 1 else 0)
+    _ok(rc, "latent_attention", made)
 
 
 def head_linear(inp, w, out, *, n_tokens: int, n_heads: int, k: int, n: int, in_strides, w_strides, out_strides,
