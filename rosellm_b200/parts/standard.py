@@ -397,6 +397,29 @@ class CausalSelfAttention(Part):
     def cache_spec(self):
         return KVCacheSpec(self.num_kv_heads, self.head_dim, self.window)
 
+    def cluster_parts(self, n_decode: int, span: int, act_dtype: torch.dtype) -> int:
+        """Into how many parts the keys of a decoded request are cut that meet as the blocks of a cluster (eight warps each), without
+        scratch and a kernel to merge them; 0: they don't.  Measured on B200 with 12, 16 and 25 heads of 64 and 8 and 16 heads of 128, 300 to
+        8,192 keys, in bfloat16 and (to 4,100 keys) 32 bits, wherever this rule has them: at most 1% behind the plans without clusters, us, without /
+        with.  Up to a quarter of the SMs: 12 heads of 64, 300 keys 3.5 / 2.9, 900 6.1 / 3.1, 3000 11.5 / 5.4; 25 heads, 544 4.9 / 3.6; 8 of 128,
+        900 12.0 / 4.6; 12 in 32 bits, 900 11.2 / 4.5.  From 4,096 keys on the plan without has four parts a request and wins while those stand on the SMs at
+        once (16 heads of 64 on 4, 8192 keys 9.8 / 11.5; of 128 17.3 / 21.5), not beyond (24 heads, 8192 18.8 / 14.1).  Up to 9/20 of them:
+        48 heads, 544 keys 5.0 / 4.0, 8192 25.2 / 22.3; 64 of 128 53.3 / 48.1; in 32 bits, 3000 20.5 / 18.5.  Just above one head an SM: 200 heads, 300 keys
+        5.8 / 5.9, 544 8.9 / 7.8, 8192 85.5 / 68.9; 192 in 32 bits, 544 17.1 / 11.6.  Between, and above 3/2 heads an SM, whole walks are as fast
+        (96 to 144 heads, 544 keys 6.4 / 6.8, 900 8.7 / 8.7; 288 13.0 / 15.1).  Larger keys (32 bits, heads of 128) lose up to 1.6 times in the few
+        parts that they would have.  Up to 256 keys the kernel takes a request whole."""
+        if self.window is not None:
+            span = min(span, self.window)
+        units, sms = n_decode * self.num_heads, K.sm_count()
+        key_bytes = 2 * self.head_dim * (2 if act_dtype == torch.bfloat16 else 4)
+        if not 300 <= span <= 8192 or key_bytes > 512:
+            return 0
+        if units <= sms // 4:
+            return max(3, min(8, span // 100)) if span < 4096 or units * (span // 1024) > sms else 0
+        if units <= sms * 9 // 20 and span >= 500:
+            return 6
+        return 2 if sms < units <= sms * 3 // 2 else 0
+
     def decode_plan_for(self, n_decode: int, span: int, act_dtype: torch.dtype = torch.bfloat16) -> tuple[int, bool]:
         """(splits, wide): over how many blocks the keys of one decoded request are split when
         ``n_decode`` requests attend over about ``span`` keys each, and whether the blocks have
@@ -409,18 +432,9 @@ class CausalSelfAttention(Part):
         units = n_decode * self.num_heads
         sms = K.sm_count()
         if units <= 2 * sms:
-            # Parts of up to eight are the blocks of a cluster (eight warps each).  Measured on B200 with heads of 64 in
-            # bfloat16, us, whole (sixteen warps a block, or eight) / in parts: 25 heads of one request, 544 keys 5.3 / 4.2, 900
-            # 7.0 / 4.6, four requests of 12 heads 5.7 / 5.1 and 8.5 / 6.4 (six parts); 200 heads, 320 keys 7.8 / 7.2, 544
-            # 11.7 / 9.4, 900 16.9 / 13.3 (two); 96 to 144 heads stand at one block an SM each and gain nothing
-            # (6.4 / 6.8, 900 keys 8.7 / 8.7), nor do 288 (13.0 / 15.1).  Up to 256 keys the kernel takes them whole.
-            if span >= 300 and 2 * self.head_dim * (2 if act_dtype == torch.bfloat16 else 4) <= 512 and span <= 8192:
-                if units <= sms // 4:
-                    return max(3, min(8, span // 100)), True
-                if units <= sms * 9 // 20 and span >= 500:
-                    return 6, True
-                if sms < units <= sms * 3 // 2:
-                    return 2, True
+            parts = self.cluster_parts(n_decode, span, act_dtype)
+            if parts:
+                return parts, True
             return max(1, min(span // 1024, 2 * sms // units, 32)), True   # up to four rounds a block
         # Narrow blocks: a few fit on an SM (shared memory); where they do not all run at once the
         # kernel takes its dense form (twice as many an SM, each slower), and what is still left
@@ -484,11 +498,15 @@ class CausalSelfAttention(Part):
         nothing to do with it)."""
         return ctx.max_tile_kv_len >= TC_ATTENTION_MIN_CONTEXT
 
+    def _decode_in_cluster(self, ctx, splits: int, wide: bool) -> bool:
+        """Whether the parts of a step's plan are those that ``cluster_parts`` has meet in clusters."""
+        return wide and splits > 1 and splits == self.cluster_parts(ctx.n_decode, self._decode_span(ctx), ctx.act_dtype)
+
     def launch_key(self, ctx) -> tuple:
-        """The longest context decides how decoded requests are split over blocks, how many warps those have, and
-        which kernel takes the prompt portions."""
+        """The longest context decides how decoded requests are split over blocks, how many warps those have and whether they are clusters,
+        and which kernel takes the prompt portions."""
         plan = ctx.extras.get("decode_plan") or self.decode_plan(ctx) if ctx.n_decode else None
-        return (plan, self.decode_sixteen_for(plan[0], self._decode_span(ctx), ctx.act_dtype) if plan else None,
+        return (plan, plan and self._decode_in_cluster(ctx, *plan), self.decode_sixteen_for(plan[0], self._decode_span(ctx), ctx.act_dtype) if plan else None,
                 self._tc_prompt_attention(ctx) if ctx.n_tiles else None)
 
     def bind(self, tensors) -> None:
@@ -541,7 +559,7 @@ class CausalSelfAttention(Part):
         o = ctx.workspace.get("attn_out", (n, self.q_width), ctx.act_dtype)
         splits, wide = ctx.extras.get("decode_plan") or self.decode_plan(ctx)
         part_o = part_ml = None
-        if splits > 8 or (splits > 1 and not wide):
+        if splits > 1 and not self._decode_in_cluster(ctx, splits, wide):
             rows = ctx.n_decode * self.num_heads * splits
             part_o = ctx.workspace.get("attn_part_o", (rows, self.head_dim), torch.float32)
             part_ml = ctx.workspace.get("attn_part_ml", (rows, 2), torch.float32)
