@@ -205,7 +205,7 @@ __global__ __launch_bounds__(THREADS, 1) void gemm_f32_tc_kernel(const __grid_co
     bool ok = true;
     for (int unit = blockIdx.x; unit < units && ok; unit += gridDim.x)
       for (int kb = 0; kb < kbs; ++kb) {
-        ok = tc::mbar_wait(full_bar(s), ph, abort_flag, p.status);
+        ok = tc::mbar_wait_warp(full_bar(s), ph, abort_flag, p.status);
         if (!ok) break;
         float4* x = reinterpret_cast<float4*>(smem + s * STAGE) + (tid - 64);
         float4* low = reinterpret_cast<float4*>(smem + s * STAGE + OPERANDS) + (tid - 64);
@@ -242,7 +242,7 @@ __global__ __launch_bounds__(THREADS, 1) void gemm_f32_tc_kernel(const __grid_co
       for (int i = 0; i < COLS; ++i) acc[i] = 0.f;
       for (int kb0 = 0; kb0 < kbs; kb0 += CHUNK, ++chunk) {
         const int buf = chunk & 1;
-        ok = __all_sync(0xffffffffu, tc::mbar_wait(acc_full(buf), (uint32_t)(chunk >> 1) & 1u, abort_flag, p.status));
+        ok = tc::mbar_wait_warp(acc_full(buf), (uint32_t)(chunk >> 1) & 1u, abort_flag, p.status);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t main = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * 2 * BN + part * COLS);

@@ -363,7 +363,7 @@ __global__ __launch_bounds__(PTHREADS, 1) void gemm_tc_persistent_kernel(const _
           if (col < N) bias0 = p.bias[col];
           if (part + 4 < BN / 32 && col + 128 < N) bias1 = p.bias[col + 128];
         }
-        ok = mbar_wait(acc_full(buf), (local >> 1) & 1u, abort_flag, p.status);
+        ok = mbar_wait_warp(acc_full(buf), (local >> 1) & 1u, abort_flag, p.status);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t acc_addr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)buf * acc_stride;
@@ -538,7 +538,7 @@ __global__ __launch_bounds__(PTHREADS, 1) void gemm_tc_persistent_kernel(const _
         const int own_c = part * splits + rank;
         float bias_own = 0.f;
         if (p.bias != nullptr && own_c < BN / 32 && n0 + own_c * 32 + lane < N) bias_own = p.bias[n0 + own_c * 32 + lane];
-        ok = mbar_wait(acc_full(0), 0u, abort_flag, p.status);
+        ok = mbar_wait_warp(acc_full(0), 0u, abort_flag, p.status);
         RL_PHASE_OF(6, 64);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         cluster_sync();
@@ -594,7 +594,7 @@ __global__ __launch_bounds__(PTHREADS, 1) void gemm_tc_persistent_kernel(const _
             if (col < N) bias0 = p.bias[col];
             if (part + 4 < BN / 32 && col + 128 < N) bias1 = p.bias[col + 128];
           }
-          ok = mbar_wait(acc_full(buf), (local >> 1) & 1u, abort_flag, p.status);
+          ok = mbar_wait_warp(acc_full(buf), (local >> 1) & 1u, abort_flag, p.status);
           if (!ok) break;
           if (local == 0) RL_PHASE_OF(6, 64);
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -654,7 +654,7 @@ __global__ __launch_bounds__(PTHREADS, 1) void gemm_tc_persistent_kernel(const _
             }
           }
         }
-        ok = mbar_wait(acc_full(buf), (local >> 1) & 1u, abort_flag, p.status);
+        ok = mbar_wait_warp(acc_full(buf), (local >> 1) & 1u, abort_flag, p.status);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll 1

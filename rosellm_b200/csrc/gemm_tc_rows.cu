@@ -181,7 +181,7 @@ __global__ __launch_bounds__(RTHREADS) void gemm_tc_rows_kernel(
   // The accumulator's lanes are output columns, its columns rows of A: every row goes to the block that finishes it, the
   // eight warps taking a quarter of the lanes and every second group of 16 rows each.
   if (warp >= 2) {
-    ok = __all_sync(0xffffffffu, mbar_wait(acc_bar, 0u, abort_flag, status));
+    ok = mbar_wait_warp(acc_bar, 0u, abort_flag, status);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (ok) {
       const int quarter = warp & 3;

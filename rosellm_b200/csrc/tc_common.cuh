@@ -90,7 +90,8 @@ __device__ __forceinline__ bool elect_one() {
   return elected != 0;
 }
 
-// mbar_wait by a whole warp, with one answer for all of its lanes.
+// mbar_wait by a whole warp, with one answer for all of its lanes: what a loop that goes on or ends by it needs, where a vote,
+// a shuffle or a barrier of the whole warp follows (lanes that gave up would leave the others waiting there, without a bound).
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status) {
   if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status));
