@@ -3,28 +3,29 @@
 //   out[M,N] = A[M,K] * W[N,K]^T  (+ bias[N]) (GELU) (or out += ..., the float32 residual stream)
 //
 // the products and epilogues of gemm_simt.cu (rosellm/rosetrainer/model.py:95, 220, 334-337; fused_mlp.py:79-113).  An
-// operand is cut into two parts of eleven significant bits, x = hi + lo, hi the nearest tf32 number to x and lo the
-// nearest to the rest, which leaves at most 2^-24 of x (half a unit in its last place).  Of the four products of the parts
-// three are made, hi hi, hi lo and lo hi, each exact in the multiplier; lo lo is below 2^-22 of the product and
-// left out (its sign is random: over a sum it stays far below one rounding).  What costs a sum on this unit its bits is the
-// accumulator, which cuts off instead of rounding: so hi hi and the two small products have an accumulator each, the small
-// one losing nothing that counts, and after CHUNK K blocks of 32 both are drained and added in registers with ordinary
-// float32 additions.  (With two blocks between the additions 5% faster, but sums of 128 positive products were further from 64 bits
-// than single FMAs.)
+// operand is the sum of three bfloat16 numbers, x = hi + mid + lo, each the nearest to what is left: 8 + 8 + 8 bits hold all 24 of a
+// float32 number, and its range is bfloat16's, so nothing is left out.  Eight of the nine products of the parts are
+// made, each exact in the multiplier; lo lo is left out, at most 2^-34 of the product.  What costs a sum on this unit its bits is the
+// accumulator, which cuts off instead of rounding: so hi hi (16 bits a product) and the seven small products have an accumulator each.  The
+// first is drained after CHUNK K blocks of 32 and added in registers with ordinary float32 additions, one rounding a drain as an FMA has
+// one a product; the small one, of 2^-8 of its size, is drained after SPAN K blocks and at the end.  (Two parts of eleven bits, in tf32, are 6 to
+// 16% faster and leave out up to 2^-21 of a product: a sum of one product was up to 7.4 x 2^-24 off, an FMA is 1.0, this 1.0.)
 //
 // One block per SM walks tiles of 128 rows x BN columns.  Its warps:
 //   warp 0      one lane copies tiles of A and W (K blocks of 32 floats = 128 bytes, 128-byte swizzle) by TMA into a ring of
 //               stages; those of W for the first stages before the wait for the kernels ahead;
-//   warps 2-9   cut what arrived: hi takes the place of x, lo goes to the stage's second half, byte for byte at the same
-//               place, so that the swizzle needs no thought;
-//   warp 1      one lane issues tcgen05.mma kind::tf32, twelve of K 8 a K block;
-//   warps 10-17 drain the accumulators (two pairs in turn) and write the tile.
-// Shared memory is what bounds it: a K block of a 128 x 128 tile is read once and written twice by the cutting warps (96 KB)
-// and read three times by the products (96 KB), about 1,500 clocks of its 128 bytes a clock where the tensor pipe needs 770.
+//   warps 2-9   cut what arrived: the 128 bytes of a row take its hi (64 bytes) and its mid behind them, the first half of a
+//               row of 128 bytes in the stage's second half its lo, all in the swizzle of the copy;
+//   warp 1      one lane issues tcgen05.mma kind::f16 (bfloat16), sixteen of K 16 a K block;
+//   warps 10-17 drain the accumulators (two of each in turn) and write the tile.
+// Shared memory is what bounds it: a K block of a 128 x 128 tile is read once and written one and a half times by the cutting warps
+// (96 KB with the conflicts of lo) and read eight times in parts by the products (128 KB), about 1,750 clocks of its 128 bytes a clock
+// where the tensor pipe needs 1,040; measured 1.04 us.  Narrow tiles are a chain of waits, 0.75 us a K block.
 //
-// Measured on B200 between the other kernels of a layer, 1,752 rows of GPT-2 124M, us (the CUDA-core tiles before, now): 2304 x 768
-// 160, 3072 x 768 226, now 82 on average; += 768 x 768 and += 768 x 3072 161 on average, now 73.  Error against 64 bits (2-norm of
-// the difference over that of the result) of those tiles and of this kernel: K 768 2.4e-7, 1.0e-7; K 3072 7.5e-7, 1.8e-7.
+// Measured on B200 in chains of products, 1,752 rows, us (the CUDA-core tiles, this kernel): 2304 x 768 157, 70; 3072 x 768 218, 104; 768 x 768
+// 65, 39; 768 x 3072 247, 118; 1600 x 6400 932, 438.  129 rows: 768 x 768 22.2, 22.4; 2304 x 768 56.6, 22.8; 1600 x 1600 73, 41.
+// Error against 64 bits (2-norm of the difference over that of the FMAs' difference): dense sums 0.25 (K 256), 0.21 (768), 0.19 (3072); sums
+// of one product 1.00, of two to sixteen 0.5 to 1.1; of positive numbers 0.26 to 0.19.
 //
 // Numbers that cannot be cut (infinities, NaN, magnitudes that round to infinity) are noticed while cutting: a block that
 // has met one works its tiles out anew with FMAs from memory, in the order of the CUDA-core kernels.
@@ -39,6 +40,7 @@ namespace f32tc {
 constexpr int BM = 128, BK = 32;
 constexpr int CUT_WARPS = 8, EPI_WARPS = 8, THREADS = 32 * (2 + CUT_WARPS + EPI_WARPS);
 constexpr int CHUNK = 1;  // K blocks between two additions in registers
+constexpr int SPAN = 128;  // K blocks between two drains of the small products' accumulator; a multiple of CHUNK
 constexpr int MAX_STAGES = 4;
 constexpr int A_BYTES = BM * BK * 4;
 __host__ __device__ constexpr int operand_bytes(int bn) { return A_BYTES + bn * BK * 4; }
@@ -61,20 +63,14 @@ struct Args {
   int* status;
 };
 
-__device__ __forceinline__ void mma_tf32(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
+// Two neighbouring numbers' nearest bfloat16 ones, the first in the lower half, and what is left of the numbers (exactly).
+__device__ __forceinline__ uint32_t take_part(float& x, float& y) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+  const uint32_t bits = *reinterpret_cast<const uint32_t*>(&h);
+  x -= __uint_as_float(bits << 16);
+  y -= __uint_as_float(bits & 0xffff0000u);
+  return bits;
 }
-// tf32 x tf32 -> float32, both operands K-major
-__host__ __device__ constexpr uint32_t instr_desc_tf32(int n) {
-  return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
-}
-// The nearest number of eleven significant bits, halves away from zero (an infinity stays one; the largest magnitudes become one).
-__device__ __forceinline__ float to_tf32(float x) { return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u); }
 // A call, not sixteen inlined copies, of four values at a time: one after the other their latencies would add up.
 __device__ __noinline__ float4 act_call(float4 v, int act) {
   return make_float4(apply_act(v.x, act), apply_act(v.y, act), apply_act(v.z, act), apply_act(v.w, act));
@@ -84,7 +80,7 @@ template <int BN>
 __global__ __launch_bounds__(THREADS, 1) void gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a,
                                                                  const __grid_constant__ CUtensorMap map_w, const Args p) {
   constexpr int OPERANDS = operand_bytes(BN), STAGE = 2 * OPERANDS, STAGES = stages_of(BN);
-  constexpr uint32_t TMEM_COLS = 4 * BN;  // two pairs of accumulators
+  constexpr uint32_t TMEM_COLS = 4 * BN;  // two accumulators of hi hi, two of the small products
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const uint32_t smem_base = tc::smem_u32(smem), bar_base = smem_base + STAGES * STAGE;
@@ -164,9 +160,11 @@ __global__ __launch_bounds__(THREADS, 1) void gemm_f32_tc_kernel(const __grid_co
     if (*abort_flag)
       for (int k = it > STAGES ? it - STAGES : 0; k < it; ++k) tc::mbar_wait_quiet(full_bar(k % STAGES), (uint32_t)(k / STAGES) & 1u);
   } else if (warp == 1) {
-    constexpr uint32_t idesc = instr_desc_tf32(BN);
+    constexpr uint32_t idesc = tc::instr_desc(BN);
     const uint64_t desc0 = tc::smem_desc(smem_base);
-    int s = 0, chunk = 0;
+    // (an accumulator of the small products is written again two spans on, when the chunk after the one it was drained with has been
+    // drained as well: the wait for the main accumulator says so)
+    int s = 0, chunk = 0, span = 0;
     uint32_t ph = 0;
     bool ok = true;
     for (int unit = blockIdx.x; unit < units && ok; unit += gridDim.x)
@@ -175,19 +173,25 @@ __global__ __launch_bounds__(THREADS, 1) void gemm_f32_tc_kernel(const __grid_co
         ok = tc::mbar_wait_warp(acc_empty(buf), ((uint32_t)(chunk >> 1) & 1u) ^ 1u, abort_flag, p.status);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t main = tmem_base + (uint32_t)(buf * 2 * BN), small = main + BN;
+        const uint32_t main = tmem_base + (uint32_t)(buf * BN), small = tmem_base + (uint32_t)((2 + (span & 1)) * BN);
         for (int kb = kb0; kb < min(kb0 + CHUNK, kbs); ++kb) {
           ok = tc::mbar_wait_warp(cut_bar(s), ph, abort_flag, p.status);
           if (!ok) break;
-          const uint64_t a_hi = desc0 + (uint64_t)(s * (STAGE >> 4)), w_hi = a_hi + (A_BYTES >> 4);
-          const uint64_t a_lo = a_hi + (OPERANDS >> 4), w_lo = w_hi + (OPERANDS >> 4);
+          const uint64_t a = desc0 + (uint64_t)(s * (STAGE >> 4)), w = a + (A_BYTES >> 4);
           if (tc::elect_one()) {
+            // the parts of a row: descriptors count 16-byte units, a K step of 16 numbers is two of them
+            constexpr uint32_t HI = 0, MID = 4, LO = OPERANDS >> 4;
 #pragma unroll
-            for (int k = 0; k < BK / 8; ++k) {  // K steps of 8 floats: 32 bytes, two units of a descriptor
-              const uint32_t more = kb > kb0 || k > 0 ? 1u : 0u;
-              mma_tf32(small, a_lo + 2 * k, w_hi + 2 * k, idesc, more);
-              mma_tf32(small, a_hi + 2 * k, w_lo + 2 * k, idesc, 1u);
-              mma_tf32(main, a_hi + 2 * k, w_hi + 2 * k, idesc, more);
+            for (int k = 0; k < BK / 16; ++k) {
+              const uint32_t more = kb > kb0 || k > 0 ? 1u : 0u, small_more = kb % SPAN != 0 || k > 0 ? 1u : 0u;
+              tc::mma_f16(small, a + LO + 2 * k, w + MID + 2 * k, idesc, small_more);
+              tc::mma_f16(small, a + MID + 2 * k, w + LO + 2 * k, idesc, 1u);
+              tc::mma_f16(small, a + LO + 2 * k, w + HI + 2 * k, idesc, 1u);
+              tc::mma_f16(small, a + HI + 2 * k, w + LO + 2 * k, idesc, 1u);
+              tc::mma_f16(small, a + MID + 2 * k, w + MID + 2 * k, idesc, 1u);
+              tc::mma_f16(small, a + MID + 2 * k, w + HI + 2 * k, idesc, 1u);
+              tc::mma_f16(small, a + HI + 2 * k, w + MID + 2 * k, idesc, 1u);
+              tc::mma_f16(main, a + HI + 2 * k, w + HI + 2 * k, idesc, more);
             }
             tc::mma_commit(empty_bar(s));
           }
@@ -196,10 +200,14 @@ __global__ __launch_bounds__(THREADS, 1) void gemm_f32_tc_kernel(const __grid_co
         }
         if (ok && tc::elect_one()) tc::mma_commit(acc_full(buf));
         __syncwarp();
+        if ((kb0 + CHUNK) % SPAN == 0 || kb0 + CHUNK >= kbs) ++span;
       }
   } else if (warp < 2 + CUT_WARPS) {
-    constexpr int PIECES = OPERANDS / 16 / (32 * CUT_WARPS);  // 16-byte pieces of a K block a thread cuts
-    static_assert(OPERANDS % (16 * 32 * CUT_WARPS) == 0, "pieces are shared evenly");
+    // A warp cuts eight rows at a time, lane (r = lane / 4, c = lane % 4) the numbers 8 c ... 8 c + 7 of row r: the 16-byte pieces 2 c and
+    // 2 c + 1 of its 128 bytes, which become piece c of hi, of mid (piece 4 + c) and of lo; piece p of row r lies at p ^ r.  Odd rows store mid
+    // first, so that eight lanes' stores meet all banks.
+    constexpr int GROUPS = (BM + BN) / 8, TURNS = (GROUPS + CUT_WARPS - 1) / CUT_WARPS;
+    const int r = lane >> 2, c = lane & 3, first = r & 1 ? 4 : 0;
     int s = 0;
     uint32_t ph = 0;
     bool ok = true;
@@ -207,21 +215,34 @@ __global__ __launch_bounds__(THREADS, 1) void gemm_f32_tc_kernel(const __grid_co
       for (int kb = 0; kb < kbs; ++kb) {
         ok = tc::mbar_wait_warp(full_bar(s), ph, abort_flag, p.status);
         if (!ok) break;
-        float4* x = reinterpret_cast<float4*>(smem + s * STAGE) + (tid - 64);
-        float4* low = reinterpret_cast<float4*>(smem + s * STAGE + OPERANDS) + (tid - 64);
-        float4 v[PIECES];
+        uint8_t* rows = smem + s * STAGE + (size_t)((warp - 2) * 8 + r) * 128;
+        float4 v[TURNS][2];
 #pragma unroll
-        for (int i = 0; i < PIECES; ++i) v[i] = x[i * 32 * CUT_WARPS];
-        float odd = 0.f;  // becomes NaN where a rest is not finite
+        for (int i = 0; i < TURNS; ++i)
+          if (warp - 2 + i * CUT_WARPS < GROUPS)
 #pragma unroll
-        for (int i = 0; i < PIECES; ++i) {
-          const float4 hi = make_float4(to_tf32(v[i].x), to_tf32(v[i].y), to_tf32(v[i].z), to_tf32(v[i].w));
-          const float4 lo = make_float4(v[i].x - hi.x, v[i].y - hi.y, v[i].z - hi.z, v[i].w - hi.w);
-          odd = fmaf(lo.x, 0.f, odd), odd = fmaf(lo.y, 0.f, odd), odd = fmaf(lo.z, 0.f, odd), odd = fmaf(lo.w, 0.f, odd);
-          x[i * 32 * CUT_WARPS] = hi;
-          low[i * 32 * CUT_WARPS] = make_float4(to_tf32(lo.x), to_tf32(lo.y), to_tf32(lo.z), to_tf32(lo.w));
-        }
-        if (odd != 0.f) *uncut_flag = 1;  // (a NaN is not equal to zero)
+            for (int h = 0; h < 2; ++h) v[i][h] = *reinterpret_cast<const float4*>(rows + i * CUT_WARPS * 1024 + (((2 * c + h) ^ r) << 4));
+        __syncwarp();  // all of the warp's rows have been read: they are written over
+        float odd = 0.f;  // becomes NaN where a rest is not finite, and is not zero where one is left
+#pragma unroll
+        for (int i = 0; i < TURNS; ++i)
+          if (warp - 2 + i * CUT_WARPS < GROUPS) {
+            float x[8] = {v[i][0].x, v[i][0].y, v[i][0].z, v[i][0].w, v[i][1].x, v[i][1].y, v[i][1].z, v[i][1].w};
+            uint32_t part[3][4];
+#pragma unroll
+            for (int q = 0; q < 3; ++q)
+#pragma unroll
+              for (int e = 0; e < 4; ++e) part[q][e] = take_part(x[2 * e], x[2 * e + 1]);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) odd += fabsf(x[e]);
+            uint8_t* row = rows + i * CUT_WARPS * 1024;
+            const uint4 hi = make_uint4(part[0][0], part[0][1], part[0][2], part[0][3]);
+            const uint4 mid = make_uint4(part[1][0], part[1][1], part[1][2], part[1][3]);
+            *reinterpret_cast<uint4*>(row + (((first + c) ^ r) << 4)) = first ? mid : hi;
+            *reinterpret_cast<uint4*>(row + (((4 - first + c) ^ r) << 4)) = first ? hi : mid;
+            *reinterpret_cast<uint4*>(row + OPERANDS + ((c ^ r) << 4)) = make_uint4(part[2][0], part[2][1], part[2][2], part[2][3]);
+          }
+        if (!(odd == 0.f)) *uncut_flag = 1;  // (a NaN is not equal to zero)
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
         if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(cut_bar(s)) : "memory");
@@ -233,7 +254,7 @@ __global__ __launch_bounds__(THREADS, 1) void gemm_f32_tc_kernel(const __grid_co
     constexpr int STEP = 16;
     const int quarter = warp & 3, part = (warp - 2 - CUT_WARPS) >> 2;
     const bool vec = p.ldo % 4 == 0 && (uintptr_t)p.out % 16 == 0;
-    int chunk = 0;
+    int chunk = 0, span = 0;
     bool ok = true;
     for (int unit = blockIdx.x; unit < units && ok; unit += gridDim.x) {
       const int row = (unit % m_tiles) * BM + quarter * 32 + lane, n0 = (unit / m_tiles) * BN + part * COLS;
@@ -245,16 +266,19 @@ __global__ __launch_bounds__(THREADS, 1) void gemm_f32_tc_kernel(const __grid_co
         ok = tc::mbar_wait_warp(acc_full(buf), (uint32_t)(chunk >> 1) & 1u, abort_flag, p.status);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t main = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * 2 * BN + part * COLS);
+        const uint32_t mine = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(part * COLS);
+        auto add = [&](uint32_t from) {
 #pragma unroll
-        for (int c = 0; c < COLS; c += STEP) {
-          uint32_t big[STEP], small[STEP];
-          tc::tmem_load16(main + c, big);
-          tc::tmem_load16(main + BN + c, small);
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          for (int c = 0; c < COLS; c += STEP) {
+            uint32_t r[STEP];
+            tc::tmem_load16(from + c, r);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-          for (int i = 0; i < STEP; ++i) acc[c + i] += __uint_as_float(big[i]) + __uint_as_float(small[i]);
-        }
+            for (int i = 0; i < STEP; ++i) acc[c + i] += __uint_as_float(r[i]);
+          }
+        };
+        add(mine + (uint32_t)(buf * BN));
+        if ((kb0 + CHUNK) % SPAN == 0 || kb0 + CHUNK >= kbs) add(mine + (uint32_t)((2 + (span++ & 1)) * BN));
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
         if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(acc_empty(buf)) : "memory");
@@ -346,7 +370,7 @@ struct WidthTime {
   int bn;
   double fixed, kb, round;
 };
-constexpr WidthTime WIDTHS[] = {{32, 5.1, 0.62, 1.2}, {64, 7.0, 0.67, 3.0}, {128, 10.5, 0.85, 7.0}};
+constexpr WidthTime WIDTHS[] = {{32, 4.6, 0.75, 1.3}, {64, 6.3, 0.82, 3.8}, {128, 10.3, 1.04, 9.0}};
 
 double time_us(int M, int N, int K, int* width) {
   const long down = ((long)M + BM - 1) / BM;
