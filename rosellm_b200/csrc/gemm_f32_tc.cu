@@ -27,8 +27,9 @@
 // Error against 64 bits (2-norm of the difference over that of the FMAs' difference): dense sums 0.25 (K 256), 0.21 (768), 0.19 (3072); sums
 // of one product 1.00, of two to sixteen 0.5 to 1.1; of positive numbers 0.26 to 0.19.
 //
-// Numbers that cannot be cut (infinities, NaN, magnitudes that round to infinity) are noticed while cutting: a block that
-// has met one works its tiles out anew with FMAs from memory, in the order of the CUDA-core kernels.
+// Sums that are not finite are worked out again with FMAs from memory, in the order of the CUDA-core kernels, each by itself: those with an
+// infinity or NaN among their operands, those that overflow on the way (a product of hi parts does before the FMA with it does), and
+// those with an operand that three parts do not hold (above 3.39e38, or with bits below 2^-133), which becomes NaN in the cutting.
 // Every wait on a barrier is bounded (status bit, abort flag), as in gemm_tc.cu.
 #include "gemm_epilogue.cuh"
 #include "gemm_f32_tc.cuh"
@@ -49,7 +50,7 @@ __host__ __device__ constexpr int stages_of(int bn) {
   return fit > MAX_STAGES ? MAX_STAGES : fit;
 }
 // 1024 for alignment | stages of (hi, in x's place | lo) | barriers full, cut, empty [MAX_STAGES], acc_full, acc_empty [2],
-// the tensor-memory address, the abort flag and the flag of a number that cannot be cut
+// the tensor-memory address and the abort flag
 __host__ __device__ constexpr int smem_bytes(int bn) { return 1024 + stages_of(bn) * 2 * operand_bytes(bn) + (3 * MAX_STAGES + 4) * 8 + 16; }
 
 struct Args {
@@ -76,6 +77,24 @@ __device__ __noinline__ float4 act_call(float4 v, int act) {
   return make_float4(apply_act(v.x, act), apply_act(v.y, act), apply_act(v.z, act), apply_act(v.w, act));
 }
 
+// A sum of the product by FMAs in ascending order, as the CUDA-core kernels add (K a multiple of 4, both on 16-byte boundaries).
+__device__ __noinline__ float sum_of_fmas(const float* a, const float* w, int K) {
+  float t = 0.f;
+  for (int k = 0; k < K; k += 32) {
+    float4 x[8], y[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {  // beyond K: the first numbers again, and not used
+      const int at = k + 4 * i < K ? k + 4 * i : 0;
+      x[i] = *reinterpret_cast<const float4*>(a + at);
+      y[i] = *reinterpret_cast<const float4*>(w + at);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (k + 4 * i < K) t = fmaf(x[i].w, y[i].w, fmaf(x[i].z, y[i].z, fmaf(x[i].y, y[i].y, fmaf(x[i].x, y[i].x, t))));
+  }
+  return t;
+}
+
 template <int BN>
 __global__ __launch_bounds__(THREADS, 1) void gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a,
                                                                  const __grid_constant__ CUtensorMap map_w, const Args p) {
@@ -91,7 +110,6 @@ __global__ __launch_bounds__(THREADS, 1) void gemm_f32_tc_kernel(const __grid_co
   auto acc_empty = [&](int b) { return bar_base + 8u * (3 * MAX_STAGES + 2 + b); };
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + STAGES * STAGE + (3 * MAX_STAGES + 4) * 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  volatile int* uncut_flag = reinterpret_cast<volatile int*>(tmem_slot + 2);
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const int m_tiles = (p.M + BM - 1) / BM, units = m_tiles * ((p.N + BN - 1) / BN), kbs = (p.K + BK - 1) / BK;
 
@@ -107,7 +125,6 @@ __global__ __launch_bounds__(THREADS, 1) void gemm_f32_tc_kernel(const __grid_co
       tc::mbar_init(acc_empty(b), EPI_WARPS);
     }
     *abort_flag = 0;
-    *uncut_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     tc::tma_prefetch_map(&map_a);
@@ -223,7 +240,6 @@ __global__ __launch_bounds__(THREADS, 1) void gemm_f32_tc_kernel(const __grid_co
 #pragma unroll
             for (int h = 0; h < 2; ++h) v[i][h] = *reinterpret_cast<const float4*>(rows + i * CUT_WARPS * 1024 + (((2 * c + h) ^ r) << 4));
         __syncwarp();  // all of the warp's rows have been read: they are written over
-        float odd = 0.f;  // becomes NaN where a rest is not finite, and is not zero where one is left
 #pragma unroll
         for (int i = 0; i < TURNS; ++i)
           if (warp - 2 + i * CUT_WARPS < GROUPS) {
@@ -233,16 +249,20 @@ __global__ __launch_bounds__(THREADS, 1) void gemm_f32_tc_kernel(const __grid_co
             for (int q = 0; q < 3; ++q)
 #pragma unroll
               for (int e = 0; e < 4; ++e) part[q][e] = take_part(x[2 * e], x[2 * e + 1]);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) odd += fabsf(x[e]);
             uint8_t* row = rows + i * CUT_WARPS * 1024;
             const uint4 hi = make_uint4(part[0][0], part[0][1], part[0][2], part[0][3]);
             const uint4 mid = make_uint4(part[1][0], part[1][1], part[1][2], part[1][3]);
             *reinterpret_cast<uint4*>(row + (((first + c) ^ r) << 4)) = first ? mid : hi;
             *reinterpret_cast<uint4*>(row + (((4 - first + c) ^ r) << 4)) = first ? hi : mid;
-            *reinterpret_cast<uint4*>(row + OPERANDS + ((c ^ r) << 4)) = make_uint4(part[2][0], part[2][1], part[2][2], part[2][3]);
+            uint4* lo = reinterpret_cast<uint4*>(row + OPERANDS + ((c ^ r) << 4));
+            *lo = make_uint4(part[2][0], part[2][1], part[2][2], part[2][3]);
+            // a rest that is not finite, or left beyond bfloat16's least number (else all are +0): NaN in its place, so that the row's sums
+            // are worked out anew
+            uint32_t rest = 0;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) rest |= __float_as_uint(x[e]);
+            if (rest != 0) lo->x = 0x7fff7fffu;
           }
-        if (!(odd == 0.f)) *uncut_flag = 1;  // (a NaN is not equal to zero)
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
         if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(cut_bar(s)) : "memory");
@@ -284,45 +304,60 @@ __global__ __launch_bounds__(THREADS, 1) void gemm_f32_tc_kernel(const __grid_co
         if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(acc_empty(buf)) : "memory");
       }
       if (!ok) break;
-      if (row >= p.M) continue;
-      if (*uncut_flag) {
-        const float* a = p.a + (size_t)row * p.lda;
-#pragma unroll
-        for (int i = 0; i < COLS; ++i) {
-          const float* w = p.w + (size_t)min(n0 + i, p.N - 1) * p.K;
-          float t = 0.f;
-#pragma unroll 1
-          for (int k = 0; k < p.K; ++k) t = fmaf(a[k], w[k], t);
-          acc[i] = t;
-        }
-      }
+      uint32_t again[(COLS + 31) / 32] = {};  // columns whose sums are not finite
       float* out = p.out + (size_t)row * p.ldo + n0;
+      if (row < p.M) {
 #pragma unroll
-      for (int c = 0; c < COLS; c += 4) {
-        if (n0 + c >= p.N) break;
-        float v[4];
+        for (int c = 0; c < COLS; c += 4) {
+          if (n0 + c >= p.N) break;
+          float v[4];
+          uint32_t odd = 0;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          v[i] = acc[c + i];
-          if (p.bias != nullptr && n0 + c + i < p.N) v[i] += p.bias[n0 + c + i];
-        }
-        if (p.act != RL_ACT_NONE) {
-          const float4 t = act_call(make_float4(v[0], v[1], v[2], v[3]), p.act);
-          v[0] = t.x, v[1] = t.y, v[2] = t.z, v[3] = t.w;
-        }
-        if (vec && n0 + c + 3 < p.N) {
-          float4 t = make_float4(v[0], v[1], v[2], v[3]);
-          if (p.residual) {
-            const float4 old = *reinterpret_cast<const float4*>(out + c);
-            t.x += old.x, t.y += old.y, t.z += old.z, t.w += old.w;
+          for (int i = 0; i < 4; ++i) {
+            v[i] = acc[c + i];
+            if (n0 + c + i >= p.N) continue;
+            odd |= (uint32_t)((__float_as_uint(v[i]) & 0x7f800000u) == 0x7f800000u) << i;
+            if (p.bias != nullptr) v[i] += p.bias[n0 + c + i];
           }
-          *reinterpret_cast<float4*>(out + c) = t;
-        } else {
+          again[c / 32] |= odd << (c % 32);
+          if (p.act != RL_ACT_NONE) {
+            const float4 t = act_call(make_float4(v[0], v[1], v[2], v[3]), p.act);
+            v[0] = t.x, v[1] = t.y, v[2] = t.z, v[3] = t.w;
+          }
+          if (vec && odd == 0 && n0 + c + 3 < p.N) {
+            float4 t = make_float4(v[0], v[1], v[2], v[3]);
+            if (p.residual) {
+              const float4 old = *reinterpret_cast<const float4*>(out + c);
+              t.x += old.x, t.y += old.y, t.z += old.z, t.w += old.w;
+            }
+            *reinterpret_cast<float4*>(out + c) = t;
+          } else {
 #pragma unroll
-          for (int i = 0; i < 4; ++i)
-            if (n0 + c + i < p.N) out[c + i] = p.residual ? out[c + i] + v[i] : v[i];
+            for (int i = 0; i < 4; ++i)
+              if (n0 + c + i < p.N && (odd >> i & 1) == 0) out[c + i] = p.residual ? out[c + i] + v[i] : v[i];
+          }
         }
       }
+      // a row at a time, its columns over the lanes
+      uint32_t any = again[0];
+      if constexpr (COLS > 32) any |= again[1];
+      for (unsigned rows = __ballot_sync(0xffffffffu, any != 0); rows != 0; rows &= rows - 1) {
+        const int src = __ffs(rows) - 1;
+        const size_t there = (size_t)(row - lane + src);
+#pragma unroll
+        for (int h = 0; h < (COLS + 31) / 32; ++h) {
+          const uint32_t columns = __shfl_sync(0xffffffffu, again[h], src);
+          if (columns >> lane & 1) {
+            const int n = n0 + 32 * h + lane;
+            float v = sum_of_fmas(p.a + there * p.lda, p.w + (size_t)n * p.K, p.K);
+            if (p.bias != nullptr) v += p.bias[n];
+            v = act_call(make_float4(v, 0.f, 0.f, 0.f), p.act).x;
+            float* at = p.out + there * p.ldo + n;
+            *at = p.residual ? *at + v : v;
+          }
+        }
+      }
+      __syncwarp();
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
