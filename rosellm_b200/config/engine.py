@@ -23,7 +23,7 @@ DTYPE_NAMES = {
 @dataclass(frozen=True)
 class EngineConfig:
     dtype: str = "bfloat16"
-    """``bfloat16``: the serving path.  ``float32``: every product and sum to 32 bits."""
+    """``bfloat16``: the serving path.  ``float32``: operands and sums in 32 bits throughout."""
     page_size: int = 16
     """Tokens per cache page (the reference fixes 64, rosellm/roseinfer/engine.py:230)."""
     num_pages: int | None = None

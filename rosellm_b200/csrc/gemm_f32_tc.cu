@@ -396,7 +396,7 @@ static int launch(const Args& p, cudaStream_t stream) {
 }
 
 bool takes(const void* a, long lda, const void* w, int K, const int* status) {
-  return K > 0 && K % 4 == 0 && lda % 4 == 0 && (uintptr_t)a % 16 == 0 && (uintptr_t)w % 16 == 0 && status != nullptr &&
+  return K > 0 && K % 4 == 0 && lda >= K && lda % 4 == 0 && (uintptr_t)a % 16 == 0 && (uintptr_t)w % 16 == 0 && status != nullptr &&
          tc::encode_fn() != nullptr;
 }
 
@@ -407,19 +407,20 @@ struct WidthTime {
 };
 constexpr WidthTime WIDTHS[] = {{32, 4.6, 0.75, 1.3}, {64, 6.3, 0.82, 3.8}, {128, 10.3, 1.04, 9.0}};
 
-double time_us(int M, int N, int K, int* width) {
+int width_for(int M, int N, int K) {
   const long down = ((long)M + BM - 1) / BM;
   const int kbs = (K + BK - 1) / BK, sms = sm_count();
   double best = 1e30;
+  int width = 128;
   for (const WidthTime& w : WIDTHS) {
     const long tiles = down * ((N + w.bn - 1) / w.bn), rounds = (tiles + sms - 1) / sms;
     const double us = w.fixed + rounds * kbs * w.kb + (rounds - 1) * w.round;
     if (us < best && tiles <= 0x7fffffff) {
       best = us;
-      *width = w.bn;
+      width = w.bn;
     }
   }
-  return best;
+  return width;
 }
 
 int run(const float* a, long lda, const float* w, const float* bias, float* out, long ldo, int M, int N, int K, int act, int residual,
@@ -437,8 +438,7 @@ RL_EXPORT int rl_gemm_f32_tc(const float* A, long lda, const float* W, const flo
                              int act, int residual, int tile_width, int* status, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (!rl::f32tc::takes(A, lda, W, K, status)) return -2;
-  int width = tile_width;
-  if (width == 0) rl::f32tc::time_us(M, N, K, &width);
+  const int width = tile_width == 0 ? rl::f32tc::width_for(M, N, K) : tile_width;
   if (width != 32 && width != 64 && width != 128) return -2;
   return rl::f32tc::run(A, lda, W, bias, out, ldo, M, N, K, act, residual, width, status, stream);
 }

@@ -1,8 +1,8 @@
 // Matrix products on the CUDA cores: out[M,N] = A[M,K] * W[N,K]^T, with the epilogues the
 // model needs fused in: + bias[N]; GELU; and accumulation into a float32 residual stream.
 //
-// This is the matrix path of the 32-bit mode (IEEE float32 FMA; products of many rows with inner sizes
-// from 256 go to gemm_f32_tc.cu, whose error is no larger), and the small-batch path of the bfloat16
+// This is the matrix path of the 32-bit mode (IEEE float32 FMA; products of many rows whose columns and inner size
+// are large go to gemm_f32_tc.cu, which holds its operands in full and rounds less often), and the small-batch path of the bfloat16
 // mode, where a product streams the weights once and is bound by memory, not arithmetic.  The formulas fused here:
 //   y = a W + b                           rosellm/rosetrainer/model.py:95, 220, 334-337
 //   gelu_tanh(u) = 0.5 u (1 + tanh(sqrt(2/pi) (u + 0.044715 u^3)))   model.py:274-277,
@@ -85,7 +85,7 @@ __global__ __launch_bounds__(256) void gemm_tile_kernel(
 // thread grid apart), K in steps of 16 that travel by cp.async, as they lie in memory, through a ring of three buffers of
 // shared memory (rows 80 bytes apart: the eight rows of a 16-byte access phase hit different banks).
 // Each output's sum runs over k in ascending order whatever M is and whatever the tile is, so a row's result does
-// not depend on which other rows share the launch.  What bounds it: reads of shared memory, 12 pieces of 16 bytes a thread for 128
+// not depend on which other rows share the launch (nor does it hang on M whether a product of many rows comes here: f32tc::ahead).  What bounds it: reads of shared memory, 12 pieces of 16 bytes a thread for 128
 // FMAs with 8 x 4 outputs (about 19 of the 37.2 TFMA/s; the form before, 64 x 64 tiles of 4 x 4 outputs transposed through registers with
 // two barriers a step, 9 to 16).  Pairs of FMAs in one instruction (fma.rn.f32x2) measured the same and add up in another order.
 template <int BM, int BN, int TM, int TN>
@@ -446,7 +446,7 @@ static double tile_time(const TileTime (&time)[POINTS], double tiles) {
 // The tile that ends first.  Over 161 products of 65 to 2048 rows (64 to 4096 columns, K 256 to 6400) the choice is 1% behind the
 // fastest form on average; by counting rounds of tiles it was 7%, up to 45% (1600 x 1600 at 300 rows: 146, 99 and 120 us on 64 x 64,
 // 32 x 64 and 32 x 32; 768 x 768 at 600 rows 66, 56 and 59).  128 x 64, and 8 x 8 outputs a thread, measured slower throughout.
-static dim3 tile_f32_for(int M, int N, double* us = nullptr) {
+static dim3 tile_f32_for(int M, int N) {
   const int sms = simt_sm_count();
   auto cost = [&](int bm, int bn, const auto& time) {
     const long down = (M + bm - 1) / bm, tiles = down * ((N + bn - 1) / bn);
@@ -454,7 +454,6 @@ static dim3 tile_f32_for(int M, int N, double* us = nullptr) {
     return tile_time(time, (double)tiles / sms);
   };
   const double large = cost(64, 64, TIME_64X64), middle = cost(32, 64, TIME_32X64), small = cost(32, 32, TIME_32X32);
-  if (us != nullptr) *us = fmin(fmin(large, middle), small);
   return large <= middle && large <= small ? dim3(64, 64) : middle <= small ? dim3(32, 64) : dim3(32, 32);
 }
 
@@ -556,14 +555,11 @@ RL_EXPORT int rl_gemm_simt(int in_dtype, int out_dtype, const void* A, long lda,
   rl::KvScatter kv{kv_pool, kv_block_table, kv_bt_stride, kv_positions, kv_req_of_token, kv_slots,
                    kv_q_width, kv_width, kv_head_dim, kv_page_size, kv_heads, kv_max_pos, status};
   int rc;
-  if (in_dtype == RL_F32 && out_dtype == RL_F32 && M > rows_limit && kv_pool == nullptr && K >= rl::f32tc::MIN_K &&
+  if (in_dtype == RL_F32 && out_dtype == RL_F32 && M > rows_limit && kv_pool == nullptr && rl::f32tc::ahead(N, K) &&
       rl::f32tc::takes(A, lda, W, K, status)) {
-    // many rows: the tensor cores where they are the faster (gemm_f32_tc.cu), which they are but for few tiles
-    double tiles_us = 0.0;
-    rl::tile_f32_for(M, N, &tiles_us);
-    int width = 0;
-    if (rl::f32tc::time_us(M, N, K, &width) < 0.95 * tiles_us * K / 768.0)
-      return rl::f32tc::run((const float*)A, lda, (const float*)W, bias, (float*)out, ldo, M, N, K, act, residual, width, status, stream);
+    rc = rl::f32tc::run((const float*)A, lda, (const float*)W, bias, (float*)out, ldo, M, N, K, act, residual,
+                        rl::f32tc::width_for(M, N, K), status, stream);
+    if (rc != -10 && rc != -11) return rc;  // without tensor maps: the CUDA cores
   }
   if (in_dtype == RL_F32 && out_dtype == RL_F32)
     rc = rl::launch_gemm<float, float>(A, lda, W, bias, out, ldo, M, N, K, act, residual, rows_limit, kv, stream);

@@ -342,7 +342,7 @@ RL_EXPORT int rl_gemm_tc_rows_fits(int M, int N, int K) {
 // bfloat16 A [M <= 128, K] (row stride lda) and W [N, K]; out bfloat16 or float32 [M, N].
 // residual != 0: out (float32) += result.  kv_pool != nullptr: output columns from kv_q_width
 // on are written into cache pages as keys and values, not to out.  Returns -7 when the sizes
-// do not fit (K too long for one block's shared memory).
+// do not fit (more than 128 rows, or K above 8192).
 RL_EXPORT int rl_gemm_tc_rows(int out_dtype, const void* A, long lda, const void* W, const float* bias, void* out,
                               long ldo, int M, int N, int K, int act, int residual, void* kv_pool,
                               const int* kv_block_table, int kv_bt_stride, const int* kv_positions,

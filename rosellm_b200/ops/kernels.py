@@ -540,7 +540,8 @@ def linear(a, weight, bias, out, *, act: int = ACT_NONE, residual: bool = False,
     at most 16 rows).  Otherwise
     a [rows, k] (row stride a multiple of 8), weight [n, k] contiguous, both float32 or both
     bfloat16; out [rows, n] of a's dtype or float32.  Which kernel runs: float32 up to 64 rows
-    the row kernel, above it tiles of FMAs or, from an inner size of 256 where it is faster, of tf32 parts; bfloat16 up to 16 rows the
+    the row kernel, above it tiles of FMAs or, by the columns and the inner size alone, the tensor cores (csrc/gemm_f32_tc.cuh: ``ahead``; operands
+    in three bfloat16 parts, which hold them in full); bfloat16 up to 16 rows the
     weight-streaming kernels (fed by TMA through a ring; for a very wide float32 output, a head, by
     bulk copies; by registers otherwise: the library chooses), above it as ``bf16_path`` and ``clustered_is_ahead`` say.  ``path``
     (for tests) forces ``"rows"``, ``"tile"``, ``"f32tc"``, ``"mma"``, ``"smem"``, ``"tc"`` or ``"tcr"``.  ``kv``: output columns from
@@ -607,8 +608,7 @@ def linear(a, weight, bias, out, *, act: int = ACT_NONE, residual: bool = False,
     if path == "mma" and m > 64:
         raise KernelError("linear: the mma row kernel takes at most 64 rows")
     if path == "tcr" and not _lib().rl_gemm_tc_rows_fits(m, n, k):
-        raise KernelError("linear: the clustered tcgen05 kernel takes at most 128 rows and an inner size that "
-                          "fits the shared memory of eight blocks")
+        raise KernelError("linear: the clustered tcgen05 kernel takes at most 128 rows and an inner size of at most 8192")
     if kv is not None and path == "tile":
         raise KernelError("linear: the 32-bit tile kernel does not write into the cache")
     if kv is not None and (act != ACT_NONE or residual):

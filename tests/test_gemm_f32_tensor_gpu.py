@@ -1,4 +1,4 @@
-"""Float32 products on the tensor cores (csrc/gemm_f32_tc.cu): operands in two tf32 parts, against float64 and against the
+"""Float32 products on the tensor cores (csrc/gemm_f32_tc.cu): operands in three bfloat16 parts, against float64 and against the
 CUDA-core kernels, whose error they may not exceed."""
 import pytest
 import torch
@@ -24,7 +24,7 @@ def test_every_width(m, n, k, width):
     ref = a.double() @ w.double().T
     out = torch.full((m, n), float("nan"), device=DEV)
     K.linear(a, w, None, out, path="f32tc", tile_width=width)
-    # a product of the parts leaves out 2^-22 of itself at most, a chunk of 32 elements adds four partial sums cut off at 2^-23 and
+    # a product leaves out 2^-34 of itself at most, a chunk of 32 elements adds two partial sums cut off at 2^-23 and
     # the chunks are added with a rounding each: all of it below k roundings of 2^-24 of sums of order 1
     assert (out.double() - ref).abs().max().item() <= 4 * (k + 64) * 2.0 ** -24 + 1e-6
     x = torch.randn(m, n + 3, device=DEV)[:, :n]
@@ -59,7 +59,7 @@ def test_error_is_no_larger_than_that_of_fmas(kind, k):
 
 
 def test_numbers_that_cannot_be_cut():
-    """Infinities, NaN and magnitudes that round to infinity: such a block's results are those of FMAs."""
+    """Infinities, NaN and magnitudes that round to infinity: the sums with them are those of FMAs."""
     a, w, b = _data(300, 200, 96)
     a[5, 7], a[200, 3], a[130, 9], w[17, 40] = float("inf"), float("nan"), 3.4028e38, float("-inf")
     out, ref = torch.empty(300, 200, device=DEV), a.double() @ w.double().T + b.double()
@@ -79,7 +79,7 @@ def test_a_row_does_not_depend_on_the_rows_beside_it(m, n, k):
     assert torch.equal(fewer, out[:m - 1])
 
 
-def test_operands_off_the_copies_boundaries_run_on_the_cuda_cores():
+def test_operands_off_a_16_byte_boundary_are_refused():
     a, w, b = _data(200, 96, 64)
     shifted = torch.empty(200 * 64 + 1, device=DEV)[1:].view(200, 64).copy_(a)  # rows four bytes off a 16-byte boundary
     with pytest.raises(K.KernelError):
