@@ -177,11 +177,14 @@ __global__ __launch_bounds__(THREADS, HALVES * PIECES == 1 ? 2 : 1) void gemm_ro
     }
   }
   // Where a warp holds one piece of eight rows (and there is no norm or choice of tokens) the loop below is walked once before the wait
-  // for the kernels ahead, over whatever lies in shared memory and to no effect: between other kernels its instructions would
+  // for the kernels ahead, over a kilobyte of the partial sums' place that nothing writes by
+  // then (never the ring, which the copies fill) and to no effect: between other kernels its instructions would
   // have to be fetched once the rows are there.  A step of GPT-2 355M, one request, 481 -> 464 us with both numbers of pieces, a pass of
   // 8 requests of GPT-2 124M 19,313 -> 18,892, one of 1.5B 51,555 -> 51,213.  Two pieces gain less (one request of 1.5B 50,740) and lose where
   // a short kernel is ahead, and the lap comes too late (8 requests of the latent-attention model 14,635 -> 14,737); sixteen rows 5% slower in chains.
   constexpr bool DRY = !NORM && !SAMPLE && HALVES * PIECES == 1;
+  constexpr int DRY_AT = WARPS * 64 * 4;  // beyond the sums that the lap itself stores; its reads end 1 KB behind, those of a second block WARPS KB on
+  static_assert(!DRY || DRY_AT + (SLOTS - 1) * WARPS * 1024 + 1024 <= 2 * ROUND * WARPS * 64 * 4, "within the partial sums' place");
   if constexpr (!DRY) asm volatile("griddepcontrol.wait;" ::: "memory");
 
   // the row's sampling options, and its best entry so far
@@ -277,13 +280,14 @@ __global__ __launch_bounds__(THREADS, HALVES * PIECES == 1 ? 2 : 1) void gemm_ro
   // The lane's two 16-byte pieces of a block: 2 j and 2 j + 1 of the row's 128 bytes, swizzled by the row.
   const uint32_t w_at = ring0 + warp * 1024 + g * 128 + ((2 * j ^ g) << 4);
   int stage = 0, buf = 0;
-  uint32_t parity = 0, w_stage = w_at;
+  uint32_t parity = 0, w_stage = DRY ? tc::smem_u32(part_s) + DRY_AT + g * 128 + ((2 * j ^ g) << 4) : w_at;
 #pragma unroll 1
   for (int g0 = DRY ? first - ROUND : first; g0 < last; g0 += ROUND, buf ^= 1) {
     const bool dry = DRY && g0 < first;
     if (DRY && g0 == first) {
       asm volatile("griddepcontrol.wait;" ::: "memory");
       load_rows(rows, pitch, 0);
+      w_stage = w_at;
     }
     const int n_here = dry ? 1 : min(ROUND, last - g0);
     float* mine = part_s + buf * (ROUND * WARPS * HALVES * 64);
