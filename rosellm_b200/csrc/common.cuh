@@ -171,6 +171,16 @@ __device__ __forceinline__ void pdl_begin() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// A load that stays behind the wait it stands behind.  What a kernel ahead writes is read after the wait, but through a pointer that is
+// __restrict__ the compiler may take an ordinary load for one of memory that does not change while the kernel runs, and move it ahead (seen
+// in head_rows_kernel: with a condition on its weights' load its input was read before the wait).  So what kernels ahead write
+// is read by this, or through pointers that are not __restrict__, where a kernel does anything before its wait.
+__device__ __forceinline__ uint4 load_in_order(const uint4* p) {
+  uint4 v;
+  asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+  return v;
+}
+
 // The split of an SM's on-chip memory between L1 and shared memory is a property of the
 // running kernel; where two kernels that follow one another want different splits, the SM
 // has to run empty in between, which costs a decode step about two microseconds per change.

@@ -87,7 +87,7 @@ __global__ void layernorm_kernel(const float* __restrict__ x, const int* __restr
 // load is unconditional (a clamped address), so that all are issued before the first is used;
 // a load under a condition would wait for the one before it.
 template <typename T, int PIECES>
-__global__ __launch_bounds__(128) void layernorm_warp_kernel(const float* __restrict__ x,
+__global__ __launch_bounds__(128) void layernorm_warp_kernel(const float* x,
                                                              const int* __restrict__ rows,
                                                              const float* __restrict__ gamma,
                                                              const float* __restrict__ beta, T* __restrict__ out,
@@ -282,7 +282,7 @@ namespace rl {
 // kernel writes them) are asked for before the wait for the kernels ahead.  Rows of at most 2048
 // elements, a multiple of 4.
 template <typename T>
-__global__ __launch_bounds__(256) void layernorm_block_kernel(const float* __restrict__ x, const int* __restrict__ rows,
+__global__ __launch_bounds__(256) void layernorm_block_kernel(const float* x, const int* __restrict__ rows,
                                                               const float* __restrict__ gamma,
                                                               const float* __restrict__ beta, T* __restrict__ out,
                                                               int n_out, int hidden, float eps) {

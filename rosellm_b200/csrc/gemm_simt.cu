@@ -183,7 +183,7 @@ __global__ __launch_bounds__((BM / TM) * (BN / TN)) void gemm_tile_f32_kernel(
 // of what it has left), then over the group's warps in shared memory: in an order that is the same for every row whatever M is.
 constexpr int ROWS_COLS = 4, ROWS_STAGES = 3;
 template <int ROWS, int PARTS>
-__global__ __launch_bounds__(256, 2) void gemm_rows_f32_kernel(const float* __restrict__ A, long lda, const float* __restrict__ W,
+__global__ __launch_bounds__(256, 2) void gemm_rows_f32_kernel(const float* A, long lda, const float* __restrict__ W,
                                                                const float* __restrict__ bias, float* __restrict__ out, long ldo,
                                                                int M, int N, int K, int act, int residual, KvScatter kv) {
   constexpr int COLS = ROWS_COLS, STAGES = ROWS_STAGES, VALUES = COLS * ROWS, AHEAD = STAGES - 1, GROUPS = 8 / PARTS;

@@ -99,10 +99,10 @@ __global__ __launch_bounds__(128) void head_linear_mma_kernel(const __nv_bfloat1
 // tiles (32 blocks, sixteen steps of K one after the other).
 constexpr int HR_WARPS = 8, HR_MAX_K = 4 * 64 * HR_WARPS;
 template <int KB>
-__global__ __launch_bounds__(32 * HR_WARPS) void head_rows_kernel(const __nv_bfloat16* __restrict__ in, long in_tok, long in_head,
+__global__ __launch_bounds__(32 * HR_WARPS) void head_rows_kernel(const __nv_bfloat16* in, long in_tok, long in_head,
                                                                   const __nv_bfloat16* __restrict__ w, long w_head, long w_n,
                                                                   __nv_bfloat16* __restrict__ out, long out_tok, long out_head,
-                                                                  int n_tokens, int n_total, int parts, const float* __restrict__ gate,
+                                                                  int n_tokens, int n_total, int parts, const float* gate,
                                                                   long gate_tok, long gate_head, long gate_n) {
   __shared__ float part_s[HR_WARPS][32][4];
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -30,8 +30,8 @@ struct HeadRowsWeights {
     for (int kb = 0; kb < KB; ++kb)
 #pragma unroll
       for (int s = 0; s < 2; ++s) {
-        a[kb][s] = reinterpret_cast<const uint4*>(lo + kb * 64 + 16 * j)[s];
-        b[kb][s] = reinterpret_cast<const uint4*>(hi + kb * 64 + 16 * j)[s];
+        a[kb][s] = load_in_order(reinterpret_cast<const uint4*>(lo + kb * 64 + 16 * j) + s);
+        b[kb][s] = load_in_order(reinterpret_cast<const uint4*>(hi + kb * 64 + 16 * j) + s);
       }
     float d[4] = {0.f, 0.f, 0.f, 0.f};
     c[0] = c[1] = c[2] = c[3] = 0.f;

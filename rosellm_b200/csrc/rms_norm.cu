@@ -90,8 +90,8 @@ __global__ __launch_bounds__(256) void rmsnorm_add_kernel(const float* __restric
 // for at once, gamma before the wait for the kernels ahead, where the kernel above reads y, sums, and then reads y, gamma and the
 // stream one round trip later (8 rows of 2048 in a decode step: 3.2 us a launch, a third of it that round trip).  The same bits.
 template <int Q>
-__global__ __launch_bounds__(256) void rmsnorm_add_row_kernel(const float* __restrict__ y, long ldy, const float* __restrict__ gamma,
-                                                              float* __restrict__ stream, long lds, __nv_bfloat16* __restrict__ copy,
+__global__ __launch_bounds__(256) void rmsnorm_add_row_kernel(const float* y, long ldy, const float* __restrict__ gamma,
+                                                              float* stream, long lds, __nv_bfloat16* __restrict__ copy,
                                                               long ldc, int width, float eps, float mult) {
   __shared__ float scratch[33];
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -198,7 +198,7 @@ struct SublayerRows {
 // summed rows).  NEXT off: the addition to the stream alone.
 template <typename TOut, int KEEP, bool EXPERTS, bool NEXT>
 __global__ __launch_bounds__(256) void rmsnorm_add_norm_vec_kernel(const SublayerRows src, const float* __restrict__ gamma,
-                                                                   float* __restrict__ stream, long lds,
+                                                                   float* stream, long lds,
                                                                    const float* __restrict__ gamma_next, TOut* __restrict__ next,
                                                                    long ldn, int width, float eps, float eps_next) {
   __shared__ float scratch[33];
