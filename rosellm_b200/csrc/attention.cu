@@ -14,14 +14,14 @@
 // clusters.  One without the other is refused.  n_tokens: rows of q; n_pages: pages of the pool (both bound the
 // TMA tensor maps of the tcgen05 kernel).
 //
-// old_keys_settled: the decode kernel is launched with programmatic dependent launch and, when
-// this is nonzero, fetches the batch description, the block table and the keys and values at
-// positions below kv_len - 1 BEFORE it waits for the kernels ahead of it on the stream.  Pass
+// old_keys_settled: the kernels are launched with programmatic dependent launch.  When this is nonzero, the tcgen05
+// kernel of the prompt portions reads the batch description and the block table, and the decode kernel those and the
+// keys and values at positions below kv_len - 1, BEFORE they wait for the kernels ahead of them on the stream.  Pass
 // nonzero only if all of those were written by work that had completed before the kernel
 // preceding this call on the stream started (inside the engine they are of earlier steps, and
 // every step begins with a copy to the device, which separates the steps' kernels).  A caller
 // that writes several positions of the cache and attends over them back to back on one stream
-// passes 0: the kernel then reads nothing before its wait.
+// passes 0: the kernels then read nothing before their wait.
 RL_EXPORT int rl_attention(int dtype, const void* q, long q_stride, const void* pool,
                            const int* block_table, int bt_stride, const int* q_start,
                            const int* kv_len, const int* slots, void* out, long out_stride,

@@ -157,6 +157,7 @@ __global__ __launch_bounds__(ATT_THREADS, 1) void attn_tc_kernel(const __grid_co
 
   // the warp's number as a value that the compiler knows to be the same in all lanes
   const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  if (!p.old_keys_settled) asm volatile("griddepcontrol.wait;" ::: "memory");  // the caller promises nothing of the table and the description
   const int tile = singly ? gridDim.y - 1 - blockIdx.y : gridDim.x - 1 - blockIdx.x;
   const int req = tiles[2 * tile], entry_t0 = tiles[2 * tile + 1];
   if (entry_t0 % ATT_Q != 0) return;  // the second half of a piece
@@ -210,7 +211,7 @@ __global__ __launch_bounds__(ATT_THREADS, 1) void attn_tc_kernel(const __grid_co
   const uint32_t tmem_pv = tmem_base + 256u;  // two tiles of 64 columns
   RL_PHASE(1);
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  // the pages of the first tile (the block table is written by no kernel of a step): looked up before the wait
+  // the pages of the first tile (the block table is of earlier work, or has been waited for): looked up before the wait
   const int* bt = p.block_table + (size_t)slot * p.bt_stride;
   const int pages_per_tile = ATT_KV / p.page_size;
   auto pages_of_tile = [&](int kv_hi, int t) { return min(pages_per_tile, (kv_hi - t * ATT_KV + p.page_size - 1) / p.page_size); };

@@ -103,13 +103,14 @@ __global__ __launch_bounds__(32 * HR_WARPS) void head_rows_kernel(const __nv_bfl
                                                                   const __nv_bfloat16* __restrict__ w, long w_head, long w_n,
                                                                   __nv_bfloat16* __restrict__ out, long out_tok, long out_head,
                                                                   int n_tokens, int n_total, int parts, const float* gate,
-                                                                  long gate_tok, long gate_head, long gate_n) {
+                                                                  long gate_tok, long gate_head, long gate_n, int w_settled) {
   __shared__ float part_s[HR_WARPS][32][4];
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, j = lane & 3;
   const int h = blockIdx.y, per_block = HR_WARPS / parts;
   const int part = warp / per_block, n0 = (blockIdx.x * per_block + warp % per_block) * 8, k0 = part * KB * 64;
   HeadRowsWeights<KB> weights;
+  if (!w_settled) asm volatile("griddepcontrol.wait;" ::: "memory");  // the caller promises nothing
   weights.load(w + (size_t)h * w_head + (size_t)min(n0 + g, n_total - 1) * w_n + k0);
   asm volatile("griddepcontrol.wait;" ::: "memory");
   const __nv_bfloat16* in_h = in + (size_t)h * in_head + k0;
@@ -140,10 +141,12 @@ __global__ __launch_bounds__(32 * HR_WARPS) void head_rows_kernel(const __nv_bfl
 // in: element (t, h, k) at in + t*in_tok + h*in_head + k; w: element (h, k, n) at
 // w + h*w_head + k*w_k + n*w_n; out: element (t, h, n) at out + t*out_tok + h*out_head + n.
 // gate: null, or float32 logits, element (t, h, n) at gate + t*gate_tok + h*gate_head + n*gate_n: out *=
-// sigmoid(gate).
+// sigmoid(gate).  w_settled: w was written by work that was over before the kernel preceding this call on the stream began (weights);
+// the kernel of up to 16 rows then asks for it before its wait for the kernels ahead.
 RL_EXPORT int rl_head_linear(int dtype, const void* in, long in_tok, long in_head, const void* w, long w_head, long w_k,
                              long w_n, void* out, long out_tok, long out_head, int n_tokens, int n_heads, int k_total,
-                             int n_total, const float* gate, long gate_tok, long gate_head, long gate_n, cudaStream_t stream) {
+                             int n_total, const float* gate, long gate_tok, long gate_head, long gate_n, int w_settled,
+                             cudaStream_t stream) {
   if (n_tokens <= 0) return 0;
   if (n_heads <= 0 || n_heads > 65535 || k_total <= 0 || n_total <= 0) return -2;
   const dim3 grid((n_tokens + rl::TG_M - 1) / rl::TG_M, (n_total + rl::TG_N - 1) / rl::TG_N, n_heads);
@@ -166,7 +169,7 @@ RL_EXPORT int rl_head_linear(int dtype, const void* in, long in_tok, long in_hea
         auto kernel = kb == 1 ? rl::head_rows_kernel<1> : kb == 2 ? rl::head_rows_kernel<2> : rl::head_rows_kernel<4>;
         rl::launch_pdl(kernel, dim3((n_total + columns - 1) / columns, n_heads), 32 * rl::HR_WARPS, 0, stream, (const __nv_bfloat16*)in,
                        in_tok, in_head, (const __nv_bfloat16*)w, w_head, w_n, (__nv_bfloat16*)out, out_tok, out_head, n_tokens, n_total,
-                       parts, gate, gate_tok, gate_head, gate_n);
+                       parts, gate, gate_tok, gate_head, gate_n, w_settled);
         RL_CHECK_LAUNCH();
         return 0;
       }

@@ -1,8 +1,8 @@
 // A warp's share of a per-head product of at most 16 rows on mma.sync m16n8k16, operands straight from memory into registers:
 // out[t, n] = sum_k in[t, k] w[n, k] for eight columns n and KB blocks of 64 elements of K.  Lane (g = lane / 4, j = lane % 4)
 // holds elements 16 j ... 16 j + 15 of row g of W and of rows g and g + 8 of the input, block by block: K is permuted alike in
-// both, so that every load is 16 bytes.  The weights (written by no kernel of a step) are asked for before the wait for the
-// kernels ahead, by a call of their own.
+// both, so that every load is 16 bytes.  The weights are asked for by a call of their own: where no kernel ahead
+// writes them, before the wait for those.
 #pragma once
 #include "common.cuh"
 

@@ -230,6 +230,7 @@ struct LatentParams {
   int n_heads, rank, row_width, page_size;
   float scale;
   int* status;
+  int table_settled;   // the step's description and the block table may be read before the wait for the kernels ahead
 };
 
 constexpr int LT_Q = 16;     // queries per block
@@ -570,7 +571,8 @@ __global__ __launch_bounds__(32 * WARPS) void latent_attn_mma_kernel(LatentParam
   constexpr int RB = 16 * (WARPS / DVS), LM_KT = 8 * NKT;
   extern __shared__ __align__(16) unsigned char latent_smem[];
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  // (the step's description and the block table are written by none of its kernels: read before the wait below)
+  // the step's description and the block table, where the caller has said that no kernel ahead writes them, are read before the wait below
+  if (!p.table_settled) asm volatile("griddepcontrol.wait;" ::: "memory");
   const int W = p.row_width, H = p.n_heads;
   const int Wk = (W + 15) & ~15, LD = Wk + 8, W8 = Wk >> 3;
   bf16* q_s = reinterpret_cast<bf16*>(latent_smem);  // [RB][LD]
@@ -1101,7 +1103,8 @@ RL_EXPORT int rl_latent_kv_write(int dtype, const float* dkv, long ld, const flo
 }
 
 // The product of at most 16 rows' queries with W_uk, their rotation and the new rows of the cache in one launch (bfloat16; see
-// LatentPrepare).  dkv null: no rows are written.  Returns -2 for sizes it does not take (the caller then makes the three calls).
+// LatentPrepare).  dkv null: no rows are written.  uk, inv_freq, positions, req_of_token, slots and the block table are read before the wait
+// for the kernels ahead: none of those may write them.  Returns -2 for sizes it does not take (the caller then makes the three calls).
 RL_EXPORT int rl_latent_prepare(const void* q, long q_stride, int head_in, int plain, const void* uk, void* rows, long rows_stride,
                                 int row_width, int rank, int rot_dim, int rot_dims, const float* inv_freq, float rot_mult,
                                 const int* positions, int n_tokens, int n_heads, const float* dkv, long ld, const float* gamma, float eps,
@@ -1149,19 +1152,21 @@ RL_EXPORT int rl_latent_q_rope(int dtype, const void* q, long q_stride, int head
 // that takes all heads of a request in one block, their keys cut into n_splits parts
 // (part_o: n_decode*heads*n_splits*rank floats, part_ml: n_decode*heads*n_splits*2); otherwise
 // they are tiles of one query.  bfloat16 runs on the tensor-core kernel (decoded requests then
-// always by request) unless simt_only is set (for comparisons) or its sizes do not fit.
+// always by request) unless simt_only is set (for comparisons) or its sizes do not fit.  table_settled: the lengths, slots, lists and the
+// block table were written by work that was over before the kernel preceding this call on the stream began; the tensor-core
+// kernel then reads them before its wait for the kernels ahead (the cached rows and the queries are read after it).
 RL_EXPORT int rl_latent_attention(int dtype, const void* q, long q_stride, const void* pool, const int* block_table,
                                   int bt_stride, const int* q_start, const int* kv_len, const int* slots, void* out,
                                   long out_stride, const float* sink, int n_heads, int rank, int row_width,
                                   int page_size, float scale, const int* tiles, int n_tiles, const int* decode_reqs,
                                   int n_decode, int decode_by_request, int n_splits, float* part_o, float* part_ml,
-                                  int simt_only, int* status, cudaStream_t stream) {
+                                  int simt_only, int table_settled, int* status, cudaStream_t stream) {
   if (!rl_latent_attention_fits(n_heads, rank, row_width) || status == nullptr) return -2;
   if (decode_by_request && !rl_latent_decode_fits(n_heads, rank, row_width)) return -3;
   if (n_splits < 1 || n_splits > 64 || (decode_by_request && n_splits > 1 && (part_o == nullptr || part_ml == nullptr)))
     return -4;  // the merge takes up to 64 parts
   rl::LatentParams p{q, q_stride, pool, block_table, bt_stride, q_start, kv_len, slots, out, out_stride, sink,
-                     n_heads, rank, row_width, page_size, scale, status};
+                     n_heads, rank, row_width, page_size, scale, status, table_settled};
   int rc = 0;
   if (dtype == RL_F32)
     rc = rl::dispatch_latent<float>(p, tiles, n_tiles, decode_reqs, n_decode, n_splits, decode_by_request != 0, part_o,

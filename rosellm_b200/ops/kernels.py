@@ -199,8 +199,8 @@ def _lib() -> ctypes.CDLL:
         lib.rl_latent_prepare.argtypes = [P, L, I, I, P, P, L, I, I, I, I, P, F, P, I, I, P, L, P, F, P, P, I, P, P, I, I, P, P]
         lib.rl_latent_prepare.restype = I
         lib.rl_latent_q_rope.argtypes = [I, P, L, I, I, P, L, I, I, I, I, P, P, I, I, F, P]
-        lib.rl_latent_attention.argtypes = [I, P, L, P, P, I, P, P, P, P, L, P, I, I, I, I, F, P, I, P, I, I, I, P, P, I, P, P]
-        lib.rl_head_linear.argtypes = [I, P, L, L, P, L, L, L, P, L, L, I, I, I, I, P, L, L, L, P]
+        lib.rl_latent_attention.argtypes = [I, P, L, P, P, I, P, P, P, P, L, P, I, I, I, I, F, P, I, P, I, I, I, P, P, I, I, P, P]
+        lib.rl_head_linear.argtypes = [I, P, L, L, P, L, L, L, P, L, L, I, I, I, I, P, L, L, L, I, P]
         lib.rl_gated_act.argtypes = [I, I, P, L, I, P, L, I, I, I, F, F, P]
         lib.rl_token_gate.argtypes = [I, P, L, P, P, L, I, I, P, L, I, I, I, P, I, P, P]
         lib.rl_moe_select.argtypes = [P, L, P, I, I, I, I, I, I, F, P, P, P, P]
@@ -365,7 +365,8 @@ def embed(token_ids, positions, table, pos_table, out, feedback=None, scale: flo
 
 
 def layernorm(x, gamma, beta, eps: float, out, rows=None) -> None:
-    """out[i] = LayerNorm(x[rows[i]] or x[i]) * gamma + beta; x float32, out float32 or bfloat16."""
+    """out[i] = LayerNorm(x[rows[i]] or x[i]) * gamma + beta; x float32, out float32 or bfloat16.  gamma and beta are weights: they may be
+    read before the kernels ahead have ended, so none of those may write them."""
     _need(x, "x", torch.float32)
     _need(gamma, "gamma", torch.float32)
     if beta is not None:
@@ -524,7 +525,9 @@ class NormInput:
 
 
 class KvTarget:
-    """Where the key and value columns of a packed qkv product go instead of the output buffer."""
+    """Where the key and value columns of a packed qkv product go instead of the output buffer.  The block table, positions,
+    requests and slots are a step's description, copied to the device before its kernels: the products of few rows read them before
+    the kernels ahead have ended, so none of those may write them."""
 
     def __init__(self, pool, block_table, positions, req_of_token, slots, q_width: int, max_pos: int) -> None:
         self.pool, self.block_table = pool, block_table
@@ -1042,9 +1045,9 @@ def attention(q, pool, block_table, q_start, kv_len, slots, out, *, n_heads: int
     ``old_keys_settled``: the caller promises that the block table and the keys and values below
     each decoded request's last position were written by work that was over before the kernel
     preceding this call on the stream began (true inside the engine, whose steps are separated
-    by a copy to the device); the decode kernel then fetches them before it waits for the
-    kernels ahead of it.  Off, it reads nothing before that wait, and a cache write issued just
-    before this call is seen.
+    by a copy to the device); the decode kernel then fetches them, and the tcgen05 kernel of the prompt portions reads the
+    step's description and the block table, before they wait for the kernels ahead of them.  Off, they read nothing before
+    that wait, and a cache write issued just before this call is seen.
     """
     _need(q, "q", contiguous=False)
     _need(pool, "pool", q.dtype)
@@ -1149,7 +1152,8 @@ def rmsnorm(x, gamma, eps: float, out, rows=None) -> None:
 
 def rmsnorm_add(y, gamma, eps: float, stream_rows, mult: float, copy=None) -> None:
     """stream_rows += mult * y / sqrt(mean(y^2) + eps) * gamma (all float32); ``copy`` (bfloat16,
-    same shape) receives the rounded new rows of the stream."""
+    same shape) receives the rounded new rows of the stream.  gamma is a weight: it may be read before the kernels ahead have ended, so
+    none of those may write it."""
     _need(y, "y", torch.float32, contiguous=False)
     _need(gamma, "gamma", torch.float32)
     _need(stream_rows, "stream_rows", torch.float32, contiguous=False)
@@ -1219,7 +1223,8 @@ def latent_prepare(q, uk, rows, inv_freq, positions, *, n_heads: int, head_in: i
                    row_width: int, rot_mult: float = 1.0, dkv=None, gamma=None, eps: float = 0.0, pool=None, block_table=None,
                    req_of_token=None, slots=None, max_pos: int = 0) -> None:
     """In one launch, for at most 16 rows of bfloat16: ``rows[t, h, :rank] = q_plain W_uk,h^T`` (``uk`` [heads, rank, plain],
-    weights: read before the kernels ahead have ended), ``latent_q_rope``, and (``dkv`` given) ``latent_kv_write``."""
+    weights), ``latent_q_rope``, and (``dkv`` given) ``latent_kv_write``.  ``uk``, ``inv_freq``, ``positions``, ``req_of_token``, ``slots`` and
+    ``block_table`` are read before the kernels ahead have ended: none of those may write them."""
     _need(q, "q", torch.bfloat16, contiguous=False)
     _need(rows, "rows", torch.bfloat16, contiguous=False)
     _need(uk, "uk", torch.bfloat16)
@@ -1266,14 +1271,16 @@ def latent_q_rope(q, rows, inv_freq, positions, *, n_heads: int, head_in: int, p
 
 def latent_attention(q, pool, block_table, q_start, kv_len, slots, out, *, sink, n_heads: int, rank: int, scale: float,
                      tiles, n_tiles: int, decode_reqs, n_decode: int, decode_by_request: bool = False,
-                     n_splits: int = 1, part_o=None, part_ml=None, simt_only: bool = False) -> None:
+                     n_splits: int = 1, part_o=None, part_ml=None, simt_only: bool = False, table_settled: bool = False) -> None:
     """Causal attention of the step's query rows ``q`` [tokens, heads * row width] over the cached
     latent rows (``pool`` [pages, 1, 1, page size, row width]); a row's first ``rank`` entries are
     its value; ``out`` [tokens, heads * rank].  ``sink`` float32 [heads] or ``None``.
     ``decode_by_request``: decoded requests take the kernel that serves all heads in one block
     and cuts a request's keys into ``n_splits`` parts (scratch ``part_o``, ``part_ml``).  bfloat16
     runs on the tensor cores where the sizes fit and decoded requests go by request;
-    ``simt_only`` (for tests and comparisons) keeps it on the CUDA-core kernels."""
+    ``simt_only`` (for tests and comparisons) keeps it on the CUDA-core kernels.  ``table_settled``: the caller promises that the
+    step's description (lengths, slots, lists) and the block table were written by work that was over before the kernel preceding this call
+    on the stream began, as in the engine; they are then read before the wait for the kernels ahead."""
     _need(q, "q", contiguous=False)
     _need(pool, "pool", q.dtype)
     _need(out, "out", q.dtype, contiguous=False)
@@ -1293,20 +1300,21 @@ def latent_attention(q, pool, block_table, q_start, kv_len, slots, out, *, sink,
                                     _ptr(q_start), _ptr(kv_len), _ptr(slots), _ptr(out), out.stride(0), _ptr(sink),
                                     n_heads, rank, row_width, page_size, float(scale), _ptr(tiles), n_tiles,
                                     _ptr(decode_reqs), n_decode, int(decode_by_request), n_splits, _ptr(part_o),
-                                    _ptr(part_ml), int(simt_only), _ptr(status_word(q.device)), _stream())
+                                    _ptr(part_ml), int(simt_only), int(table_settled), _ptr(status_word(q.device)), _stream())
     if rc in (-2, -3):
         raise KernelError(f"latent_attention: sizes not taken (heads {n_heads}, value width {rank}, row width {row_width})")
     _ok(rc, "latent_attention", made)
 
 
 def head_linear(inp, w, out, *, n_tokens: int, n_heads: int, k: int, n: int, in_strides, w_strides, out_strides,
-                gate=None, gate_strides=(0, 0, 1)) -> None:
+                gate=None, gate_strides=(0, 0, 1), w_settled: bool = False) -> None:
     """out[t, h, :n] = inp[t, h, :k] @ W_h for every head: element (t, h, i) of ``inp`` at
     ``t*in_strides[0] + h*in_strides[1] + i``, element (h, i, j) of ``w`` at ``h*w_strides[0] +
     i*w_strides[1] + j*w_strides[2]``, element (t, h, j) of ``out`` at ``t*out_strides[0] +
     h*out_strides[1] + j`` (strides in elements; the tensors give base addresses and dtype).  ``gate``: float32
     logits, element (t, h, j) at ``t*gate_strides[0] + h*gate_strides[1] + j*gate_strides[2]`` (a last stride of 0: one
-    logit a head): the result times their sigmoid."""
+    logit a head): the result times their sigmoid.  ``w_settled``: the caller promises that ``w`` was written by work that was over before the
+    kernel preceding this call on the stream began (weights); it is then asked for before the wait for the kernels ahead."""
     _need(inp, "inp", contiguous=False)
     _need(w, "w", inp.dtype)
     _need(out, "out", inp.dtype, contiguous=False)
@@ -1314,7 +1322,7 @@ def head_linear(inp, w, out, *, n_tokens: int, n_heads: int, k: int, n: int, in_
         _need(gate, "gate", torch.float32, contiguous=False)
     rc = _lib().rl_head_linear(_code(inp), _ptr(inp), in_strides[0], in_strides[1], _ptr(w), w_strides[0], w_strides[1],
                                w_strides[2], _ptr(out), out_strides[0], out_strides[1], n_tokens, n_heads, k, n,
-                               _ptr(gate), *gate_strides, _stream())
+                               _ptr(gate), *gate_strides, int(w_settled), _stream())
     _ok(rc, "head_linear")
 
 

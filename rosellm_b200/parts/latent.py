@@ -179,7 +179,7 @@ class LatentAttention(Part):
         K.latent_attention(rows, pool, table, ctx.q_start, ctx.kv_len, ctx.slots, o_lat, sink=self.sink, n_heads=H,
                            rank=rank, scale=self.scale, tiles=ctx.tiles, n_tiles=ctx.n_tiles,
                            decode_reqs=ctx.decode_reqs, n_decode=ctx.n_decode, decode_by_request=by_request,
-                           n_splits=splits, part_o=part_o, part_ml=part_ml)
+                           n_splits=splits, part_o=part_o, part_ml=part_ml, table_settled=True)  # a step begins with a copy to the device
         # the heads' values: (sum of probabilities x latents) W_uv,h^T, then the output product
         if self.heads_padded != self.heads_width:
             o = ws.get_zeroed(f"latent_heads_{self.heads_width}", (n, self.heads_padded), act)
@@ -191,7 +191,7 @@ class LatentAttention(Part):
             gate_strides = (proj.stride(0), self.value_dim, 1) if self.gate_kind == "element" else (proj.stride(0), 1, 0)
         K.head_linear(o_lat, self.uv_weight, o, n_tokens=n, n_heads=H, k=rank, n=self.value_dim,
                       in_strides=(H * rank, rank), w_strides=(self.value_dim * rank, 1, rank),
-                      out_strides=(self.heads_padded, self.value_dim), gate=gate, gate_strides=gate_strides)
+                      out_strides=(self.heads_padded, self.value_dim), gate=gate, gate_strides=gate_strides, w_settled=True)
         K.linear(o, self.o_weight, None, x, residual=add)
 
     def _prepare(self, ctx, q, dkv, rows, freq, pool, table) -> None:
@@ -203,7 +203,7 @@ class LatentAttention(Part):
                               max_pos=ctx.cache.max_seq_len, rot_mult=self.rotary.mult)
         K.head_linear(q, self.uk_weight, rows, n_tokens=n, n_heads=H, k=self.plain_dim, n=rank,
                       in_strides=(q.stride(0), self.head_in), w_strides=(self.plain_dim * rank, 1, self.plain_dim),
-                      out_strides=(H * W, W))
+                      out_strides=(H * W, W), w_settled=True)
         K.latent_q_rope(q, rows, freq, ctx.positions, n_heads=H, head_in=self.head_in, plain=self.plain_dim,
                         rank=rank, rot_dim=self.rot_dim, rot_dims=self.rotary.dims, row_width=W,
                         rot_mult=self.rotary.mult)
