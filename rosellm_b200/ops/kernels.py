@@ -461,7 +461,11 @@ def clustered_is_ahead(rows: int, n_out: int, k: int, *, out_f32: bool = False, 
     instead (csrc/gemm_tc_rows.cu), by what it takes between the other kernels of a layer (GPT-2 of three sizes at 64 rows, us, the
     other kernel / clustered): 3072 x 1024 7.4 / 6.7, 4096 x 1024 6.9 / 6.3, 4800 x 1600 9.0 / 8.7, 6400 x 1600 9.6 / 8.1, += 1600 x
     6400 11.5 / 10.9.  Smaller products lose what their clusters wait for places that the kernels ahead leave: 2304 x 768 5.6 / 6.8, += 768 x
-    768 5.2 / 6.4, += 1600 x 1600 6.0 / 7.6, though in chains of their own they gain as well (3072 x 768 6.2 / 4.8).  Float32 outputs that
+    768 5.2 / 6.4, += 1600 x 1600 6.0 / 7.6, though in chains of their own they gain as well (3072 x 768 6.2 / 4.8).  Between those sizes, whole
+    layers of decoded tokens, without / with this rule at 17, 33 and 64 rows: width 896 27.9 / 28.0, 36.2 / 36.2, 42.9 / 42.8; 1024 29.5 / 29.4,
+    37.4 / 36.9, 46.2 / 45.3; 1152 37.5 / 33.8, 39.2 / 38.5, 49.1 / 48.8; 1280 39.5 / 34.4, 45.1 / 42.8, 50.7 / 49.9; 1408 40.3 / 35.6, 46.0 /
+    41.1, 54.1 / 52.5; 1536 39.9 / 38.1, 46.1 / 44.8, 54.9 / 55.0; 1600 45.9 / 38.7, 49.6 / 46.2, 57.1 / 57.3.  += 1536 x 6144 would gain 0.4 to
+    0.6 of a layer's 40 to 55; += 1408 x 5632 and what is smaller and added to lose at one number of rows or another.  Float32 outputs that
     are not added to, logits among them, stay with the kernels that tokens are drawn from."""
     if not 17 <= rows <= 64 or k > 8192 or (out_f32 and not residual) or -(-n_out // 64) >= sm_count():
         return False
@@ -611,7 +615,8 @@ def linear(a, weight, bias, out, *, act: int = ACT_NONE, residual: bool = False,
     if path == "mma" and m > 64:
         raise KernelError("linear: the mma row kernel takes at most 64 rows")
     if path == "tcr" and not _lib().rl_gemm_tc_rows_fits(m, n, k):
-        raise KernelError("linear: the clustered tcgen05 kernel takes at most 128 rows and an inner size of at most 8192")
+        raise KernelError("linear: the clustered tcgen05 kernel takes at most 128 rows and an inner size of at most "
+                          "8192 (the ring that it walks fits the shared memory at any)")
     if kv is not None and path == "tile":
         raise KernelError("linear: the 32-bit tile kernel does not write into the cache")
     if kv is not None and (act != ACT_NONE or residual):
