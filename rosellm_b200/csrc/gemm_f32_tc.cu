@@ -18,12 +18,13 @@
 //               row of 128 bytes in the stage's second half its lo, all in the swizzle of the copy;
 //   warp 1      one lane issues tcgen05.mma kind::f16 (bfloat16), sixteen of K 16 a K block;
 //   warps 10-17 drain the accumulators (two of each in turn) and write the tile.
-// Shared memory is what bounds it: a K block of a 128 x 128 tile is read once and written one and a half times by the cutting warps
-// (96 KB with the conflicts of lo) and read eight times in parts by the products (128 KB), about 1,750 clocks of its 128 bytes a clock
-// where the tensor pipe needs 1,040; measured 1.04 us.  Narrow tiles are a chain of waits, 0.75 us a K block.
+// What bounds it: a K block goes through four roles, each with a wait on the one before; no unit is full.  Of 3072 x 768 at 1,752
+// rows (ncu, 128 columns): tensor pipe 40%, shared memory's pipe 57% (a K block of 128 x 128 is read once and written one and a half times by the
+// cutting warps and read eight times in parts by the products), issue slots 46%.  A K block takes 1.04 us where the tensor pipe needs 0.55; narrow
+// tiles are all chain, 0.75 us a K block.
 //
-// Measured on B200 in chains of products, 1,752 rows, us (the CUDA-core tiles, this kernel): 2304 x 768 157, 70; 3072 x 768 218, 104; 768 x 768
-// 65, 39; 768 x 3072 247, 118; 1600 x 6400 932, 438.  129 rows: 768 x 768 22.2, 22.4; 2304 x 768 56.6, 22.8; 1600 x 1600 73, 41.
+// Measured on B200 in chains of products, 1,752 rows, us (the CUDA-core tiles, this kernel): 2304 x 768 157, 70; 3072 x 768 218, 103; 768 x 768
+// 65, 38; 768 x 3072 247, 116; 1600 x 6400 932, 428.  129 rows: 768 x 768 22.2, 22.5; 2304 x 768 56.6, 22.7; 1600 x 1600 73, 41.
 // Error against 64 bits (2-norm of the difference over that of the FMAs' difference): dense sums 0.25 (K 256), 0.21 (768), 0.19 (3072); sums
 // of one product 1.00, of two to sixteen 0.5 to 1.1; of positive numbers 0.26 to 0.19.
 //

@@ -832,9 +832,9 @@ def separate_is_faster(rows: int, hidden: int, attention_fused: bool) -> bool:
 
     both fused, width 576, 8 rows    16.4 > 17.1   17.3 > 17.1   18.7 > 18.2   21.8 > 20.5
                 704, 5               16.6 > 16.8   17.4 > 16.8   18.7 > 17.8   21.3 > 20.1
-                768, 1               16.7 > 15.3   16.7 > 15.6   16.7 > 16.7   16.9 > 18.9
-                768, 4               16.8 > 16.7   17.1 > 16.7   17.8 > 17.7   19.4 > 20.0
-                768, 8               18.0 > 17.5   19.9 > 17.6   20.3 > 18.8   23.2 > 21.1
+                768, 1               16.4 > 14.8   16.7 > 15.2   16.8 > 15.4   16.9 > 15.4
+                768, 4               17.0 > 15.9   17.1 > 16.0   17.9 > 16.2   19.3 > 17.8
+                768, 8               17.8 > 17.0   18.9 > 17.1   20.2 > 18.3   23.6 > 20.6
                 768, 12              18.8 > 21.0   21.4 > 21.3   23.8 > 22.7   29.3 > 25.1
                 832, 8               18.7 > 18.4   19.7 > 18.4   21.5 > 19.5   24.6 > 22.0
                 896, 1               17.7 > 17.9   17.6 > 18.0   17.8 > 19.1   17.9 > 21.5
@@ -849,7 +849,9 @@ def separate_is_faster(rows: int, hidden: int, attention_fused: bool) -> bool:
                 1024, 8              22.0 > 20.9   22.2 > 20.9   23.4 > 22.0   25.7 > 24.6
                 1024, 16             25.5 > 24.2   28.2 > 26.2   29.9 > 29.7   34.8 > 36.3
 
-    Both at 1024 columns are not to be had (sixteen heads of clusters are more than the device holds).  There the separate
+    At 768 columns the separate form is ahead at every context since decode attention cuts keys over clusters and the ring-fed product
+    walks an empty lap first; up to four rows the fused one is kept all the same (tests/test_layer_form_gpu.py states it; a pass of one request
+    of GPT-2 124M differs by 1 to 3%).  Both at 1024 columns are not to be had (sixteen heads of clusters are more than the device holds).  There the separate
     form is taken for all rows, though from eleven to fifteen rows and 512 tokens on it is up to 9% behind: the fused
     feed-forward reads a copy of its output weights, 250 MB for the 24 layers of GPT-2 355M."""
     if hidden > FUSED_LAYER_MAX_WIDTH:
